@@ -1095,85 +1095,175 @@ __global__ void __launch_bounds__(256) sort_scatter_kernel(GatherArgs g) {
   }
 }
 
-// Chunk gather into the data section.  Regions (reg_chunk, reg_slot, reg_len)
-// are sorted by slot; every 16-byte unit of the data section is written once.
-// Each block owns a contiguous range of units, so a thread locates its region
-// once by binary search and then walks forward.
-__global__ void copy_kernel(GatherArgs g) {
-  pdl_enter();
-  if (!g.lay->ok) return;
-  const uint32_t R = g.lay->num_distinct;
-  const uint64_t nslots = g.lay->chunk_counter;
-  if (R == 0 || nslots == 0) return;
-  uint8_t* dst = g.stage + g.lay->pad + g.lay->data_off;
-  const uint64_t cs = g.cs;
-  const uint64_t last = (uint64_t)g.N - 1;
-  const uint64_t tail_len = g.len - last * cs;  // bytes of the last chunk
-  const uint64_t nunits = nslots * cs / 16;
-  const uint64_t per_block = ((nunits + gridDim.x - 1) / gridDim.x + blockDim.x - 1) / blockDim.x * blockDim.x;
-  const uint64_t u0 = (uint64_t)blockIdx.x * per_block, u1 = min(u0 + per_block, nunits);
-  uint64_t u = u0 + threadIdx.x;
-  if (u >= u1) return;
-  // 16-byte units per chunk; a power of two (every usual chunk size) is a shift
-  const uint64_t upc = cs / 16;
-  const int lg = (upc & (upc - 1)) == 0 ? __ffsll((long long)upc) - 1 : -1;
-  auto slot_of_unit = [&](uint64_t uu) { return lg >= 0 ? uu >> lg : uu / upc; };
-  uint64_t slot = slot_of_unit(u);
-  uint32_t lo = 0, hi = R - 1;
-  while (lo < hi) {
-    uint32_t mid = (lo + hi + 1) >> 1;
-    if (g.reg_slot[mid] <= slot) lo = mid; else hi = mid - 1;
-  }
-  uint32_t r = lo;
-  // one 16-byte unit of the data section; chunks past the end of the buffer
-  // stay zero (the reference reads out of bounds there)
-  auto load = [&](uint64_t uu) {
-    const uint64_t sl = slot_of_unit(uu);
-    while (r + 1 < R && g.reg_slot[r + 1] <= sl) r++;
-    const uint64_t within = (uu - sl * upc) * 16;
-    const uint64_t chunk = (uint64_t)g.reg_chunk[r] + (sl - g.reg_slot[r]);
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (chunk < last || (chunk == last && within + 16 <= tail_len)) {
-      v = __ldcs(reinterpret_cast<const uint4*>(g.data + chunk * cs + within));
-    } else if (chunk == last && within < tail_len) {
-      uint32_t w[4] = {0, 0, 0, 0};
-      for (uint32_t b = 0; b < 16 && within + b < tail_len; b++) w[b >> 2] |= (uint32_t)g.data[chunk * cs + within + b] << (8 * (b & 3));
-      v = make_uint4(w[0], w[1], w[2], w[3]);
-    }
-    return v;
-  };
-  // two units in flight per thread: both loads issue before either store
-  for (; u < u1; u += 2 * (uint64_t)blockDim.x) {
-    const uint64_t ub = u + blockDim.x;
-    const uint4 va = load(u);
-    const uint4 vb = ub < u1 ? load(ub) : make_uint4(0, 0, 0, 0);
-    __stcs(reinterpret_cast<uint4*>(dst + u * 16), va);
-    if (ub < u1) __stcs(reinterpret_cast<uint4*>(dst + ub * 16), vb);
-  }
+// Chunk gather into the data section.  Regions (reg_chunk, reg_slot) are
+// sorted by slot; every 16-byte unit of the data section is written once, by
+// one 16-byte store (the section starts on a 16-byte boundary).
+//
+// Bound by HBM (the chunks read once, written once).  A tile is 32 KiB of the
+// data section, or 256 slots of chunks shorter than 128 bytes; a block owns a
+// contiguous range of tiles, so it searches the region list once and then
+// carries its position along.  Per tile the regions are staged in shared
+// memory and every slot's chunk is found there once, so a unit costs a lookup
+// in shared memory whatever the regions' lengths: threads that walked the
+// list one region at a time took 372 us for 3.1 M regions of one 64-byte
+// chunk and 1481 us for one region of 4 GiB, a search per byte 819 us for
+// 64 MB in chunks of 100 bytes.
+constexpr uint32_t kCopyTileUnits = 2048;
+constexpr uint32_t kCopySlots = 256 + 2;  // slots that a tile can touch
+constexpr int kCopyPer = 4;               // units in flight per thread
+
+// Words of 16 bytes from address A: byte i of the result is the byte at A + i
+// for i in [lo, hi).  Loads only aligned words that hold one of these bytes.
+__device__ __forceinline__ uint4 load_window(uint64_t A, uint32_t lo, uint32_t hi) {
+  const uint32_t d = (uint32_t)(A & 15);
+  const uint4* w = reinterpret_cast<const uint4*>(A - d);
+  uint4 w0 = make_uint4(0, 0, 0, 0), w1 = make_uint4(0, 0, 0, 0);
+  if (lo + d < 16) w0 = __ldg(w);
+  if (hi + d > 16) w1 = __ldg(w + 1);
+  return cut16(w0, w1, d);
+}
+// mask of the bytes of word q (bytes 4q .. 4q + 3) that lie below n
+__device__ __forceinline__ uint32_t bytes_below(int n, int q) {
+  const int k = n - 4 * q;
+  return k <= 0 ? 0u : k >= 4 ? ~0u : (1u << (8 * k)) - 1;
 }
 
-// Byte-granular gather for chunk sizes that are not multiples of 16 or
-// buffers that are not 16-byte aligned.
-__global__ void copy_bytes_kernel(GatherArgs g) {
+// kVec: chunks of whole 16-byte words from a 16-byte aligned buffer, one load
+// per unit.  Otherwise a unit is cut out of the aligned words around each of
+// its pieces (one piece, or two where it crosses into a slot of another
+// region; more only for chunks shorter than 16 bytes).
+template <bool kVec>
+__global__ void __launch_bounds__(256) copy_kernel(GatherArgs g) {
   pdl_enter();
   if (!g.lay->ok) return;
   const uint32_t R = g.lay->num_distinct;
   const uint64_t nslots = g.lay->chunk_counter;
   if (R == 0 || nslots == 0) return;
+  __shared__ uint32_t rs[kCopySlots + 1], rc[kCopySlots + 1], ch[kCopySlots];
+  __shared__ uint32_t s_r;      // region of the tile's first slot
+  __shared__ uint32_t s_j[2];   // region (from the tile's first) of the last slot, of the slot after it
   uint8_t* dst = g.stage + g.lay->pad + g.lay->data_off;
   const uint64_t cs = g.cs;
+  const uint32_t tid = threadIdx.x;
   const uint64_t nbytes = nslots * cs;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nbytes; b += stride) {
-    uint64_t slot = b / cs;
-    uint32_t lo = 0, hi = R - 1;
+  const uint64_t nunits = (nbytes + 15) / 16;
+  const uint32_t ut = cs >= 128 ? kCopyTileUnits : 16 * (uint32_t)cs;
+  const uint64_t ntiles = (nunits + ut - 1) / ut;
+  const uint64_t per_block = (ntiles + gridDim.x - 1) / gridDim.x;
+  const uint64_t tile0 = (uint64_t)blockIdx.x * per_block;
+  const uint64_t tile1 = tile0 + per_block < ntiles ? tile0 + per_block : ntiles;
+  if (tile0 >= tile1) return;
+  const int lg = (cs & (cs - 1)) == 0 ? __ffsll((long long)cs) - 1 : -1;
+  // slot of byte x, counted from the tile's first slot (x < cs + 32 KiB: at
+  // most one slot on for chunks longer than a tile)
+  auto slot_of = [&](uint64_t x) -> uint32_t {
+    if (x < cs) return 0;
+    if (cs > 16 * kCopyTileUnits) return 1;
+    return lg >= 0 ? (uint32_t)(x >> lg) : (uint32_t)x / (uint32_t)cs;
+  };
+  if (tid < 32) {
+    const uint32_t s0 = (uint32_t)(tile0 * ut * 16 / cs);
+    uint32_t lo = 0, hi = R - 1;  // last region that starts at or before s0
+    if (R == nslots) lo = hi = s0;
     while (lo < hi) {
-      uint32_t mid = (lo + hi + 1) >> 1;
-      if (g.reg_slot[mid] <= slot) lo = mid; else hi = mid - 1;
+      const uint32_t step = (hi - lo) / 32 + 1;
+      const uint64_t p = (uint64_t)lo + (uint64_t)tid * step;
+      const uint32_t b = __ballot_sync(0xffffffffu, p <= hi && g.reg_slot[p] <= s0);
+      lo += (31 - __clz(b)) * step;
+      if ((uint64_t)lo + step - 1 < hi) hi = lo + step - 1;
     }
-    const uint64_t chunk = (uint64_t)g.reg_chunk[lo] + (slot - g.reg_slot[lo]);
-    const uint64_t src = chunk * cs + (b - slot * cs);
-    dst[b] = src < g.len ? g.data[src] : 0;
+    if (tid == 0) s_r = lo;
+  }
+  __syncthreads();
+  for (uint64_t tile = tile0; tile < tile1; tile++) {
+    const uint64_t u0 = tile * ut;
+    const uint32_t nu = (uint32_t)(nunits - u0 < ut ? nunits - u0 : ut);
+    const uint64_t b0 = u0 * 16, b1 = b0 + 16ull * nu < nbytes ? b0 + 16ull * nu : nbytes;
+    const uint32_t s0 = (uint32_t)(lg >= 0 ? b0 >> lg : b0 / cs);
+    const uint64_t rel = b0 - s0 * cs;
+    const uint32_t ns = slot_of(rel + (b1 - 1 - b0)) + 1;
+    const uint32_t r0 = s_r;
+    const uint32_t m = R - r0 < ns + 1 ? R - r0 : ns + 1;
+    for (uint32_t i = tid; i < m; i += 256) {
+      rs[i] = g.reg_slot[r0 + i];
+      rc[i] = g.reg_chunk[r0 + i];
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i <= ns; i += 256) {
+      uint32_t lo = 0, hi = m - 1;
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (rs[mid] <= s0 + i) lo = mid; else hi = mid - 1;
+      }
+      if (i < ns) ch[i] = rc[lo] + (s0 + i - rs[lo]);
+      if (i + 1 >= ns) s_j[i + 1 - ns] = lo;
+    }
+    __syncthreads();
+    // the next tile starts in this tile's last slot, or in the one after it
+    if (tid == 0) s_r = r0 + s_j[rel + (b1 - b0) >= ns * cs ? 1 : 0];
+    uint4* out = reinterpret_cast<uint4*>(dst) + u0;
+    for (uint32_t k0 = tid; k0 < nu; k0 += 256 * kCopyPer) {
+      uint4 v[kCopyPer];
+#pragma unroll
+      for (int q = 0; q < kCopyPer; q++) {
+        const uint32_t k = k0 + 256u * q;
+        v[q] = make_uint4(0, 0, 0, 0);
+        if (k >= nu) continue;
+        const uint64_t x = rel + 16ull * k;
+        uint32_t si = slot_of(x);
+        if (kVec) {
+          // bytes past the end of the buffer stay zero (the reference reads
+          // out of bounds there)
+          const uint64_t off = ch[si] * cs + (x - si * cs);
+          if (off + 16 <= g.len) {
+            v[q] = __ldcs(reinterpret_cast<const uint4*>(g.data + off));
+          } else if (off < g.len) {
+            // an aligned word of the buffer's allocation
+            const int hi = (int)(g.len - off);
+            const uint4 w = __ldcs(reinterpret_cast<const uint4*>(g.data + off));
+            v[q] = make_uint4(w.x & bytes_below(hi, 0), w.y & bytes_below(hi, 1), w.z & bytes_below(hi, 2),
+                              w.w & bytes_below(hi, 3));
+          }
+        } else {
+          uint32_t pos = 0;
+          uint64_t within = x - si * cs;
+          const uint32_t want = (uint32_t)(nbytes - (b0 + 16ull * k) < 16 ? nbytes - (b0 + 16ull * k) : 16);
+          while (pos < want) {
+            const uint64_t off = ch[si] * cs + within;  // source of byte pos
+            uint32_t end = cs - within < want - pos ? pos + (uint32_t)(cs - within) : want;
+            const uint32_t s1 = si;
+            if (end < want && cs >= 16 && ch[si + 1] == ch[si] + 1) end = want;  // one run of bytes
+            uint32_t hi = off >= g.len ? pos : g.len - off < end - pos ? pos + (uint32_t)(g.len - off) : end;
+            if (hi > pos) {
+              const uint4 w = load_window(reinterpret_cast<uint64_t>(g.data) + off - pos, pos, hi);
+              v[q].x |= w.x & bytes_below(hi, 0) & ~bytes_below(pos, 0);
+              v[q].y |= w.y & bytes_below(hi, 1) & ~bytes_below(pos, 1);
+              v[q].z |= w.z & bytes_below(hi, 2) & ~bytes_below(pos, 2);
+              v[q].w |= w.w & bytes_below(hi, 3) & ~bytes_below(pos, 3);
+            }
+            pos = end;
+            si = s1 + 1;
+            within = 0;
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kCopyPer; q++) {
+        const uint32_t k = k0 + 256u * q;
+        if (k >= nu) continue;
+        const uint64_t left = nbytes - (b0 + 16ull * k);
+        if (kVec || left >= 16) {
+          __stcs(out + k, v[q]);
+        } else {
+#pragma unroll
+          for (uint32_t b = 0; b < 15; b++) {
+            const uint32_t w = b < 4 ? v[q].x : b < 8 ? v[q].y : b < 12 ? v[q].z : v[q].w;
+            if (b < left) reinterpret_cast<uint8_t*>(out + k)[b] = (uint8_t)(w >> (8 * (b & 3)));
+          }
+        }
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -1357,11 +1447,11 @@ cudaError_t launch_assemble(const GatherArgs& g, uint64_t max_entries, cudaStrea
     note_launch(2);
   }
   const bool vec = (g.cs % 16 == 0) && ((reinterpret_cast<uintptr_t>(g.data) & 15) == 0);
-  static const bool reg = (register_input_kernel(reinterpret_cast<const void*>(copy_kernel), INPUT_GATHER),
-                           register_input_kernel(reinterpret_cast<const void*>(copy_bytes_kernel), INPUT_GATHER), true);
+  static const bool reg = (register_input_kernel(reinterpret_cast<const void*>(copy_kernel<true>), INPUT_GATHER),
+                           register_input_kernel(reinterpret_cast<const void*>(copy_kernel<false>), INPUT_GATHER), true);
   (void)reg;
-  if (vec) launch_k(copy_kernel, num_sms() * 8, 256, 0, s, g);
-  else launch_k(copy_bytes_kernel, num_sms() * 8, 256, 0, s, g);
+  if (vec) launch_k(copy_kernel<true>, num_sms() * 8, 256, 0, s, g);
+  else launch_k(copy_kernel<false>, num_sms() * 8, 256, 0, s, g);
   note_launch();
   return cudaGetLastError();
 }

@@ -54,6 +54,22 @@ __device__ __forceinline__ void st_digest(Digest* p, const Digest& d) {
   *reinterpret_cast<uint4*>(p) = make_uint4(d.w[0], d.w[1], d.w[2], d.w[3]);
 }
 
+// Bytes d .. d + 15 (d < 16) of the 32 bytes in w0, w1.
+__device__ __forceinline__ uint4 cut16(const uint4& w0, const uint4& w1, uint32_t d) {
+  uint32_t v[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+  uint32_t o[5];
+  const uint32_t sh = (d & 3) * 8;
+  switch (d >> 2) {
+    case 0: o[0] = v[0]; o[1] = v[1]; o[2] = v[2]; o[3] = v[3]; o[4] = v[4]; break;
+    case 1: o[0] = v[1]; o[1] = v[2]; o[2] = v[3]; o[3] = v[4]; o[4] = v[5]; break;
+    case 2: o[0] = v[2]; o[1] = v[3]; o[2] = v[4]; o[3] = v[5]; o[4] = v[6]; break;
+    default: o[0] = v[3]; o[1] = v[4]; o[2] = v[5]; o[3] = v[6]; o[4] = v[7]; break;
+  }
+  if (sh == 0) return make_uint4(o[0], o[1], o[2], o[3]);
+  return make_uint4(__funnelshift_r(o[0], o[1], sh), __funnelshift_r(o[1], o[2], sh), __funnelshift_r(o[2], o[3], sh),
+                    __funnelshift_r(o[3], o[4], sh));
+}
+
 // ---------------------------------------------------------------------------
 // Murmur3 variant of the reference (include/kokkos_murmur3.hpp:213-292):
 // MurmurHash3_x64_128 with seed 0 in which rotl64 returns uint32_t, so each

@@ -889,20 +889,6 @@ __device__ __forceinline__ void resolve_chunk(const RArgs& a, const OwnMasks& ow
 //    aligned 16-byte words, the word after a unit taken from the next lane,
 //    and the unit is cut out with funnel shifts; every load stays inside a
 //    16-byte word holding at least one byte of the source region.
-__device__ __forceinline__ uint4 cut16(const uint4& w0, const uint4& w1, uint32_t d) {
-  uint32_t v[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-  uint32_t o[5];
-  const uint32_t sh = (d & 3) * 8;
-  switch (d >> 2) {
-    case 0: o[0] = v[0]; o[1] = v[1]; o[2] = v[2]; o[3] = v[3]; o[4] = v[4]; break;
-    case 1: o[0] = v[1]; o[1] = v[2]; o[2] = v[3]; o[3] = v[4]; o[4] = v[5]; break;
-    case 2: o[0] = v[2]; o[1] = v[3]; o[2] = v[4]; o[3] = v[5]; o[4] = v[6]; break;
-    default: o[0] = v[3]; o[1] = v[4]; o[2] = v[5]; o[3] = v[6]; o[4] = v[7]; break;
-  }
-  if (sh == 0) return make_uint4(o[0], o[1], o[2], o[3]);
-  return make_uint4(__funnelshift_r(o[0], o[1], sh), __funnelshift_r(o[1], o[2], sh), __funnelshift_r(o[2], o[3], sh),
-                    __funnelshift_r(o[3], o[4], sh));
-}
 constexpr int kCopyUnroll = 4;
 __device__ __forceinline__ void copy_tile(const RArgs& a, uint64_t c0, const uint8_t* src, uint32_t nb) {
   const uint32_t lane = threadIdx.x & 31;
