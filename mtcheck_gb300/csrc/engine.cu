@@ -410,7 +410,7 @@ int Engine::enqueue(const uint8_t* data, uint64_t len, bool timed) {
   int rc = (mode_ == MODE_LIST || mode_ == MODE_BASIC) ? run_list_basic(data, len) : run_tree(data, len, baseline_path_);
   if (rc) return rc;
   if (timed) MTC_TRY(mark(2));
-  MTC_CUDA(launch_assemble(gather_args(data, len), (uint64_t)N_ + 1, stream_));
+  MTC_CUDA(launch_assemble(gather_args(data, len), (uint64_t)N_ + 1, fresh_, stream_));
   if (timed) MTC_TRY(mark(3));
   // results (layout, error word, map size) written to pinned memory by a
   // kernel, not queued on a copy engine behind other streams' transfers

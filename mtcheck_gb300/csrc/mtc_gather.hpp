@@ -92,7 +92,8 @@ cudaError_t launch_chunk_compaction(const uint8_t* labels, uint32_t n_chunks, in
                                     uint32_t* sh_list, Layout* lay, uint64_t* scan_scratch, uint64_t* scan_total,
                                     cudaStream_t s);
 // Assemble the diff into g.stage; max_entries bounds F and S (N + 1).
-cudaError_t launch_assemble(const GatherArgs& g, uint64_t max_entries, cudaStream_t s);
+// whole: most chunks are expected in the diff (a baseline).
+cudaError_t launch_assemble(const GatherArgs& g, uint64_t max_entries, bool whole, cudaStream_t s);
 // Rebuild `from` into the empty table `to` (capacity change), preserving values.
 cudaError_t launch_map_rehash(const DigestMap& from, uint64_t from_cap, const DigestMap& to, uint32_t* err,
                               cudaStream_t s);
