@@ -134,7 +134,7 @@ __device__ __forceinline__ uint8_t forest_node(const ForestArgs& a, int pass, in
     if (baseline) {
       Digest dg = hash_pair(a.hash_kind, ld_digest(a.tree + l), ld_digest(a.tree + rr));
       st_digest(a.tree + n, dg);
-      if (map_insert_serial(a.map, dg, (uint32_t)n, cur_id, epoch_all, a.err)) atomicAdd(a.map.size, 1u);
+      if (map_insert_serial(a.map, dg, (uint32_t)n, cur_id, epoch_all, true, a.err)) atomicAdd(a.map.size, 1u);
     }
   }
   if (store) a.labels[n] = lab_n;
@@ -577,7 +577,8 @@ __device__ __forceinline__ void drain_inserts(const ForestArgs& a, uint32_t b0, 
   uint32_t created = 0;
   for (uint32_t k = (blockIdx.x - b0) * blockDim.x + threadIdx.x; k < n; k += nb * blockDim.x) {
     const uint32_t node = a.ins_queue[k];
-    created += map_insert_serial(a.map, ld_digest(a.tree + node), node, cur_id, epoch_fo, a.err);
+    // a first occurrence's digest is new: its leaves' are
+    created += map_insert_serial(a.map, ld_digest(a.tree + node), node, cur_id, epoch_fo, false, a.err);
   }
   count_new_entries(a.map, created);
 }
@@ -1301,7 +1302,7 @@ __global__ void map_rehash_kernel(DigestMap from, uint64_t from_cap, DigestMap t
     const uint4 v = *reinterpret_cast<const uint4*>(s.key);
     if (key_empty(v)) continue;
     uint64_t slot;
-    if (map_claim(to, Digest{{v.x, v.y, v.z, v.w}}, &slot, err) != INS_NEW) continue;
+    if (map_claim(to, Digest{{v.x, v.y, v.z, v.w}}, false, &slot, err) != INS_NEW) continue;
     to.slots[slot].win = s.win;
     to.slots[slot].tree = s.tree;
     created++;

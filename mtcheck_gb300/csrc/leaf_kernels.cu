@@ -103,38 +103,86 @@ __device__ __forceinline__ void note_dup(const LeafArgs& a, uint32_t note) {
 // advanced (the header overload) leaves in place: the reference lowers its
 // node and keeps the chunk a first occurrence there too.  The creator of an
 // entry waits for nothing after its claim.
+// Lanes of a warp that hold one digest (runs of equal chunks) insert it once,
+// through their first lane and with their lowest chunk, as if the lowest had
+// come first.  The slot is read before it is claimed only once the block has
+// met a digest that was there already (and for each thread's first chunk):
+// with random accesses the bound, new digests save the read.
 template <int EPI>
-__global__ void leaf_insert_kernel(LeafArgs a) {
+__global__ void __launch_bounds__(256) leaf_insert_kernel(LeafArgs a) {
   pdl_enter();
+  __shared__ volatile uint32_t s_dups;
   const uint32_t n = *a.changed_count;
   const uint32_t cur = a.sp->cur, epoch = a.sp->epoch;
+  const uint32_t lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) s_dups = 0;
+  __syncthreads();
+  bool first = true;
   uint32_t created = 0;
-  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t c = a.changed_list[k];
-    const Digest dg = map_key(ld_digest(a.prev + c));
-    const uint32_t node = EPI == EPI_TREE ? a.leaf_base + c : c;
+  // whole warps step together
+  for (uint64_t kw = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); kw < n;
+       kw += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t k = kw + lane;
+    const bool in = k < n;
+    const uint32_t c = in ? a.changed_list[k] : 0xffffffffu;
+    Digest dg{{0, 0, 0, 0}};
+    if (in) dg = map_key(ld_digest(a.prev + c));
+    const unsigned act = __ballot_sync(0xffffffffu, in);
+    unsigned peers = 1u << lane;
+    uint32_t low = c;
+    const unsigned like = in ? __match_any_sync(act, dg.w[0]) : 0;
+    if (like & (like - 1)) {
+      const int src = __ffs(like) - 1;
+      const uint32_t w1 = __shfl_sync(like, dg.w[1], src), w2 = __shfl_sync(like, dg.w[2], src),
+                     w3 = __shfl_sync(like, dg.w[3], src);
+      const bool same = dg.w[1] == w1 && dg.w[2] == w2 && dg.w[3] == w3;
+      const unsigned all = __ballot_sync(like, same);
+      if (same) {
+        peers = all;
+        low = __reduce_min_sync(all, c);
+      }
+    }
+    const int lead = __ffs(peers) - 1;
     uint64_t slot = 0;
+    int r = INS_FAILED;
+    unsigned long long old = kWinEmpty;
+    bool here = false;  // an older entry that carries this checkpoint's id
+    if (in && (int)lane == lead) {
+      const uint32_t node = EPI == EPI_TREE ? a.leaf_base + low : low;
+      r = map_claim(a.map, dg, first || s_dups != 0, &slot, a.err);
+      MapSlot* s = &a.map.slots[slot];
+      if (r == INS_NEW) {
+        slot_init(s, win_of(epoch, node), cur, low);
+        created++;
+      } else if (r == INS_EXISTING) {
+        old = win_min(s, win_of(epoch, node));
+        if (old != kWinEmpty && win_epoch(old) != epoch && EPI == EPI_TREE && __ldcg(&s->tree) == cur) {
+          // lowest node within the older entry (the reference's atomic_min,
+          // src/tree_approach.cpp:337-339): the entry's high bits (epoch and
+          // serial level) are fixed, since every insert of this launch carries
+          // a larger epoch and leaves them alone, so lowering the whole word
+          // lowers exactly its node
+          if (win_node(old) > node) win_min(s, (old & ~0xffffffffull) | node);
+          here = true;
+        }
+      }
+    }
+    first = false;
+    if (__any_sync(0xffffffffu, r == INS_EXISTING) && lane == 0) s_dups = 1;
+    r = __shfl_sync(0xffffffffu, r, lead);
+    slot = __shfl_sync(0xffffffffu, slot, lead);
+    old = __shfl_sync(0xffffffffu, old, lead);
+    here = __shfl_sync(0xffffffffu, (int)here, lead) != 0;
+    if (!in) continue;
     uint8_t label = SHIFT_DUPL;
-    const int r = map_claim(a.map, dg, &slot, a.err);
-    MapSlot* s = &a.map.slots[slot];
     if (r == INS_NEW) {
-      s->tree = cur;
-      s->first_chunk = c;
-      atomicMin(&s->win, win_of(epoch, node));
       label = FIRST_OCUR;
-      created++;
+      if (c != low) note_dup(a, (uint32_t)k | kCheckCreator);
     } else if (r == INS_EXISTING) {
-      const unsigned long long old = win_min(&s->win, win_of(epoch, node));
       if (old == kWinEmpty || win_epoch(old) == epoch) {
         label = FIRST_OCUR;  // first seen by this launch: the lowest chunk keeps it
         note_dup(a, (uint32_t)k | kCheckCreator);
-      } else if (EPI == EPI_TREE && __ldcg(&s->tree) == cur) {
-        // lowest node within the older entry (the reference's atomic_min,
-        // src/tree_approach.cpp:337-339): the entry's high bits (epoch and
-        // serial level) are fixed, since every insert of this launch carries
-        // a larger epoch and leaves them alone, so one atomicMin on the
-        // whole word lowers exactly its node
-        if (win_node(old) > node) win_min(&s->win, (old & ~0xffffffffull) | node);
+      } else if (here) {
         label = FIRST_OCUR;
         note_dup(a, (uint32_t)k);
       }
@@ -782,7 +830,7 @@ cudaError_t batch_leaf_node_params(const BatchLeafParams& p, cudaKernelNodeParam
 }
 
 cudaError_t launch_leaf_inserts(const LeafArgs& a, cudaStream_t s) {
-  const uint32_t grid = (uint32_t)num_sms() * 8;
+  const uint32_t grid = (uint32_t)num_sms() * 6;
   if (a.epi == EPI_TREE) launch_k(leaf_insert_kernel<EPI_TREE>, grid, 256, 0, s, a);
   else launch_k(leaf_insert_kernel<EPI_LIST>, grid, 256, 0, s, a);
   launch_k(leaf_demote_kernel, grid, 256, 0, s, a);

@@ -316,7 +316,7 @@ __host__ __device__ __forceinline__ uint32_t leftmost_leaf(uint32_t node, uint32
 // slots.  A slot is claimed by one 128-bit compare-and-swap of its key
 // (all-ones = empty; a digest equal to that pattern is stored with its lowest
 // bit cleared).  `win` packs (epoch << 38) | priority and starts all-ones;
-// every insert of a key, its creator's included, applies atomicMin to it, so
+// every insert of a key, its creator's included, lowers it to its own, so
 //   * an entry created by an earlier launch (smaller epoch) is kept,
 //   * among the inserts of one launch the lowest priority wins: the lowest
 //     chunk or node (the reference's atomic_min), or the serial order of a
@@ -325,7 +325,8 @@ __host__ __device__ __forceinline__ uint32_t leftmost_leaf(uint32_t node, uint32
 // than its launch.  The node is win's low 32 bits.  `tree` (the checkpoint id
 // of the first occurrence) is written by the creator and read by later
 // launches; so is `first_chunk`, the chunk whose leaf insert created the
-// entry (read by that checkpoint's demote pass).  No insert waits on another
+// entry (read by that checkpoint's demote pass).  Both halves of a slot are
+// only written by 16-byte compare-and-swaps.  No insert waits on another
 // thread.
 // ---------------------------------------------------------------------------
 struct __align__(32) MapSlot {
@@ -367,49 +368,81 @@ __device__ __forceinline__ uint64_t slot_of(const Digest& k, uint64_t mask) {
   return a & mask;
 }
 
-// 128-bit compare-and-swap of a slot's key from empty to k; returns the key
-// that was there (empty: the caller now owns the slot).
-__device__ __forceinline__ uint4 claim_key(MapSlot* s, const Digest& k) {
-  const unsigned long long e = ~0ull;
-  const unsigned long long vlo = ((unsigned long long)k.w[1] << 32) | k.w[0];
-  const unsigned long long vhi = ((unsigned long long)k.w[3] << 32) | k.w[2];
-  unsigned long long olo, ohi;
+// 128-bit compare-and-swap of one aligned half of a slot.
+struct Half { unsigned long long lo, hi; };
+__device__ __forceinline__ bool half_eq(const Half& a, const Half& b) { return a.lo == b.lo && a.hi == b.hi; }
+__device__ __forceinline__ Half cas_half(void* p, const Half& expect, const Half& v) {
+  Half o;
   asm volatile(
       "{\n\t.reg .b128 c, v, o;\n\t"
       "mov.b128 c, {%2, %3};\n\t"
       "mov.b128 v, {%4, %5};\n\t"
       "atom.relaxed.gpu.global.cas.b128 o, [%6], c, v;\n\t"
       "mov.b128 {%0, %1}, o;\n\t}"
-      : "=l"(olo), "=l"(ohi)
-      : "l"(e), "l"(e), "l"(vlo), "l"(vhi), "l"(s->key)
+      : "=l"(o.lo), "=l"(o.hi)
+      : "l"(expect.lo), "l"(expect.hi), "l"(v.lo), "l"(v.hi), "l"(p)
       : "memory");
-  return make_uint4((uint32_t)olo, (uint32_t)(olo >> 32), (uint32_t)ohi, (uint32_t)(ohi >> 32));
+  return o;
+}
+__device__ __forceinline__ Half empty_half() { return Half{~0ull, ~0ull}; }
+
+// Claims a slot's key from empty to k; returns the key that was there
+// (empty: the caller now owns the slot).
+__device__ __forceinline__ uint4 claim_key(MapSlot* s, const Digest& k) {
+  const Half o = cas_half(s->key, empty_half(), Half{((unsigned long long)k.w[1] << 32) | k.w[0],
+                                                    ((unsigned long long)k.w[3] << 32) | k.w[2]});
+  return make_uint4((uint32_t)o.lo, (uint32_t)(o.lo >> 32), (uint32_t)o.hi, (uint32_t)(o.hi >> 32));
 }
 
-// atomicMin on an entry's win word, read first: win only decreases, so a
-// value read at or below `w` (a stale read can only be higher than the
-// current one) means the atomic would change nothing, and the read stands in
-// for the value it would have returned: its epoch is the current one, and a
-// node read too high only makes a caller lower it once more, which changes
-// nothing either.
-__device__ __forceinline__ unsigned long long win_min(unsigned long long* p, unsigned long long w) {
-  const unsigned long long cur = __ldcg(p);
-  return cur <= w ? cur : atomicMin(p, w);
+// The values of an entry this thread has just created, in one operation: the
+// half is still empty unless another insert of the key has lowered its win
+// word first, and then keeps the lower one.  With the claim, two operations
+// per new entry; a claim, two stores and a minimum cost 865 us for 2^23 random
+// inserts into a 2 GiB table, these 665 us (470 us without the read before
+// the claim), each operation on the line costing about the same.
+__device__ __forceinline__ void slot_init(MapSlot* s, unsigned long long win, uint32_t tree, uint32_t first_chunk) {
+  const unsigned long long hi = ((unsigned long long)first_chunk << 32) | tree;
+  Half seen = empty_half();
+  while (true) {
+    const Half o = cas_half(&s->win, seen, Half{seen.lo < win ? seen.lo : win, hi});
+    if (half_eq(o, seen)) return;
+    seen = o;
+  }
+}
+
+// Lowers an entry's win word to w if it is above, and returns the word that
+// was there.  Read first: the word only decreases, so one read at or below w
+// (a stale read can only be higher than the current one) needs no atomic, and
+// a node read too high only makes a caller lower it once more, which changes
+// nothing.  Every retry follows another insert's success.
+__device__ __forceinline__ unsigned long long win_min(MapSlot* s, unsigned long long w) {
+  const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2*>(&s->win));
+  Half seen{v.x, v.y};
+  while (seen.lo > w) {
+    const Half o = cas_half(&s->win, seen, Half{w, seen.hi});
+    if (half_eq(o, seen)) break;
+    seen = o;
+  }
+  return seen.lo;
 }
 
 // The slot of k, claimed if absent: INS_NEW (this thread created the entry),
 // INS_EXISTING, or INS_FAILED (table full, error word set).
-// A key, once claimed, never changes within a launch, so the slot is read
-// before the compare-and-swap: a key that is already there (every duplicate
-// of a digest, thousands of times over in a run of equal chunks) costs a
-// load instead of an atomic on one contended line.  Only a read equal to k
-// is taken as it is; anything else (another key, an empty slot, or a 16-byte
-// read that saw half of a concurrent claim) goes through the atomic.
-__device__ inline int map_claim(const DigestMap& m, const Digest& k, uint64_t* slot, uint32_t* err) {
+// A key, once claimed, never changes within a launch.  `read`: look at the
+// slot before the compare-and-swap, so that a key that is already there
+// (every duplicate of a digest, thousands of times over in a run of equal
+// chunks) costs a load instead of an atomic on one contended line (about 6 ns
+// each).  Only a read equal to k is taken as it is; anything else (another
+// key, an empty slot, or a 16-byte read that saw half of a concurrent claim)
+// goes through the atomic.  Where keys are expected to be new, the read is
+// one more trip to a random line (665 against 470 us, above) and is left out.
+__device__ inline int map_claim(const DigestMap& m, const Digest& k, bool read, uint64_t* slot, uint32_t* err) {
   uint64_t i = slot_of(k, m.mask);
   for (uint64_t probe = 0; probe <= m.mask; probe++) {
-    const uint4 seen = __ldcg(reinterpret_cast<const uint4*>(m.slots[i].key));
-    if (key_eq(seen, k)) { *slot = i; return INS_EXISTING; }
+    if (read) {
+      const uint4 seen = __ldcg(reinterpret_cast<const uint4*>(m.slots[i].key));
+      if (key_eq(seen, k)) { *slot = i; return INS_EXISTING; }
+    }
     const uint4 old = claim_key(&m.slots[i], k);
     if (key_empty(old)) { *slot = i; return INS_NEW; }
     if (key_eq(old, k)) { *slot = i; return INS_EXISTING; }
@@ -417,22 +450,6 @@ __device__ inline int map_claim(const DigestMap& m, const Digest& k, uint64_t* s
   }
   raise_err(err, DERR_MAP_FULL);
   return INS_FAILED;
-}
-
-// Insert (k -> win, tree) with the priority rule above.  *old_win receives the
-// entry's previous win: kWinEmpty for an entry created by this launch whose
-// creator has not applied its own yet.  A new entry is not counted in
-// m.size: the caller adds it (count_new_entries).
-__device__ __forceinline__ int map_insert_win(const DigestMap& m, const Digest& k0, unsigned long long win,
-                                              uint32_t tree, uint64_t* slot, unsigned long long* old_win,
-                                              uint32_t* err) {
-  const Digest k = map_key(k0);
-  const int r = map_claim(m, k, slot, err);
-  if (r == INS_FAILED) return r;
-  MapSlot* s = &m.slots[*slot];
-  if (r == INS_NEW) s->tree = tree;
-  *old_win = win_min(&s->win, win);
-  return r;
 }
 
 // Warp total of new entries added to m.size (every lane of the warp calls it).
@@ -464,12 +481,16 @@ __device__ __forceinline__ uint64_t serial_prio(uint32_t node) {
 }
 // Insert for a pass that spans several levels in one launch: an entry from an
 // earlier launch is kept; among inserts of this pass the serially first wins.
-// Returns 1 when the entry is new.
+// Returns 1 when the entry is new; the caller adds it to m.size
+// (count_new_entries).  `read` as in map_claim.
 __device__ __forceinline__ uint32_t map_insert_serial(const DigestMap& m, const Digest& k, uint32_t node,
-                                                      uint32_t tree, uint32_t epoch, uint32_t* err) {
+                                                      uint32_t tree, uint32_t epoch, bool read, uint32_t* err) {
   uint64_t slot;
-  unsigned long long old;
-  return map_insert_win(m, k, win_of(epoch, serial_prio(node)), tree, &slot, &old, err) == INS_NEW ? 1u : 0u;
+  const unsigned long long win = win_of(epoch, serial_prio(node));
+  const int r = map_claim(m, map_key(k), read, &slot, err);
+  if (r == INS_NEW) slot_init(&m.slots[slot], win, tree, 0xffffffffu);
+  else if (r == INS_EXISTING) win_min(&m.slots[slot], win);
+  return r == INS_NEW ? 1u : 0u;
 }
 
 // Plain read of a slot's value after the launch that wrote it has finished.
