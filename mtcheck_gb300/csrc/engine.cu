@@ -307,8 +307,12 @@ int Engine::run_tree(const uint8_t* data, uint64_t len, bool baseline_path) {
   // the forest's first-occurrence inserts
   fa.ins_queue = changed_list_.p;
   fa.ins_count = changed_count_.p + 2;
-  MTC_CUDA(launch_forest(fa, 0, 0, N, stream_));                         // first-occurrence forest
-  MTC_CUDA(launch_forest(fa, 1, baseline_path ? 1 : 0, N, stream_));  // duplicate forest
+  if (baseline_path && fresh_) {
+    MTC_CUDA(launch_forest(fa, 3, 1, N, stream_));  // both passes of a baseline on cleared digests
+  } else {
+    MTC_CUDA(launch_forest(fa, 0, 0, N, stream_));                      // first-occurrence forest
+    MTC_CUDA(launch_forest(fa, 1, baseline_path ? 1 : 0, N, stream_));  // duplicate forest
+  }
   MTC_CUDA(launch_root_compaction(fa, N, M, fo_list_.p, sh_list_.p, lay_.p, scan_.p, scan_total_.p, stream_));
   return ST_OK;
 }

@@ -44,7 +44,19 @@ __device__ __forceinline__ uint8_t child_flag(uint8_t lab) {
 // (src/tree_approach.cpp:378-404); pass 1: duplicate forest (:413-477), with
 // baseline != 0 the baseline variant that tests the not-yet-hashed digest and
 // then hashes and inserts every interior node (:155-227); pass 2: both
-// incremental passes in one traversal (ForestArgs::fuse_gate).
+// incremental passes in one traversal (ForestArgs::fuse_gate); pass 3: both
+// passes of a baseline on cleared digests in one traversal, which hashes
+// every node and leaves the inserts to forest_insert_all_kernel.
+//
+// Pass 3.  A node is a first occurrence in the baseline's second pass exactly
+// when it is one in the first (both only look at the leaves' labels), with the
+// same digest, so its second hash and insert change nothing.  The shift test
+// reads a digest that is still cleared, so it asks one question of the map:
+// whether it holds the all-zero digest.  Which of the passes a node's insert
+// belongs to is kept in its epoch, and a map entry keeps the lowest (epoch,
+// priority), so the inserts may follow in any order.  4 GiB in 512-byte
+// chunks: the two passes took 2.10 ms (bottom 0.23, inserts 1.16, a barrier
+// per level with a second hash and insert of every node 0.71).
 constexpr uint32_t kSpanLevels = 9;     // 256 nodes on the bottom level of a span
 constexpr uint32_t kBottomLevels = 12;  // bottom span: 16 leaves per thread, 4096 per block
 constexpr uint32_t kBottomSink = 2048;  // queued inserts a bottom block holds in shared memory
@@ -134,7 +146,8 @@ __device__ __forceinline__ uint8_t forest_node(const ForestArgs& a, int pass, in
     if (baseline) {
       Digest dg = hash_pair(a.hash_kind, ld_digest(a.tree + l), ld_digest(a.tree + rr));
       st_digest(a.tree + n, dg);
-      if (map_insert_serial(a.map, dg, (uint32_t)n, cur_id, epoch_all, true, a.err)) atomicAdd(a.map.size, 1u);
+      if (pass == 1 && map_insert_serial(a.map, dg, (uint32_t)n, cur_id, epoch_all, true, a.err))
+        atomicAdd(a.map.size, 1u);
     }
   }
   if (store) a.labels[n] = lab_n;
@@ -206,13 +219,33 @@ __device__ __forceinline__ bool digest_wanted(int pass, uint8_t lab) {
 // One interior node n of an incremental pass (first-occurrence forest
 // src/tree_approach.cpp:378-404, duplicate forest :413-477, or both: pass 2)
 // given its children's labels and digests; `dg` receives n's digest when n is
-// hashed.  First-occurrence inserts go to the block's sink.
-template <int HK>
+// hashed.  First-occurrence inserts go to the block's sink.  BASE: pass 3,
+// every node hashed and its label kept for the inserts that follow.
+template <int HK, bool BASE>
 __device__ __forceinline__ uint8_t span_node(const ForestArgs& a, int pass, uint32_t n, uint8_t ll, uint8_t lr,
                                              const Digest& dl, const Digest& dr, Digest& dg, bool store,
                                              IdSink* sink) {
   const uint32_t l = 2 * n + 1, rr = l + 1;
   uint8_t lab_n;
+  if (BASE) {
+    uint8_t fl = ROOT_NONE, fr = ROOT_NONE;
+    lab_n = DONE;
+    if (ll != lr) {
+      fl = child_flag(ll);
+      fr = child_flag(lr);
+    } else if (ll == FIXED_DUPL || ll == FIRST_OCUR) {
+      lab_n = ll;
+    } else if (ll == SHIFT_DUPL) {
+      if (map_find(a.map, ld_digest(a.tree + n), a.err) >= 0) lab_n = SHIFT_DUPL;
+      else fl = fr = ROOT_SHIFT;
+    }
+    if (fl != ROOT_NONE) a.rflag[canon_pos(a, l)] = fl;
+    if (fr != ROOT_NONE) a.rflag[canon_pos(a, rr)] = fr;
+    dg = hash_pair(HK, dl, dr);
+    st_digest(a.tree + n, dg);
+    a.labels[n] = lab_n;
+    return lab_n;
+  }
   if (pass == 0) {
     if (ll == FIRST_OCUR && lr == FIRST_OCUR) {
       lab_n = FIRST_OCUR;
@@ -259,16 +292,16 @@ __device__ __forceinline__ uint8_t span_node(const ForestArgs& a, int pass, uint
 
 // Node n on the deepest interior level: a leaf there (a ragged last level)
 // keeps its label and stored digest; an interior node is computed.
-template <int HK>
+template <int HK, bool BASE>
 __device__ __forceinline__ uint8_t span_label(const ForestArgs& a, int pass, uint64_t n, uint64_t last_interior,
                                               uint64_t M, uint8_t ll, uint8_t lr, const Digest& dl,
                                               const Digest& dr, Digest& dg, IdSink* sink) {
   if (n > last_interior) {
     const uint8_t lab = n < M ? a.labels[n] : DONE;
-    if (digest_wanted(pass, lab)) dg = ld_digest(a.tree + n);
+    if (BASE ? n < M : digest_wanted(pass, lab)) dg = ld_digest(a.tree + n);
     return lab;
   }
-  return span_node<HK>(a, pass, (uint32_t)n, ll, lr, dl, dr, dg, false, sink);
+  return span_node<HK, BASE>(a, pass, (uint32_t)n, ll, lr, dl, dr, dg, false, sink);
 }
 
 __device__ __forceinline__ Digest shfl_digest(const Digest& d, int src) {
@@ -282,7 +315,7 @@ __device__ __forceinline__ Digest shfl_digest(const Digest& d, int src) {
 // five inside each warp (children's labels and digests by shuffle), then
 // three in warp 0 from the eight warps' results.  Stores r's label.  Every
 // node here is interior.
-template <int HK>
+template <int HK, bool BASE>
 __device__ __forceinline__ void upper_levels(const ForestArgs& a, int pass, uint64_t r, uint8_t lab, Digest dg,
                                              IdSink* sink, uint8_t* top8, Digest* topdg) {
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -293,14 +326,14 @@ __device__ __forceinline__ void upper_levels(const ForestArgs& a, int pass, uint
     const uint8_t cl = (uint8_t)__shfl_sync(kFull, lab, sl);
     const uint8_t cr = (uint8_t)__shfl_sync(kFull, lab, sr);
     Digest dl{{0, 0, 0, 0}}, dr{{0, 0, 0, 0}};
-    if (__any_sync(kFull, digest_wanted(pass, lab))) {
+    if (BASE || __any_sync(kFull, digest_wanted(pass, lab))) {
       dl = shfl_digest(dg, sl);
       dr = shfl_digest(dg, sr);
     }
     const uint32_t width = 32u >> step;
     if (lane < width) {
       const uint64_t n = (r + 1) * (256u >> step) - 1 + warp * width + lane;
-      lab = span_node<HK>(a, pass, (uint32_t)n, cl, cr, dl, dr, dg, false, sink);
+      lab = span_node<HK, BASE>(a, pass, (uint32_t)n, cl, cr, dl, dr, dg, false, sink);
     }
   }
   if (lane == 0) {
@@ -320,7 +353,7 @@ __device__ __forceinline__ void upper_levels(const ForestArgs& a, int pass, uint
       const uint32_t width = 256u >> step;
       if (lane < width) {
         const uint64_t n = (r + 1) * width - 1 + lane;
-        lab = span_node<HK>(a, pass, (uint32_t)n, cl, cr, dl, dr, dg, step == 8, sink);
+        lab = span_node<HK, BASE>(a, pass, (uint32_t)n, cl, cr, dl, dr, dg, step == 8, sink);
       }
     }
   }
@@ -331,7 +364,7 @@ __device__ __forceinline__ void upper_levels(const ForestArgs& a, int pass, uint
 // come from memory, the rest by upper_levels -- one block barrier instead of
 // nine, and no digest goes through memory between levels (they are still
 // stored: the tree keeps every digest for the next checkpoint).
-template <int HK>
+template <int HK, bool BASE>
 __global__ void __launch_bounds__(256) forest_span9_warp_kernel(ForestArgs a, int pass, uint32_t N, uint32_t d_top) {
   pdl_enter();
   __shared__ uint8_t top8[8];
@@ -356,15 +389,15 @@ __global__ void __launch_bounds__(256) forest_span9_warp_kernel(ForestArgs a, in
       const uint64_t c = 2 * n + 1;
       ll = c < M ? a.labels[c] : DONE;
       lr = c + 1 < M ? a.labels[c + 1] : DONE;
-      if (ll == lr && digest_wanted(pass, ll)) {
+      if (BASE || (ll == lr && digest_wanted(pass, ll))) {
         dl = ld_digest(a.tree + c);
         dr = ld_digest(a.tree + c + 1);
       }
     }
-    lab = span_label<HK>(a, pass, n, last_interior, M, ll, lr, dl, dr, dg, &sink);
+    lab = span_label<HK, BASE>(a, pass, n, last_interior, M, ll, lr, dl, dr, dg, &sink);
   }
-  upper_levels<HK>(a, pass, r, lab, dg, &sink, top8, topdg);
-  if (pass != 1) flush_sink(a, sink, &ids_base);
+  upper_levels<HK, BASE>(a, pass, r, lab, dg, &sink, top8, topdg);
+  if (!BASE && pass != 1) flush_sink(a, sink, &ids_base);
 }
 
 // Byte-parallel labelling of four (left, right) pairs per 32-bit word, the
@@ -403,7 +436,7 @@ __device__ __forceinline__ void set_byte(uint32_t& w, int b, uint32_t v) {
 // deepest interior level are all interior: the 16 children's labels in c[4]
 // (byte j = child j).  Returns the label of the thread's top node and its
 // digest in dg when a parent reads it.
-template <int HK>
+template <int HK, bool BASE>
 __device__ __forceinline__ uint8_t thread_levels_bytewise(const ForestArgs& a, int pass, uint64_t r, uint32_t t,
                                                           uint32_t c[4], IdSink* sink, Digest (*work)[256],
                                                           Digest& dg) {
@@ -420,6 +453,7 @@ __device__ __forceinline__ uint8_t thread_levels_bytewise(const ForestArgs& a, i
 #pragma unroll
     for (int q = 0; q < 2; q++) {
       uint32_t X = XF[q] | XS[q];
+      if (BASE) X = lvl == 0 ? ~0u : q == 1 ? 0u : lvl == 1 ? ~0u : lvl == 2 ? 0xffffu : 0xffu;  // every node
       while (X) {
         const int b = (__ffs(X) - 1) >> 3;
         X &= ~(0xffu << (8 * b));
@@ -434,6 +468,17 @@ __device__ __forceinline__ uint8_t thread_levels_bytewise(const ForestArgs& a, i
           dr = work[2 * i + 1][t];
         }
         const Digest d = hash_pair(HK, dl, dr);
+        if (BASE) {
+          if ((XS[q] >> (8 * b)) & 1 && map_find(a.map, ld_digest(a.tree + n), a.err) < 0) {
+            set_byte(P[q], b, DONE);
+            set_byte(FL[q], b, ROOT_SHIFT);
+            set_byte(FR[q], b, ROOT_SHIFT);
+          }
+          st_digest(a.tree + n, d);
+          a.labels[n] = (uint8_t)(P[q] >> (8 * b));
+          work[i][t] = d;
+          continue;
+        }
         st_digest(a.tree + n, d);
         if ((XF[q] >> (8 * b)) & 1) {
           queue_insert(a, sink, (uint32_t)n);
@@ -470,7 +515,7 @@ __device__ __forceinline__ uint8_t thread_levels_bytewise(const ForestArgs& a, i
     nb = (nb - 1) / 2;
   }
   const uint8_t lab = (uint8_t)c[0];
-  if (digest_wanted(pass, lab)) dg = work[0][t];
+  if (BASE || digest_wanted(pass, lab)) dg = work[0][t];
   return lab;
 }
 
@@ -482,7 +527,7 @@ __device__ __forceinline__ uint8_t thread_levels_bytewise(const ForestArgs& a, i
 // thread whose 16 children are all unchanged (fixed duplicates) has nothing
 // to hash, flag or insert.  upper_levels does the rest.  Loops rather than
 // unrolled levels keep the kernel small enough for the instruction cache.
-template <int HK>
+template <int HK, bool BASE>
 __global__ void __launch_bounds__(256) forest_bottom12_kernel(ForestArgs a, int pass, uint32_t N, uint32_t d_top) {
   pdl_enter();
   __shared__ uint8_t top8[8];
@@ -523,11 +568,11 @@ __global__ void __launch_bounds__(256) forest_bottom12_kernel(ForestArgs a, int 
   uint8_t lab;
   Digest dg{{0, 0, 0, 0}};
   constexpr uint64_t kFixed8 = 0x0101010101010101ull * FIXED_DUPL;
-  if (lo == kFixed8 && hi == kFixed8 && nb1 + 7 <= last_interior) {
+  if (!BASE && lo == kFixed8 && hi == kFixed8 && nb1 + 7 <= last_interior) {
     lab = pass == 0 ? DONE : FIXED_DUPL;
   } else if (nb1 + 7 <= last_interior) {
     uint32_t c[4] = {(uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32)};
-    lab = thread_levels_bytewise<HK>(a, pass, r, t, c, &sink, work, dg);
+    lab = thread_levels_bytewise<HK, BASE>(a, pass, r, t, c, &sink, work, dg);
   } else {
     uint64_t nb = nb1;
     uint32_t width = 8;
@@ -541,7 +586,7 @@ __global__ void __launch_bounds__(256) forest_bottom12_kernel(ForestArgs a, int 
         const uint8_t lr = (uint8_t)((j + 1 < 8 ? lo >> (8 * (j + 1)) : hi >> (8 * (j - 7))) & 0xff);
         const uint64_t n = nb + i;
         Digest dl{{0, 0, 0, 0}}, dr{{0, 0, 0, 0}}, d{{0, 0, 0, 0}};
-        if (ll == lr && digest_wanted(pass, ll)) {
+        if (BASE || (ll == lr && digest_wanted(pass, ll))) {
           if (lvl == 0) {
             if (n <= last_interior) {
               dl = ld_digest(a.tree + 2 * n + 1);
@@ -552,9 +597,9 @@ __global__ void __launch_bounds__(256) forest_bottom12_kernel(ForestArgs a, int 
             dr = work[j + 1][t];
           }
         }
-        const uint8_t l = lvl == 0 ? span_label<HK>(a, pass, n, last_interior, M, ll, lr, dl, dr, d, &sink)
-                                   : span_node<HK>(a, pass, (uint32_t)n, ll, lr, dl, dr, d, false, &sink);
-        if (digest_wanted(pass, l)) work[i][t] = d;  // read back only at the next level, from a higher index
+        const uint8_t l = lvl == 0 ? span_label<HK, BASE>(a, pass, n, last_interior, M, ll, lr, dl, dr, d, &sink)
+                                   : span_node<HK, BASE>(a, pass, (uint32_t)n, ll, lr, dl, dr, d, false, &sink);
+        if (BASE || digest_wanted(pass, l)) work[i][t] = d;  // read back only at the next level, from a higher index
         out |= (uint64_t)l << (8 * i);
         if (lvl == 3) dg = d;
       }
@@ -565,8 +610,8 @@ __global__ void __launch_bounds__(256) forest_bottom12_kernel(ForestArgs a, int 
     }
     lab = (uint8_t)lo;
   }
-  upper_levels<HK>(a, pass, r, lab, dg, &sink, top8, topdg);
-  if (pass != 1) flush_sink(a, sink, &ids_base);
+  upper_levels<HK, BASE>(a, pass, r, lab, dg, &sink, top8, topdg);
+  if (!BASE && pass != 1) flush_sink(a, sink, &ids_base);
 }
 
 // The queued first-occurrence inserts of a pass, one thread per node, over
@@ -579,6 +624,28 @@ __device__ __forceinline__ void drain_inserts(const ForestArgs& a, uint32_t b0, 
     const uint32_t node = a.ins_queue[k];
     // a first occurrence's digest is new: its leaves' are
     created += map_insert_serial(a.map, ld_digest(a.tree + node), node, cur_id, epoch_fo, false, a.err);
+  }
+  count_new_entries(a.map, created);
+}
+// After pass 3: every interior node's digest into the map.  First occurrences
+// carry the first pass's epoch, the others the second's, among which equal
+// digests abound (runs of equal chunks): those of a warp insert once.  Bound by the
+// random accesses (two operations on each line).
+__global__ void __launch_bounds__(256) forest_insert_all_kernel(ForestArgs a, uint32_t n_interior) {
+  pdl_enter();
+  const uint32_t cur_id = a.sp->cur, epoch = a.sp->epoch;
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t created = 0;
+  for (uint64_t nw = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); nw < n_interior;
+       nw += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t n = (uint32_t)nw + lane;
+    const bool in = nw + lane < n_interior;
+    const bool fo = in && a.labels[n] == FIRST_OCUR;
+    Digest d{{0, 0, 0, 0}};
+    if (in) d = ld_digest(a.tree + n);
+    if (fo) created += map_insert_serial(a.map, d, n, cur_id, epoch + 1, false, a.err);
+    if (__any_sync(0xffffffffu, in && !fo))
+      created += warp_insert_serial(a.map, in && !fo, d, n, cur_id, epoch + 2, a.err);
   }
   count_new_entries(a.map, created);
 }
@@ -1338,7 +1405,7 @@ cudaError_t launch_map_rebase(const DigestMap& m, uint64_t cap, cudaStream_t s) 
 // ---------------------------------------------------------------------------
 cudaError_t launch_forest(const ForestArgs& a, int pass, int baseline, uint32_t N, cudaStream_t s) {
   if (N < 2) return cudaSuccess;
-  if (pass == 0) {
+  if (pass == 0 || pass == 3) {
     // the duplicate pass (alone or fused into the first) writes only the
     // flags of roots; every other position (node 1 .. M-1 in canonical
     // order) reads ROOT_NONE
@@ -1350,13 +1417,15 @@ cudaError_t launch_forest(const ForestArgs& a, int pass, int baseline, uint32_t 
   uint32_t dmax = 0;
   while (((2ull << dmax) - 1) <= (uint64_t)(N - 2)) dmax++;
   const bool dup_baseline = pass == 1 && baseline;
+  const bool md5 = a.hash_kind == HASH_MD5;
   int bot = (int)dmax;
   if (!dup_baseline && dmax + 1 >= kBottomLevels) {
     const uint32_t top = dmax - (kBottomLevels - 1);
     const uint64_t first = (1ull << top) - 1;
     const uint64_t count = std::min<uint64_t>(1ull << top, (uint64_t)N - 1 - first);
-    if (a.hash_kind == HASH_MD5) launch_k(forest_bottom12_kernel<HASH_MD5>, (uint32_t)count, 256, 0, s, a, pass, N, top);
-    else launch_k(forest_bottom12_kernel<HASH_MURMUR3>, (uint32_t)count, 256, 0, s, a, pass, N, top);
+    auto k = pass == 3 ? (md5 ? forest_bottom12_kernel<HASH_MD5, true> : forest_bottom12_kernel<HASH_MURMUR3, true>)
+                       : (md5 ? forest_bottom12_kernel<HASH_MD5, false> : forest_bottom12_kernel<HASH_MURMUR3, false>);
+    launch_k(k, (uint32_t)count, 256, 0, s, a, pass, N, top);
     note_launch();
     bot = (int)top - 1;
   }
@@ -1364,16 +1433,19 @@ cudaError_t launch_forest(const ForestArgs& a, int pass, int baseline, uint32_t 
     const uint32_t top = bot >= (int)kSpanLevels - 1 ? (uint32_t)bot - (kSpanLevels - 1) : 0;
     const uint64_t first = (1ull << top) - 1;
     const uint64_t count = std::min<uint64_t>(1ull << top, (uint64_t)N - 1 - first);
+    auto k9 = pass == 3
+                  ? (md5 ? forest_span9_warp_kernel<HASH_MD5, true> : forest_span9_warp_kernel<HASH_MURMUR3, true>)
+                  : (md5 ? forest_span9_warp_kernel<HASH_MD5, false> : forest_span9_warp_kernel<HASH_MURMUR3, false>);
     if (!dup_baseline && (uint32_t)bot - top == kSpanLevels - 1)
-      if (a.hash_kind == HASH_MD5) launch_k(forest_span9_warp_kernel<HASH_MD5>, (uint32_t)count, 256, 0, s, a, pass, N, top);
-      else launch_k(forest_span9_warp_kernel<HASH_MURMUR3>, (uint32_t)count, 256, 0, s, a, pass, N, top);
+      launch_k(k9, (uint32_t)count, 256, 0, s, a, pass, N, top);
     else
       launch_k(forest_span_kernel, (uint32_t)count, 256, 0, s, a, pass, baseline, N, top, (uint32_t)bot);
     note_launch();
     if (top == 0) break;
   }
-  if (pass == 0) {
-    launch_k(forest_insert_kernel, grid_for(N, 256), 256, 0, s, a);
+  if (pass == 0 || pass == 3) {
+    if (pass == 0) launch_k(forest_insert_kernel, grid_for(N, 256), 256, 0, s, a);
+    else launch_k(forest_insert_all_kernel, grid_for(N - 1, 256), 256, 0, s, a, N - 1);
     note_launch();
   }
   return cudaGetLastError();

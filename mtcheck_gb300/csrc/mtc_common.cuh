@@ -493,6 +493,28 @@ __device__ __forceinline__ uint32_t map_insert_serial(const DigestMap& m, const 
   return r == INS_NEW ? 1u : 0u;
 }
 
+// The same for a whole warp: lanes that hold one digest insert it once, with
+// their serially first node (the lowest, for nodes of one depth; `node` must
+// ascend with the lanes there).  Every lane of the warp calls it, with one
+// epoch.
+__device__ __forceinline__ uint32_t warp_insert_serial(const DigestMap& m, bool in, const Digest& k, uint32_t node,
+                                                       uint32_t tree, uint32_t epoch, uint32_t* err) {
+  const uint32_t lane = threadIdx.x & 31;
+  const unsigned act = __ballot_sync(0xffffffffu, in);
+  if (!in) return 0;
+  const uint32_t depth = 31 - __clz(node + 1);
+  const unsigned like = __match_any_sync(act, k.w[0] ^ depth);
+  if (like & (like - 1)) {
+    const int src = __ffs(like) - 1;
+    const uint32_t w0 = __shfl_sync(like, k.w[0], src), w1 = __shfl_sync(like, k.w[1], src),
+                   w2 = __shfl_sync(like, k.w[2], src), w3 = __shfl_sync(like, k.w[3], src),
+                   dp = __shfl_sync(like, depth, src);
+    const bool same = k.w[0] == w0 && k.w[1] == w1 && k.w[2] == w2 && k.w[3] == w3 && depth == dp;
+    if (same && (int)lane != src) return 0;
+  }
+  return map_insert_serial(m, k, node, tree, epoch, true, err);
+}
+
 // Plain read of a slot's value after the launch that wrote it has finished.
 struct NodeIdDev { uint32_t node, tree; };
 __device__ __forceinline__ NodeIdDev slot_value(const DigestMap& m, int64_t slot) {

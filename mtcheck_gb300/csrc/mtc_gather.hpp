@@ -83,7 +83,8 @@ struct GatherArgs {
 };
 
 // All levels of one forest pass in a few launches (9 levels each).
-// pass 0 = first-occurrence forest, 1 = duplicate forest.
+// pass 0 = first-occurrence forest, 1 = duplicate forest, 3 = both, and the
+// inserts, of a baseline whose digests were cleared (baseline = 1).
 cudaError_t launch_forest(const ForestArgs& a, int pass, int baseline, uint32_t N, cudaStream_t s);
 cudaError_t launch_root_compaction(const ForestArgs& fa, uint32_t N, uint32_t M, uint32_t* fo_list,
                                    uint32_t* sh_list, Layout* lay, uint64_t* scan_scratch, uint64_t* scan_total,
