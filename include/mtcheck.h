@@ -326,9 +326,8 @@ typedef struct mtc_tune {
   int32_t threads_per_chunk; /* 1 (0 taken as 1): one thread per chunk; 32: one warp
                                 per chunk (chunks of at most 4096 bytes; the warp loads
                                 the chunk, one lane hashes it: the digests are serial) */
-  int32_t untimed;      /* 1: replay an incremental checkpoint as one graph, without the
-                           events between its phases (one graph launch instead of five);
-                           the phase times and the log timers then read 0 */
+  int32_t untimed;      /* 1: no readings of the device clock between the phases of a
+                           checkpoint; the phase times and the log timers then read 0 */
 } mtc_tune_t;
 int mtc_set_tuning(mtc_dedup_t* h, const mtc_tune_t* t);
 int mtc_get_tuning(const mtc_dedup_t* h, mtc_tune_t* out);

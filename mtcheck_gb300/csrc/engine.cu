@@ -21,12 +21,14 @@ static __global__ void set_word_kernel(uint32_t* p, uint32_t v) { *p = v; }
 // would wait behind it on the copy engine, and a kernel reading mapped host
 // memory behind it on the link.  A replayed graph gets each step's values
 // by an update of this node (Engine::replay_own).
-static __global__ void params_in_kernel(StepParams p, StepParams* dev, uint32_t* err) {
+static __global__ void params_in_kernel(StepParams p, ParamsOut o) {
   pdl_enter();
+  stamp(o.clk, CLK_BEGIN);
   if (threadIdx.x == 0) {
-    *dev = p;
-    *err = 0;
+    *o.sp = p;
+    *o.err = 0;
   }
+  stamp(o.clk, CLK_SETUP_DONE);
 }
 
 // Polls of an injected stall's bounded waits (about a millisecond).
@@ -34,8 +36,10 @@ constexpr uint32_t kInjectedSpinLimit = 1u << 14;
 
 static __global__ void readback_kernel(Readback r) {
   pdl_enter();
+  stamp(r.clk, CLK_END);
+  __syncwarp();
 #pragma unroll
-  for (int k = 0; k < 3; k++)
+  for (int k = 0; k < 4; k++)
     for (uint32_t i = threadIdx.x; i < r.words[k]; i += blockDim.x) r.dst[k][i] = r.src[k][i];
 }
 
@@ -66,6 +70,7 @@ Engine::Engine(int mode, int hash_kind, uint32_t chunk_size)
   cudaMallocHost(&lay_host_, sizeof(Layout));
   cudaMallocHost(&err_host_, 2 * sizeof(uint32_t));
   cudaMallocHost(&sp_host_, sizeof(StepParams));
+  cudaMallocHost(&clk_host_, CLK_COUNT * sizeof(uint64_t));
   std::memset(lay_host_, 0, sizeof(Layout));
   std::memset(sp_host_, 0, sizeof(StepParams));
   // test hook: start the launch epochs near their limit to exercise the rebase
@@ -85,6 +90,7 @@ Engine::~Engine() {
   if (lay_host_) cudaFreeHost(lay_host_);
   if (err_host_) cudaFreeHost(err_host_);
   if (sp_host_) cudaFreeHost(sp_host_);
+  if (clk_host_) cudaFreeHost(clk_host_);
   if (hdr_host_) cudaFreeHost(hdr_host_);
   if (rdi_ev_) cudaEventDestroy(rdi_ev_);
   if (rdi_host_) cudaFreeHost(rdi_host_);
@@ -197,6 +203,7 @@ int Engine::ensure_state(uint32_t N, bool fresh, uint32_t id_headroom) {
     MTC_CUDA(scan_total2_.ensure(1, stream_));
     MTC_CUDA(lay_.ensure(1, stream_));
     MTC_CUDA(sp_.ensure(1, stream_));
+    MTC_CUDA(clk_.ensure(CLK_COUNT, stream_));
     if (mode_ != MODE_BASIC) {
       // room for the baseline's inserts and the worst case of the next
       // checkpoint, so that the first incremental checkpoint does not grow it
@@ -232,6 +239,7 @@ GatherArgs Engine::gather_args(const uint8_t* data, uint64_t len) {
   g.digests = digests_.p;
   g.map = DigestMap{slots_.p, map_cap_ ? map_cap_ - 1 : 0, map_size_.p};
   g.err = err_.p;
+  g.clk = timed_ ? clk_.p : nullptr;
   g.fo_list = fo_list_.p;
   g.sh_list = sh_list_.p;
   g.fo_val = fo_val_.p;
@@ -269,6 +277,7 @@ int Engine::run_tree(const uint8_t* data, uint64_t len, bool baseline_path) {
   la.sp = sp_.p;
   la.leaf_base = N - 1;
   la.err = err_.p;
+  la.clk = timed_ ? clk_.p : nullptr;
   la.hash_kind = hash_kind_;
   la.epi = EPI_TREE;
   la.changed_list = changed_list_.p;
@@ -285,7 +294,6 @@ int Engine::run_tree(const uint8_t* data, uint64_t len, bool baseline_path) {
   MTC_CUDA(cudaMemsetAsync(changed_count_.p, 0, 4 * sizeof(uint32_t), stream_));
   if (leaf_hook_) MTC_TRY(leaf_hook_->on_leaves(this, la, stream_));
   else MTC_CUDA(launch_leaves(la, &tma_, stream_, leaf_tune_));
-  if (timed_) MTC_TRY(mark(4));
   MTC_CUDA(launch_leaf_inserts(la, stream_));
 
   ForestArgs fa{};
@@ -330,6 +338,7 @@ int Engine::run_list_basic(const uint8_t* data, uint64_t len) {
   la.sp = sp_.p;
   la.leaf_base = 0;
   la.err = err_.p;
+  la.clk = timed_ ? clk_.p : nullptr;
   la.hash_kind = hash_kind_;
   la.epi = mode_ == MODE_LIST ? EPI_LIST : EPI_BASIC;
   la.basic_first = current_id == 0 ? 1 : 0;  // never true in a captured sequence
@@ -345,10 +354,9 @@ int Engine::run_list_basic(const uint8_t* data, uint64_t len) {
   MTC_CUDA(cudaMemsetAsync(changed_count_.p, 0, 4 * sizeof(uint32_t), stream_));
   if (leaf_hook_) MTC_TRY(leaf_hook_->on_leaves(this, la, stream_));
   else MTC_CUDA(launch_leaves(la, &tma_, stream_, leaf_tune_));
-  if (timed_) MTC_TRY(mark(4));
   if (mode_ == MODE_LIST) MTC_CUDA(launch_leaf_inserts(la, stream_));
   MTC_CUDA(launch_chunk_compaction(labels_.p, N_, mode_ == MODE_BASIC ? 1 : 0, fo_list_.p, sh_list_.p, lay_.p, scan_.p,
-                                   scan_total_.p, stream_));
+                                   scan_total_.p, la.clk, stream_));
   return ST_OK;
 }
 
@@ -389,19 +397,17 @@ void Engine::stage_params() {
 
 int Engine::enqueue(const uint8_t* data, uint64_t len, bool timed) {
   timed_ = timed;
-  if (timed) MTC_TRY(mark(0));
   if (mode_ == MODE_FULL) {
     // FullDeduplicator: the checkpoint is the raw buffer (src/full_approach.cpp:66-72)
-    if (timed) MTC_TRY(mark(1));
-    if (timed) MTC_TRY(mark(2));
+    if (timed) MTC_CUDA(cudaEventRecord(ev_[0], stream_));
     MTC_CUDA(cudaMemcpyAsync(stage_.p, data, len, cudaMemcpyDeviceToDevice, stream_));
-    if (timed) MTC_TRY(mark(3));
+    if (timed) MTC_CUDA(cudaEventRecord(ev_[1], stream_));
     return ST_OK;
   }
   if (params_by_value_) {
     static const bool reg = (register_input_kernel(reinterpret_cast<const void*>(params_in_kernel), INPUT_PARAMS), true);
     (void)reg;
-    launch_k(params_in_kernel, 1, 32, 0, stream_, *sp_host_, sp_.p, err_.p);
+    launch_k(params_in_kernel, 1, 32, 0, stream_, *sp_host_, ParamsOut{sp_.p, err_.p, timed ? clk_.p : nullptr});
     note_launch();
     MTC_CUDA(cudaGetLastError());
   } else {
@@ -410,12 +416,9 @@ int Engine::enqueue(const uint8_t* data, uint64_t len, bool timed) {
     MTC_CUDA(cudaMemcpyAsync(sp_.p, sp_host_, sizeof(StepParams), cudaMemcpyHostToDevice, stream_));
     MTC_CUDA(cudaMemsetAsync(err_.p, 0, sizeof(uint32_t), stream_));
   }
-  if (timed) MTC_TRY(mark(1));
   int rc = (mode_ == MODE_LIST || mode_ == MODE_BASIC) ? run_list_basic(data, len) : run_tree(data, len, baseline_path_);
   if (rc) return rc;
-  if (timed) MTC_TRY(mark(2));
   MTC_CUDA(launch_assemble(gather_args(data, len), (uint64_t)N_ + 1, fresh_, stream_));
-  if (timed) MTC_TRY(mark(3));
   // results (layout, error word, map size) written to pinned memory by a
   // kernel, not queued on a copy engine behind other streams' transfers
   static_assert(sizeof(Layout) % 4 == 0, "layout copied as words");
@@ -431,23 +434,28 @@ int Engine::enqueue(const uint8_t* data, uint64_t len, bool timed) {
     rb.dst[2] = rb.dst[1] + 1;
     rb.words[2] = 1;
   }
+  if (timed) {
+    rb.src[3] = reinterpret_cast<const uint32_t*>(clk_.p);
+    rb.dst[3] = static_cast<uint32_t*>(host_alias(clk_host_));
+    rb.words[3] = CLK_COUNT * 2;
+    rb.clk = clk_.p;
+  }
   MTC_CUDA(launch_readback(rb, stream_));
   return ST_OK;
 }
 
 int Engine::order_inputs() {
   if (!order_after_legacy_) return ST_OK;
-  MTC_CUDA(cudaEventRecord(ev_[5], cudaStreamLegacy));
-  MTC_CUDA(cudaStreamWaitEvent(stream_, ev_[5], 0));
+  MTC_CUDA(cudaEventRecord(ev_[2], cudaStreamLegacy));
+  MTC_CUDA(cudaStreamWaitEvent(stream_, ev_[2], 0));
   return ST_OK;
 }
 
 void Engine::drop_own_graph() {
-  for (auto& sg : own_segs_) {
-    if (sg.exec) cudaGraphExecDestroy(sg.exec);
-    if (sg.graph) cudaGraphDestroy(sg.graph);
-  }
-  own_segs_.clear();
+  if (own_exec_) cudaGraphExecDestroy(own_exec_);
+  if (own_seq_) cudaGraphDestroy(own_seq_);
+  own_exec_ = nullptr;
+  own_seq_ = nullptr;
   input_nodes_.clear();
   own_sig_ = 0;
   own_data_ = nullptr;
@@ -479,7 +487,7 @@ int Engine::retarget_own(const uint8_t* data, uint64_t len) {
     cudaKernelNodeParams q = in.p;
     q.kernelParams = args;
     q.extra = nullptr;
-    MTC_CUDA(cudaGraphExecKernelNodeSetParams(own_segs_[in.seg].exec, in.node, &q));
+    MTC_CUDA(cudaGraphExecKernelNodeSetParams(own_exec_, in.node, &q));
   }
   own_data_ = data;
   return ST_OK;
@@ -491,11 +499,11 @@ int Engine::update_own_params() {
   for (auto& in : input_nodes_) {
     if (in.kind != INPUT_PARAMS) continue;
     StepParams sp = *sp_host_;
-    void* args[3] = {&sp, &in.sp_dev, &in.err_dev};
+    void* args[2] = {&sp, &in.po};
     cudaKernelNodeParams q = in.p;
     q.kernelParams = args;
     q.extra = nullptr;
-    MTC_CUDA(cudaGraphExecKernelNodeSetParams(own_segs_[in.seg].exec, in.node, &q));
+    MTC_CUDA(cudaGraphExecKernelNodeSetParams(own_exec_, in.node, &q));
   }
   return ST_OK;
 }
@@ -510,110 +518,69 @@ void Engine::set_own_graph(bool on) {
   if (!on) drop_own_graph();
 }
 
-// A timing mark of the launch sequence: an event on the stream, or, while
-// the sequence is being captured, the end of one segment and the start of the
-// next (an event recorded by a graph cannot be timed, so the events are
-// recorded between the segments' launches).
-int Engine::mark(int i) {
-  if (!seg_capture_) {
-    MTC_CUDA(cudaEventRecord(ev_[i], stream_));
-    return ST_OK;
-  }
-  if (untimed_) return ST_OK;  // one graph, no phase events
-  cudaGraph_t g = nullptr;
-  MTC_CUDA(cudaStreamEndCapture(cap_stream_, &g));
-  seg_graphs_.emplace_back(seg_mark_, g);
-  seg_mark_ = i;
-  MTC_CUDA(cudaStreamBeginCapture(cap_stream_, cudaStreamCaptureModeRelaxed));
-  return ST_OK;
-}
-
-// The launch sequence of an incremental checkpoint as a few graph launches:
-// each replay updates the step values (an argument of the first kernel) and,
-// for a new input buffer, the nodes that read the input, so one capture
-// serves every checkpoint until a device buffer or the launch shape changes
-// (the signature).
+// The launch sequence of an incremental checkpoint as one graph launch: each
+// replay updates the step values (an argument of the first kernel) and, for a
+// new input buffer, the nodes that read the input, so one capture serves
+// every checkpoint until a device buffer or the launch shape changes (the
+// signature).  The phases are timed by the kernels themselves (CLK_*): events
+// between them cut the sequence into five graphs, whose launches and gaps
+// took 10-15 us of a 145 us checkpoint of 64 MiB in 128-byte chunks.
 int Engine::replay_own(const uint8_t* data, uint64_t len) {
   const uint64_t sig = shape_signature(data, len);
-  if (!own_segs_.empty() && sig == own_sig_ && data != own_data_) MTC_TRY(retarget_own(data, len));
-  if (own_segs_.empty() || sig != own_sig_) {
+  if (own_exec_ && sig == own_sig_ && data != own_data_) MTC_TRY(retarget_own(data, len));
+  if (!own_exec_ || sig != own_sig_) {
     drop_own_graph();
     if (!cap_stream_) MTC_CUDA(cudaStreamCreateWithFlags(&cap_stream_, cudaStreamNonBlocking));
     const uint64_t l0 = launch_count();
-    seg_graphs_.clear();
-    seg_mark_ = -1;
     MTC_CUDA(cudaStreamBeginCapture(cap_stream_, cudaStreamCaptureModeRelaxed));
     cudaStream_t keep = stream_;
     stream_ = cap_stream_;
-    seg_capture_ = true;
-    int rc = enqueue(data, len, true);
-    seg_capture_ = false;
+    const int rc = enqueue(data, len, !untimed_);
     stream_ = keep;
-    cudaGraph_t g = nullptr;
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(cap_stream_, &st);
-    const cudaError_t ee = st == cudaStreamCaptureStatusActive ? cudaStreamEndCapture(cap_stream_, &g) : cudaSuccess;
-    if (g) seg_graphs_.emplace_back(seg_mark_, g);
-    cudaError_t ie = cudaSuccess;
-    if (rc == ST_OK && ee == cudaSuccess) {
-      for (auto& sg : seg_graphs_) {
-        size_t n = 0;
-        cudaGraphGetNodes(sg.second, nullptr, &n);
-        cudaGraphExec_t x = nullptr;
-        if (n && ie == cudaSuccess) ie = cudaGraphInstantiate(&x, sg.second, 0);
-        own_segs_.push_back(OwnSeg{sg.first, sg.second, x});
-        sg.second = nullptr;  // owned by own_segs_ (node handles stay valid for updates)
-        if (!n || ie != cudaSuccess) continue;
-        std::vector<cudaGraphNode_t> nodes(n);
-        cudaGraphGetNodes(own_segs_.back().graph, nodes.data(), &n);
-        for (cudaGraphNode_t nd : nodes) {
-          cudaGraphNodeType ty;
-          if (cudaGraphNodeGetType(nd, &ty) != cudaSuccess || ty != cudaGraphNodeTypeKernel) continue;
-          InputNode in{};
-          if (cudaGraphKernelNodeGetParams(nd, &in.p) != cudaSuccess) continue;
-          in.kind = input_kernel_kind(in.p.func);
-          if (in.kind == INPUT_NONE) continue;
-          in.seg = own_segs_.size() - 1;
-          in.node = nd;
-          if (in.kind == INPUT_LEAF_TMA) {
-            std::memcpy(&in.tmap, in.p.kernelParams[0], sizeof(CUtensorMap));
-            std::memcpy(&in.la, in.p.kernelParams[1], sizeof(LeafArgs));
-            std::memcpy(&in.u[0], in.p.kernelParams[2], sizeof(uint32_t));
-          } else if (in.kind == INPUT_LEAF_DIRECT) {
-            std::memcpy(&in.la, in.p.kernelParams[0], sizeof(LeafArgs));
-            std::memcpy(&in.u[0], in.p.kernelParams[1], sizeof(uint32_t));
-            std::memcpy(&in.u[1], in.p.kernelParams[2], sizeof(uint32_t));
-          } else if (in.kind == INPUT_PARAMS) {
-            std::memcpy(&in.sp_dev, in.p.kernelParams[1], sizeof(StepParams*));
-            std::memcpy(&in.err_dev, in.p.kernelParams[2], sizeof(uint32_t*));
-          } else {
-            std::memcpy(&in.ga, in.p.kernelParams[0], sizeof(GatherArgs));
-          }
-          in.p.kernelParams = nullptr;
-          input_nodes_.push_back(in);
-        }
+    cudaError_t ce = cudaStreamEndCapture(cap_stream_, &own_seq_);
+    size_t n = 0;
+    if (rc == ST_OK && ce == cudaSuccess) ce = cudaGraphInstantiate(&own_exec_, own_seq_, 0);
+    if (rc == ST_OK && ce == cudaSuccess) ce = cudaGraphGetNodes(own_seq_, nullptr, &n);
+    std::vector<cudaGraphNode_t> nodes(n);
+    if (n) cudaGraphGetNodes(own_seq_, nodes.data(), &n);
+    for (cudaGraphNode_t nd : nodes) {
+      cudaGraphNodeType ty;
+      if (cudaGraphNodeGetType(nd, &ty) != cudaSuccess || ty != cudaGraphNodeTypeKernel) continue;
+      InputNode in{};
+      if (cudaGraphKernelNodeGetParams(nd, &in.p) != cudaSuccess) continue;
+      in.kind = input_kernel_kind(in.p.func);
+      if (in.kind == INPUT_NONE) continue;
+      in.node = nd;
+      if (in.kind == INPUT_LEAF_TMA) {
+        std::memcpy(&in.tmap, in.p.kernelParams[0], sizeof(CUtensorMap));
+        std::memcpy(&in.la, in.p.kernelParams[1], sizeof(LeafArgs));
+        std::memcpy(&in.u[0], in.p.kernelParams[2], sizeof(uint32_t));
+      } else if (in.kind == INPUT_LEAF_DIRECT) {
+        std::memcpy(&in.la, in.p.kernelParams[0], sizeof(LeafArgs));
+        std::memcpy(&in.u[0], in.p.kernelParams[1], sizeof(uint32_t));
+        std::memcpy(&in.u[1], in.p.kernelParams[2], sizeof(uint32_t));
+      } else if (in.kind == INPUT_PARAMS) {
+        std::memcpy(&in.po, in.p.kernelParams[1], sizeof(ParamsOut));
+      } else {
+        std::memcpy(&in.ga, in.p.kernelParams[0], sizeof(GatherArgs));
       }
+      in.p.kernelParams = nullptr;
+      input_nodes_.push_back(in);
     }
-    for (auto& sg : seg_graphs_)
-      if (sg.second) cudaGraphDestroy(sg.second);
-    seg_graphs_.clear();
-    if (rc != ST_OK || ee != cudaSuccess || ie != cudaSuccess) {
+    if (rc != ST_OK || ce != cudaSuccess) {
       drop_own_graph();
       cudaGetLastError();
       if (rc != ST_OK) return rc;
-      return fail(ST_ECUDA, std::string("graph capture: ") + cudaGetErrorString(ee != cudaSuccess ? ee : ie));
+      return fail(ST_ECUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
     }
     own_sig_ = sig;
     own_data_ = data;
-    own_kernels_ = launch_count() - l0;  // counted while capturing, run by the launches below
+    own_kernels_ = launch_count() - l0;  // counted while capturing, run by the launch below
   } else {
     MTC_TRY(update_own_params());
     note_launch((uint32_t)own_kernels_);
   }
-  for (auto& sg : own_segs_) {
-    if (sg.mark >= 0) MTC_CUDA(cudaEventRecord(ev_[sg.mark], stream_));
-    if (sg.exec) MTC_CUDA(cudaGraphLaunch(sg.exec, stream_));
-  }
+  MTC_CUDA(cudaGraphLaunch(own_exec_, stream_));
   timed_ = !untimed_;
   return ST_OK;
 }
@@ -648,15 +615,19 @@ static float event_ms(cudaEvent_t a, cudaEvent_t b) {
 }
 
 int Engine::complete(uint64_t len, HeaderHost* header) {
-  float ms[3] = {0, 0, 0};
-  if (timed_) {
-    ms[0] = event_ms(ev_[0], ev_[1]);
-    ms[1] = event_ms(ev_[1], ev_[2]);
-    ms[2] = event_ms(ev_[2], ev_[3]);
-    timers[0] = ms[0] * 1e-3; timers[1] = ms[1] * 1e-3; timers[2] = ms[2] * 1e-3;
-  } else {
-    timers[0] = timers[1] = timers[2] = 0;
-    phase_times[0] = phase_times[1] = phase_times[2] = 0;
+  timers[0] = timers[1] = timers[2] = 0;
+  phase_times[0] = phase_times[1] = phase_times[2] = 0;
+  if (timed_ && mode_ == MODE_FULL) {
+    timers[2] = event_ms(ev_[0], ev_[1]) * 1e-3;
+  } else if (timed_) {
+    // seconds between two readings of the device clock
+    auto span = [&](int from, int to) { return (double)(int64_t)(clk_host_[to] - clk_host_[from]) * 1e-9; };
+    timers[0] = span(CLK_BEGIN, CLK_SETUP_DONE);
+    timers[1] = span(CLK_SETUP_DONE, CLK_ROOTS_DONE);
+    timers[2] = span(CLK_ROOTS_DONE, CLK_END);
+    phase_times[0] = span(CLK_SETUP_DONE, CLK_LEAVES_DONE);
+    phase_times[1] = span(CLK_LEAVES_DONE, CLK_ROOTS_DONE);
+    phase_times[2] = timers[2];
   }
   if (mode_ == MODE_FULL) {
     diff_len_ = len;
@@ -669,10 +640,6 @@ int Engine::complete(uint64_t len, HeaderHost* header) {
   const Layout& L = *lay_host_;
   last_device_error = err_host_[0];
   if (map_size_.p) map_size_host_ = err_host_[1];
-  if (timed_) {
-    const float leaf = event_ms(ev_[1], ev_[4]), rest = event_ms(ev_[4], ev_[2]);
-    phase_times[0] = leaf * 1e-3; phase_times[1] = rest * 1e-3; phase_times[2] = ms[2] * 1e-3;
-  }
   if (last_device_error & DERR_SPIN) {
     // some chunks' digests may already be stored: the next checkpoint starts
     // from scratch as a baseline
@@ -720,7 +687,7 @@ uint64_t Engine::shape_signature(const uint8_t* data, uint64_t len) const {
                         (uint64_t)sh_key_.p, (uint64_t)sh_prev_.p, (uint64_t)hist_.p, hist_.n, (uint64_t)rep_.p,
                         (uint64_t)rank_.p, (uint64_t)fo_val_.p, (uint64_t)sort_mat_.p, sort_mat_.n, (uint64_t)scan_.p,
                         (uint64_t)scan_total_.p, (uint64_t)scan2_.p, (uint64_t)scan_total2_.p, (uint64_t)stage_.p,
-                        stage_.n, (uint64_t)lay_.p, (uint64_t)sp_.p, (uint64_t)baseline_path_, (uint64_t)mode_,
+                        stage_.n, (uint64_t)lay_.p, (uint64_t)sp_.p, (uint64_t)clk_.p, (uint64_t)baseline_path_, (uint64_t)mode_,
                         (uint64_t)leaf_tune_.rows, (uint64_t)leaf_tune_.ctas_per_sm, (uint64_t)leaf_tune_.direct,
                         (uint64_t)leaf_tune_.threads_per_chunk};
   uint64_t h = 1469598103934665603ull;
@@ -733,7 +700,7 @@ void Engine::for_each_buf(F f) {
   f(digests_); f(labels_); f(rflag_); f(chunk_slot_); f(changed_list_); f(changed_count_); f(slots_);
   f(map_size_); f(err_); f(fo_list_); f(sh_list_); f(reg_chunk_); f(reg_slot_); f(reg_len_); f(sh_key_);
   f(sh_prev_); f(hist_); f(rep_); f(rank_); f(fo_val_); f(sort_mat_); f(scan_); f(scan_total_); f(scan2_);
-  f(scan_total2_); f(stage_); f(lay_); f(sp_);
+  f(scan_total2_); f(stage_); f(lay_); f(sp_); f(clk_);
 }
 
 void Engine::set_pool(cudaMemPool_t pool) {
@@ -810,7 +777,7 @@ uint64_t Engine::device_bytes() const {
                              rep_.n + rank_.n) +
          sizeof(MapSlot) * slots_.n +
          sizeof(uint64_t) * (fo_val_.n + sort_mat_.n + scan_.n + scan_total_.n + scan2_.n + scan_total2_.n) + stage_.n +
-         sizeof(Layout) * lay_.n + sizeof(StepParams) * sp_.n;
+         sizeof(Layout) * lay_.n + sizeof(StepParams) * sp_.n + sizeof(uint64_t) * clk_.n;
 }
 
 const uint8_t* Engine::diff_device() const { return stage_.p ? stage_.p + diff_pad_ : nullptr; }

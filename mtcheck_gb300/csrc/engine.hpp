@@ -157,8 +157,7 @@ class Engine {
   // signature changes (on by default; a Batch never uses it).
   void set_own_graph(bool on);
   bool own_graph() const { return own_graph_; }
-  // Replay an incremental checkpoint as one graph without the phase events
-  // between its segments; its timers and phase times then read 0.
+  // Take checkpoints without timing them: their timers and phase times read 0.
   void set_untimed(bool on);
   bool untimed() const { return untimed_; }
   // Batch members read their step values from the pinned block at run time.
@@ -273,17 +272,11 @@ class Engine {
   uint32_t N_ = 0, M_ = 0;
   bool own_graph_ = true;
   bool untimed_ = false;
-  // the captured sequence, cut at the timing marks: the event recorded
-  // before each segment (or -1) and the segment's graph (null when empty)
-  struct OwnSeg {
-    int mark;
-    cudaGraph_t graph;
-    cudaGraphExec_t exec;
-  };
-  std::vector<OwnSeg> own_segs_;
+  // the captured launch sequence
+  cudaGraph_t own_seq_ = nullptr;
+  cudaGraphExec_t own_exec_ = nullptr;
   // kernel nodes that read the input buffer, with their captured arguments
   struct InputNode {
-    size_t seg;
     cudaGraphNode_t node;
     int kind;
     cudaKernelNodeParams p;
@@ -291,8 +284,7 @@ class Engine {
     LeafArgs la;
     uint32_t u[2];
     GatherArgs ga;
-    StepParams* sp_dev;  // INPUT_PARAMS: the kernel's pointer arguments
-    uint32_t* err_dev;
+    ParamsOut po;
   };
   std::vector<InputNode> input_nodes_;
   const uint8_t* own_data_ = nullptr;  // input pointer the graphs currently read
@@ -300,11 +292,7 @@ class Engine {
   uint64_t own_sig_ = 0, own_kernels_ = 0;
   int retarget_own(const uint8_t* data, uint64_t len);
   int update_own_params();
-  bool seg_capture_ = false;  // enqueue runs under a capture cut at each mark
-  int seg_mark_ = -1;
-  std::vector<std::pair<int, cudaGraph_t>> seg_graphs_;
   int replay_own(const uint8_t* data, uint64_t len);
-  int mark(int i);
   void drop_own_graph();
   bool stream_work_ = false;
   LeafHook* leaf_hook_ = nullptr;
@@ -325,13 +313,15 @@ class Engine {
   DevBuf<uint8_t> stage_;
   DevBuf<Layout> lay_;
   DevBuf<StepParams> sp_;
+  DevBuf<uint64_t> clk_;            // device times of a checkpoint's phases (CLK_*)
   StepParams* sp_host_ = nullptr;   // pinned
   Layout* lay_host_ = nullptr;      // pinned
   uint32_t* err_host_ = nullptr;    // pinned [err, map size]
+  uint64_t* clk_host_ = nullptr;    // pinned copy of clk_
   bool params_by_value_ = true;     // false for batch members (their graphs copy sp_host_)
   uint64_t diff_len_ = 0, diff_pad_ = 0;
   TmaCache tma_;
-  cudaEvent_t ev_[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  cudaEvent_t ev_[3] = {nullptr, nullptr, nullptr};  // two timing events, one ordering event
   RestartScratch* rs_ = nullptr;  // restart buffers, created on first use
   // restart: a second stream for the work that does not depend on the main
   // sequence (clears, the chain tables beside the main scatter, the copy of

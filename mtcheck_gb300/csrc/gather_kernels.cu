@@ -887,6 +887,7 @@ __device__ __forceinline__ void shift_prep(const GatherArgs& g) {
 // Both root lists' lookups in one launch.
 __global__ void roots_prep_kernel(GatherArgs g) {
   pdl_enter();
+  stamp(g.clk, CLK_ROOTS_DONE);
   shift_prep(g);
   fo_prep(g);
 }
@@ -1353,8 +1354,9 @@ struct ChunkEmit {
     if (v >> 32) sh_list[(uint32_t)(ex >> 32)] = (uint32_t)c;
   }
 };
-__global__ void chunk_totals_kernel(const uint64_t* total, Layout* lay) {
+__global__ void chunk_totals_kernel(const uint64_t* total, Layout* lay, uint64_t* clk) {
   pdl_enter();
+  stamp(clk, CLK_LEAVES_DONE);
   lay->root_fo = 0;
   lay->F = (uint32_t)(*total);
   lay->S = (uint32_t)(*total >> 32);
@@ -1473,11 +1475,11 @@ cudaError_t launch_root_compaction(const ForestArgs& fa, uint32_t N, uint32_t M,
 
 cudaError_t launch_chunk_compaction(const uint8_t* labels, uint32_t n_chunks, int basic, uint32_t* fo_list,
                                     uint32_t* sh_list, Layout* lay, uint64_t* scan_scratch, uint64_t* scan_total,
-                                    cudaStream_t s) {
+                                    uint64_t* clk, cudaStream_t s) {
   cudaError_t e = grid_scan(ChunkVal{labels, basic}, ChunkEmit{fo_list, sh_list}, nullptr, n_chunks, scan_scratch,
                             scan_total, s);
   if (e != cudaSuccess) return e;
-  launch_k(chunk_totals_kernel, 1, 1, 0, s, scan_total, lay);
+  launch_k(chunk_totals_kernel, 1, 1, 0, s, scan_total, lay, basic ? clk : nullptr);
   note_launch();
   return cudaGetLastError();
 }

@@ -36,6 +36,15 @@ __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// One thread of a launch records the device clock in clk[i] (null: no record).
+__device__ __forceinline__ void stamp(uint64_t* clk, int i) {
+  if (clk && blockIdx.x == 0 && threadIdx.x == 0) {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    clk[i] = t;
+  }
+}
+
 // Raise bits in a device error word (a launch given none records nothing).
 __device__ __forceinline__ void raise_err(uint32_t* err, uint32_t bits) {
   if (err) atomicOr(err, bits);

@@ -69,6 +69,7 @@ struct GatherArgs {
   const Digest* digests;  // tree heap (by node) or hash list (by chunk)
   DigestMap map;
   uint32_t* err;
+  uint64_t* clk;          // CLK_ROOTS_DONE is written by the first launch
   const uint32_t* fo_list;
   const uint32_t* sh_list;
   uint64_t* fo_val;
@@ -91,7 +92,7 @@ cudaError_t launch_root_compaction(const ForestArgs& fa, uint32_t N, uint32_t M,
                                    cudaStream_t s);
 cudaError_t launch_chunk_compaction(const uint8_t* labels, uint32_t n_chunks, int basic, uint32_t* fo_list,
                                     uint32_t* sh_list, Layout* lay, uint64_t* scan_scratch, uint64_t* scan_total,
-                                    cudaStream_t s);
+                                    uint64_t* clk, cudaStream_t s);
 // Assemble the diff into g.stage; max_entries bounds F and S (N + 1).
 // whole: most chunks are expected in the diff (a baseline).
 cudaError_t launch_assemble(const GatherArgs& g, uint64_t max_entries, bool whole, cudaStream_t s);

@@ -31,6 +31,19 @@ struct StepParams {
 };
 constexpr uint32_t kEpochsPerCheckpoint = 3;
 
+// Device clock readings of a checkpoint's phases, written by one thread of the
+// first kernel of each (%globaltimer, 32 ns steps): the phases are timed
+// inside the replayed launch sequence, which an event between its kernels
+// would cut in pieces.
+enum : int { CLK_BEGIN = 0, CLK_SETUP_DONE = 1, CLK_LEAVES_DONE = 2, CLK_ROOTS_DONE = 3, CLK_END = 4, CLK_COUNT = 5 };
+
+// What the first kernel of a checkpoint writes.
+struct ParamsOut {
+  StepParams* sp;
+  uint32_t* err;
+  uint64_t* clk;
+};
+
 struct LeafArgs {
   const uint8_t* data = nullptr;  // device buffer being checkpointed
   uint64_t len = 0;               // bytes
@@ -44,6 +57,7 @@ struct LeafArgs {
   const StepParams* sp = nullptr; // current checkpoint id and launch epoch (device)
   uint32_t leaf_base = 0;         // node id of chunk 0 (N-1 for the tree, 0 for the list)
   uint32_t* err = nullptr;        // device error word
+  uint64_t* clk = nullptr;        // CLK_LEAVES_DONE is written by the insert pass (may be null)
   uint32_t* changed_list = nullptr;  // chunks whose digest changed (tree, list)
   uint32_t* changed_count = nullptr;
   uint32_t* demoted = nullptr;    // set to 1 when a first occurrence is demoted (tree; may be null)
@@ -136,19 +150,21 @@ int num_sms();
 // Small device results to pinned host memory, written by a kernel through the
 // memory's device mapping instead of copied: copies of a few bytes would
 // queue on the copy engines behind large transfers of other streams (an
-// upload, another process's spill).  Up to three (src, dst, words) segments;
+// upload, another process's spill).  Up to four (src, dst, words) segments;
 // dst is the device alias of pinned memory (host_alias).
 struct Readback {
-  const uint32_t* src[3];
-  uint32_t* dst[3];
-  uint32_t words[3];
+  const uint32_t* src[4];
+  uint32_t* dst[4];
+  uint32_t words[4];
+  uint64_t* clk;  // CLK_END is written here first (may be null)
 };
 cudaError_t launch_readback(const Readback& r, cudaStream_t s);
 // The device address of pinned host memory (the same pointer under unified
 // addressing).
 void* host_alias(void* pinned);
 
-// Kernel launch with programmatic stream serialization (see pdl_enter): the
+// Kernel launch with programmatic stream serialization (see pdl_enter; launch_with
+// false: without): the
 // kernel may be scheduled while its predecessor finishes, hiding the launch
 // gap between the dependent kernels of a checkpoint.  Off when MTCHECK_PDL=0,
 // and while a thread holds a PdlSuppress (captures that become child graphs).
@@ -158,8 +174,8 @@ struct PdlSuppress {
   ~PdlSuppress();
 };
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                            Args... args) {
+inline cudaError_t launch_with(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                               Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -169,8 +185,13 @@ inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  cfg.numAttrs = pdl && pdl_enabled() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                            Args... args) {
+  return launch_with(true, kernel, grid, block, smem, s, args...);
 }
 // Running count of kernel launches issued by the library (all handles).
 void note_launch(uint32_t n = 1);
@@ -184,7 +205,7 @@ enum : int {
   INPUT_LEAF_TMA = 1,     // (const CUtensorMap, LeafArgs, uint32_t)
   INPUT_LEAF_DIRECT = 2,  // (LeafArgs, uint32_t, uint32_t)
   INPUT_GATHER = 3,       // (GatherArgs)
-  INPUT_PARAMS = 4,       // (StepParams, StepParams*, uint32_t*): the step values
+  INPUT_PARAMS = 4,       // (StepParams, ParamsOut): the step values
 };
 void register_input_kernel(const void* func, int kind);
 int input_kernel_kind(const void* func);
