@@ -21,14 +21,24 @@ static __global__ void set_word_kernel(uint32_t* p, uint32_t v) { *p = v; }
 // would wait behind it on the copy engine, and a kernel reading mapped host
 // memory behind it on the link.  A replayed graph gets each step's values
 // by an update of this node (Engine::replay_own).
-static __global__ void params_in_kernel(StepParams p, ParamsOut o) {
-  pdl_enter();
+__device__ __forceinline__ void params_store(const StepParams& p, const ParamsOut& o) {
   stamp(o.clk, CLK_BEGIN);
   if (threadIdx.x == 0) {
     *o.sp = p;
     *o.err = 0;
   }
+  if (threadIdx.x < kCounters) o.counters[threadIdx.x] = 0;
   stamp(o.clk, CLK_SETUP_DONE);
+}
+static __global__ void params_in_kernel(StepParams p, ParamsOut o) {
+  pdl_enter();
+  params_store(p, o);
+}
+// A batch member's sequence, replayed inside the batch's graph, reads the step
+// values staged in the pinned block.
+static __global__ void params_host_kernel(const volatile StepParams* host, ParamsOut o) {
+  pdl_enter();
+  params_store(StepParams{host->cur, host->baseline_id, host->epoch, host->pad}, o);
 }
 
 // Polls of an injected stall's bounded waits (about a millisecond).
@@ -161,7 +171,11 @@ int Engine::ensure_sort(uint32_t K) {
   // reallocate on every call
   K = (uint32_t)next_pow2(std::max<uint32_t>(K, 64));
   const uint64_t T = (uint64_t)(N_ + 1 + kSortTile - 1) / kSortTile + 1;
-  MTC_CUDA(hist_.ensure(K, stream_));
+  if (hist_.n < K) {
+    // zero between checkpoints (the layout kernel clears what it has read)
+    MTC_CUDA(hist_.ensure(K, stream_));
+    MTC_CUDA(cudaMemsetAsync(hist_.p, 0, sizeof(uint32_t) * hist_.n, stream_));
+  }
   MTC_CUDA(rep_.ensure(K, stream_));
   MTC_CUDA(rank_.ensure(K, stream_));
   MTC_CUDA(sort_mat_.ensure((size_t)K * T, stream_));
@@ -182,10 +196,13 @@ int Engine::ensure_state(uint32_t N, bool fresh, uint32_t id_headroom) {
     MTC_CUDA(digests_.ensure(nd, stream_));
     MTC_CUDA(cudaMemsetAsync(digests_.p, 0, sizeof(Digest) * nd, stream_));
     MTC_CUDA(labels_.ensure(nd, stream_));
-    MTC_CUDA(rflag_.ensure(tree ? M : 1, stream_));
+    // root flags, read in 16-byte words: zero between checkpoints (the root
+    // compaction clears what it has read)
+    MTC_CUDA(rflag_.ensure(tree ? ((size_t)M + 15) / 16 * 16 : 16, stream_));
+    MTC_CUDA(cudaMemsetAsync(rflag_.p, 0, rflag_.n, stream_));
     MTC_CUDA(chunk_slot_.ensure(N, stream_));
     MTC_CUDA(changed_list_.ensure(N, stream_));
-    MTC_CUDA(changed_count_.ensure(4, stream_));  // [changed chunks, leaves demoted, forest inserts, duplicate notes]
+    MTC_CUDA(changed_count_.ensure(kCounters, stream_));
     MTC_CUDA(map_size_.ensure(1, stream_));
     MTC_CUDA(err_.ensure(1, stream_));
     MTC_CUDA(fo_list_.ensure(N + 1, stream_));
@@ -291,7 +308,6 @@ int Engine::run_tree(const uint8_t* data, uint64_t len, bool baseline_path) {
     la.stall = 1;
     la.spin_limit = kInjectedSpinLimit;
   }
-  MTC_CUDA(cudaMemsetAsync(changed_count_.p, 0, 4 * sizeof(uint32_t), stream_));
   if (leaf_hook_) MTC_TRY(leaf_hook_->on_leaves(this, la, stream_));
   else MTC_CUDA(launch_leaves(la, &tma_, stream_, leaf_tune_));
   MTC_CUDA(launch_leaf_inserts(la, stream_));
@@ -351,7 +367,6 @@ int Engine::run_list_basic(const uint8_t* data, uint64_t len) {
     la.stall = 1;
     la.spin_limit = kInjectedSpinLimit;
   }
-  MTC_CUDA(cudaMemsetAsync(changed_count_.p, 0, 4 * sizeof(uint32_t), stream_));
   if (leaf_hook_) MTC_TRY(leaf_hook_->on_leaves(this, la, stream_));
   else MTC_CUDA(launch_leaves(la, &tma_, stream_, leaf_tune_));
   if (mode_ == MODE_LIST) MTC_CUDA(launch_leaf_inserts(la, stream_));
@@ -404,18 +419,18 @@ int Engine::enqueue(const uint8_t* data, uint64_t len, bool timed) {
     if (timed) MTC_CUDA(cudaEventRecord(ev_[1], stream_));
     return ST_OK;
   }
+  // one kernel for the step values and every clear: each memset or copy of a
+  // few bytes was a node of its own in the replayed sequence
+  const ParamsOut po{sp_.p, err_.p, timed ? clk_.p : nullptr, changed_count_.p};
   if (params_by_value_) {
     static const bool reg = (register_input_kernel(reinterpret_cast<const void*>(params_in_kernel), INPUT_PARAMS), true);
     (void)reg;
-    launch_k(params_in_kernel, 1, 32, 0, stream_, *sp_host_, ParamsOut{sp_.p, err_.p, timed ? clk_.p : nullptr});
-    note_launch();
-    MTC_CUDA(cudaGetLastError());
+    launch_k(params_in_kernel, 1, 32, 0, stream_, *sp_host_, po);
   } else {
-    // a batch member: its sequence, replayed inside the batch's graph, copies
-    // the step values staged in the pinned block
-    MTC_CUDA(cudaMemcpyAsync(sp_.p, sp_host_, sizeof(StepParams), cudaMemcpyHostToDevice, stream_));
-    MTC_CUDA(cudaMemsetAsync(err_.p, 0, sizeof(uint32_t), stream_));
+    launch_k(params_host_kernel, 1, 32, 0, stream_, (const volatile StepParams*)host_alias(sp_host_), po);
   }
+  note_launch();
+  MTC_CUDA(cudaGetLastError());
   int rc = (mode_ == MODE_LIST || mode_ == MODE_BASIC) ? run_list_basic(data, len) : run_tree(data, len, baseline_path_);
   if (rc) return rc;
   MTC_CUDA(launch_assemble(gather_args(data, len), (uint64_t)N_ + 1, fresh_, stream_));

@@ -687,22 +687,14 @@ __device__ __forceinline__ uint64_t count_word(uint32_t w) {
   return (uint64_t)__popc(w & 0x01010101u) | ((uint64_t)__popc(w & 0x02020202u) << 32);
 }
 
-// The thread's flags starting at p (p a multiple of 16); bytes at or past n
-// read as ROOT_NONE.
+// The thread's flags starting at p (p a multiple of 16); the array is padded to
+// whole words of ROOT_NONE.
 __device__ __forceinline__ uint64_t load_flags(const uint8_t* f, uint64_t p, uint64_t n, uint4 v[kRootVec]) {
   uint64_t c = 0;
 #pragma unroll
   for (int k = 0; k < kRootVec; k++) {
     const uint64_t q = p + 16 * (uint64_t)k;
-    if (q + 16 <= n) {
-      v[k] = *reinterpret_cast<const uint4*>(f + q);
-    } else {
-      uint32_t w[4] = {0, 0, 0, 0};
-#pragma unroll
-      for (int j = 0; j < 16; j++)
-        if (q + j < n) w[j >> 2] |= (uint32_t)f[q + j] << (8 * (j & 3));
-      v[k] = make_uint4(w[0], w[1], w[2], w[3]);
-    }
+    v[k] = q < n ? *reinterpret_cast<const uint4*>(f + q) : make_uint4(0, 0, 0, 0);
     c += count_word(v[k].x) + count_word(v[k].y) + count_word(v[k].z) + count_word(v[k].w);
   }
   return c;
@@ -769,6 +761,9 @@ __global__ void __launch_bounds__(kScanThreads) root_emit_kernel(ForestArgs a, u
   if (!c) return;
 #pragma unroll
   for (int k = 0; k < kRootVec; k++) {
+    // cleared for the next checkpoint
+    if (v[k].x | v[k].y | v[k].z | v[k].w)
+      *reinterpret_cast<uint4*>(a.rflag + p + 16 * (uint64_t)k) = make_uint4(0, 0, 0, 0);
     const uint32_t w4[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
 #pragma unroll
     for (int j = 0; j < 4; j++) {
@@ -976,7 +971,10 @@ __global__ void layout_kernel(GatherArgs g) {
     }
   }
   __syncthreads();
-  if (!lay->ok) return;
+  if (!lay->ok) {
+    for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) g.hist[k] = 0;
+    return;
+  }
   uint8_t* diff = g.stage + pad;
   if (threadIdx.x == 0) {
     // header_t, include/utils.hpp:29-37
@@ -1035,7 +1033,10 @@ __global__ void layout_kernel(GatherArgs g) {
   }
   __syncthreads();
   for (uint32_t k = threadIdx.x; k < K; k += blockDim.x)
-    if (g.hist[k] > 0) g.rep[k] = g.rank[g.rep[k]];
+    if (g.hist[k] > 0) {
+      g.rep[k] = g.rank[g.rep[k]];
+      g.hist[k] = 0;  // for the next checkpoint
+    }
   if (threadIdx.x == 0) {
     lay->nkeys = run;
     const uint32_t T = (S + kSortTile - 1) / kSortTile;
@@ -1407,14 +1408,6 @@ cudaError_t launch_map_rebase(const DigestMap& m, uint64_t cap, cudaStream_t s) 
 // ---------------------------------------------------------------------------
 cudaError_t launch_forest(const ForestArgs& a, int pass, int baseline, uint32_t N, cudaStream_t s) {
   if (N < 2) return cudaSuccess;
-  if (pass == 0 || pass == 3) {
-    // the duplicate pass (alone or fused into the first) writes only the
-    // flags of roots; every other position (node 1 .. M-1 in canonical
-    // order) reads ROOT_NONE
-    cudaError_t e = cudaMemsetAsync(a.rflag, ROOT_NONE, 2ull * N - 2, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(a.ins_count, 0, sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
-  }
   // deepest interior depth: that of node N-2
   uint32_t dmax = 0;
   while (((2ull << dmax) - 1) <= (uint64_t)(N - 2)) dmax++;
@@ -1490,7 +1483,6 @@ cudaError_t launch_assemble(const GatherArgs& g, uint64_t max_entries, bool whol
   // pad depends on F, P, S; P needs the histogram.  Order: shift prep
   // (histogram), FO prep + scan (region sizes), layout (pad, table, header),
   // FO emit (metadata + regions), sort, copy.
-  cudaMemsetAsync(g.hist, 0, sizeof(uint32_t) * (size_t)g.k_cap, s);
   const uint32_t gs = grid_for(max_entries, 256);
   launch_k(roots_prep_kernel, gs, 256, 0, s, g);
   // region totals first (phase 1+2 of the scan), then layout, then emit

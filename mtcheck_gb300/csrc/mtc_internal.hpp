@@ -42,7 +42,11 @@ struct ParamsOut {
   StepParams* sp;
   uint32_t* err;
   uint64_t* clk;
+  uint32_t* counters;  // kCounters words, cleared
 };
+// Counters of a checkpoint: changed chunks, demoted leaves, queued forest
+// inserts, notes of the insert pass.
+constexpr int kCounters = 4;
 
 struct LeafArgs {
   const uint8_t* data = nullptr;  // device buffer being checkpointed
