@@ -202,6 +202,10 @@ int Engine::ensure_state(uint32_t N, bool fresh, uint32_t id_headroom) {
     MTC_CUDA(cudaMemsetAsync(rflag_.p, 0, rflag_.n, stream_));
     MTC_CUDA(chunk_slot_.ensure(N, stream_));
     MTC_CUDA(changed_list_.ensure(N, stream_));
+    if (tree) {
+      MTC_CUDA(span_done_.ensure(forest_done_words(N), stream_));
+      MTC_CUDA(cudaMemsetAsync(span_done_.p, 0, sizeof(uint32_t) * span_done_.n, stream_));
+    }
     MTC_CUDA(changed_count_.ensure(kCounters, stream_));
     MTC_CUDA(map_size_.ensure(1, stream_));
     MTC_CUDA(err_.ensure(1, stream_));
@@ -331,6 +335,7 @@ int Engine::run_tree(const uint8_t* data, uint64_t len, bool baseline_path) {
   // the forest's first-occurrence inserts
   fa.ins_queue = changed_list_.p;
   fa.ins_count = changed_count_.p + 2;
+  fa.span_done = span_done_.p;
   if (baseline_path && fresh_) {
     MTC_CUDA(launch_forest(fa, 3, 1, N, stream_));  // both passes of a baseline on cleared digests
   } else {
@@ -702,7 +707,7 @@ uint64_t Engine::shape_signature(const uint8_t* data, uint64_t len) const {
                         (uint64_t)sh_key_.p, (uint64_t)sh_prev_.p, (uint64_t)hist_.p, hist_.n, (uint64_t)rep_.p,
                         (uint64_t)rank_.p, (uint64_t)fo_val_.p, (uint64_t)sort_mat_.p, sort_mat_.n, (uint64_t)scan_.p,
                         (uint64_t)scan_total_.p, (uint64_t)scan2_.p, (uint64_t)scan_total2_.p, (uint64_t)stage_.p,
-                        stage_.n, (uint64_t)lay_.p, (uint64_t)sp_.p, (uint64_t)clk_.p, (uint64_t)baseline_path_, (uint64_t)mode_,
+                        stage_.n, (uint64_t)lay_.p, (uint64_t)sp_.p, (uint64_t)clk_.p, (uint64_t)span_done_.p, (uint64_t)baseline_path_, (uint64_t)mode_,
                         (uint64_t)leaf_tune_.rows, (uint64_t)leaf_tune_.ctas_per_sm, (uint64_t)leaf_tune_.direct,
                         (uint64_t)leaf_tune_.threads_per_chunk};
   uint64_t h = 1469598103934665603ull;
@@ -715,7 +720,7 @@ void Engine::for_each_buf(F f) {
   f(digests_); f(labels_); f(rflag_); f(chunk_slot_); f(changed_list_); f(changed_count_); f(slots_);
   f(map_size_); f(err_); f(fo_list_); f(sh_list_); f(reg_chunk_); f(reg_slot_); f(reg_len_); f(sh_key_);
   f(sh_prev_); f(hist_); f(rep_); f(rank_); f(fo_val_); f(sort_mat_); f(scan_); f(scan_total_); f(scan2_);
-  f(scan_total2_); f(stage_); f(lay_); f(sp_); f(clk_);
+  f(scan_total2_); f(stage_); f(lay_); f(sp_); f(clk_); f(span_done_);
 }
 
 void Engine::set_pool(cudaMemPool_t pool) {
@@ -789,7 +794,7 @@ uint64_t Engine::device_bytes() const {
   return sizeof(Digest) * digests_.n + labels_.n + rflag_.n +
          sizeof(uint32_t) * (chunk_slot_.n + changed_list_.n + changed_count_.n + map_size_.n + err_.n + fo_list_.n +
                              sh_list_.n + reg_chunk_.n + reg_slot_.n + reg_len_.n + sh_key_.n + sh_prev_.n + hist_.n +
-                             rep_.n + rank_.n) +
+                             rep_.n + rank_.n + span_done_.n) +
          sizeof(MapSlot) * slots_.n +
          sizeof(uint64_t) * (fo_val_.n + sort_mat_.n + scan_.n + scan_total_.n + scan2_.n + scan_total2_.n) + stage_.n +
          sizeof(Layout) * lay_.n + sizeof(StepParams) * sp_.n + sizeof(uint64_t) * clk_.n;

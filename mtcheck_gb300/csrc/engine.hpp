@@ -313,6 +313,7 @@ class Engine {
   DevBuf<uint8_t> stage_;
   DevBuf<Layout> lay_;
   DevBuf<StepParams> sp_;
+  DevBuf<uint32_t> span_done_;      // forest passes: finished subtrees per span
   DevBuf<uint64_t> clk_;            // device times of a checkpoint's phases (CLK_*)
   StepParams* sp_host_ = nullptr;   // pinned
   Layout* lay_host_ = nullptr;      // pinned

@@ -37,16 +37,11 @@ __device__ __forceinline__ uint8_t child_flag(uint8_t lab) {
   return (lab == FIXED_DUPL || lab == DONE) ? ROOT_NONE : (lab == SHIFT_DUPL ? ROOT_SHIFT : ROOT_FO);
 }
 
-// Several levels per launch: CTA b owns the subtree of interior node
-// r = 2^d_top - 1 + b and computes its interior nodes from depth d_bot up to
-// d_top.  Only the bottom children, leaves met on the way, digests and the
-// results touch global memory.  pass 0: first-occurrence forest
-// (src/tree_approach.cpp:378-404); pass 1: duplicate forest (:413-477), with
-// baseline != 0 the baseline variant that tests the not-yet-hashed digest and
-// then hashes and inserts every interior node (:155-227); pass 2: both
-// incremental passes in one traversal (ForestArgs::fuse_gate); pass 3: both
-// passes of a baseline on cleared digests in one traversal, which hashes
-// every node and leaves the inserts to forest_insert_all_kernel.
+// Passes.  0: first-occurrence forest (src/tree_approach.cpp:378-404); 1:
+// duplicate forest (:413-477); 2: both incremental passes in one traversal
+// (ForestArgs::fuse_gate); 3: both passes of a baseline (:115-227) on cleared
+// digests in one traversal, which hashes every node and leaves the inserts to
+// forest_insert_all_kernel.
 //
 // Pass 3.  A node is a first occurrence in the baseline's second pass exactly
 // when it is one in the first (both only look at the leaves' labels), with the
@@ -57,130 +52,90 @@ __device__ __forceinline__ uint8_t child_flag(uint8_t lab) {
 // priority), so the inserts may follow in any order.  4 GiB in 512-byte
 // chunks: the two passes took 2.10 ms (bottom 0.23, inserts 1.16, a barrier
 // per level with a second hash and insert of every node 0.71).
+//
+// Launches.  A pass is one launch.  Block b of forest_kernel owns the 12 lowest
+// levels below one node; the last block to finish below a node nine levels up
+// goes on with those nine levels, and so on to the root, so that no level
+// waits for a launch (the upper levels as launches of their own took 5-8 us of
+// a 47 us labelling of 2^19 chunks, and as much again for the duplicate pass
+// that usually returns at once).  Trees of at most 2048 leaves are one block.
 constexpr uint32_t kSpanLevels = 9;     // 256 nodes on the bottom level of a span
 constexpr uint32_t kBottomLevels = 12;  // bottom span: 16 leaves per thread, 4096 per block
-constexpr uint32_t kBottomSink = 2048;  // queued inserts a bottom block holds in shared memory
+constexpr uint32_t kSmallLeaves = 2048; // forest_small_kernel
 
-// First-occurrence inserts are queued (node ids in ForestArgs::ins_queue) and
-// issued by forest_insert_kernel after the pass's last launch: the
-// first-occurrence pass never looks an entry up, the fused pass looks up only
-// digests that no queued insert can equal, and the serial-order rule of
-// map_insert_serial does not depend on arrival order.  A span block collects
-// its ids in shared memory and appends them with one atomic.
+__device__ __forceinline__ bool forest_fused(const ForestArgs& a) { return a.fuse_gate && *a.fuse_gate == 0; }
+
+// First-occurrence nodes of a span, collected in shared memory as positions in
+// the subtree of the span's root r: position h at relative depth k = log2 h is
+// node h - 1 + (r << k).  `off` is (r << k) - 1 of the level being computed.
 struct IdSink {
-  uint32_t* ids;  // shared memory
-  uint32_t* n;    // shared counter
-  uint32_t cap;   // ids beyond it go to the global queue directly
+  uint16_t* ids;
+  uint32_t* n;
+  uint32_t off;
 };
-__device__ __forceinline__ void queue_insert(const ForestArgs& a, IdSink* sink, uint32_t n) {
-  if (sink) {
-    const uint32_t k = atomicAdd(sink->n, 1u);
-    if (k < sink->cap) {
-      sink->ids[k] = n;
-      return;
-    }
-  }
-  a.ins_queue[atomicAdd(a.ins_count, 1u)] = n;
+__device__ __forceinline__ void sink_level(IdSink& sink, uint64_t r, int k) { sink.off = (uint32_t)((r << k) - 1); }
+__device__ __forceinline__ void queue_insert(IdSink& sink, uint32_t n) {
+  sink.ids[atomicAdd(sink.n, 1u)] = (uint16_t)(n - sink.off);
 }
-__device__ __forceinline__ void flush_sink(const ForestArgs& a, const IdSink& sink, uint32_t* base) {
+// The span's inserts, by its block: issued at once when the duplicate pass is
+// still to come and will look them up; queued when the passes are fused (a
+// fused pass looks nothing up that they could add), for launches that have
+// other work to hide them (drain_inserts).  Each node's digest is new, as its
+// leaves' are; the serial-order rule does not depend on the inserts' order.
+__device__ __forceinline__ void flush_sink(const ForestArgs& a, bool fused, uint64_t r, const IdSink& sink,
+                                           uint32_t* base) {
   __syncthreads();
-  const uint32_t cnt = min(*sink.n, sink.cap);
-  if (cnt == 0) return;
-  if (threadIdx.x == 0) *base = atomicAdd(a.ins_count, cnt);
+  const uint32_t cnt = *sink.n;
+  auto node = [&](uint32_t k) {
+    const uint32_t h = sink.ids[k];
+    return (uint32_t)(h - 1 + (r << (31 - __clz(h))));
+  };
+  if (fused) {
+    if (cnt && threadIdx.x == 0) *base = atomicAdd(a.ins_count, cnt);
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < cnt; k += blockDim.x) a.ins_queue[*base + k] = node(k);
+  } else {
+    const uint32_t cur_id = a.sp->cur, epoch_fo = a.sp->epoch + 1;
+    uint32_t created = 0;
+    for (uint32_t k = threadIdx.x; k < cnt; k += blockDim.x)
+      created += map_insert_serial(a.map, ld_digest(a.tree + node(k)), node(k), cur_id, epoch_fo, false, a.err);
+    count_new_entries(a.map, created);
+  }
   __syncthreads();
-  const uint32_t b = *base;
-  for (uint32_t k = threadIdx.x; k < cnt; k += blockDim.x) a.ins_queue[b + k] = sink.ids[k];
+  if (threadIdx.x == 0) *sink.n = 0;
 }
 
-// One interior node n of a forest pass, given its children's labels: the
-// hashing, map insert or lookup and children's root flags of the reference's
-// level loops.  Writes n's label only when `store` is set (a span's top
-// level, read by the next launch, or the baseline); only flags other than
-// ROOT_NONE are written, the flag array being cleared before the first pass.
-__device__ __forceinline__ uint8_t forest_node(const ForestArgs& a, int pass, int baseline, uint64_t n, uint8_t ll,
-                                               uint8_t lr, uint32_t cur_id, uint32_t epoch_all, bool store) {
+// One interior node n of a baseline's duplicate pass on digests that are not
+// cleared (a second checkpoint under id 0): tests the not-yet-hashed digest,
+// then hashes and inserts every interior node (:155-227).
+__device__ __forceinline__ uint8_t forest_node(const ForestArgs& a, uint64_t n, uint8_t ll, uint8_t lr,
+                                               uint32_t cur_id, uint32_t epoch_all) {
   const uint32_t l = 2 * (uint32_t)n + 1, rr = l + 1;
-  uint8_t lab_n;
-  if (pass == 0) {
-    if (ll == FIRST_OCUR && lr == FIRST_OCUR) {
-      lab_n = FIRST_OCUR;
-      st_digest(a.tree + n, hash_pair(a.hash_kind, ld_digest(a.tree + l), ld_digest(a.tree + rr)));
-      queue_insert(a, nullptr, (uint32_t)n);
-    } else {
-      lab_n = DONE;
-    }
-  } else {
-    uint8_t fl = ROOT_NONE, fr = ROOT_NONE;
-    if (ll != lr) {
-      lab_n = DONE;
-      fl = child_flag(ll);
-      fr = child_flag(lr);
-    } else if (ll == FIXED_DUPL) {
-      lab_n = FIXED_DUPL;
-    } else if (ll == SHIFT_DUPL) {
-      Digest dg;
-      if (baseline) {
-        dg = ld_digest(a.tree + n);
-      } else {
-        dg = hash_pair(a.hash_kind, ld_digest(a.tree + l), ld_digest(a.tree + rr));
-        st_digest(a.tree + n, dg);
-      }
-      if (map_find(a.map, dg, a.err) >= 0) {
-        lab_n = SHIFT_DUPL;
-      } else {
-        lab_n = DONE;
-        fl = ROOT_SHIFT;
-        fr = ROOT_SHIFT;
-      }
-    } else if (ll == FIRST_OCUR) {
-      lab_n = FIRST_OCUR;
-      if (pass == 2) {
-        st_digest(a.tree + n, hash_pair(a.hash_kind, ld_digest(a.tree + l), ld_digest(a.tree + rr)));
-        queue_insert(a, nullptr, (uint32_t)n);
-      }
-    } else {
-      lab_n = DONE;  // both first duplicates, or both done
-    }
-    if (fl != ROOT_NONE) a.rflag[canon_pos(a, l)] = fl;
-    if (fr != ROOT_NONE) a.rflag[canon_pos(a, rr)] = fr;
-    if (baseline) {
-      Digest dg = hash_pair(a.hash_kind, ld_digest(a.tree + l), ld_digest(a.tree + rr));
-      st_digest(a.tree + n, dg);
-      if (pass == 1 && map_insert_serial(a.map, dg, (uint32_t)n, cur_id, epoch_all, true, a.err))
-        atomicAdd(a.map.size, 1u);
-    }
+  uint8_t lab_n = DONE, fl = ROOT_NONE, fr = ROOT_NONE;
+  if (ll != lr) {
+    fl = child_flag(ll);
+    fr = child_flag(lr);
+  } else if (ll == FIXED_DUPL || ll == FIRST_OCUR) {
+    lab_n = ll;
+  } else if (ll == SHIFT_DUPL) {
+    if (map_find(a.map, ld_digest(a.tree + n), a.err) >= 0) lab_n = SHIFT_DUPL;
+    else fl = fr = ROOT_SHIFT;
   }
-  if (store) a.labels[n] = lab_n;
+  if (fl != ROOT_NONE) a.rflag[canon_pos(a, l)] = fl;
+  if (fr != ROOT_NONE) a.rflag[canon_pos(a, rr)] = fr;
+  const Digest dg = hash_pair(a.hash_kind, ld_digest(a.tree + l), ld_digest(a.tree + rr));
+  st_digest(a.tree + n, dg);
+  if (map_insert_serial(a.map, dg, (uint32_t)n, cur_id, epoch_all, true, a.err)) atomicAdd(a.map.size, 1u);
+  a.labels[n] = lab_n;
   return lab_n;
 }
 
-// Label of node n at a level of a span: final for a leaf (or DONE past the
-// end), otherwise computed from the children's labels.
-__device__ __forceinline__ uint8_t forest_label(const ForestArgs& a, int pass, int baseline, uint64_t n,
-                                                uint64_t last_interior, uint64_t M, uint8_t ll, uint8_t lr,
-                                                uint32_t cur_id, uint32_t epoch_all, bool store) {
-  if (n > last_interior) return n < M ? a.labels[n] : DONE;
-  return forest_node(a, pass, baseline, n, ll, lr, cur_id, epoch_all, store);
-}
-
-// Resolves the pass of an incremental launch: with the fuse gate open the
-// first-occurrence launch runs both passes (2) and the duplicate launch has
-// nothing left to do (-1).
-__device__ __forceinline__ int resolve_pass(const ForestArgs& a, int pass) {
-  if (a.fuse_gate && *a.fuse_gate == 0) return pass == 1 ? -1 : 2;
-  return pass;
-}
-
-// Levels d_bot .. d_top of the subtree rooted at depth d_top, node labels in
-// shared memory, one barrier per level.  Serves every span shape, and the
-// baseline's duplicate pass, whose shift test must see every insert of the
-// levels below it.
-__global__ void __launch_bounds__(256) forest_span_kernel(ForestArgs a, int pass, int baseline, uint32_t N,
-                                                          uint32_t d_top, uint32_t d_bot) {
+// Levels d_bot .. d_top of the subtree rooted at depth d_top for that pass,
+// node labels in shared memory, one barrier per level: its shift test must
+// see every insert of the levels below it.
+__global__ void __launch_bounds__(256) forest_span_kernel(ForestArgs a, uint32_t N, uint32_t d_top, uint32_t d_bot) {
   pdl_enter();
   __shared__ uint8_t lab[2][2 << (kSpanLevels - 1)];
-  pass = resolve_pass(a, pass);
-  if (pass < 0) return;
   const uint32_t cur_id = a.sp->cur, epoch_all = a.sp->epoch + 2;
   const uint64_t r = ((1ull << d_top) - 1) + blockIdx.x;
   const uint64_t last_interior = (uint64_t)N - 2, M = 2ull * N - 1;
@@ -199,9 +154,11 @@ __global__ void __launch_bounds__(256) forest_span_kernel(ForestArgs a, int pass
   for (int d = (int)d_bot; d >= (int)d_top; d--) {
     const uint32_t width = 1u << (d - d_top);
     const uint64_t first = (r + 1) * width - 1;
-    for (uint32_t i = threadIdx.x; i < width; i += blockDim.x)
-      cur[i] = forest_label(a, pass, baseline, first + i, last_interior, M, child[2 * i], child[2 * i + 1], cur_id,
-                            epoch_all, baseline || d == (int)d_top);
+    for (uint32_t i = threadIdx.x; i < width; i += blockDim.x) {
+      const uint64_t n = first + i;
+      cur[i] = n > last_interior ? (n < M ? a.labels[n] : (uint8_t)DONE)
+                                 : forest_node(a, n, child[2 * i], child[2 * i + 1], cur_id, epoch_all);
+    }
     __syncthreads();
     uint8_t* t = child;
     child = cur;
@@ -216,77 +173,55 @@ __device__ __forceinline__ bool digest_wanted(int pass, uint8_t lab) {
   return pass == 0 ? lab == FIRST_OCUR : pass == 1 ? lab == SHIFT_DUPL : (lab == FIRST_OCUR || lab == SHIFT_DUPL);
 }
 
-// One interior node n of an incremental pass (first-occurrence forest
-// src/tree_approach.cpp:378-404, duplicate forest :413-477, or both: pass 2)
-// given its children's labels and digests; `dg` receives n's digest when n is
-// hashed.  First-occurrence inserts go to the block's sink.  BASE: pass 3,
-// every node hashed and its label kept for the inserts that follow.
+// One interior node n of a pass given its children's labels and digests; `dg`
+// receives n's digest when n is hashed.  First occurrences go to the block's
+// sink; n's label is written when `store` is set (the top of a span); only
+// flags other than ROOT_NONE are written, the flag array being clear before
+// the first pass.  BASE: pass 3, every node hashed and its label kept for the
+// inserts that follow.
 template <int HK, bool BASE>
 __device__ __forceinline__ uint8_t span_node(const ForestArgs& a, int pass, uint32_t n, uint8_t ll, uint8_t lr,
                                              const Digest& dl, const Digest& dr, Digest& dg, bool store,
-                                             IdSink* sink) {
+                                             IdSink& sink) {
   const uint32_t l = 2 * n + 1, rr = l + 1;
-  uint8_t lab_n;
-  if (BASE) {
-    uint8_t fl = ROOT_NONE, fr = ROOT_NONE;
-    lab_n = DONE;
-    if (ll != lr) {
-      fl = child_flag(ll);
-      fr = child_flag(lr);
-    } else if (ll == FIXED_DUPL || ll == FIRST_OCUR) {
-      lab_n = ll;
-    } else if (ll == SHIFT_DUPL) {
-      if (map_find(a.map, ld_digest(a.tree + n), a.err) >= 0) lab_n = SHIFT_DUPL;
-      else fl = fr = ROOT_SHIFT;
-    }
-    if (fl != ROOT_NONE) a.rflag[canon_pos(a, l)] = fl;
-    if (fr != ROOT_NONE) a.rflag[canon_pos(a, rr)] = fr;
-    dg = hash_pair(HK, dl, dr);
-    st_digest(a.tree + n, dg);
-    a.labels[n] = lab_n;
-    return lab_n;
-  }
-  if (pass == 0) {
+  uint8_t lab_n = DONE;
+  uint8_t fl = ROOT_NONE, fr = ROOT_NONE;
+  if (!BASE && pass == 0) {
     if (ll == FIRST_OCUR && lr == FIRST_OCUR) {
       lab_n = FIRST_OCUR;
       dg = hash_pair(HK, dl, dr);
       st_digest(a.tree + n, dg);
-      queue_insert(a, sink, n);
-    } else {
-      lab_n = DONE;
+      queue_insert(sink, n);
     }
   } else {
-    uint8_t fl = ROOT_NONE, fr = ROOT_NONE;
     if (ll != lr) {
-      lab_n = DONE;
       fl = child_flag(ll);
       fr = child_flag(lr);
     } else if (ll == FIXED_DUPL) {
       lab_n = FIXED_DUPL;
     } else if (ll == SHIFT_DUPL) {
-      dg = hash_pair(HK, dl, dr);
-      st_digest(a.tree + n, dg);
-      if (map_find(a.map, dg, a.err) >= 0) {
-        lab_n = SHIFT_DUPL;
-      } else {
-        lab_n = DONE;
-        fl = ROOT_SHIFT;
-        fr = ROOT_SHIFT;
-      }
-    } else if (ll == FIRST_OCUR) {
-      lab_n = FIRST_OCUR;
-      if (pass == 2) {
+      if (!BASE) {
         dg = hash_pair(HK, dl, dr);
         st_digest(a.tree + n, dg);
-        queue_insert(a, sink, n);
       }
-    } else {
-      lab_n = DONE;  // both first duplicates, or both done
-    }
+      if (map_find(a.map, BASE ? ld_digest(a.tree + n) : dg, a.err) >= 0) lab_n = SHIFT_DUPL;
+      else fl = fr = ROOT_SHIFT;
+    } else if (ll == FIRST_OCUR) {
+      lab_n = FIRST_OCUR;
+      if (!BASE && pass == 2) {
+        dg = hash_pair(HK, dl, dr);
+        st_digest(a.tree + n, dg);
+        queue_insert(sink, n);
+      }
+    }  // both first duplicates, or both done: DONE
     if (fl != ROOT_NONE) a.rflag[canon_pos(a, l)] = fl;
     if (fr != ROOT_NONE) a.rflag[canon_pos(a, rr)] = fr;
   }
-  if (store) a.labels[n] = lab_n;
+  if (BASE) {
+    dg = hash_pair(HK, dl, dr);
+    st_digest(a.tree + n, dg);
+  }
+  if (BASE || store) a.labels[n] = lab_n;
   return lab_n;
 }
 
@@ -295,7 +230,7 @@ __device__ __forceinline__ uint8_t span_node(const ForestArgs& a, int pass, uint
 template <int HK, bool BASE>
 __device__ __forceinline__ uint8_t span_label(const ForestArgs& a, int pass, uint64_t n, uint64_t last_interior,
                                               uint64_t M, uint8_t ll, uint8_t lr, const Digest& dl,
-                                              const Digest& dr, Digest& dg, IdSink* sink) {
+                                              const Digest& dr, Digest& dg, IdSink& sink) {
   if (n > last_interior) {
     const uint8_t lab = n < M ? a.labels[n] : DONE;
     if (BASE ? n < M : digest_wanted(pass, lab)) dg = ld_digest(a.tree + n);
@@ -310,18 +245,20 @@ __device__ __forceinline__ Digest shfl_digest(const Digest& d, int src) {
                  __shfl_sync(kFull, d.w[3], src)}};
 }
 
-// The eight upper levels of a span below node r, from one node per thread
-// (relative depth 8, node (r+1)*256-1+threadIdx.x, label `lab`, digest `dg`):
-// five inside each warp (children's labels and digests by shuffle), then
-// three in warp 0 from the eight warps' results.  Stores r's label.  Every
-// node here is interior.
+// The levels of an L-level span above its bottom one, from one node per thread
+// (relative depth L - 1, node (r+1) * 2^(L-1) - 1 + threadIdx.x, label `lab`,
+// digest `dg`, threads below 2^(L-1)): up to five inside each warp (children's
+// labels and digests by shuffle), then up to three in warp 0 from the eight
+// warps' results.  Stores r's label (L > 1).  Every node here is interior.
 template <int HK, bool BASE>
-__device__ __forceinline__ void upper_levels(const ForestArgs& a, int pass, uint64_t r, uint8_t lab, Digest dg,
-                                             IdSink* sink, uint8_t* top8, Digest* topdg) {
+__device__ __forceinline__ void upper_levels(const ForestArgs& a, int pass, uint64_t r, uint32_t L, uint8_t lab,
+                                             Digest dg, IdSink& sink, uint8_t* top8, Digest* topdg) {
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t w = 1u << (L - 1);
   constexpr unsigned kFull = 0xffffffffu;
+  const uint32_t in_warp = L - 1 < 5 ? L - 1 : 5;
 #pragma unroll 1
-  for (uint32_t step = 1; step <= 5; step++) {
+  for (uint32_t step = 1; step <= in_warp; step++) {
     const int sl = (2 * lane) & 31, sr = (2 * lane + 1) & 31;
     const uint8_t cl = (uint8_t)__shfl_sync(kFull, lab, sl);
     const uint8_t cr = (uint8_t)__shfl_sync(kFull, lab, sr);
@@ -330,12 +267,14 @@ __device__ __forceinline__ void upper_levels(const ForestArgs& a, int pass, uint
       dl = shfl_digest(dg, sl);
       dr = shfl_digest(dg, sr);
     }
-    const uint32_t width = 32u >> step;
-    if (lane < width) {
-      const uint64_t n = (r + 1) * (256u >> step) - 1 + warp * width + lane;
-      lab = span_node<HK, BASE>(a, pass, (uint32_t)n, cl, cr, dl, dr, dg, false, sink);
+    const uint32_t width = 32u >> step, i = warp * width + lane;
+    if (lane < width && i < (w >> step)) {
+      sink_level(sink, r, (int)(L - 1 - step));
+      const uint64_t n = (r + 1) * (w >> step) - 1 + i;
+      lab = span_node<HK, BASE>(a, pass, (uint32_t)n, cl, cr, dl, dr, dg, step == L - 1, sink);
     }
   }
+  if (L <= 6) return;
   if (lane == 0) {
     top8[warp] = lab;
     topdg[warp] = dg;
@@ -345,59 +284,65 @@ __device__ __forceinline__ void upper_levels(const ForestArgs& a, int pass, uint
     lab = lane < 8 ? top8[lane] : DONE;
     if (lane < 8) dg = topdg[lane];
 #pragma unroll 1
-    for (uint32_t step = 6; step <= 8; step++) {
+    for (uint32_t step = 6; step <= L - 1; step++) {
       const int sl = (2 * lane) & 31, sr = (2 * lane + 1) & 31;
       const uint8_t cl = (uint8_t)__shfl_sync(kFull, lab, sl);
       const uint8_t cr = (uint8_t)__shfl_sync(kFull, lab, sr);
       const Digest dl = shfl_digest(dg, sl), dr = shfl_digest(dg, sr);
-      const uint32_t width = 256u >> step;
-      if (lane < width) {
-        const uint64_t n = (r + 1) * width - 1 + lane;
-        lab = span_node<HK, BASE>(a, pass, (uint32_t)n, cl, cr, dl, dr, dg, step == 8, sink);
+      if (lane < (w >> step)) {
+        sink_level(sink, r, (int)(L - 1 - step));
+        const uint64_t n = (r + 1) * (w >> step) - 1 + lane;
+        lab = span_node<HK, BASE>(a, pass, (uint32_t)n, cl, cr, dl, dr, dg, step == L - 1, sink);
       }
     }
   }
 }
 
-// A full span of 9 levels (256 nodes on its bottom level) for the incremental
-// passes and the baseline's first-occurrence pass: the bottom nodes' children
-// come from memory, the rest by upper_levels -- one block barrier instead of
-// nine, and no digest goes through memory between levels (they are still
-// stored: the tree keeps every digest for the next checkpoint).
+// The spans above the block's own, whose root is node i of depth d: the last
+// block to finish below a span's root takes the span.  The counters return to
+// zero for the next pass.  Thread 0 wrote the label and digest of the block's
+// root, so its fence publishes them; they are read past the L1.
 template <int HK, bool BASE>
-__global__ void __launch_bounds__(256) forest_span9_warp_kernel(ForestArgs a, int pass, uint32_t N, uint32_t d_top) {
-  pdl_enter();
-  __shared__ uint8_t top8[8];
-  __shared__ Digest topdg[8];
-  __shared__ uint32_t ids[(1u << kSpanLevels) - 1];  // one per interior node: never overflows
-  __shared__ uint32_t ids_n, ids_base;
-  const uint64_t r = ((1ull << d_top) - 1) + blockIdx.x;
-  const uint64_t last_interior = (uint64_t)N - 2, M = 2ull * N - 1;
-  if (r > last_interior) return;
-  pass = resolve_pass(a, pass);
-  if (pass < 0) return;
-  if (threadIdx.x == 0) ids_n = 0;
-  __syncthreads();
-  IdSink sink{ids, &ids_n, (1u << kSpanLevels) - 1};
-  uint8_t lab;
-  Digest dg{{0, 0, 0, 0}};
-  {
-    const uint64_t n = (r + 1) * 256 - 1 + threadIdx.x;
-    uint8_t ll = DONE, lr = DONE;
-    Digest dl{{0, 0, 0, 0}}, dr{{0, 0, 0, 0}};
-    if (n <= last_interior) {
-      const uint64_t c = 2 * n + 1;
-      ll = c < M ? a.labels[c] : DONE;
-      lr = c + 1 < M ? a.labels[c + 1] : DONE;
-      if (BASE || (ll == lr && digest_wanted(pass, ll))) {
-        dl = ld_digest(a.tree + c);
-        dr = ld_digest(a.tree + c + 1);
-      }
+__device__ __forceinline__ void upper_spans(const ForestArgs& a, int pass, bool fused, uint32_t d, uint32_t i,
+                                            IdSink& sink, uint32_t* base, uint8_t* top8, Digest* topdg,
+                                            uint32_t* s_last) {
+  uint32_t* done = a.span_done;
+#pragma unroll 1
+  while (d > 0) {
+    const uint32_t L = d < kSpanLevels ? d : kSpanLevels, p = i >> L;
+    d -= L;
+    if (threadIdx.x == 0) {
+      __threadfence();
+      const bool last = atomicAdd(&done[p], 1u) + 1 == (1u << L);
+      if (last) done[p] = 0;
+      __threadfence();
+      *s_last = last ? 1u : 0u;
     }
-    lab = span_label<HK, BASE>(a, pass, n, last_interior, M, ll, lr, dl, dr, dg, &sink);
+    __syncthreads();
+    if (!*s_last) return;
+    const uint64_t r = ((1ull << d) - 1) + p;
+    const uint32_t w = 1u << (L - 1);
+    uint8_t lab = DONE;
+    Digest dg{{0, 0, 0, 0}};
+    if (threadIdx.x < w) {
+      const uint64_t n = (r + 1) * w - 1 + threadIdx.x, c = 2 * n + 1;
+      const uint8_t ll = __ldcg(a.labels + c), lr = __ldcg(a.labels + c + 1);
+      Digest dl{{0, 0, 0, 0}}, dr{{0, 0, 0, 0}};
+      if (BASE || (ll == lr && digest_wanted(pass, ll))) {
+        const uint4 vl = __ldcg(reinterpret_cast<const uint4*>(a.tree + c)),
+                    vr = __ldcg(reinterpret_cast<const uint4*>(a.tree + c + 1));
+        dl = Digest{{vl.x, vl.y, vl.z, vl.w}};
+        dr = Digest{{vr.x, vr.y, vr.z, vr.w}};
+      }
+      sink_level(sink, r, (int)L - 1);
+      lab = span_node<HK, BASE>(a, pass, (uint32_t)n, ll, lr, dl, dr, dg, L == 1, sink);
+    }
+    upper_levels<HK, BASE>(a, pass, r, L, lab, dg, sink, top8, topdg);
+    if (!BASE && pass != 1) flush_sink(a, fused, r, sink, base);
+    __syncthreads();
+    done += 1ull << d;
+    i = p;
   }
-  upper_levels<HK, BASE>(a, pass, r, lab, dg, &sink, top8, topdg);
-  if (!BASE && pass != 1) flush_sink(a, sink, &ids_base);
 }
 
 // Byte-parallel labelling of four (left, right) pairs per 32-bit word, the
@@ -438,12 +383,13 @@ __device__ __forceinline__ void set_byte(uint32_t& w, int b, uint32_t v) {
 // digest in dg when a parent reads it.
 template <int HK, bool BASE>
 __device__ __forceinline__ uint8_t thread_levels_bytewise(const ForestArgs& a, int pass, uint64_t r, uint32_t t,
-                                                          uint32_t c[4], IdSink* sink, Digest (*work)[256],
+                                                          uint32_t c[4], IdSink& sink, Digest (*work)[256],
                                                           Digest& dg) {
   uint64_t nb = (r + 1) * 2048 - 1 + 8ull * t;  // first parent of the level
 #pragma unroll 1
   for (int lvl = 0; lvl < 4; lvl++) {
     uint32_t P[2], FL[2], FR[2], XF[2], XS[2];
+    sink_level(sink, r, (int)kBottomLevels - 1 - lvl);
 #pragma unroll
     for (int q = 0; q < 2; q++)
       label_pairs4(pass, __byte_perm(c[2 * q], c[2 * q + 1], 0x6420), __byte_perm(c[2 * q], c[2 * q + 1], 0x7531),
@@ -481,7 +427,7 @@ __device__ __forceinline__ uint8_t thread_levels_bytewise(const ForestArgs& a, i
         }
         st_digest(a.tree + n, d);
         if ((XF[q] >> (8 * b)) & 1) {
-          queue_insert(a, sink, (uint32_t)n);
+          queue_insert(sink, (uint32_t)n);
           work[i][t] = d;
         } else if (map_find(a.map, d, a.err) >= 0) {
           work[i][t] = d;  // parent stays SHIFT_DUPL
@@ -519,102 +465,148 @@ __device__ __forceinline__ uint8_t thread_levels_bytewise(const ForestArgs& a, i
   return lab;
 }
 
-// The bottom span of an incremental pass (and of the baseline's
-// first-occurrence pass): 12 levels, 4096 leaves per block.  Each thread
-// reads the labels of its 16 children with one aligned 16-byte load (the
-// first byte comes from the lane before) and computes its 8, 4, 2 and 1 nodes
-// in a loop, labels packed in a 64-bit word, digests in shared memory; a
-// thread whose 16 children are all unchanged (fixed duplicates) has nothing
-// to hash, flag or insert.  upper_levels does the rest.  Loops rather than
+// A pass over a tree of more than kSmallLeaves leaves.  Bottom span: 12 levels,
+// 4096 leaves per block.  Each thread reads the labels of its 16 children with
+// one aligned 16-byte load (the first byte comes from the lane before) and
+// computes its 8, 4, 2 and 1 nodes in a loop, labels packed in a 64-bit word,
+// digests in shared memory; a thread whose 16 children are all unchanged
+// (fixed duplicates) has nothing to hash, flag or insert.  upper_levels does
+// the rest of the span, upper_spans the rest of the tree.  Loops rather than
 // unrolled levels keep the kernel small enough for the instruction cache.
+// The duplicate pass (1) has nothing left to do when the passes were fused: it
+// is launched as one wave, whose blocks return or take several subtrees.
 template <int HK, bool BASE>
-__global__ void __launch_bounds__(256) forest_bottom12_kernel(ForestArgs a, int pass, uint32_t N, uint32_t d_top) {
+__global__ void __launch_bounds__(256) forest_kernel(ForestArgs a, int pass, uint32_t N, uint32_t d_top,
+                                                     uint32_t count) {
   pdl_enter();
   __shared__ uint8_t top8[8];
   __shared__ Digest topdg[8];
-  __shared__ uint32_t ids[kBottomSink];
-  __shared__ uint32_t ids_n, ids_base;
+  __shared__ uint16_t ids[BASE ? 1 : 4096];
+  __shared__ uint32_t ids_n, ids_base, s_last;
   __shared__ Digest work[8][256];  // [node of the thread's level][thread]: 16-byte lanes, no bank conflicts
-  const uint64_t r = ((1ull << d_top) - 1) + blockIdx.x;
+  const bool fused = forest_fused(a);
+  if (fused) {
+    if (pass == 1) return;
+    pass = 2;
+  }
   const uint64_t last_interior = (uint64_t)N - 2, M = 2ull * N - 1;
-  if (r > last_interior) return;
-  pass = resolve_pass(a, pass);
-  if (pass < 0) return;
-  if (threadIdx.x == 0) ids_n = 0;
-  __syncthreads();
-  IdSink sink{ids, &ids_n, kBottomSink};
   const uint32_t t = threadIdx.x, lane = t & 31;
   constexpr unsigned kFull = 0xffffffffu;
-  // children (relative depth 12) cb .. cb+15; cb + 1 is a multiple of 16
-  const uint64_t cb = (r + 1) * 4096 - 1 + 16ull * t;
-  uint4 v;
-  if (cb + 17 <= M) {
-    v = *reinterpret_cast<const uint4*>(a.labels + cb + 1);
-  } else {
-    uint32_t w[4] = {0, 0, 0, 0};
+  if (t == 0) ids_n = 0;
+  __syncthreads();
+  IdSink sink{ids, &ids_n, 0};
+#pragma unroll 1
+  for (uint32_t blk = blockIdx.x; blk < count; blk += gridDim.x) {
+    const uint64_t r = ((1ull << d_top) - 1) + blk;
+    // children (relative depth 12) cb .. cb+15; cb + 1 is a multiple of 16
+    const uint64_t cb = (r + 1) * 4096 - 1 + 16ull * t;
+    uint4 v;
+    if (cb + 17 <= M) {
+      v = *reinterpret_cast<const uint4*>(a.labels + cb + 1);
+    } else {
+      uint32_t w[4] = {0, 0, 0, 0};
 #pragma unroll
-    for (int j = 0; j < 16; j++) {
-      const uint64_t c = cb + 1 + j;
-      w[j >> 2] |= (uint32_t)(c < M ? a.labels[c] : DONE) << (8 * (j & 3));
-    }
-    v = make_uint4(w[0], w[1], w[2], w[3]);
-  }
-  uint32_t first = __shfl_up_sync(kFull, v.w, 1) >> 24;  // byte 15 of the lane before = child cb
-  if (lane == 0) first = cb < M ? a.labels[cb] : DONE;
-  // child j's label is byte j of (lo, hi)
-  uint64_t lo = ((uint64_t)((v.y << 8) | (v.x >> 24)) << 32) | ((v.x << 8) | first);
-  uint64_t hi = ((uint64_t)((v.w << 8) | (v.z >> 24)) << 32) | ((v.y >> 24) | (v.z << 8));
-  const uint64_t nb1 = (r + 1) * 2048 - 1 + 8ull * t;  // relative depth 11: the deepest interior level
-  uint8_t lab;
-  Digest dg{{0, 0, 0, 0}};
-  constexpr uint64_t kFixed8 = 0x0101010101010101ull * FIXED_DUPL;
-  if (!BASE && lo == kFixed8 && hi == kFixed8 && nb1 + 7 <= last_interior) {
-    lab = pass == 0 ? DONE : FIXED_DUPL;
-  } else if (nb1 + 7 <= last_interior) {
-    uint32_t c[4] = {(uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32)};
-    lab = thread_levels_bytewise<HK, BASE>(a, pass, r, t, c, &sink, work, dg);
-  } else {
-    uint64_t nb = nb1;
-    uint32_t width = 8;
-#pragma unroll 1
-    for (int lvl = 0; lvl < 4; lvl++) {
-      uint64_t out = 0;
-#pragma unroll 1
-      for (uint32_t i = 0; i < width; i++) {
-        const uint32_t j = 2 * i;
-        const uint8_t ll = (uint8_t)((j < 8 ? lo >> (8 * j) : hi >> (8 * (j - 8))) & 0xff);
-        const uint8_t lr = (uint8_t)((j + 1 < 8 ? lo >> (8 * (j + 1)) : hi >> (8 * (j - 7))) & 0xff);
-        const uint64_t n = nb + i;
-        Digest dl{{0, 0, 0, 0}}, dr{{0, 0, 0, 0}}, d{{0, 0, 0, 0}};
-        if (BASE || (ll == lr && digest_wanted(pass, ll))) {
-          if (lvl == 0) {
-            if (n <= last_interior) {
-              dl = ld_digest(a.tree + 2 * n + 1);
-              dr = ld_digest(a.tree + 2 * n + 2);
-            }
-          } else {
-            dl = work[j][t];
-            dr = work[j + 1][t];
-          }
-        }
-        const uint8_t l = lvl == 0 ? span_label<HK, BASE>(a, pass, n, last_interior, M, ll, lr, dl, dr, d, &sink)
-                                   : span_node<HK, BASE>(a, pass, (uint32_t)n, ll, lr, dl, dr, d, false, &sink);
-        if (BASE || digest_wanted(pass, l)) work[i][t] = d;  // read back only at the next level, from a higher index
-        out |= (uint64_t)l << (8 * i);
-        if (lvl == 3) dg = d;
+      for (int j = 0; j < 16; j++) {
+        const uint64_t c = cb + 1 + j;
+        w[j >> 2] |= (uint32_t)(c < M ? a.labels[c] : DONE) << (8 * (j & 3));
       }
-      lo = out;
-      hi = 0;
-      nb = (nb - 1) / 2;  // parent of the level's first node
-      width >>= 1;
+      v = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    lab = (uint8_t)lo;
+    uint32_t first = __shfl_up_sync(kFull, v.w, 1) >> 24;  // byte 15 of the lane before = child cb
+    if (lane == 0) first = cb < M ? a.labels[cb] : DONE;
+    // child j's label is byte j of (lo, hi)
+    uint64_t lo = ((uint64_t)((v.y << 8) | (v.x >> 24)) << 32) | ((v.x << 8) | first);
+    uint64_t hi = ((uint64_t)((v.w << 8) | (v.z >> 24)) << 32) | ((v.y >> 24) | (v.z << 8));
+    const uint64_t nb1 = (r + 1) * 2048 - 1 + 8ull * t;  // relative depth 11: the deepest interior level
+    uint8_t lab;
+    Digest dg{{0, 0, 0, 0}};
+    constexpr uint64_t kFixed8 = 0x0101010101010101ull * FIXED_DUPL;
+    if (!BASE && lo == kFixed8 && hi == kFixed8 && nb1 + 7 <= last_interior) {
+      lab = pass == 0 ? DONE : FIXED_DUPL;
+    } else if (nb1 + 7 <= last_interior) {
+      uint32_t c[4] = {(uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32)};
+      lab = thread_levels_bytewise<HK, BASE>(a, pass, r, t, c, sink, work, dg);
+    } else {
+      uint64_t nb = nb1;
+      uint32_t width = 8;
+#pragma unroll 1
+      for (int lvl = 0; lvl < 4; lvl++) {
+        uint64_t out = 0;
+        sink_level(sink, r, (int)kBottomLevels - 1 - lvl);
+#pragma unroll 1
+        for (uint32_t i = 0; i < width; i++) {
+          const uint32_t j = 2 * i;
+          const uint8_t ll = (uint8_t)((j < 8 ? lo >> (8 * j) : hi >> (8 * (j - 8))) & 0xff);
+          const uint8_t lr = (uint8_t)((j + 1 < 8 ? lo >> (8 * (j + 1)) : hi >> (8 * (j - 7))) & 0xff);
+          const uint64_t n = nb + i;
+          Digest dl{{0, 0, 0, 0}}, dr{{0, 0, 0, 0}}, d{{0, 0, 0, 0}};
+          if (BASE || (ll == lr && digest_wanted(pass, ll))) {
+            if (lvl == 0) {
+              if (n <= last_interior) {
+                dl = ld_digest(a.tree + 2 * n + 1);
+                dr = ld_digest(a.tree + 2 * n + 2);
+              }
+            } else {
+              dl = work[j][t];
+              dr = work[j + 1][t];
+            }
+          }
+          const uint8_t l = lvl == 0 ? span_label<HK, BASE>(a, pass, n, last_interior, M, ll, lr, dl, dr, d, sink)
+                                     : span_node<HK, BASE>(a, pass, (uint32_t)n, ll, lr, dl, dr, d, false, sink);
+          // read back only at the next level, from a higher index
+          if (BASE || digest_wanted(pass, l)) work[i][t] = d;
+          out |= (uint64_t)l << (8 * i);
+          if (lvl == 3) dg = d;
+        }
+        lo = out;
+        hi = 0;
+        nb = (nb - 1) / 2;  // parent of the level's first node
+        width >>= 1;
+      }
+      lab = (uint8_t)lo;
+    }
+    upper_levels<HK, BASE>(a, pass, r, kSpanLevels, lab, dg, sink, top8, topdg);
+    if (!BASE && pass != 1) flush_sink(a, fused, r, sink, &ids_base);
+    upper_spans<HK, BASE>(a, pass, fused, d_top, blk, sink, &ids_base, top8, topdg, &s_last);
+    __syncthreads();
   }
-  upper_levels<HK, BASE>(a, pass, r, lab, dg, &sink, top8, topdg);
-  if (!BASE && pass != 1) flush_sink(a, sink, &ids_base);
 }
 
-// The queued first-occurrence inserts of a pass, one thread per node, over
+// A pass over a tree of at most kSmallLeaves leaves, by one block: labels in
+// shared memory, a barrier per level.
+template <int HK, bool BASE>
+__global__ void __launch_bounds__(512) forest_small_kernel(ForestArgs a, int pass, uint32_t N, uint32_t dmax) {
+  pdl_enter();
+  __shared__ uint8_t lab[2 * kSmallLeaves];
+  __shared__ uint16_t ids[BASE ? 1 : kSmallLeaves];
+  __shared__ uint32_t ids_n, ids_base;
+  const bool fused = forest_fused(a);
+  if (fused) {
+    if (pass == 1) return;
+    pass = 2;
+  }
+  if (threadIdx.x == 0) ids_n = 0;
+  for (uint32_t n = N - 1 + threadIdx.x; n < 2 * N - 1; n += blockDim.x) lab[n] = a.labels[n];
+  __syncthreads();
+  IdSink sink{ids, &ids_n, 0};
+  for (int d = (int)dmax; d >= 0; d--) {
+    const uint32_t first = (1u << d) - 1, last = min(2 * first, N - 2);
+    sink_level(sink, 0, d);
+    for (uint32_t n = first + threadIdx.x; n <= last; n += blockDim.x) {
+      const uint8_t ll = lab[2 * n + 1], lr = lab[2 * n + 2];
+      Digest dl{{0, 0, 0, 0}}, dr{{0, 0, 0, 0}}, dg;
+      if (BASE || (ll == lr && digest_wanted(pass, ll))) {
+        dl = ld_digest(a.tree + 2 * n + 1);
+        dr = ld_digest(a.tree + 2 * n + 2);
+      }
+      lab[n] = span_node<HK, BASE>(a, pass, n, ll, lr, dl, dr, dg, d == 0, sink);
+    }
+    __syncthreads();
+  }
+  if (!BASE && pass != 1) flush_sink(a, fused, 0, sink, &ids_base);
+}
+
+// The queued first-occurrence inserts of a fused pass, one thread per node, over
 // blocks b0 .. b0+nb-1 of the launch.
 __device__ __forceinline__ void drain_inserts(const ForestArgs& a, uint32_t b0, uint32_t nb) {
   const uint32_t n = *a.ins_count;
@@ -649,17 +641,6 @@ __global__ void __launch_bounds__(256) forest_insert_all_kernel(ForestArgs a, ui
   }
   count_new_entries(a.map, created);
 }
-__device__ __forceinline__ bool forest_fused(const ForestArgs& a) { return a.fuse_gate && *a.fuse_gate == 0; }
-
-// After the first-occurrence pass: the duplicate pass that follows looks its
-// digests up.  A fused pass looks nothing up that these inserts could add,
-// so its inserts wait for the root count (root_count_kernel's extra blocks).
-__global__ void forest_insert_kernel(ForestArgs a) {
-  pdl_enter();
-  if (forest_fused(a)) return;
-  drain_inserts(a, 0, gridDim.x);
-}
-
 // ---------------------------------------------------------------------------
 // Root compaction in serial push order.  rflag holds the flags at canonical
 // positions, so the lists are a stable compaction of one byte array.
@@ -1406,41 +1387,38 @@ cudaError_t launch_map_rebase(const DigestMap& m, uint64_t cap, cudaStream_t s) 
 // ---------------------------------------------------------------------------
 // Host launchers
 // ---------------------------------------------------------------------------
+size_t forest_done_words(uint32_t N) { return ((size_t)N >> 19) + 16; }
+
 cudaError_t launch_forest(const ForestArgs& a, int pass, int baseline, uint32_t N, cudaStream_t s) {
   if (N < 2) return cudaSuccess;
   // deepest interior depth: that of node N-2
   uint32_t dmax = 0;
   while (((2ull << dmax) - 1) <= (uint64_t)(N - 2)) dmax++;
-  const bool dup_baseline = pass == 1 && baseline;
   const bool md5 = a.hash_kind == HASH_MD5;
-  int bot = (int)dmax;
-  if (!dup_baseline && dmax + 1 >= kBottomLevels) {
-    const uint32_t top = dmax - (kBottomLevels - 1);
-    const uint64_t first = (1ull << top) - 1;
-    const uint64_t count = std::min<uint64_t>(1ull << top, (uint64_t)N - 1 - first);
-    auto k = pass == 3 ? (md5 ? forest_bottom12_kernel<HASH_MD5, true> : forest_bottom12_kernel<HASH_MURMUR3, true>)
-                       : (md5 ? forest_bottom12_kernel<HASH_MD5, false> : forest_bottom12_kernel<HASH_MURMUR3, false>);
-    launch_k(k, (uint32_t)count, 256, 0, s, a, pass, N, top);
-    note_launch();
-    bot = (int)top - 1;
+  if (pass == 1 && baseline) {
+    for (int bot = (int)dmax; bot >= 0; bot -= kSpanLevels) {
+      const uint32_t top = bot >= (int)kSpanLevels - 1 ? (uint32_t)bot - (kSpanLevels - 1) : 0;
+      const uint64_t first = (1ull << top) - 1;
+      const uint64_t count = std::min<uint64_t>(1ull << top, (uint64_t)N - 1 - first);
+      launch_k(forest_span_kernel, (uint32_t)count, 256, 0, s, a, N, top, (uint32_t)bot);
+      note_launch();
+    }
+    return cudaGetLastError();
   }
-  for (; bot >= 0; bot -= kSpanLevels) {
-    const uint32_t top = bot >= (int)kSpanLevels - 1 ? (uint32_t)bot - (kSpanLevels - 1) : 0;
-    const uint64_t first = (1ull << top) - 1;
-    const uint64_t count = std::min<uint64_t>(1ull << top, (uint64_t)N - 1 - first);
-    auto k9 = pass == 3
-                  ? (md5 ? forest_span9_warp_kernel<HASH_MD5, true> : forest_span9_warp_kernel<HASH_MURMUR3, true>)
-                  : (md5 ? forest_span9_warp_kernel<HASH_MD5, false> : forest_span9_warp_kernel<HASH_MURMUR3, false>);
-    if (!dup_baseline && (uint32_t)bot - top == kSpanLevels - 1)
-      launch_k(k9, (uint32_t)count, 256, 0, s, a, pass, N, top);
-    else
-      launch_k(forest_span_kernel, (uint32_t)count, 256, 0, s, a, pass, baseline, N, top, (uint32_t)bot);
-    note_launch();
-    if (top == 0) break;
+  if (N <= kSmallLeaves) {
+    auto k = pass == 3 ? (md5 ? forest_small_kernel<HASH_MD5, true> : forest_small_kernel<HASH_MURMUR3, true>)
+                       : (md5 ? forest_small_kernel<HASH_MD5, false> : forest_small_kernel<HASH_MURMUR3, false>);
+    launch_k(k, 1, 512, 0, s, a, pass, N, dmax);
+  } else {
+    auto k = pass == 3 ? (md5 ? forest_kernel<HASH_MD5, true> : forest_kernel<HASH_MURMUR3, true>)
+                       : (md5 ? forest_kernel<HASH_MD5, false> : forest_kernel<HASH_MURMUR3, false>);
+    const uint32_t top = dmax - (kBottomLevels - 1), count = 1u << top;
+    launch_k(k, pass == 1 ? std::min<uint32_t>(count, (uint32_t)num_sms() * 5) : count, 256, 0, s, a, pass, N, top,
+             count);
   }
-  if (pass == 0 || pass == 3) {
-    if (pass == 0) launch_k(forest_insert_kernel, grid_for(N, 256), 256, 0, s, a);
-    else launch_k(forest_insert_all_kernel, grid_for(N - 1, 256), 256, 0, s, a, N - 1);
+  note_launch();
+  if (pass == 3) {
+    launch_k(forest_insert_all_kernel, grid_for(N - 1, 256), 256, 0, s, a, N - 1);
     note_launch();
   }
   return cudaGetLastError();

@@ -44,6 +44,7 @@ struct ForestArgs {
   const uint32_t* fuse_gate;
   uint32_t* ins_queue;  // first-occurrence nodes awaiting their map insert (N entries)
   uint32_t* ins_count;
+  uint32_t* span_done;  // forest_done_words(N) counters, zero between passes
 };
 
 // Position of node x (>= 1) in the canonical root order.
@@ -83,9 +84,10 @@ struct GatherArgs {
   Layout* lay;
 };
 
-// All levels of one forest pass in a few launches (9 levels each).
-// pass 0 = first-occurrence forest, 1 = duplicate forest, 3 = both, and the
-// inserts, of a baseline whose digests were cleared (baseline = 1).
+// One forest pass.  pass 0 = first-occurrence forest, 1 = duplicate forest, 3 =
+// both, and the inserts, of a baseline whose digests were cleared (baseline =
+// 1).
+size_t forest_done_words(uint32_t N);
 cudaError_t launch_forest(const ForestArgs& a, int pass, int baseline, uint32_t N, cudaStream_t s);
 cudaError_t launch_root_compaction(const ForestArgs& fa, uint32_t N, uint32_t M, uint32_t* fo_list,
                                    uint32_t* sh_list, Layout* lay, uint64_t* scan_scratch, uint64_t* scan_total,
