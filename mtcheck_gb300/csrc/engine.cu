@@ -46,11 +46,7 @@ constexpr uint32_t kInjectedSpinLimit = 1u << 14;
 
 static __global__ void readback_kernel(Readback r) {
   pdl_enter();
-  stamp(r.clk, CLK_END);
-  __syncwarp();
-#pragma unroll
-  for (int k = 0; k < 4; k++)
-    for (uint32_t i = threadIdx.x; i < r.words[k]; i += blockDim.x) r.dst[k][i] = r.src[k][i];
+  readback(r);
 }
 
 cudaError_t launch_readback(const Readback& r, cudaStream_t s) {
@@ -195,7 +191,8 @@ int Engine::ensure_state(uint32_t N, bool fresh, uint32_t id_headroom) {
     const size_t nd = tree ? M : N;
     MTC_CUDA(digests_.ensure(nd, stream_));
     MTC_CUDA(cudaMemsetAsync(digests_.p, 0, sizeof(Digest) * nd, stream_));
-    MTC_CUDA(labels_.ensure(nd, stream_));
+    // read in 16-byte words by the list and basic compaction
+    MTC_CUDA(labels_.ensure((nd + 15) / 16 * 16, stream_));
     // root flags, read in 16-byte words: zero between checkpoints (the root
     // compaction clears what it has read)
     MTC_CUDA(rflag_.ensure(tree ? ((size_t)M + 15) / 16 * 16 : 16, stream_));
@@ -214,13 +211,11 @@ int Engine::ensure_state(uint32_t N, bool fresh, uint32_t id_headroom) {
     MTC_CUDA(fo_val_.ensure(N + 1, stream_));
     MTC_CUDA(reg_chunk_.ensure(N + 1, stream_));
     MTC_CUDA(reg_slot_.ensure(N + 1, stream_));
-    MTC_CUDA(reg_len_.ensure(N + 1, stream_));
+    MTC_CUDA(fo_tile_.ensure(tree ? N + 1 : 1, stream_));
     MTC_CUDA(sh_key_.ensure(N + 1, stream_));
     MTC_CUDA(sh_prev_.ensure(N + 1, stream_));
-    // tile sums: scans of 4096 entries over max(M, N+1), or of 512 regions over N+1
-    MTC_CUDA(scan_.ensure(std::max<size_t>((size_t)(std::max(M, N + 1) + kScanTile - 1) / kScanTile,
-                                           ((size_t)N + 1 + 511) / 512) + 2, stream_));
-    MTC_CUDA(scan_total_.ensure(1, stream_));
+    // per tile of 8192 flags: root counts, then region sums
+    MTC_CUDA(scan_.ensure(2 * root_tiles(), stream_));
     MTC_CUDA(scan_total2_.ensure(1, stream_));
     MTC_CUDA(lay_.ensure(1, stream_));
     MTC_CUDA(sp_.ensure(1, stream_));
@@ -247,6 +242,18 @@ int Engine::ensure_state(uint32_t N, bool fresh, uint32_t id_headroom) {
   return ensure_sort(current_id + 1 + id_headroom);
 }
 
+// Tiles of the root compaction (8192 flags each), one more for alignment's sake.
+size_t Engine::root_tiles() const { return ((size_t)std::max(M_, N_) + 8191) / 8192 + 1; }
+
+RootOrder Engine::root_order() const {
+  RootOrder o{};
+  if (mode_ == MODE_LIST || mode_ == MODE_BASIC) return o;
+  o.ascending = mode_ == MODE_TREE_LOW_OFFSET_REF ? 1 : 0;
+  while (((2ull << o.D) - 1) <= (uint64_t)(M_ - 1)) o.D++;  // depth of node M-1
+  o.sizeD = (uint64_t)M_ - ((1ull << o.D) - 1);
+  return o;
+}
+
 GatherArgs Engine::gather_args(const uint8_t* data, uint64_t len) {
   GatherArgs g{};
   g.approach = mode_ == MODE_LIST ? APPROACH_LIST : mode_ == MODE_BASIC ? APPROACH_BASIC : APPROACH_TREE;
@@ -266,25 +273,52 @@ GatherArgs Engine::gather_args(const uint8_t* data, uint64_t len) {
   g.fo_val = fo_val_.p;
   g.reg_chunk = reg_chunk_.p;
   g.reg_slot = reg_slot_.p;
-  g.reg_len = reg_len_.p;
+  g.fo_tile = fo_tile_.p;
   g.sh_key = sh_key_.p;
   g.sh_prev = sh_prev_.p;
   g.hist = hist_.p;
   g.rep = rep_.p;
   g.rank = rank_.p;
   g.sort_mat = sort_mat_.p;
-  g.scan_scratch = scan_.p;
-  g.scan_total = scan_total_.p;
+  g.tile_counts = scan_.p;
+  g.tile_regions = scan_.p + root_tiles();
   g.scan_scratch2 = scan2_.p;
   g.scan_total2 = scan_total2_.p;
   g.stage = stage_.p;
   g.stage_cap = stage_.n;
   g.lay = lay_.p;
+  g.counters = changed_count_.p;
+  const bool tree = g.approach == APPROACH_TREE;
+  g.flags = tree ? rflag_.p : labels_.p;
+  g.n_flags = tree ? (uint64_t)M_ - 1 : N_;  // every node but the root, or every chunk
+  g.labels = labels_.p;
+  g.order = root_order();
+  if (tree && !baseline_path_) {
+    g.fuse_gate = changed_count_.p + COUNT_DEMOTED;
+    g.ins_queue = changed_list_.p;
+    g.ins_count = changed_count_.p + COUNT_INSERTS;
+  }
+  // results (layout, error word, map size, phase times) written to pinned
+  // memory by a kernel, not queued on a copy engine behind other streams'
+  // transfers
+  static_assert(sizeof(Layout) % 4 == 0, "layout copied as words");
+  Readback& rb = g.results;
+  auto to_host = [&](int k, const void* src, void* host, uint32_t words) {
+    rb.src[k] = static_cast<const uint32_t*>(src);
+    rb.dst[k] = static_cast<uint32_t*>(host);
+    rb.words[k] = words;
+  };
+  uint32_t* err_dst = static_cast<uint32_t*>(host_alias(err_host_));
+  to_host(0, lay_.p, host_alias(lay_host_), sizeof(Layout) / 4);
+  to_host(1, err_.p, err_dst, 1);
+  if (map_size_.p) to_host(2, map_size_.p, err_dst + 1, 1);
+  if (timed_) to_host(3, clk_.p, host_alias(clk_host_), CLK_COUNT * 2);
+  rb.clk = g.clk;
   return g;
 }
 
 int Engine::run_tree(const uint8_t* data, uint64_t len, bool baseline_path) {
-  const uint32_t N = N_, M = M_;
+  const uint32_t N = N_;
   DigestMap map{slots_.p, map_cap_ - 1, map_size_.p};
   LeafArgs la;
   la.data = data;
@@ -302,11 +336,11 @@ int Engine::run_tree(const uint8_t* data, uint64_t len, bool baseline_path) {
   la.hash_kind = hash_kind_;
   la.epi = EPI_TREE;
   la.changed_list = changed_list_.p;
-  la.changed_count = changed_count_.p;
-  la.demoted = changed_count_.p + 1;
+  la.changed_count = changed_count_.p + COUNT_CHANGED;
+  la.demoted = changed_count_.p + COUNT_DEMOTED;
   // the first-occurrence root list is free until the root compaction
   la.dup_list = fo_list_.p;
-  la.dup_count = changed_count_.p + 3;
+  la.dup_count = changed_count_.p + COUNT_NOTES;
   la.dup_cap = (uint32_t)fo_list_.n;
   if (stall_now_) {
     la.stall = 1;
@@ -324,17 +358,14 @@ int Engine::run_tree(const uint8_t* data, uint64_t len, bool baseline_path) {
   fa.sp = sp_.p;
   fa.err = err_.p;
   fa.hash_kind = hash_kind_;
-  fa.ascending = mode_ == MODE_TREE_LOW_OFFSET_REF ? 1 : 0;
-  fa.D = 0;
-  while (((2ull << fa.D) - 1) <= (uint64_t)(M - 1)) fa.D++;  // depth of node M-1
-  fa.sizeD = (uint64_t)M - ((1ull << fa.D) - 1);
+  fa.order = root_order();
   // an incremental checkpoint without demoted leaves runs both passes in one
   // traversal (the launches of the duplicate pass then return at once)
   fa.fuse_gate = baseline_path ? nullptr : la.demoted;
   // the changed-chunk list is free once the leaf inserts are done: it queues
   // the forest's first-occurrence inserts
   fa.ins_queue = changed_list_.p;
-  fa.ins_count = changed_count_.p + 2;
+  fa.ins_count = changed_count_.p + COUNT_INSERTS;
   fa.span_done = span_done_.p;
   if (baseline_path && fresh_) {
     MTC_CUDA(launch_forest(fa, 3, 1, N, stream_));  // both passes of a baseline on cleared digests
@@ -342,7 +373,6 @@ int Engine::run_tree(const uint8_t* data, uint64_t len, bool baseline_path) {
     MTC_CUDA(launch_forest(fa, 0, 0, N, stream_));                      // first-occurrence forest
     MTC_CUDA(launch_forest(fa, 1, baseline_path ? 1 : 0, N, stream_));  // duplicate forest
   }
-  MTC_CUDA(launch_root_compaction(fa, N, M, fo_list_.p, sh_list_.p, lay_.p, scan_.p, scan_total_.p, stream_));
   return ST_OK;
 }
 
@@ -364,9 +394,9 @@ int Engine::run_list_basic(const uint8_t* data, uint64_t len) {
   la.epi = mode_ == MODE_LIST ? EPI_LIST : EPI_BASIC;
   la.basic_first = current_id == 0 ? 1 : 0;  // never true in a captured sequence
   la.changed_list = changed_list_.p;
-  la.changed_count = changed_count_.p;
+  la.changed_count = changed_count_.p + COUNT_CHANGED;
   la.dup_list = fo_list_.p;  // free until the chunk compaction
-  la.dup_count = changed_count_.p + 3;
+  la.dup_count = changed_count_.p + COUNT_NOTES;
   la.dup_cap = (uint32_t)fo_list_.n;
   if (stall_now_) {
     la.stall = 1;
@@ -375,8 +405,6 @@ int Engine::run_list_basic(const uint8_t* data, uint64_t len) {
   if (leaf_hook_) MTC_TRY(leaf_hook_->on_leaves(this, la, stream_));
   else MTC_CUDA(launch_leaves(la, &tma_, stream_, leaf_tune_));
   if (mode_ == MODE_LIST) MTC_CUDA(launch_leaf_inserts(la, stream_));
-  MTC_CUDA(launch_chunk_compaction(labels_.p, N_, mode_ == MODE_BASIC ? 1 : 0, fo_list_.p, sh_list_.p, lay_.p, scan_.p,
-                                   scan_total_.p, la.clk, stream_));
   return ST_OK;
 }
 
@@ -439,28 +467,6 @@ int Engine::enqueue(const uint8_t* data, uint64_t len, bool timed) {
   int rc = (mode_ == MODE_LIST || mode_ == MODE_BASIC) ? run_list_basic(data, len) : run_tree(data, len, baseline_path_);
   if (rc) return rc;
   MTC_CUDA(launch_assemble(gather_args(data, len), (uint64_t)N_ + 1, fresh_, stream_));
-  // results (layout, error word, map size) written to pinned memory by a
-  // kernel, not queued on a copy engine behind other streams' transfers
-  static_assert(sizeof(Layout) % 4 == 0, "layout copied as words");
-  Readback rb{};
-  rb.src[0] = reinterpret_cast<const uint32_t*>(lay_.p);
-  rb.dst[0] = static_cast<uint32_t*>(host_alias(lay_host_));
-  rb.words[0] = sizeof(Layout) / 4;
-  rb.src[1] = err_.p;
-  rb.dst[1] = static_cast<uint32_t*>(host_alias(err_host_));
-  rb.words[1] = 1;
-  if (map_size_.p) {
-    rb.src[2] = map_size_.p;
-    rb.dst[2] = rb.dst[1] + 1;
-    rb.words[2] = 1;
-  }
-  if (timed) {
-    rb.src[3] = reinterpret_cast<const uint32_t*>(clk_.p);
-    rb.dst[3] = static_cast<uint32_t*>(host_alias(clk_host_));
-    rb.words[3] = CLK_COUNT * 2;
-    rb.clk = clk_.p;
-  }
-  MTC_CUDA(launch_readback(rb, stream_));
   return ST_OK;
 }
 
@@ -703,10 +709,10 @@ uint64_t Engine::shape_signature(const uint8_t* data, uint64_t len) const {
   const uint64_t v[] = {(uint64_t)data & 15, len, (uint64_t)digests_.p, (uint64_t)labels_.p, (uint64_t)rflag_.p,
                         (uint64_t)chunk_slot_.p, (uint64_t)changed_list_.p, (uint64_t)changed_count_.p,
                         (uint64_t)slots_.p, map_cap_, (uint64_t)map_size_.p, (uint64_t)err_.p, (uint64_t)fo_list_.p,
-                        (uint64_t)sh_list_.p, (uint64_t)reg_chunk_.p, (uint64_t)reg_slot_.p, (uint64_t)reg_len_.p,
+                        (uint64_t)sh_list_.p, (uint64_t)reg_chunk_.p, (uint64_t)reg_slot_.p, (uint64_t)fo_tile_.p,
                         (uint64_t)sh_key_.p, (uint64_t)sh_prev_.p, (uint64_t)hist_.p, hist_.n, (uint64_t)rep_.p,
                         (uint64_t)rank_.p, (uint64_t)fo_val_.p, (uint64_t)sort_mat_.p, sort_mat_.n, (uint64_t)scan_.p,
-                        (uint64_t)scan_total_.p, (uint64_t)scan2_.p, (uint64_t)scan_total2_.p, (uint64_t)stage_.p,
+                        (uint64_t)scan2_.p, (uint64_t)scan_total2_.p, (uint64_t)stage_.p,
                         stage_.n, (uint64_t)lay_.p, (uint64_t)sp_.p, (uint64_t)clk_.p, (uint64_t)span_done_.p, (uint64_t)baseline_path_, (uint64_t)mode_,
                         (uint64_t)leaf_tune_.rows, (uint64_t)leaf_tune_.ctas_per_sm, (uint64_t)leaf_tune_.direct,
                         (uint64_t)leaf_tune_.threads_per_chunk};
@@ -718,8 +724,8 @@ uint64_t Engine::shape_signature(const uint8_t* data, uint64_t len) const {
 template <class F>
 void Engine::for_each_buf(F f) {
   f(digests_); f(labels_); f(rflag_); f(chunk_slot_); f(changed_list_); f(changed_count_); f(slots_);
-  f(map_size_); f(err_); f(fo_list_); f(sh_list_); f(reg_chunk_); f(reg_slot_); f(reg_len_); f(sh_key_);
-  f(sh_prev_); f(hist_); f(rep_); f(rank_); f(fo_val_); f(sort_mat_); f(scan_); f(scan_total_); f(scan2_);
+  f(map_size_); f(err_); f(fo_list_); f(sh_list_); f(reg_chunk_); f(reg_slot_); f(fo_tile_); f(sh_key_);
+  f(sh_prev_); f(hist_); f(rep_); f(rank_); f(fo_val_); f(sort_mat_); f(scan_); f(scan2_);
   f(scan_total2_); f(stage_); f(lay_); f(sp_); f(clk_); f(span_done_);
 }
 
@@ -793,10 +799,10 @@ void Engine::release_restart_scratch() {
 uint64_t Engine::device_bytes() const {
   return sizeof(Digest) * digests_.n + labels_.n + rflag_.n +
          sizeof(uint32_t) * (chunk_slot_.n + changed_list_.n + changed_count_.n + map_size_.n + err_.n + fo_list_.n +
-                             sh_list_.n + reg_chunk_.n + reg_slot_.n + reg_len_.n + sh_key_.n + sh_prev_.n + hist_.n +
+                             sh_list_.n + reg_chunk_.n + reg_slot_.n + fo_tile_.n + sh_key_.n + sh_prev_.n + hist_.n +
                              rep_.n + rank_.n + span_done_.n) +
          sizeof(MapSlot) * slots_.n +
-         sizeof(uint64_t) * (fo_val_.n + sort_mat_.n + scan_.n + scan_total_.n + scan2_.n + scan_total2_.n) + stage_.n +
+         sizeof(uint64_t) * (fo_val_.n + sort_mat_.n + scan_.n + scan2_.n + scan_total2_.n) + stage_.n +
          sizeof(Layout) * lay_.n + sizeof(StepParams) * sp_.n + sizeof(uint64_t) * clk_.n;
 }
 

@@ -259,6 +259,8 @@ class Engine {
   int run_tree(const uint8_t* data, uint64_t len, bool baseline_path);
   int run_list_basic(const uint8_t* data, uint64_t len);
   GatherArgs gather_args(const uint8_t* data, uint64_t len);
+  size_t root_tiles() const;
+  RootOrder root_order() const;
 
   int mode_, hash_kind_;
   uint32_t cs_;
@@ -308,8 +310,8 @@ class Engine {
   DevBuf<uint32_t> chunk_slot_, changed_list_, changed_count_;
   DevBuf<MapSlot> slots_;
   DevBuf<uint32_t> map_size_, err_;
-  DevBuf<uint32_t> fo_list_, sh_list_, reg_chunk_, reg_slot_, reg_len_, sh_key_, sh_prev_, hist_, rep_, rank_;
-  DevBuf<uint64_t> fo_val_, sort_mat_, scan_, scan_total_, scan2_, scan_total2_;
+  DevBuf<uint32_t> fo_list_, sh_list_, reg_chunk_, reg_slot_, fo_tile_, sh_key_, sh_prev_, hist_, rep_, rank_;
+  DevBuf<uint64_t> fo_val_, sort_mat_, scan_, scan2_, scan_total2_;
   DevBuf<uint8_t> stage_;
   DevBuf<Layout> lay_;
   DevBuf<StepParams> sp_;

@@ -606,18 +606,17 @@ __global__ void __launch_bounds__(512) forest_small_kernel(ForestArgs a, int pas
   if (!BASE && pass != 1) flush_sink(a, fused, 0, sink, &ids_base);
 }
 
-// The queued first-occurrence inserts of a fused pass, one thread per node, over
-// blocks b0 .. b0+nb-1 of the launch.
-__device__ __forceinline__ void drain_inserts(const ForestArgs& a, uint32_t b0, uint32_t nb) {
-  const uint32_t n = *a.ins_count;
-  const uint32_t cur_id = a.sp->cur, epoch_fo = a.sp->epoch + 1;
+// The queued first-occurrence inserts of a fused pass, one thread per node, by
+// nblk blocks.
+__device__ __forceinline__ void drain_inserts(const GatherArgs& g, uint32_t blk, uint32_t nblk) {
+  const uint32_t n = *g.ins_count;
+  const uint32_t cur_id = g.sp->cur, epoch_fo = g.sp->epoch + 1;
   uint32_t created = 0;
-  for (uint32_t k = (blockIdx.x - b0) * blockDim.x + threadIdx.x; k < n; k += nb * blockDim.x) {
-    const uint32_t node = a.ins_queue[k];
-    // a first occurrence's digest is new: its leaves' are
-    created += map_insert_serial(a.map, ld_digest(a.tree + node), node, cur_id, epoch_fo, false, a.err);
+  for (uint32_t k = blk * blockDim.x + threadIdx.x; k < n; k += nblk * blockDim.x) {
+    const uint32_t node = g.ins_queue[k];
+    created += map_insert_serial(g.map, ld_digest(g.digests + node), node, cur_id, epoch_fo, false, g.err);
   }
-  count_new_entries(a.map, created);
+  count_new_entries(g.map, created);
 }
 // After pass 3: every interior node's digest into the map.  First occurrences
 // carry the first pass's epoch, the others the second's, among which equal
@@ -642,10 +641,18 @@ __global__ void __launch_bounds__(256) forest_insert_all_kernel(ForestArgs a, ui
   count_new_entries(a.map, created);
 }
 // ---------------------------------------------------------------------------
-// Root compaction in serial push order.  rflag holds the flags at canonical
-// positions, so the lists are a stable compaction of one byte array.
+// Root compaction in serial push order, and what the diff's layout needs to
+// know of each root.  Tree: the flag bytes lie at canonical positions, so the
+// lists are a stable compaction of one byte array.  List and basic: the same of
+// the chunks' labels.
+//
+// From here to the finished diff there are four launches, each a chain of a few
+// dependent accesses, so the time is mostly latency and launches: 64 MiB in
+// 128-byte chunks spent 44 us of an increment in the eleven launches (counts,
+// roots, lookups, region sums, layout, metadata, four for the sort, copy,
+// results) that these replace.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t node_at(const ForestArgs& a, uint64_t p) {
+__device__ __forceinline__ uint32_t node_at(const RootOrder& a, uint64_t p) {
   if (a.ascending) return (uint32_t)p + 1;
   if (p < a.sizeD) return (uint32_t)(((1ull << a.D) - 1) + p);
   // levels D-1, D-2, ... follow with sizes 2^(D-1), 2^(D-2), ...: position q
@@ -655,386 +662,378 @@ __device__ __forceinline__ uint32_t node_at(const ForestArgs& a, uint64_t p) {
   return (uint32_t)(((1ull << d) - 1) + ((2ull << d) - x));
 }
 
-// 64 contiguous flags per thread (four 16-byte loads), 32 Ki flags per
-// tile; counts packed as (shift << 32) | fo.  Flag bytes are 0, 1 (first
-// occurrence) or 2 (shifted duplicate), so bit 0 and bit 1 of each byte
-// count the two kinds.
-constexpr int kRootVec = 4;
-constexpr uint64_t kRootPerThread = 16 * kRootVec;
+// 16 contiguous flags per thread, 8 Ki flags per tile: a tile's roots are
+// looked up by its block, so many small tiles keep a dense diff's lookups
+// spread over the GPU.
+constexpr uint64_t kRootPerThread = 16;
 constexpr uint64_t kRootTile = kRootPerThread * kScanThreads;
-static_assert(ROOT_FO == 1 && ROOT_SHIFT == 2, "flag bytes counted by bit");
+constexpr uint32_t kRootReduceTiles = 4096;  // up to here blocks sum the tiles before theirs
 
-__device__ __forceinline__ uint64_t count_word(uint32_t w) {
-  return (uint64_t)__popc(w & 0x01010101u) | ((uint64_t)__popc(w & 0x02020202u) << 32);
+// Masks (0x01 per byte) of the first occurrences and shifted duplicates among
+// four flags or labels.
+template <int APPROACH>
+__device__ __forceinline__ void kinds4(uint32_t w, uint32_t& fo, uint32_t& sh) {
+  constexpr uint32_t one = 0x01010101u;
+  if (APPROACH == APPROACH_TREE) {
+    static_assert(ROOT_FO == 1 && ROOT_SHIFT == 2, "flag bytes told apart by bit");
+    fo = w & one;
+    sh = (w >> 1) & one;
+  } else if (APPROACH == APPROACH_LIST) {
+    fo = __vcmpeq4(w, FIRST_OCUR * one) & one;
+    sh = __vcmpeq4(w, SHIFT_DUPL * one) & one;
+  } else {
+    fo = __vcmpeq4(w, one) & one;
+    sh = 0;
+  }
 }
 
-// The thread's flags starting at p (p a multiple of 16); the array is padded to
-// whole words of ROOT_NONE.
-__device__ __forceinline__ uint64_t load_flags(const uint8_t* f, uint64_t p, uint64_t n, uint4 v[kRootVec]) {
+// The thread's 16 flags at p (a multiple of 16; the arrays are padded to whole
+// words): masks per word, none at or past n.
+template <int APPROACH>
+__device__ __forceinline__ uint64_t load_kinds(const uint8_t* f, uint64_t p, uint64_t n, uint32_t fo[4], uint32_t sh[4]) {
   uint64_t c = 0;
+  uint4 v = make_uint4(0, 0, 0, 0);
+  if (p < n) v = *reinterpret_cast<const uint4*>(f + p);
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-  for (int k = 0; k < kRootVec; k++) {
-    const uint64_t q = p + 16 * (uint64_t)k;
-    v[k] = q < n ? *reinterpret_cast<const uint4*>(f + q) : make_uint4(0, 0, 0, 0);
-    c += count_word(v[k].x) + count_word(v[k].y) + count_word(v[k].z) + count_word(v[k].w);
+  for (int q = 0; q < 4; q++) {
+    kinds4<APPROACH>(w[q], fo[q], sh[q]);
+    const uint64_t at = p + 4 * q;
+    const uint32_t in = at + 4 <= n ? ~0u : at >= n ? 0u : (1u << (8 * (uint32_t)(n - at))) - 1;
+    fo[q] &= in;
+    sh[q] &= in;
+    c += (uint64_t)__popc(fo[q]) | ((uint64_t)__popc(sh[q]) << 32);
   }
   return c;
 }
 
-// The root itself is pushed only for N >= 2 in the incremental and baseline
-// passes (src/tree_approach.cpp:384-393); the serial reference inserts it
-// whenever it is a first occurrence (include/reference_impl.hpp:105-106).
-__device__ __forceinline__ void root_prologue(const uint8_t* labels, uint32_t N, int ascending, uint32_t* fo_list,
-                                              Layout* lay) {
-  const uint32_t root = (labels[0] == FIRST_OCUR && (ascending || N >= 2)) ? 1u : 0u;
-  lay->root_fo = root;
-  if (root) fo_list[0] = 0;
+// Block-wide: exclusive prefix in place over n words, their total returned.
+__device__ __forceinline__ uint64_t scan_in_place(uint64_t* v, uint32_t n, uint64_t* sh) {
+  const uint32_t per = (n + blockDim.x - 1) / blockDim.x;
+  const uint32_t lo = min(threadIdx.x * per, n), hi = min(lo + per, n);
+  uint64_t s = 0;
+  for (uint32_t i = lo; i < hi; i++) s += __ldcg(v + i);
+  uint64_t total;
+  uint64_t ex = block_excl_scan(s, sh, &total);
+  for (uint32_t i = lo; i < hi; i++) {
+    const uint64_t x = __ldcg(v + i);
+    v[i] = ex;
+    ex += x;
+  }
+  return total;
 }
 
-// The first `nd` blocks issue a fused forest pass's queued inserts (only the
-// assembly's ownership test and later checkpoints read them), the others
-// count one tile each.
-__global__ void __launch_bounds__(kScanThreads) root_count_kernel(ForestArgs a, uint32_t N, uint64_t n,
-                                                                  uint64_t* tile_sums, uint32_t* fo_list,
-                                                                  Layout* lay, uint32_t nd) {
+// True in every thread of the last block of a part of `nblocks` blocks to get
+// here; what the others wrote before is visible to it past the L1.
+__device__ __forceinline__ bool last_block(uint32_t* done, uint32_t nblocks, uint32_t* s_last) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    *s_last = atomicAdd(done, 1u) + 1 == nblocks ? 1u : 0u;
+    __threadfence();
+  }
+  __syncthreads();
+  return *s_last != 0;
+}
+
+// Flags per tile, packed as (shift << 32) | fo.  The root itself is pushed only
+// for N >= 2 in the incremental and baseline passes
+// (src/tree_approach.cpp:384-393); the serial reference inserts it whenever it
+// is a first occurrence (include/reference_impl.hpp:105-106).
+template <int APPROACH>
+__global__ void __launch_bounds__(kScanThreads) root_count_kernel(GatherArgs g) {
   pdl_enter();
   __shared__ uint64_t sh[33];
-  if (blockIdx.x < nd) {
-    if (forest_fused(a)) drain_inserts(a, 0, nd);
-    return;
+  if (APPROACH == APPROACH_BASIC) stamp(g.clk, CLK_LEAVES_DONE);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const bool root = APPROACH == APPROACH_TREE && g.labels[0] == FIRST_OCUR && (g.order.ascending || g.N >= 2);
+    g.lay->root_fo = root ? 1 : 0;
+    if (root) g.fo_list[0] = 0;
   }
-  const uint32_t tile = blockIdx.x - nd;
-  if (tile == 0 && threadIdx.x == 0) root_prologue(a.labels, N, a.ascending, fo_list, lay);
-  const uint64_t p = (uint64_t)tile * kRootTile + (uint64_t)threadIdx.x * kRootPerThread;
-  uint4 v[kRootVec];
-  const uint64_t c = p < n ? load_flags(a.rflag, p, n, v) : 0;
+  const uint64_t p = (uint64_t)blockIdx.x * kRootTile + (uint64_t)threadIdx.x * kRootPerThread;
+  uint32_t fo[4], shf[4];
+  const uint64_t c = load_kinds<APPROACH>(g.flags, p, g.n_flags, fo, shf);
   uint64_t total;
   block_excl_scan(c, sh, &total);
-  if (threadIdx.x == 0) tile_sums[tile] = total;
+  if (threadIdx.x == 0) g.tile_counts[blockIdx.x] = total;
 }
 
-// Emits the roots in serial push order.  kReduce: the tile offset is the sum of
-// the earlier tiles' counts (few tiles), and the last tile sets F and S;
-// otherwise tile_off holds scanned offsets and root_epilogue_kernel follows.
-template <bool kReduce>
-__global__ void __launch_bounds__(kScanThreads) root_emit_kernel(ForestArgs a, uint64_t n, const uint64_t* tile_off,
-                                                                 uint32_t* fo_list, uint32_t* sh_list, Layout* lay) {
+// First-occurrence root: (1 << 32) | chunks if it owns its digest, else 0.  A
+// first-occurrence leaf owns its digest: the leaf pass demotes every other one
+// (same checkpoint id, another owner).  The inserts of a fused pass may still
+// wait: a digest that is not in the map then is the root's own.
+__device__ __forceinline__ uint64_t fo_region(const GatherArgs& g, uint32_t node, bool fused, uint32_t cur) {
+  bool owner = node >= g.N - 1;
+  if (!owner) {
+    const int64_t slot = map_find(g.map, ld_digest(g.digests + node), g.err);
+    const NodeIdDev prev = slot_value(g.map, slot);
+    owner = slot < 0 ? fused : prev.node == node && prev.tree == cur;
+  }
+  return owner ? (1ull << 32) | num_leaf_descendents(node, g.M) : 0;
+}
+
+// One block, once every root is listed: repeat-count table, layout, header; bin
+// representatives for the list approach's BinOp1D.  The tiles' region sums
+// become offsets in place.
+template <int APPROACH>
+__device__ void build_layout(const GatherArgs& g, uint32_t ntiles, uint64_t* sh) {
+  volatile Layout* lay = g.lay;
+  const uint32_t F = lay->F, S = lay->S;
+  uint64_t regions = ((uint64_t)F << 32) | F;  // list / basic: one chunk per entry
+  if (APPROACH == APPROACH_TREE) regions = scan_in_place(g.tile_regions, ntiles, sh);
+  const uint32_t nd = (uint32_t)(regions >> 32), chunks = (uint32_t)regions;
+  const uint32_t cur = g.sp->cur;
+  const uint32_t K = cur + 1, tid = threadIdx.x, nt = blockDim.x;
+  constexpr bool kMeta = APPROACH != APPROACH_BASIC;
+  // P = number of source checkpoints that occur; max_key = largest of them
+  __shared__ uint32_t smax;
+  if (tid == 0) smax = 0;
+  __syncthreads();
+  uint32_t P = 0;
+  if (kMeta && S)
+    for (uint32_t b = 0; b < K; b += nt) {
+      const uint32_t k = b + tid;
+      const bool nz = k < K && __ldcg(g.hist + k) > 0;
+      P += (uint32_t)__syncthreads_count(nz);
+      if (nz) atomicMax(&smax, k);
+    }
+  __syncthreads();
+  const uint32_t max_key = smax;
+  const uint64_t fo_off = 32;
+  const uint64_t data_off = fo_off + 4ull * F + (kMeta ? 8ull * P + 8ull * S : 0);
+  const uint64_t pad = (16 - (data_off & 15)) & 15;
+  const uint64_t diff_len = data_off + (uint64_t)chunks * g.cs;
+  const bool ok = pad + diff_len <= g.stage_cap;
+  const uint64_t table_off = fo_off + 4ull * nd;
+  // sort representative of each key: stable sort by BinOp1D bin equals stable
+  // sort by the smallest key sharing the bin
+  const uint32_t nbins = APPROACH == APPROACH_TREE ? cur : S;
+  const double range = (double)(APPROACH == APPROACH_TREE ? cur : max_key);
+  const bool plain = range <= (double)nbins;  // every key is its own bin
+  uint8_t* diff = g.stage + pad;
+  if (tid == 0) {
+    lay->num_distinct = nd;
+    lay->chunk_counter = chunks;
+    lay->P = P;
+    lay->pad = pad;
+    lay->data_off = data_off;
+    lay->table_off = table_off;
+    lay->pairs_off = table_off + 8ull * P;
+    lay->nkeys = plain ? P : 0;
+    lay->sort_n = 0;
+    lay->sort_tiles = 0;
+    lay->diff_len = ok ? diff_len : 0;
+    lay->ok = ok ? 1 : 0;
+    if (!ok) atomicOr(g.err, DERR_CAPACITY);
+    // datasizes as the reference's collect_diff returns them
+    if (APPROACH == APPROACH_TREE) {
+      const uint64_t meta = 4ull * F + 8ull * P + 8ull * S;
+      lay->size_data = diff_len - meta;  // src/tree_approach.cpp:707-709
+      lay->size_meta = meta;
+    } else {
+      // src/list_approach.cpp:241-246; src/basic_approach.cpp:141-142 (32-bit product)
+      const uint64_t dsz = APPROACH == APPROACH_LIST ? (uint64_t)g.cs * F : (uint64_t)(uint32_t)(F * g.cs);
+      lay->size_data = dsz;
+      lay->size_meta = diff_len - dsz;
+    }
+    if (ok) {
+      // header_t, include/utils.hpp:29-37
+      uint32_t* h32 = reinterpret_cast<uint32_t*>(diff);
+      h32[0] = g.sp->baseline_id;
+      h32[1] = cur;
+      h32[2] = (uint32_t)g.len;
+      h32[3] = (uint32_t)(g.len >> 32);
+      h32[4] = g.cs;
+      h32[5] = F;
+      h32[6] = P;
+      h32[7] = kMeta ? S : 0;
+    }
+  }
+  if (!kMeta) return;
+  // zero bytes that the reference leaves at zero when F != num_distinct
+  if (ok)
+    for (uint64_t b = 32 + 4ull * nd + 8ull * P + 8ull * S + tid; b < data_off; b += nt) diff[b] = 0;
+  if (!S) return;
+  // (checkpoint id, count) table in ascending id (src/tree_approach.cpp:657-665),
+  // each key's dense index, and the histogram cleared for the next checkpoint
+  uint32_t base = 0;
+  for (uint32_t b = 0; b < K; b += nt) {
+    const uint32_t k = b + tid;
+    const uint32_t h = k < K ? __ldcg(g.hist + k) : 0;
+    uint64_t t;
+    const uint32_t at = base + (uint32_t)block_excl_scan(h > 0 ? 1 : 0, sh, &t);
+    if (h > 0) {
+      if (ok) {
+        uint32_t* e = reinterpret_cast<uint32_t*>(diff + table_off + 8ull * at);
+        e[0] = k;
+        e[1] = h;
+      }
+      g.hist[k] = 0;
+    }
+    if (k < K) {
+      if (plain) {
+        g.rep[k] = at;
+      } else {
+        const double mul = (double)nbins / range;
+        const int bk = (int)(mul * (double)k);
+        uint32_t rep = k;
+        while (rep > 0 && (int)(mul * (double)(rep - 1)) == bk) rep--;
+        g.rep[k] = rep | (h > 0 ? 0x80000000u : 0u);
+        g.rank[k] = 0;
+      }
+    }
+    base += (uint32_t)t;
+  }
+  uint32_t nkeys = P;
+  if (!plain) {
+    // dense index of each representative that some present key maps to
+    __syncthreads();
+    for (uint32_t k = tid; k < K; k += nt)
+      if (g.rep[k] >> 31) g.rank[g.rep[k] & 0x7fffffffu] = 1;
+    __syncthreads();
+    nkeys = 0;
+    for (uint32_t b = 0; b < K; b += nt) {
+      const uint32_t k = b + tid;
+      const uint64_t v = k < K ? __ldcg(g.rank + k) : 0;
+      uint64_t t;
+      const uint64_t ex = block_excl_scan(v, sh, &t);
+      if (k < K) g.rank[k] = nkeys + (uint32_t)ex;
+      nkeys += (uint32_t)t;
+    }
+    __syncthreads();
+    for (uint32_t k = tid; k < K; k += nt)
+      if (g.rep[k] >> 31) g.rep[k] = __ldcg(g.rank + (g.rep[k] & 0x7fffffffu));
+  }
+  if (tid == 0) {
+    const uint32_t T = (S + kSortTile - 1) / kSortTile;
+    lay->nkeys = nkeys;
+    lay->sort_tiles = T;
+    lay->sort_n = nkeys * T;
+    if (nkeys > kSortFastKeys) atomicOr(g.err, DERR_SORTKEYS);
+  }
+}
+
+// Emits the roots in serial push order (the tile offset is the sum of the
+// earlier tiles' counts, or with kReduce false a scanned offset: a block that
+// scans them for the others takes 2-6 us longer), clears the flags, and looks up the tile's own roots: region sizes of the first
+// occurrences, prefixed within the tile, and (source checkpoint, source node)
+// of the shifted duplicates with a histogram of their sources (warp-aggregated:
+// most share a few).  The last block lays the diff out.
+template <int APPROACH, bool kReduce>
+__global__ void __launch_bounds__(kScanThreads) root_emit_kernel(GatherArgs g) {
   pdl_enter();
+  stamp(g.clk, CLK_ROOTS_DONE);
   __shared__ uint64_t sh[33];
+  __shared__ uint32_t s_last;
+  constexpr bool kTree = APPROACH == APPROACH_TREE;
+  const uint32_t tile = blockIdx.x, tid = threadIdx.x;
+  const uint64_t p = (uint64_t)tile * kRootTile + (uint64_t)tid * kRootPerThread;
+  uint32_t fo[4], shf[4];
+  const uint64_t c = load_kinds<APPROACH>(g.flags, p, g.n_flags, fo, shf);
   uint64_t off = 0;
   if (kReduce) {
     uint64_t part = 0;
-    for (uint32_t k = threadIdx.x; k < blockIdx.x; k += blockDim.x) part += tile_off[k];
+    for (uint32_t k = tid; k < tile; k += blockDim.x) part += g.tile_counts[k];
     block_excl_scan(part, sh, &off);
   } else {
-    off = tile_off[blockIdx.x];
+    off = g.tile_counts[tile];
   }
-  const uint64_t p = (uint64_t)blockIdx.x * kRootTile + (uint64_t)threadIdx.x * kRootPerThread;
-  uint4 v[kRootVec];
-  const uint64_t c = p < n ? load_flags(a.rflag, p, n, v) : 0;
-  uint64_t tile_total;
-  uint64_t ex = block_excl_scan(c, sh, &tile_total) + off;
-  const uint32_t root = lay->root_fo;
-  if (kReduce && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
-    lay->F = root + (uint32_t)(off + tile_total);
-    lay->S = (uint32_t)((off + tile_total) >> 32);
+  uint64_t total;
+  uint64_t ex = block_excl_scan(c, sh, &total) + off;
+  const uint32_t root = g.lay->root_fo;
+  if (tile == gridDim.x - 1 && tid == 0) {
+    g.lay->F = root + (uint32_t)(off + total);
+    g.lay->S = (uint32_t)((off + total) >> 32);
   }
-  if (!c) return;
-#pragma unroll
-  for (int k = 0; k < kRootVec; k++) {
+  if (c) {
     // cleared for the next checkpoint
-    if (v[k].x | v[k].y | v[k].z | v[k].w)
-      *reinterpret_cast<uint4*>(a.rflag + p + 16 * (uint64_t)k) = make_uint4(0, 0, 0, 0);
-    const uint32_t w4[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+    if (kTree) *reinterpret_cast<uint4*>(g.flags + p) = make_uint4(0, 0, 0, 0);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      uint32_t w = w4[j];
+    for (int q = 0; q < 4; q++) {
+      uint32_t w = fo[q] | shf[q];
       while (w) {
-        const int bit = __ffs(w) - 1;  // lowest set flag bit: byte order = serial order
-        const int byte = bit >> 3;
-        const uint8_t f = (uint8_t)(w >> (8 * byte));
-        const uint64_t pos = p + 16 * (uint64_t)k + 4 * j + byte;
-        if (f == ROOT_FO) { fo_list[root + (uint32_t)ex] = node_at(a, pos); ex += 1; }
-        else { sh_list[(uint32_t)(ex >> 32)] = node_at(a, pos); ex += 1ull << 32; }
-        w &= ~(0xffu << (8 * byte));
+        const int bit = __ffs(w) - 1;  // byte order = serial order
+        const uint64_t pos = p + 4 * q + (bit >> 3);
+        const uint32_t id = kTree ? node_at(g.order, pos) : (uint32_t)pos;
+        if ((fo[q] >> bit) & 1) { g.fo_list[root + (uint32_t)ex] = id; ex += 1; }
+        else { g.sh_list[(uint32_t)(ex >> 32)] = id; ex += 1ull << 32; }
+        w &= w - 1;
       }
     }
   }
-}
-
-__global__ void root_epilogue_kernel(const uint64_t* total, Layout* lay) {
-  pdl_enter();
-  lay->F = lay->root_fo + (uint32_t)(*total);
-  lay->S = (uint32_t)(*total >> 32);
+  __syncthreads();
+  const uint32_t cur = g.sp->cur;
+  if (kTree) {
+    // the tile's first occurrences, the root ahead of tile 0's
+    const bool fused = g.fuse_gate && *g.fuse_gate == 0;
+    const uint32_t f0 = tile == 0 ? 0 : root + (uint32_t)off, f1 = root + (uint32_t)off + (uint32_t)total;
+    uint64_t carry = 0;
+    for (uint32_t b = f0; b < f1; b += blockDim.x) {
+      const uint32_t i = b + tid;
+      const uint64_t v = i < f1 ? fo_region(g, g.fo_list[i], fused, cur) : 0;
+      uint64_t t;
+      const uint64_t before = carry + block_excl_scan(v, sh, &t);
+      if (i < f1) {
+        g.fo_val[i] = before | (v ? 1ull << 63 : 0);
+        g.fo_tile[i] = tile;
+      }
+      carry += t;
+    }
+    if (tid == 0) g.tile_regions[tile] = carry;
+  }
+  if (APPROACH != APPROACH_BASIC) {
+    const uint32_t s0 = (uint32_t)(off >> 32), s1 = s0 + (uint32_t)(total >> 32);
+    const uint32_t lane = tid & 31;
+    for (uint32_t b = s0; b < s1; b += blockDim.x) {
+      const uint32_t i = b + tid;
+      uint32_t key = 0xffffffffu;
+      if (i < s1) {
+        const int64_t slot = map_find(g.map, ld_digest(g.digests + g.sh_list[i]), g.err);
+        NodeIdDev prev = slot_value(g.map, slot);
+        if (slot < 0 || prev.tree > cur) { atomicOr(g.err, DERR_MISSING); prev.tree = 0; prev.node = 0; }
+        g.sh_key[i] = prev.tree;
+        g.sh_prev[i] = prev.node;
+        key = prev.tree;
+      }
+      const uint32_t peers = __match_any_sync(0xffffffffu, key);
+      if (key != 0xffffffffu && lane == (uint32_t)(__ffs(peers) - 1)) atomicAdd(&g.hist[key], (uint32_t)__popc(peers));
+    }
+  }
+  if (last_block(g.counters + COUNT_ROOTS_DONE, gridDim.x, &s_last)) build_layout<APPROACH>(g, gridDim.x, sh);
 }
 
 // ---------------------------------------------------------------------------
 // Diff assembly
 // ---------------------------------------------------------------------------
-// First-occurrence roots: region size if the root owns its digest.
-__device__ __forceinline__ void fo_prep(const GatherArgs& g) {
+// First-occurrence entries: metadata and regions, by entry.
+__device__ __forceinline__ void emit_regions(const GatherArgs& g, uint32_t blk, uint32_t nblk) {
   const uint32_t F = g.lay->F;
-  const uint32_t cur = g.sp->cur;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < F; i += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t node = g.fo_list[i];
-    uint64_t v = 0;
-    if (g.approach == APPROACH_TREE) {
-      // a first-occurrence leaf owns its digest: the leaf pass demotes every
-      // other one (same checkpoint id, another owner)
-      bool owner = node >= g.N - 1;
-      if (!owner) {
-        NodeIdDev prev = slot_value(g.map, map_find(g.map, ld_digest(g.digests + node), g.err));
-        owner = prev.node == node && prev.tree == cur;
-      }
-      if (owner) v = (1ull << 32) | num_leaf_descendents(node, g.M);
-    } else {
-      v = (1ull << 32) | 1ull;  // list / basic: one chunk per entry
-    }
-    g.fo_val[i] = v;
-  }
-}
-struct FoEmit {
-  GatherArgs g;
-  __device__ __forceinline__ void operator()(uint64_t i, uint64_t ex, uint64_t v) const {
-    if (!(v >> 32)) return;
-    const uint32_t r = (uint32_t)(ex >> 32);
+  const bool ok = g.lay->ok;
+  uint8_t* meta = g.stage + g.lay->pad + 32;
+  for (uint64_t i = (uint64_t)blk * blockDim.x + threadIdx.x; i < F; i += (uint64_t)nblk * blockDim.x) {
     const uint32_t node = g.fo_list[i];
-    g.reg_slot[r] = (uint32_t)ex;
-    g.reg_len[r] = (uint32_t)v;
-    g.reg_chunk[r] = g.approach == APPROACH_TREE ? leftmost_leaf(node, g.M) - (g.N - 1) : node;
-    // FO metadata: node ids (tree) or chunk ids (list, basic), 4-byte aligned
-    if (g.lay->ok) *reinterpret_cast<uint32_t*>(g.stage + g.lay->pad + 32 + 4ull * r) = node;
-  }
-};
-
-// Region sizes scanned with one first-occurrence root per thread (tiles of
-// kFoTile) over a persistent grid: the tile count follows F on the device.
-constexpr uint32_t kFoTile = kScanThreads;
-__global__ void __launch_bounds__(kScanThreads) fo_tile_sums_kernel(GatherArgs g) {
-  pdl_enter();
-  __shared__ uint64_t sh[33];
-  const uint32_t F = g.lay->F;
-  const uint32_t nt = (F + kFoTile - 1) / kFoTile;
-  for (uint32_t t = blockIdx.x; t < nt; t += gridDim.x) {
-    const uint32_t i = t * kFoTile + threadIdx.x;
-    uint64_t total;
-    block_excl_scan(i < F ? g.fo_val[i] : 0, sh, &total);
-    if (threadIdx.x == 0) g.scan_scratch[t] = total;
-  }
-}
-__global__ void __launch_bounds__(kScanThreads) fo_emit_kernel(GatherArgs g) {
-  pdl_enter();
-  __shared__ uint64_t sh[33];
-  const uint32_t F = g.lay->F;
-  const uint32_t nt = (F + kFoTile - 1) / kFoTile;
-  const FoEmit emit{g};
-  for (uint32_t t = blockIdx.x; t < nt; t += gridDim.x) {
-    const uint32_t i = t * kFoTile + threadIdx.x;
-    const uint64_t v = i < F ? g.fo_val[i] : 0;
-    const uint64_t ex = block_excl_scan(v, sh, nullptr) + g.scan_scratch[t];
-    if (i < F) emit(i, ex, v);
-  }
-}
-
-// Shifted duplicates: (source checkpoint, source node) of each root.
-// The histogram of source checkpoints is warp-aggregated: most entries share
-// a few keys.
-__device__ __forceinline__ void shift_prep(const GatherArgs& g) {
-  const uint32_t S = g.lay->S;
-  const uint32_t cur = g.sp->cur;
-  const uint32_t lane = threadIdx.x & 31;
-  for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x; b < S; b += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t i = b + threadIdx.x;
-    uint32_t key = 0xffffffffu;
-    if (i < S) {
-      uint32_t node = g.sh_list[i];
-      int64_t slot = map_find(g.map, ld_digest(g.digests + node), g.err);
-      NodeIdDev prev = slot_value(g.map, slot);
-      if (slot < 0 || prev.tree > cur) { atomicOr(g.err, DERR_MISSING); prev.tree = 0; prev.node = 0; }
-      g.sh_key[i] = prev.tree;
-      g.sh_prev[i] = prev.node;
-      key = prev.tree;
-    }
-    const uint32_t peers = __match_any_sync(0xffffffffu, key);
-    if (key != 0xffffffffu && lane == (uint32_t)(__ffs(peers) - 1)) atomicAdd(&g.hist[key], (uint32_t)__popc(peers));
-  }
-}
-
-// Both root lists' lookups in one launch.
-__global__ void roots_prep_kernel(GatherArgs g) {
-  pdl_enter();
-  stamp(g.clk, CLK_ROOTS_DONE);
-  shift_prep(g);
-  fo_prep(g);
-}
-
-// One block: repeat-count table, layout, header; bin representatives for the
-// list approach's BinOp1D.
-// First, the tile sums of the region-size scan become tile offsets in place,
-// and their total gives the region count and the data chunk count.
-__global__ void layout_kernel(GatherArgs g) {
-  pdl_enter();
-  __shared__ uint64_t sh[33];
-  Layout* lay = g.lay;
-  {
-    const uint32_t ntiles = (lay->F + kFoTile - 1) / kFoTile;
-    uint64_t carry = 0;
-    for (uint32_t b = 0; b < ntiles; b += blockDim.x) {
-      const uint32_t i = b + threadIdx.x;
-      const uint64_t v = i < ntiles ? g.scan_scratch[i] : 0;
-      uint64_t t;
-      const uint64_t ex = block_excl_scan(v, sh, &t);
-      if (i < ntiles) g.scan_scratch[i] = carry + ex;
-      carry += t;
-    }
-    if (threadIdx.x == 0) {
-      lay->num_distinct = (uint32_t)(carry >> 32);
-      lay->chunk_counter = (uint32_t)carry;
-    }
-    __syncthreads();
-  }
-  const uint32_t cur = g.sp->cur;
-  const uint32_t K = cur + 1;
-  const uint32_t F = lay->F, S = lay->S, nd = lay->num_distinct;
-  // P = number of source checkpoints that occur; max_key = largest of them
-  __shared__ uint32_t smax;
-  if (threadIdx.x == 0) {
-    smax = 0;
-    lay->nkeys = 0;  // set below once the keys are known
-    lay->sort_n = 0;
-    lay->sort_tiles = 0;
-  }
-  __syncthreads();
-  uint32_t P = 0;
-  for (uint32_t b = 0; b < K; b += blockDim.x) {
-    uint32_t k = b + threadIdx.x;
-    uint64_t nz = (k < K && g.hist[k] > 0) ? 1 : 0;
-    uint64_t t;
-    block_excl_scan(nz, sh, &t);
-    P += (uint32_t)t;
-    if (nz) atomicMax(&smax, k);
-  }
-  __syncthreads();
-  const uint32_t max_key = smax;
-  const uint64_t fo_off = 32;
-  const uint64_t meta_meta = g.approach == APPROACH_BASIC ? 0 : 1;
-  const uint64_t data_off = fo_off + 4ull * F + meta_meta * (8ull * P + 8ull * S);
-  const uint64_t pad = (16 - (data_off & 15)) & 15;
-  const uint64_t data_len_bytes = (uint64_t)lay->chunk_counter * g.cs;
-  uint64_t diff_len = data_off + data_len_bytes;
-  if (threadIdx.x == 0) {
-    lay->P = meta_meta ? P : 0;
-    lay->pad = pad;
-    lay->data_off = data_off;
-    lay->table_off = fo_off + 4ull * nd;
-    lay->pairs_off = fo_off + 4ull * nd + 8ull * P;
-    if (pad + diff_len > g.stage_cap) {
-      atomicOr(g.err, DERR_CAPACITY);
-      lay->diff_len = 0;
-      lay->ok = 0;
-    } else {
-      lay->diff_len = diff_len;
-      lay->ok = 1;
-    }
-    // datasizes as the reference's collect_diff returns them
+    uint32_t r = (uint32_t)i, slot = (uint32_t)i, chunk = node;
     if (g.approach == APPROACH_TREE) {
-      uint64_t meta = 4ull * F + 8ull * P + 8ull * S;
-      lay->size_data = diff_len - meta;  // src/tree_approach.cpp:707-709
-      lay->size_meta = meta;
-    } else if (g.approach == APPROACH_LIST) {
-      uint64_t dsz = (uint64_t)g.cs * F;  // src/list_approach.cpp:241-246
-      lay->size_data = dsz;
-      lay->size_meta = diff_len - dsz;
-    } else {
-      uint32_t dsz = F * g.cs;  // src/basic_approach.cpp:141-142 (32-bit product)
-      lay->size_data = dsz;
-      lay->size_meta = diff_len - dsz;
+      const uint64_t v = g.fo_val[i];
+      if (!(v >> 63)) continue;
+      const uint64_t ex = (v & ~(1ull << 63)) + g.tile_regions[g.fo_tile[i]];
+      r = (uint32_t)(ex >> 32);
+      slot = (uint32_t)ex;
+      chunk = leftmost_leaf(node, g.M) - (g.N - 1);
     }
-  }
-  __syncthreads();
-  if (!lay->ok) {
-    for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) g.hist[k] = 0;
-    return;
-  }
-  uint8_t* diff = g.stage + pad;
-  if (threadIdx.x == 0) {
-    // header_t, include/utils.hpp:29-37
-    uint32_t* h32 = reinterpret_cast<uint32_t*>(diff);
-    h32[0] = g.sp->baseline_id;
-    h32[1] = cur;
-    h32[2] = (uint32_t)g.len;
-    h32[3] = (uint32_t)(g.len >> 32);
-    h32[4] = g.cs;
-    h32[5] = F;
-    h32[6] = meta_meta ? P : 0;
-    h32[7] = meta_meta ? S : 0;
-  }
-  if (!meta_meta) return;
-  // zero bytes that the reference leaves at zero when F != num_distinct
-  for (uint64_t b = 32 + 4ull * nd + 8ull * P + 8ull * S + threadIdx.x; b < data_off; b += blockDim.x) diff[b] = 0;
-  // (checkpoint id, count) table in ascending id (src/tree_approach.cpp:657-665)
-  uint32_t base = 0;
-  for (uint32_t b = 0; b < K; b += blockDim.x) {
-    uint32_t k = b + threadIdx.x;
-    uint64_t nz = (k < K && g.hist[k] > 0) ? 1 : 0;
-    uint64_t t;
-    uint64_t ex = block_excl_scan(nz, sh, &t);
-    if (nz) {
-      uint32_t* e = reinterpret_cast<uint32_t*>(diff + lay->table_off + 8ull * (base + ex));
-      e[0] = k;
-      e[1] = g.hist[k];
-    }
-    base += (uint32_t)t;
-  }
-  // sort representative of each key: stable sort by BinOp1D bin equals stable
-  // sort by the smallest key sharing the bin
-  const uint32_t nbins = g.approach == APPROACH_TREE ? cur : S;
-  const double range = (double)(g.approach == APPROACH_TREE ? cur : max_key);
-  const double mul = (range <= (double)nbins) ? 1.0 : (double)nbins / range;
-  for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) {
-    int bk = (int)(mul * (double)k);
-    uint32_t rep = k;
-    while (rep > 0 && (int)(mul * (double)(rep - 1)) == bk) rep--;
-    g.rep[k] = rep;
-    g.rank[k] = 0;
-  }
-  __syncthreads();
-  // dense index of each representative that some present key maps to
-  for (uint32_t k = threadIdx.x; k < K; k += blockDim.x)
-    if (g.hist[k] > 0) g.rank[g.rep[k]] = 1;
-  __syncthreads();
-  uint32_t run = 0;
-  for (uint32_t b0 = 0; b0 < K; b0 += blockDim.x) {
-    uint32_t k = b0 + threadIdx.x;
-    uint64_t v = k < K ? g.rank[k] : 0;
-    uint64_t t;
-    uint64_t ex = block_excl_scan(v, sh, &t);
-    if (k < K) g.rank[k] = run + (uint32_t)ex;
-    run += (uint32_t)t;
-  }
-  __syncthreads();
-  for (uint32_t k = threadIdx.x; k < K; k += blockDim.x)
-    if (g.hist[k] > 0) {
-      g.rep[k] = g.rank[g.rep[k]];
-      g.hist[k] = 0;  // for the next checkpoint
-    }
-  if (threadIdx.x == 0) {
-    lay->nkeys = run;
-    const uint32_t T = (S + kSortTile - 1) / kSortTile;
-    lay->sort_tiles = T;
-    lay->sort_n = run * T;
-    if (run > kSortFastKeys) atomicOr(g.err, DERR_SORTKEYS);
+    g.reg_slot[r] = slot;
+    g.reg_chunk[r] = chunk;
+    // FO metadata: node ids (tree) or chunk ids (list, basic), 4-byte aligned
+    if (ok) *reinterpret_cast<uint32_t*>(meta + 4ull * r) = node;
   }
 }
 
 // Stable counting sort of the shift entries by representative key.
 // Tile t counts its keys; matrix[key * T + t] (key-major).
-__global__ void sort_count_kernel(GatherArgs g) {
-  pdl_enter();
-  extern __shared__ uint32_t cnt[];
+__device__ __forceinline__ void sort_count(const GatherArgs& g, uint32_t blk, uint32_t nblk, uint32_t* cnt) {
   const uint32_t K = g.lay->nkeys, S = g.lay->S, T = g.lay->sort_tiles;
   if (K > kSortFastKeys) return;
-  for (uint32_t t = blockIdx.x; t < T; t += gridDim.x) {
+  for (uint32_t t = blk; t < T; t += nblk) {
     for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) cnt[k] = 0;
     __syncthreads();
     const uint64_t b = (uint64_t)t * kSortTile;
@@ -1056,6 +1055,25 @@ __global__ void sort_count_kernel(GatherArgs g) {
     __syncthreads();
   }
 }
+
+// Metadata and regions (the first n_emit blocks) beside the sort's counts (the
+// others, whose last block turns the counts into positions unless the matrix
+// is large: sort_scan false).
+__global__ void __launch_bounds__(256) emit_count_kernel(GatherArgs g) {
+  pdl_enter();
+  extern __shared__ uint32_t cnt[];
+  __shared__ uint64_t sh[33];
+  __shared__ uint32_t s_last;
+  if (blockIdx.x < g.n_emit) {
+    emit_regions(g, blockIdx.x, g.n_emit);
+    return;
+  }
+  const uint32_t nblk = gridDim.x - g.n_emit;
+  sort_count(g, blockIdx.x - g.n_emit, nblk, cnt);
+  if (g.sort_scan && last_block(g.counters + COUNT_SORT_DONE, nblk, &s_last) && g.lay->nkeys <= kSortFastKeys)
+    scan_in_place(g.sort_mat, g.lay->sort_n, sh);
+}
+
 struct MatVal {
   const uint64_t* m;
   __device__ __forceinline__ uint64_t operator()(uint64_t i) const { return m[i]; }
@@ -1069,17 +1087,18 @@ struct MatEmit {
 // memory), then the per-key counts of earlier warps and the tile's global
 // base (key-major scan of sort_mat) give each entry its position.
 constexpr int kSortWarps = 8;
-__global__ void __launch_bounds__(256) sort_scatter_kernel(GatherArgs g) {
-  pdl_enter();
-  __shared__ uint32_t keys[kSortTile];
-  __shared__ uint32_t lrank[kSortTile];
-  extern __shared__ uint32_t cnt[];  // [kSortWarps][K]
+struct SortShared {
+  uint16_t keys[kSortTile], lrank[kSortTile];
+};
+static_assert(kSortFastKeys <= 0x10000 && kSortTile <= 0x10000, "keys and ranks kept in 16 bits");
+__device__ __forceinline__ void sort_scatter(const GatherArgs& g, uint32_t blk, uint32_t nblk, SortShared& sm,
+                                             uint32_t* cnt) {  // cnt: [kSortWarps][K]
   const uint32_t K = g.lay->nkeys, S = g.lay->S, T = g.lay->sort_tiles;
   if (!g.lay->ok || K > kSortFastKeys) return;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr uint32_t kSlice = kSortTile / kSortWarps;
   uint8_t* pairs = g.stage + g.lay->pad + g.lay->pairs_off;
-  for (uint32_t t = blockIdx.x; t < T; t += gridDim.x) {
+  for (uint32_t t = blk; t < T; t += nblk) {
     const uint64_t b = (uint64_t)t * kSortTile;
     if (b >= S) break;
     const uint32_t n = (uint32_t)(S - b < kSortTile ? S - b : kSortTile);
@@ -1094,7 +1113,7 @@ __global__ void __launch_bounds__(256) sort_scatter_kernel(GatherArgs g) {
 #pragma unroll
       for (int j = 0; j < kPer; j++) {
         const uint32_t i = threadIdx.x + 256u * j;
-        if (i < n) keys[i] = g.rep[kk[j]];
+        if (i < n) sm.keys[i] = (uint16_t)g.rep[kk[j]];
       }
     }
     for (uint32_t k = threadIdx.x; k < kSortWarps * K; k += blockDim.x) cnt[k] = 0;
@@ -1103,13 +1122,13 @@ __global__ void __launch_bounds__(256) sort_scatter_kernel(GatherArgs g) {
     for (uint32_t i0 = warp * kSlice; i0 < (warp + 1) * kSlice && i0 < n; i0 += 32) {
       const uint32_t i = i0 + lane;
       const bool v = i < n && i < (warp + 1) * kSlice;
-      const uint32_t key = v ? keys[i] : 0xffffffffu;
+      const uint32_t key = v ? sm.keys[i] : 0xffffffffu;
       const uint32_t peers = __match_any_sync(0xffffffffu, key);
       const uint32_t rank = __popc(peers & ((1u << lane) - 1));
       uint32_t base = v ? wc[key] : 0;
       __syncwarp();
       if (v) {
-        lrank[i] = base + rank;
+        sm.lrank[i] = (uint16_t)(base + rank);
         if (lane == (uint32_t)(__ffs(peers) - 1)) wc[key] = base + __popc(peers);
       }
       __syncwarp();
@@ -1136,7 +1155,7 @@ __global__ void __launch_bounds__(256) sort_scatter_kernel(GatherArgs g) {
       for (int j = 0; j < kPer; j++) {
         const uint32_t i = threadIdx.x + 256u * j;
         if (i >= n) continue;
-        const uint32_t pos = cnt[(i / kSlice) * K + keys[i]] + lrank[i];
+        const uint32_t pos = cnt[(i / kSlice) * K + sm.keys[i]] + sm.lrank[i];
         uint32_t* e = reinterpret_cast<uint32_t*>(pairs + 8ull * pos);  // 4-byte aligned only
         e[0] = nd[j];
         e[1] = pv[j];
@@ -1183,16 +1202,20 @@ __device__ __forceinline__ uint32_t bytes_below(int n, int q) {
 // per unit.  Otherwise a unit is cut out of the aligned words around each of
 // its pieces (one piece, or two where it crosses into a slot of another
 // region; more only for chunks shorter than 16 bytes).
+struct CopyShared {
+  uint32_t rs[kCopySlots + 1], rc[kCopySlots + 1], ch[kCopySlots];
+  uint32_t r;     // region of the tile's first slot
+  uint32_t j[2];  // region (from the tile's first) of the last slot, of the slot after it
+};
 template <bool kVec>
-__global__ void __launch_bounds__(256) copy_kernel(GatherArgs g) {
-  pdl_enter();
+__device__ __forceinline__ void copy_tiles(const GatherArgs& g, uint32_t blk, uint32_t nblk, CopyShared& sm) {
   if (!g.lay->ok) return;
   const uint32_t R = g.lay->num_distinct;
   const uint64_t nslots = g.lay->chunk_counter;
   if (R == 0 || nslots == 0) return;
-  __shared__ uint32_t rs[kCopySlots + 1], rc[kCopySlots + 1], ch[kCopySlots];
-  __shared__ uint32_t s_r;      // region of the tile's first slot
-  __shared__ uint32_t s_j[2];   // region (from the tile's first) of the last slot, of the slot after it
+  uint32_t* rs = sm.rs;
+  uint32_t* rc = sm.rc;
+  uint32_t* ch = sm.ch;
   uint8_t* dst = g.stage + g.lay->pad + g.lay->data_off;
   const uint64_t cs = g.cs;
   const uint32_t tid = threadIdx.x;
@@ -1200,8 +1223,8 @@ __global__ void __launch_bounds__(256) copy_kernel(GatherArgs g) {
   const uint64_t nunits = (nbytes + 15) / 16;
   const uint32_t ut = cs >= 128 ? kCopyTileUnits : 16 * (uint32_t)cs;
   const uint64_t ntiles = (nunits + ut - 1) / ut;
-  const uint64_t per_block = (ntiles + gridDim.x - 1) / gridDim.x;
-  const uint64_t tile0 = (uint64_t)blockIdx.x * per_block;
+  const uint64_t per_block = (ntiles + nblk - 1) / nblk;
+  const uint64_t tile0 = (uint64_t)blk * per_block;
   const uint64_t tile1 = tile0 + per_block < ntiles ? tile0 + per_block : ntiles;
   if (tile0 >= tile1) return;
   const int lg = (cs & (cs - 1)) == 0 ? __ffsll((long long)cs) - 1 : -1;
@@ -1223,7 +1246,7 @@ __global__ void __launch_bounds__(256) copy_kernel(GatherArgs g) {
       lo += (31 - __clz(b)) * step;
       if ((uint64_t)lo + step - 1 < hi) hi = lo + step - 1;
     }
-    if (tid == 0) s_r = lo;
+    if (tid == 0) sm.r = lo;
   }
   __syncthreads();
   for (uint64_t tile = tile0; tile < tile1; tile++) {
@@ -1233,7 +1256,7 @@ __global__ void __launch_bounds__(256) copy_kernel(GatherArgs g) {
     const uint32_t s0 = (uint32_t)(lg >= 0 ? b0 >> lg : b0 / cs);
     const uint64_t rel = b0 - s0 * cs;
     const uint32_t ns = slot_of(rel + (b1 - 1 - b0)) + 1;
-    const uint32_t r0 = s_r;
+    const uint32_t r0 = sm.r;
     const uint32_t m = R - r0 < ns + 1 ? R - r0 : ns + 1;
     for (uint32_t i = tid; i < m; i += 256) {
       rs[i] = g.reg_slot[r0 + i];
@@ -1247,11 +1270,11 @@ __global__ void __launch_bounds__(256) copy_kernel(GatherArgs g) {
         if (rs[mid] <= s0 + i) lo = mid; else hi = mid - 1;
       }
       if (i < ns) ch[i] = rc[lo] + (s0 + i - rs[lo]);
-      if (i + 1 >= ns) s_j[i + 1 - ns] = lo;
+      if (i + 1 >= ns) sm.j[i + 1 - ns] = lo;
     }
     __syncthreads();
     // the next tile starts in this tile's last slot, or in the one after it
-    if (tid == 0) s_r = r0 + s_j[rel + (b1 - b0) >= ns * cs ? 1 : 0];
+    if (tid == 0) sm.r = r0 + sm.j[rel + (b1 - b0) >= ns * cs ? 1 : 0];
     uint4* out = reinterpret_cast<uint4*>(dst) + u0;
     for (uint32_t k0 = tid; k0 < nu; k0 += 256 * kCopyPer) {
       uint4 v[kCopyPer];
@@ -1318,30 +1341,34 @@ __global__ void __launch_bounds__(256) copy_kernel(GatherArgs g) {
   }
 }
 
-// list / basic: flags over chunks -> ascending FO (changed) and SHIFT lists
-struct ChunkVal {
-  const uint8_t* labels;
-  int basic;
-  __device__ __forceinline__ uint64_t operator()(uint64_t c) const {
-    uint8_t l = labels[c];
-    if (basic) return l ? 1ull : 0ull;
-    return (l == FIRST_OCUR ? 1ull : 0ull) | (l == SHIFT_DUPL ? (1ull << 32) : 0ull);
-  }
-};
-struct ChunkEmit {
-  uint32_t* fo_list;
-  uint32_t* sh_list;
-  __device__ __forceinline__ void operator()(uint64_t c, uint64_t ex, uint64_t v) const {
-    if (v & 1ull) fo_list[(uint32_t)ex] = (uint32_t)c;
-    if (v >> 32) sh_list[(uint32_t)(ex >> 32)] = (uint32_t)c;
-  }
-};
-__global__ void chunk_totals_kernel(const uint64_t* total, Layout* lay, uint64_t* clk) {
+// The gather of a whole checkpoint, a block per tile, in a launch of its own:
+// counting 2^17 finished blocks (below) would cost more than the launch.
+template <bool kVec>
+__global__ void __launch_bounds__(256, 5) copy_kernel(GatherArgs g) {
   pdl_enter();
-  stamp(clk, CLK_LEAVES_DONE);
-  lay->root_fo = 0;
-  lay->F = (uint32_t)(*total);
-  lay->S = (uint32_t)(*total >> 32);
+  __shared__ CopyShared sm;
+  copy_tiles<kVec>(g, blockIdx.x, gridDim.x, sm);
+}
+
+// The rest of a checkpoint in one launch, by block: the sorted shift entries
+// (n_sort blocks), the map inserts a fused forest pass has queued (n_drain:
+// only later checkpoints read them, and the copy hides their random accesses),
+// the chunk gather (the others).  The last block to finish writes the results
+// to pinned host memory.
+template <bool kVec>
+__global__ void __launch_bounds__(256, 5) final_kernel(GatherArgs g) {
+  pdl_enter();
+  extern __shared__ uint32_t cnt[];
+  __shared__ union {
+    SortShared sort;
+    CopyShared copy;
+  } sm;
+  __shared__ uint32_t s_last;
+  const uint32_t blk = blockIdx.x;
+  if (blk < g.n_sort) sort_scatter(g, blk, g.n_sort, sm.sort, cnt);
+  else if (blk < g.n_sort + g.n_drain) drain_inserts(g, blk - g.n_sort, g.n_drain);
+  else if (g.n_copy) copy_tiles<kVec>(g, blk - g.n_sort - g.n_drain, g.n_copy, sm.copy);
+  if (last_block(g.counters + COUNT_FINAL_DONE, gridDim.x, &s_last)) readback(g.results);
 }
 
 // Entries of a table moved into a larger one (keys are stored already
@@ -1424,88 +1451,70 @@ cudaError_t launch_forest(const ForestArgs& a, int pass, int baseline, uint32_t 
   return cudaGetLastError();
 }
 
-cudaError_t launch_root_compaction(const ForestArgs& fa, uint32_t N, uint32_t M, uint32_t* fo_list,
-                                   uint32_t* sh_list, Layout* lay, uint64_t* scan_scratch, uint64_t* scan_total,
-                                   cudaStream_t s) {
-  const uint64_t n = (uint64_t)M - 1;  // every node but the root
-  uint32_t ntiles = (uint32_t)((n + kRootTile - 1) / kRootTile);
-  if (ntiles == 0) ntiles = 1;
-  const uint32_t nd = 2 * num_sms();
-  launch_k(root_count_kernel, ntiles + nd, kScanThreads, 0, s, fa, N, n, scan_scratch, fo_list, lay, nd);
-  if (ntiles <= reduce_tile_limit()) {
-    launch_k(root_emit_kernel<true>, ntiles, kScanThreads, 0, s, fa, n, scan_scratch, fo_list, sh_list, lay);
-    note_launch(2);
-    return cudaGetLastError();
+cudaError_t launch_assemble(GatherArgs g, uint64_t max_entries, bool whole, cudaStream_t s) {
+  const uint32_t tiles = (uint32_t)std::max<uint64_t>(1, (g.n_flags + kRootTile - 1) / kRootTile);
+  const bool reduce = tiles <= std::min<uint32_t>(kRootReduceTiles, 2 * reduce_tile_limit());
+  const bool tree = g.approach == APPROACH_TREE, basic = g.approach == APPROACH_BASIC;
+  auto count = tree ? root_count_kernel<APPROACH_TREE>
+               : basic ? root_count_kernel<APPROACH_BASIC> : root_count_kernel<APPROACH_LIST>;
+  auto emit = tree ? (reduce ? root_emit_kernel<APPROACH_TREE, true> : root_emit_kernel<APPROACH_TREE, false>)
+              : basic ? (reduce ? root_emit_kernel<APPROACH_BASIC, true> : root_emit_kernel<APPROACH_BASIC, false>)
+                      : (reduce ? root_emit_kernel<APPROACH_LIST, true> : root_emit_kernel<APPROACH_LIST, false>);
+  launch_k(count, tiles, kScanThreads, 0, s, g);
+  if (!reduce) {
+    launch_k(scan_tile_offsets_kernel, 1, 1024, 0, s, g.tile_counts, tiles, (uint64_t*)nullptr);
+    note_launch();
   }
-  launch_k(scan_tile_offsets_kernel, 1, 1024, 0, s, scan_scratch, ntiles, scan_total);
-  launch_k(root_emit_kernel<false>, ntiles, kScanThreads, 0, s, fa, n, scan_scratch, fo_list, sh_list, lay);
-  launch_k(root_epilogue_kernel, 1, 1, 0, s, scan_total, lay);
-  note_launch(4);
-  return cudaGetLastError();
-}
+  launch_k(emit, tiles, kScanThreads, 0, s, g);
 
-cudaError_t launch_chunk_compaction(const uint8_t* labels, uint32_t n_chunks, int basic, uint32_t* fo_list,
-                                    uint32_t* sh_list, Layout* lay, uint64_t* scan_scratch, uint64_t* scan_total,
-                                    uint64_t* clk, cudaStream_t s) {
-  cudaError_t e = grid_scan(ChunkVal{labels, basic}, ChunkEmit{fo_list, sh_list}, nullptr, n_chunks, scan_scratch,
-                            scan_total, s);
-  if (e != cudaSuccess) return e;
-  launch_k(chunk_totals_kernel, 1, 1, 0, s, scan_total, lay, basic ? clk : nullptr);
-  note_launch();
-  return cudaGetLastError();
-}
-
-cudaError_t launch_assemble(const GatherArgs& g, uint64_t max_entries, bool whole, cudaStream_t s) {
-  cudaError_t e;
-  // the FO metadata is written while scanning, so the pad must be known first:
-  // pad depends on F, P, S; P needs the histogram.  Order: shift prep
-  // (histogram), FO prep + scan (region sizes), layout (pad, table, header),
-  // FO emit (metadata + regions), sort, copy.
-  const uint32_t gs = grid_for(max_entries, 256);
-  launch_k(roots_prep_kernel, gs, 256, 0, s, g);
-  // region totals first (phase 1+2 of the scan), then layout, then emit
-  const uint32_t gfo = (uint32_t)std::min<uint64_t>((max_entries + kFoTile - 1) / kFoTile + 1, 4ull * num_sms());
-  launch_k(fo_tile_sums_kernel, gfo, kScanThreads, 0, s, g);
-  launch_k(layout_kernel, 1, 1024, 0, s, g);
-  launch_k(fo_emit_kernel, gfo, kScanThreads, 0, s, g);
-  note_launch(4);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if (g.approach != APPROACH_BASIC) {
-    // bound on the distinct keys (source checkpoints): at most k_cap, which
-    // covers every checkpoint id that this launch sequence can see
-    const uint32_t K = std::min<uint32_t>(g.k_cap, kSortFastKeys);
-    const uint32_t T = (uint32_t)((max_entries + kSortTile - 1) / kSortTile) + 1;
-    const size_t smem_cnt = sizeof(uint32_t) * (size_t)K;
-    const size_t smem_sc = sizeof(uint32_t) * (size_t)K * kSortWarps;
-    static size_t attr_sc = 0;
-    if (smem_sc > 16 * 1024 && smem_sc > attr_sc) {
-      cudaFuncSetAttribute(sort_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_sc);
-      attr_sc = smem_sc;
-    }
-    // tiles of the actual shift entries, read on the device: small grids
-    const uint32_t gsort = std::min<uint32_t>(T, 2 * num_sms());
-    launch_k(sort_count_kernel, gsort, 256, smem_cnt, s, g);
-    e = grid_scan(MatVal{g.sort_mat}, MatEmit{g.sort_mat}, &g.lay->sort_n, (uint64_t)K * T, g.scan_scratch2,
-                  g.scan_total2, s);
+  // metadata, regions, and the sort's counts.  Bound on the distinct keys
+  // (source checkpoints): at most k_cap, which covers every checkpoint id that
+  // this launch sequence can see
+  const uint32_t K = std::min<uint32_t>(g.k_cap, kSortFastKeys);
+  const uint32_t T = (uint32_t)((max_entries + kSortTile - 1) / kSortTile) + 1;
+  g.n_emit = (uint32_t)std::min<uint64_t>((max_entries + 255) / 256, 4ull * num_sms());
+  // tiles of the actual shift entries, read on the device: small grids
+  g.n_sort = basic ? 0 : std::min<uint32_t>(T, 2 * num_sms());
+  // one block scans the counts of all tiles; for larger matrices two launches
+  // over the whole GPU
+  g.sort_scan = (uint64_t)K * T <= (1u << 18) ? 1 : 0;
+  launch_k(emit_count_kernel, g.n_emit + g.n_sort, 256, basic ? 0 : sizeof(uint32_t) * (size_t)K, s, g);
+  note_launch(3);
+  if (!basic && !g.sort_scan) {
+    cudaError_t e = grid_scan(MatVal{g.sort_mat}, MatEmit{g.sort_mat}, &g.lay->sort_n, (uint64_t)K * T, g.scan_scratch2,
+                              g.scan_total2, s);
     if (e != cudaSuccess) return e;
-    launch_k(sort_scatter_kernel, gsort, 256, smem_sc, s, g);
-    note_launch(2);
   }
+
   const bool vec = (g.cs % 16 == 0) && ((reinterpret_cast<uintptr_t>(g.data) & 15) == 0);
-  static const bool reg = (register_input_kernel(reinterpret_cast<const void*>(copy_kernel<true>), INPUT_GATHER),
-                           register_input_kernel(reinterpret_cast<const void*>(copy_kernel<false>), INPUT_GATHER), true);
+  static const bool reg = (register_input_kernel(reinterpret_cast<const void*>(final_kernel<true>), INPUT_GATHER),
+                           register_input_kernel(reinterpret_cast<const void*>(final_kernel<false>), INPUT_GATHER), true);
   (void)reg;
+  auto k = vec ? final_kernel<true> : final_kernel<false>;
+  const size_t smem = basic ? 0 : sizeof(uint32_t) * (size_t)K * kSortWarps;
+  if (smem > 16 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)(sizeof(uint32_t) * kSortFastKeys * kSortWarps));
+    if (e != cudaSuccess) return e;
+  }
   // A first or whole checkpoint gathers (nearly) every chunk: a block per tile
   // keeps the copy at the bandwidth of a plain one (4 GiB: 1.21 ms against
   // 1.46 ms for a persistent grid).  An incremental one gathers a few percent
   // and gets one wave of blocks: a block per possible tile costs more to
   // launch than the copy takes.
   const uint64_t tile_bytes = 16ull * (g.cs >= 128 ? kCopyTileUnits : 16 * g.cs);
-  const uint64_t tiles = ((uint64_t)g.N * g.cs + tile_bytes - 1) / tile_bytes;
-  const uint32_t wave = (uint32_t)num_sms() * 6;
-  const uint32_t grid = (uint32_t)std::min<uint64_t>(tiles, whole ? 1u << 20 : wave);
-  if (vec) launch_k(copy_kernel<true>, grid, 256, 0, s, g);
-  else launch_k(copy_kernel<false>, grid, 256, 0, s, g);
+  const uint64_t ctiles = ((uint64_t)g.N * g.cs + tile_bytes - 1) / tile_bytes;
+  const uint32_t wave = (uint32_t)num_sms() * 5;
+  uint32_t copies = (uint32_t)std::min<uint64_t>(ctiles, whole ? 1u << 20 : wave);
+  if (whole && copies > wave) {  // never in a captured sequence
+    launch_k(vec ? copy_kernel<true> : copy_kernel<false>, copies, 256, 0, s, g);
+    note_launch();
+    copies = 0;
+  }
+  g.n_drain = g.fuse_gate ? std::min<uint32_t>(2 * num_sms(), (g.N + 255) / 256) : 0;
+  g.n_copy = copies;
+  const uint32_t grid = std::max(1u, g.n_sort + g.n_drain + copies);
+  launch_k(k, grid, 256, smem, s, g);
   note_launch();
   return cudaGetLastError();
 }

@@ -25,6 +25,13 @@ struct Layout {
   uint32_t sort_n, sort_tiles;            // nkeys * sort tiles; tiles of kSortTile shift entries
 };
 
+// The canonical (serial push) order of a tree's nodes.
+struct RootOrder {
+  int ascending;   // 0 = deeper levels first, 1 = ascending node id
+  uint32_t D;      // depth of node M-1
+  uint64_t sizeD;  // nodes on depth D
+};
+
 struct ForestArgs {
   Digest* tree;
   uint8_t* labels;
@@ -33,9 +40,7 @@ struct ForestArgs {
   const StepParams* sp;  // cur, epochs (device)
   uint32_t* err;
   int hash_kind;
-  int ascending;   // canonical order: 0 = deeper levels first (serial push order), 1 = ascending node id
-  uint32_t D;      // depth of node M-1
-  uint64_t sizeD;  // nodes on depth D
+  RootOrder order;
   // Incremental checkpoints: word that is 0 when no leaf was demoted to a
   // shifted duplicate of a digest first seen in this checkpoint.  Then no
   // shifted pair can hash to a digest inserted by the first-occurrence pass
@@ -49,14 +54,14 @@ struct ForestArgs {
 
 // Position of node x (>= 1) in the canonical root order.
 __host__ __device__ __forceinline__ uint64_t canon_pos(const ForestArgs& a, uint32_t x) {
-  if (a.ascending) return (uint64_t)x - 1;
+  if (a.order.ascending) return (uint64_t)x - 1;
 #ifdef __CUDA_ARCH__
   const uint32_t d = 31 - __clz(x + 1);
 #else
   uint32_t d = 0;
   while (((2ull << d) - 1) <= (uint64_t)x) d++;
 #endif
-  const uint64_t fp = d == a.D ? 0 : a.sizeD + ((1ull << a.D) - (2ull << d));
+  const uint64_t fp = d == a.order.D ? 0 : a.order.sizeD + ((1ull << a.order.D) - (2ull << d));
   return fp + (x - ((1ull << d) - 1));
 }
 
@@ -70,18 +75,32 @@ struct GatherArgs {
   const Digest* digests;  // tree heap (by node) or hash list (by chunk)
   DigestMap map;
   uint32_t* err;
-  uint64_t* clk;          // CLK_ROOTS_DONE is written by the first launch
-  const uint32_t* fo_list;
-  const uint32_t* sh_list;
-  uint64_t* fo_val;
-  uint32_t *reg_chunk, *reg_slot, *reg_len;
+  uint64_t* clk;          // phase times (may be null)
+  uint32_t* counters;     // COUNT_*
+  // what is compacted: root flags at canonical positions (tree) or the chunks'
+  // labels, padded to whole 16-byte words
+  uint8_t* flags;
+  uint64_t n_flags;
+  const uint8_t* labels;  // tree: node labels
+  RootOrder order;
+  uint64_t *tile_counts, *tile_regions;  // per tile of flags
+  uint32_t* fo_list;
+  uint32_t* sh_list;
+  uint64_t* fo_val;       // tree: regions and chunks before the entry in its tile, bit 63 if it is a region
+  uint32_t* fo_tile;      // tree: the entry's tile
+  uint32_t *reg_chunk, *reg_slot;
   uint32_t *sh_key, *sh_prev;
   uint32_t *hist, *rep, *rank;
   uint64_t* sort_mat;
-  uint64_t *scan_scratch, *scan_total, *scan_scratch2, *scan_total2;
+  uint64_t *scan_scratch2, *scan_total2;
+  // inserts queued by a fused forest pass (fuse_gate as in ForestArgs)
+  const uint32_t* fuse_gate;
+  const uint32_t *ins_queue, *ins_count;
   uint8_t* stage;
   uint64_t stage_cap;
   Layout* lay;
+  Readback results;       // written by the last launch
+  uint32_t n_emit, n_sort, n_drain, n_copy, sort_scan;  // set by launch_assemble
 };
 
 // One forest pass.  pass 0 = first-occurrence forest, 1 = duplicate forest, 3 =
@@ -89,15 +108,9 @@ struct GatherArgs {
 // 1).
 size_t forest_done_words(uint32_t N);
 cudaError_t launch_forest(const ForestArgs& a, int pass, int baseline, uint32_t N, cudaStream_t s);
-cudaError_t launch_root_compaction(const ForestArgs& fa, uint32_t N, uint32_t M, uint32_t* fo_list,
-                                   uint32_t* sh_list, Layout* lay, uint64_t* scan_scratch, uint64_t* scan_total,
-                                   cudaStream_t s);
-cudaError_t launch_chunk_compaction(const uint8_t* labels, uint32_t n_chunks, int basic, uint32_t* fo_list,
-                                    uint32_t* sh_list, Layout* lay, uint64_t* scan_scratch, uint64_t* scan_total,
-                                    uint64_t* clk, cudaStream_t s);
-// Assemble the diff into g.stage; max_entries bounds F and S (N + 1).
-// whole: most chunks are expected in the diff (a baseline).
-cudaError_t launch_assemble(const GatherArgs& g, uint64_t max_entries, bool whole, cudaStream_t s);
+// Roots listed and the diff assembled into g.stage; max_entries bounds F and S
+// (N + 1).  whole: most chunks are expected in the diff (a baseline).
+cudaError_t launch_assemble(GatherArgs g, uint64_t max_entries, bool whole, cudaStream_t s);
 // Rebuild `from` into the empty table `to` (capacity change), preserving values.
 cudaError_t launch_map_rehash(const DigestMap& from, uint64_t from_cap, const DigestMap& to, uint32_t* err,
                               cudaStream_t s);

@@ -45,8 +45,12 @@ struct ParamsOut {
   uint32_t* counters;  // kCounters words, cleared
 };
 // Counters of a checkpoint: changed chunks, demoted leaves, queued forest
-// inserts, notes of the insert pass.
-constexpr int kCounters = 4;
+// inserts, notes of the insert pass; finished blocks of the assembly's
+// launches.
+enum : int {
+  COUNT_CHANGED = 0, COUNT_DEMOTED = 1, COUNT_INSERTS = 2, COUNT_NOTES = 3,
+  COUNT_ROOTS_DONE = 4, COUNT_SORT_DONE = 5, COUNT_FINAL_DONE = 6, kCounters = 8
+};
 
 struct LeafArgs {
   const uint8_t* data = nullptr;  // device buffer being checkpointed

@@ -43,6 +43,20 @@ __device__ __forceinline__ uint64_t block_excl_scan(uint64_t v, uint64_t* sh, ui
   return r;
 }
 
+// One block writes a launch sequence's results to pinned host memory.
+__device__ __forceinline__ void readback(const Readback& r) {
+  if (r.clk && threadIdx.x == 0) {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    r.clk[CLK_END] = t;
+    __threadfence_block();
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    for (uint32_t i = threadIdx.x; i < r.words[k]; i += blockDim.x) r.dst[k][i] = __ldcg(r.src[k] + i);
+}
+
 // Grid-level exclusive scan of u64 values produced by a functor, three phases.
 //   phase 1: tile sums         (grid over tiles)
 //   phase 2: scan of tile sums (one block)
