@@ -461,11 +461,18 @@ __device__ inline int map_claim(const DigestMap& m, const Digest& k, bool read, 
   return INS_FAILED;
 }
 
-// Warp total of new entries added to m.size (every lane of the warp calls it).
+// Block total of new entries added to m.size (every thread of the block calls
+// it): one atomic per block, since a launch's all go to one word (one per warp
+// took 40 of 340 us of a baseline's labels, 1 GiB in 512-byte chunks).
 __device__ __forceinline__ void count_new_entries(const DigestMap& m, uint32_t n) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-  if ((threadIdx.x & 31) == 0 && n) atomicAdd(m.size, n);
+  __shared__ uint32_t s_new;
+  __syncthreads();
+  if (threadIdx.x == 0) s_new = 0;
+  __syncthreads();
+  const uint32_t w = __reduce_add_sync(0xffffffffu, n);
+  if ((threadIdx.x & 31) == 0 && w) atomicAdd(&s_new, w);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_new) atomicAdd(m.size, s_new);
 }
 
 // Slot index of key, or -1.  Plain loads: a key inserted by an earlier launch
