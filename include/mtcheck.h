@@ -199,13 +199,14 @@ int mtc_basic_checkpoint_noalloc(int hash, const void* dev_data, uint64_t len, u
  * its own stream.  mtc_batch_checkpoint checkpoints every member in one call:
  * the baseline step runs eagerly with all members overlapped; later steps
  * replay one CUDA graph holding every member's kernels as parallel branches
- * (captured again only when a member's device buffers move).  Each member's
+ * (captured again only when a member's device buffers change; an input that
+ * has moved is updated in place).  Each member's
  * diff, header and counters are byte-identical to those of a lone handle
  * given the same buffers; read them through the member handles. */
 typedef struct mtc_batch mtc_batch_t;
 typedef struct mtc_batch_info {
   uint64_t steps;
-  uint64_t graph_captures;
+  uint64_t graph_captures; /* members' sequences captured, or pointed at an input that has moved */
   uint64_t graph_nodes;
   uint64_t kernels_per_step;
   double last_device_ms;   /* fork to join of the last step (CUDA events) */

@@ -94,6 +94,10 @@ void Batch::drop_graph() {
   in_kernel_.assign(engs_.size(), 0);
   recs_.assign(engs_.size(), MemberLeaf{});
   sigs_.assign(engs_.size(), 0);
+  cap_data_.assign(engs_.size(), nullptr);
+  exec_data_.assign(engs_.size(), nullptr);
+  children_.assign(engs_.size(), nullptr);
+  inputs_.assign(engs_.size(), {});
   nodes_.assign(engs_.size(), 0);
   kernels_.assign(engs_.size(), 0);
 }
@@ -192,7 +196,8 @@ int Batch::capture_member(size_t i, const uint8_t* data, uint64_t len) {
   if (post_[i]) cudaGraphGetNodes(post_[i], nullptr, &n2);
   nodes_[i] = n + n2;
   kernels_[i] = launch_count() - l0;
-  sigs_[i] = engs_[i]->signature(data, len);
+  sigs_[i] = leaf_batching_ ? engs_[i]->signature(data, len) : engs_[i]->shape_signature(data, len);
+  cap_data_[i] = data;
   stats_.captures++;
   return ST_OK;
 }
@@ -253,6 +258,7 @@ int Batch::build_parent() {
   for (size_t i = 0; i < engs_.size(); i++) {
     cudaGraphNode_t a = nullptr;
     MTC_BCUDA(cudaGraphAddChildGraphNode(&a, parent_, nullptr, 0, pre_[i]));
+    children_[i] = a;
     if (in_kernel_[i]) before.push_back(a);
   }
   if (!order.empty()) {
@@ -273,6 +279,14 @@ int Batch::build_parent() {
     drop_parent();
     return fail(ST_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(ie));
   }
+  // the members' input nodes, as they lie in the step graph
+  for (size_t i = 0; i < engs_.size() && !leaf_batching_; i++) {
+    cudaGraph_t g = nullptr;
+    MTC_BCUDA(cudaGraphChildGraphNodeGetGraph(children_[i], &g));
+    const int rc = engs_[i]->collect_inputs(g, &inputs_[i]);
+    if (rc) return fail(rc, "member " + std::to_string(i) + ": " + engs_[i]->last_error);
+  }
+  exec_data_ = cap_data_;
   return ST_OK;
 }
 
@@ -297,9 +311,12 @@ int Batch::checkpoint(const uint8_t* const* data, const uint64_t* lens, bool mak
   std::vector<char> join(engs_.size(), 0);
   if (graph) {
     bool rebuild = !parent_exec_;
+    const std::vector<const uint8_t*> before = exec_data_;
     for (size_t i = 0; i < engs_.size(); i++) {
       if (engs_[i]->take_stream_work()) join[i] = 1;
-      if (!pre_[i] || sigs_[i] != engs_[i]->signature(data[i], lens[i])) {
+      const uint64_t sig = leaf_batching_ ? engs_[i]->signature(data[i], lens[i])
+                                          : engs_[i]->shape_signature(data[i], lens[i]);
+      if (!pre_[i] || sigs_[i] != sig) {
         int rc = capture_member(i, data[i], lens[i]);
         if (rc) return rc;
         join[i] = 1;
@@ -309,6 +326,18 @@ int Batch::checkpoint(const uint8_t* const* data, const uint64_t* lens, bool mak
     if (rebuild) {
       int rc = build_parent();
       if (rc) return rc;
+    }
+    // inputs that have moved: the nodes that read them are updated in place
+    // (capturing 24 members again took 1.6 of a step's 2.1 ms)
+    for (size_t i = 0; i < engs_.size() && !leaf_batching_; i++) {
+      if (exec_data_[i] == data[i]) continue;
+      const int rc = engs_[i]->retarget(parent_exec_, inputs_[i], data[i], lens[i]);
+      if (rc) {
+        drop_parent();
+        return fail(rc, "member " + std::to_string(i) + ": " + engs_[i]->last_error);
+      }
+      exec_data_[i] = data[i];
+      if (before[i] != data[i]) stats_.captures++;
     }
   }
   // 3. issue: the step starts after the work already on the legacy default

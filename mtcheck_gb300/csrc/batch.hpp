@@ -85,6 +85,11 @@ class Batch : public Engine::LeafHook {
   std::vector<char> in_kernel_;      // the member's leaves run in the batched launch
   std::vector<MemberLeaf> recs_;     // their records (host copy)
   std::vector<uint64_t> sigs_, nodes_, kernels_;
+  // the input each member's sequence was captured with, the one its nodes in
+  // the step graph read now, and those nodes
+  std::vector<const uint8_t*> cap_data_, exec_data_;
+  std::vector<cudaGraphNode_t> children_;
+  std::vector<std::vector<Engine::InputNode>> inputs_;
   size_t cur_ = 0;                   // member being captured
   // step graph: [head reset, members' pre_] -> batched leaf launch -> members' post_
   cudaGraph_t parent_ = nullptr;

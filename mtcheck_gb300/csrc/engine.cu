@@ -487,13 +487,54 @@ void Engine::drop_own_graph() {
   own_data_ = nullptr;
 }
 
-// Points the captured sequence at another input buffer of the same length
-// and alignment: the leaf kernels' descriptor and pointer, the chunk gather's
-// pointer (no other kernel reads the input).
-int Engine::retarget_own(const uint8_t* data, uint64_t len) {
-  for (auto& in : input_nodes_) {
+int Engine::collect_inputs(cudaGraph_t g, std::vector<InputNode>* out) {
+  out->clear();
+  size_t n = 0;
+  MTC_CUDA(cudaGraphGetNodes(g, nullptr, &n));
+  std::vector<cudaGraphNode_t> nodes(n);
+  if (n) MTC_CUDA(cudaGraphGetNodes(g, nodes.data(), &n));
+  for (cudaGraphNode_t nd : nodes) {
+    cudaGraphNodeType ty;
+    InputNode in{};
+    in.node = nd;
+    MTC_CUDA(cudaGraphNodeGetType(nd, &ty));
+    if (ty == cudaGraphNodeTypeMemcpy && mode_ == MODE_FULL) {
+      in.kind = INPUT_COPY;
+      out->push_back(in);
+    }
+    if (ty != cudaGraphNodeTypeKernel) continue;
+    MTC_CUDA(cudaGraphKernelNodeGetParams(nd, &in.p));
+    in.kind = input_kernel_kind(in.p.func);
+    if (in.kind == INPUT_NONE) continue;
+    if (in.kind == INPUT_LEAF_TMA) {
+      std::memcpy(&in.tmap, in.p.kernelParams[0], sizeof(CUtensorMap));
+      std::memcpy(&in.la, in.p.kernelParams[1], sizeof(LeafArgs));
+      std::memcpy(&in.u[0], in.p.kernelParams[2], sizeof(uint32_t));
+    } else if (in.kind == INPUT_LEAF_DIRECT) {
+      std::memcpy(&in.la, in.p.kernelParams[0], sizeof(LeafArgs));
+      std::memcpy(&in.u[0], in.p.kernelParams[1], sizeof(uint32_t));
+      std::memcpy(&in.u[1], in.p.kernelParams[2], sizeof(uint32_t));
+    } else if (in.kind == INPUT_PARAMS) {
+      std::memcpy(&in.po, in.p.kernelParams[1], sizeof(ParamsOut));
+    } else {
+      std::memcpy(&in.ga, in.p.kernelParams[0], sizeof(GatherArgs));
+    }
+    in.p.kernelParams = nullptr;
+    out->push_back(in);
+  }
+  return ST_OK;
+}
+
+// The leaf kernels' descriptor and pointer and the chunk gather's pointer (no
+// other kernel reads the input).
+int Engine::retarget(cudaGraphExec_t exec, std::vector<InputNode>& nodes, const uint8_t* data, uint64_t len) {
+  for (auto& in : nodes) {
     void* args[3] = {nullptr, nullptr, nullptr};
     if (in.kind == INPUT_PARAMS) continue;
+    if (in.kind == INPUT_COPY) {
+      MTC_CUDA(cudaGraphExecMemcpyNodeSetParams1D(exec, in.node, stage_.p, data, len, cudaMemcpyDeviceToDevice));
+      continue;
+    }
     if (in.kind == INPUT_LEAF_TMA) {
       if (!input_tmap(&tma_, data, len, cs_, leaf_tune_)) return fail(ST_ECUDA, "tensor map for the new input");
       in.tmap = tma_.map;
@@ -513,9 +554,8 @@ int Engine::retarget_own(const uint8_t* data, uint64_t len) {
     cudaKernelNodeParams q = in.p;
     q.kernelParams = args;
     q.extra = nullptr;
-    MTC_CUDA(cudaGraphExecKernelNodeSetParams(own_exec_, in.node, &q));
+    MTC_CUDA(cudaGraphExecKernelNodeSetParams(exec, in.node, &q));
   }
-  own_data_ = data;
   return ST_OK;
 }
 
@@ -553,7 +593,10 @@ void Engine::set_own_graph(bool on) {
 // took 10-15 us of a 145 us checkpoint of 64 MiB in 128-byte chunks.
 int Engine::replay_own(const uint8_t* data, uint64_t len) {
   const uint64_t sig = shape_signature(data, len);
-  if (own_exec_ && sig == own_sig_ && data != own_data_) MTC_TRY(retarget_own(data, len));
+  if (own_exec_ && sig == own_sig_ && data != own_data_) {
+    MTC_TRY(retarget(own_exec_, input_nodes_, data, len));
+    own_data_ = data;
+  }
   if (!own_exec_ || sig != own_sig_) {
     drop_own_graph();
     if (!cap_stream_) MTC_CUDA(cudaStreamCreateWithFlags(&cap_stream_, cudaStreamNonBlocking));
@@ -564,35 +607,8 @@ int Engine::replay_own(const uint8_t* data, uint64_t len) {
     const int rc = enqueue(data, len, !untimed_);
     stream_ = keep;
     cudaError_t ce = cudaStreamEndCapture(cap_stream_, &own_seq_);
-    size_t n = 0;
     if (rc == ST_OK && ce == cudaSuccess) ce = cudaGraphInstantiate(&own_exec_, own_seq_, 0);
-    if (rc == ST_OK && ce == cudaSuccess) ce = cudaGraphGetNodes(own_seq_, nullptr, &n);
-    std::vector<cudaGraphNode_t> nodes(n);
-    if (n) cudaGraphGetNodes(own_seq_, nodes.data(), &n);
-    for (cudaGraphNode_t nd : nodes) {
-      cudaGraphNodeType ty;
-      if (cudaGraphNodeGetType(nd, &ty) != cudaSuccess || ty != cudaGraphNodeTypeKernel) continue;
-      InputNode in{};
-      if (cudaGraphKernelNodeGetParams(nd, &in.p) != cudaSuccess) continue;
-      in.kind = input_kernel_kind(in.p.func);
-      if (in.kind == INPUT_NONE) continue;
-      in.node = nd;
-      if (in.kind == INPUT_LEAF_TMA) {
-        std::memcpy(&in.tmap, in.p.kernelParams[0], sizeof(CUtensorMap));
-        std::memcpy(&in.la, in.p.kernelParams[1], sizeof(LeafArgs));
-        std::memcpy(&in.u[0], in.p.kernelParams[2], sizeof(uint32_t));
-      } else if (in.kind == INPUT_LEAF_DIRECT) {
-        std::memcpy(&in.la, in.p.kernelParams[0], sizeof(LeafArgs));
-        std::memcpy(&in.u[0], in.p.kernelParams[1], sizeof(uint32_t));
-        std::memcpy(&in.u[1], in.p.kernelParams[2], sizeof(uint32_t));
-      } else if (in.kind == INPUT_PARAMS) {
-        std::memcpy(&in.po, in.p.kernelParams[1], sizeof(ParamsOut));
-      } else {
-        std::memcpy(&in.ga, in.p.kernelParams[0], sizeof(GatherArgs));
-      }
-      in.p.kernelParams = nullptr;
-      input_nodes_.push_back(in);
-    }
+    if (rc == ST_OK && ce == cudaSuccess) MTC_TRY(collect_inputs(own_seq_, &input_nodes_));
     if (rc != ST_OK || ce != cudaSuccess) {
       drop_own_graph();
       cudaGetLastError();
@@ -704,8 +720,8 @@ uint64_t Engine::signature(const uint8_t* data, uint64_t len) const {
 
 uint64_t Engine::shape_signature(const uint8_t* data, uint64_t len) const {
   // the signature without the input's address, only its alignment (which
-  // chooses the kernels that read it): the single-call graph follows a moved
-  // input by retarget_own
+  // chooses the kernels that read it): a captured sequence follows a moved
+  // input by retarget
   const uint64_t v[] = {(uint64_t)data & 15, len, (uint64_t)digests_.p, (uint64_t)labels_.p, (uint64_t)rflag_.p,
                         (uint64_t)chunk_slot_.p, (uint64_t)changed_list_.p, (uint64_t)changed_count_.p,
                         (uint64_t)slots_.p, map_cap_, (uint64_t)map_size_.p, (uint64_t)err_.p, (uint64_t)fo_list_.p,

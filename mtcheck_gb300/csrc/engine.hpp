@@ -233,6 +233,22 @@ class Engine {
   void set_order_after_legacy(bool on) { order_after_legacy_ = on; }
   int order_inputs();
   uint32_t launches() const { return launches_; }
+  // The nodes of a captured sequence that read the input buffer (or, in a lone
+  // handle's, carry the step values), with their captured arguments; and the
+  // same nodes, in a graph instantiated from that sequence, pointed at another
+  // input of the same length and alignment.
+  struct InputNode {
+    cudaGraphNode_t node;
+    int kind;
+    cudaKernelNodeParams p;
+    CUtensorMap tmap;
+    LeafArgs la;
+    uint32_t u[2];
+    GatherArgs ga;
+    ParamsOut po;
+  };
+  int collect_inputs(cudaGraph_t g, std::vector<InputNode>* out);
+  int retarget(cudaGraphExec_t exec, std::vector<InputNode>& nodes, const uint8_t* data, uint64_t len);
   // A batch takes over the leaf pass of its members' captured sequences:
   // while a hook is set, the sequence calls it where it would launch the
   // leaf kernels.
@@ -277,22 +293,10 @@ class Engine {
   // the captured launch sequence
   cudaGraph_t own_seq_ = nullptr;
   cudaGraphExec_t own_exec_ = nullptr;
-  // kernel nodes that read the input buffer, with their captured arguments
-  struct InputNode {
-    cudaGraphNode_t node;
-    int kind;
-    cudaKernelNodeParams p;
-    CUtensorMap tmap;
-    LeafArgs la;
-    uint32_t u[2];
-    GatherArgs ga;
-    ParamsOut po;
-  };
   std::vector<InputNode> input_nodes_;
   const uint8_t* own_data_ = nullptr;  // input pointer the graphs currently read
   cudaStream_t cap_stream_ = nullptr;  // private stream the sequence is captured on
   uint64_t own_sig_ = 0, own_kernels_ = 0;
-  int retarget_own(const uint8_t* data, uint64_t len);
   int update_own_params();
   int replay_own(const uint8_t* data, uint64_t len);
   void drop_own_graph();

@@ -214,6 +214,7 @@ enum : int {
   INPUT_LEAF_DIRECT = 2,  // (LeafArgs, uint32_t, uint32_t)
   INPUT_GATHER = 3,       // (GatherArgs)
   INPUT_PARAMS = 4,       // (StepParams, ParamsOut): the step values
+  INPUT_COPY = 5,         // a copy of the whole input (the full approach)
 };
 void register_input_kernel(const void* func, int kind);
 int input_kernel_kind(const void* func);
