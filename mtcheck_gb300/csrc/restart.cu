@@ -889,6 +889,76 @@ __device__ __forceinline__ void resolve_chunk(const RArgs& a, const OwnMasks& ow
 //    aligned 16-byte words, the word after a unit taken from the next lane,
 //    and the unit is cut out with funnel shifts; every load stays inside a
 //    16-byte word holding at least one byte of the source region.
+// Mask of the bytes of word q (bytes 4q .. 4q + 3) in [lo, hi).
+__device__ __forceinline__ uint32_t byte_mask(int lo, int hi, int q) {
+  const int a = lo - 4 * q, b = hi - 4 * q;
+  const uint32_t below_b = b <= 0 ? 0u : b >= 4 ? ~0u : (1u << (8 * b)) - 1;
+  const uint32_t below_a = a <= 0 ? 0u : a >= 4 ? ~0u : (1u << (8 * a)) - 1;
+  return below_b & ~below_a;
+}
+
+// Chunk sizes that are no multiple of 16 bytes, or an output that is not 16-byte
+// aligned: the warp writes the aligned 16-byte units of its 32 chunks' range,
+// each put together from the chunks it meets (two at most for chunks of 16
+// bytes or more), every piece cut out of the aligned words around it.  A unit
+// of which not every byte is restored is written byte by byte.  64 MB in chunks
+// of 100 bytes, a byte per lane: 218 us.
+__device__ __forceinline__ void copy_tile_any(const RArgs& a, uint64_t c0, const uint8_t* src, uint32_t nb) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t cs = a.cs, total = 32 * cs;
+  const unsigned long long sp = reinterpret_cast<unsigned long long>(src);
+  const uint64_t d0 = reinterpret_cast<uint64_t>(a.out) + c0 * cs;
+  const uint64_t u0 = d0 & ~15ull, nu = (d0 + total - u0 + 15) / 16;
+  const int pieces = cs >= 16 ? 2 : (int)((15 + cs) / cs) + 1;
+  for (uint64_t f0 = 0; f0 < nu; f0 += 32) {
+    const uint64_t u = u0 + 16 * (f0 + lane);
+    int pos = u < d0 ? (int)(d0 - u) : 0;
+    const int end = u >= d0 + total ? 0 : d0 + total - u < 16 ? (int)(d0 + total - u) : 16;
+    const uint64_t x = u + pos - d0;
+    uint64_t q64 = 0;
+    if (pos < end && x >= cs) q64 = total <= 0xffffffffull ? (uint32_t)x / (uint32_t)cs : x / cs;
+    uint32_t q = (uint32_t)q64;
+    uint64_t within = pos < end ? x - q64 * cs : 0;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    uint4 m = make_uint4(0, 0, 0, 0);  // bytes of v that are restored
+    for (int k = 0; k < pieces; k++) {
+      const unsigned long long s = __shfl_sync(0xffffffffu, sp, q & 31);
+      const uint32_t n = __shfl_sync(0xffffffffu, nb, q & 31);
+      if (pos < end) {
+        const int stop = cs - within < (uint64_t)(end - pos) ? pos + (int)(cs - within) : end;
+        // bytes pos .. hi of the unit come from s + within on
+        const int hi = within >= n ? pos : n - within < (uint64_t)(stop - pos) ? pos + (int)(n - within) : stop;
+        if (hi > pos) {
+          const uint64_t A = s + within - pos;
+          const int d = (int)(A & 15);
+          const uint4* w = reinterpret_cast<const uint4*>(A - d);
+          uint4 w0 = make_uint4(0, 0, 0, 0), w1 = make_uint4(0, 0, 0, 0);
+          if (pos + d < 16) w0 = __ldcs(w);
+          if (hi + d > 16) w1 = __ldcs(w + 1);
+          const uint4 c = cut16(w0, w1, (uint32_t)d);
+          const uint32_t m0 = byte_mask(pos, hi, 0), m1 = byte_mask(pos, hi, 1), m2 = byte_mask(pos, hi, 2),
+                         m3 = byte_mask(pos, hi, 3);
+          v.x |= c.x & m0; v.y |= c.y & m1; v.z |= c.z & m2; v.w |= c.w & m3;
+          m.x |= m0; m.y |= m1; m.z |= m2; m.w |= m3;
+        }
+        pos = stop;
+        q++;
+        within = 0;
+      }
+    }
+    if ((m.x & m.y & m.z & m.w) == ~0u) {
+      *reinterpret_cast<uint4*>(u) = v;
+    } else if (m.x | m.y | m.z | m.w) {
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        const uint32_t vw = i < 4 ? v.x : i < 8 ? v.y : i < 12 ? v.z : v.w;
+        const uint32_t mw = i < 4 ? m.x : i < 8 ? m.y : i < 12 ? m.z : m.w;
+        if ((mw >> (8 * (i & 3))) & 1) *reinterpret_cast<uint8_t*>(u + i) = (uint8_t)(vw >> (8 * (i & 3)));
+      }
+    }
+  }
+}
+
 constexpr int kCopyUnroll = 4;
 __device__ __forceinline__ void copy_tile(const RArgs& a, uint64_t c0, const uint8_t* src, uint32_t nb) {
   const uint32_t lane = threadIdx.x & 31;
@@ -896,14 +966,7 @@ __device__ __forceinline__ void copy_tile(const RArgs& a, uint64_t c0, const uin
   const unsigned long long sp = reinterpret_cast<unsigned long long>(src);
   uint8_t* out0 = a.out + c0 * cs;
   if ((cs & 15) != 0 || (reinterpret_cast<uintptr_t>(a.out) & 15) != 0) {
-    // byte by byte (odd chunk sizes)
-    const uint64_t total = (uint64_t)cs * 32;
-    for (uint64_t f = lane; f < total; f += 32) {
-      const uint32_t q = (uint32_t)(f / cs), b = (uint32_t)(f - (uint64_t)q * cs);
-      const uint8_t* s = reinterpret_cast<const uint8_t*>(__shfl_sync(0xffffffffu, sp, q));
-      const uint32_t n = __shfl_sync(0xffffffffu, nb, q);
-      if (b < n) out0[(uint64_t)q * cs + b] = s[b];
-    }
+    copy_tile_any(a, c0, src, nb);
     return;
   }
   const uint32_t upc = cs >> 4;
