@@ -341,7 +341,6 @@ class Engine {
   void* rdi_host_ = nullptr;
   size_t rdi_host_bytes_ = 0;
   cudaEvent_t rdi_ev_ = nullptr;
-  DevBuf<uint8_t> hdr_dev_;         // read_headers: gathered headers
  public:
   // A host chain copied to device memory for a restart (the staging path of
   // mtc_restart); kept between restarts, released with the restart tables.

@@ -40,8 +40,11 @@ struct DiffInfo {
   uint64_t len;
   uint64_t fo_off, cnt_off, map_off, data_off;
   uint32_t F, P, S, id;
-  uint32_t fo_begin, sh_begin, rrs_begin, pad;
+  uint32_t fo_begin, sh_begin, rrs_begin;
+  uint32_t fo_tile, sh_tile;  // its first tile of FO and of shift entries
+  uint32_t pad[3];
 };
+static_assert(sizeof(DiffInfo) % 16 == 0, "copied as 16-byte words");
 
 struct RArgs {
   int approach;
@@ -54,8 +57,9 @@ struct RArgs {
   uint32_t F0, S0;               // FO and shift entries of the main checkpoint
   uint32_t fo_cb, sh_cb;         // first FO / shift entry of the chain (nfo / nsh without one)
   uint64_t tag;                  // this restart's epoch << 32 (chain table cells)
-  uint32_t *fo_node, *fo_seg, *fo_clen;
-  uint64_t* fo_excl;
+  uint32_t *fo_node, *fo_seg;
+  uint32_t* fo_clen;             // tree: chunks of the entry's diff before the entry
+  uint64_t* fo_excl;             // tree, main checkpoint: the same
   uint32_t *sh_node, *sh_prev, *sh_tree, *sh_seg;
   uint64_t *sh_off, *sh_excl;
   uint32_t* rrs;
@@ -70,7 +74,9 @@ struct RArgs {
   uint32_t* sbm;                 // [KW][32 W steps][dm, rm] bitmaps: the step's map holds the key
   uint32_t KW;                   // 32-key words per bitmap
   uint64_t* dm_excl;            // per chain FO entry: item prefix of the distinct-map table
-  uint4* fo_rng;                // chain FO entries: leaf key ranges {lo0, n0, lo1, n1}
+  uint4* fo_rng;                // interior chain FO entries (tree): leaf key ranges {lo0, n0, lo1, n1}
+  uint64_t *tile_len, *tile_items, *tile_sh;  // per tile of entries: FO chunks and table items, shift items
+  uint32_t n_fo_tiles, n_sh_tiles, n_rrs;     // tiles, blocks of the repeat tables
   uint64_t *tot;                // [0] dm items, [2] main FO chunks, [3] main shift chunks, [4] [3] + rm items
   uint8_t* out;
   uint32_t* err;
@@ -84,43 +90,26 @@ __device__ __forceinline__ uint32_t rd32(const uint8_t* p) {
   return v;
 }
 
-__device__ __forceinline__ uint32_t seg_of(const DiffInfo* di, uint32_t ndiff, uint32_t g, bool fo) {
-  uint32_t lo = 0, hi = ndiff - 1;
-  while (lo < hi) {
-    uint32_t mid = (lo + hi + 1) >> 1;
-    if ((fo ? di[mid].fo_begin : di[mid].sh_begin) <= g) lo = mid; else hi = mid - 1;
-  }
-  return lo;
+// The chain's descriptors from pinned host memory, and the restart's small
+// clears, in one launch.
+__global__ void setup_kernel(const uint4* host_di, uint4* di, uint32_t n16, uint32_t* err, uint64_t* tot) {
+  for (uint32_t i = threadIdx.x; i < n16; i += blockDim.x) di[i] = host_di[i];
+  if (threadIdx.x == 0) *err = 0;
+  if (threadIdx.x < 5) tot[threadIdx.x] = 0;
 }
 
-// 1. decode FO and shift entries of every diff
-__global__ void load_entries_kernel(RArgs a) {
-  const uint64_t total = (uint64_t)a.nfo + a.nsh;
-  for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < total; g += (uint64_t)gridDim.x * blockDim.x) {
-    if (g < a.nfo) {
-      uint32_t s = seg_of(a.di, a.ndiff, (uint32_t)g, true);
-      const DiffInfo& d = a.di[s];
-      uint32_t i = (uint32_t)g - d.fo_begin;
-      uint32_t node = rd32(d.base + d.fo_off + 4ull * i);
-      if (a.approach == APPROACH_TREE ? node > a.M : node >= a.N) { atomicOr(a.err, DERR_RANGE); node = 0; }
-      a.fo_node[g] = node;
-      a.fo_seg[g] = s;
-    } else {
-      uint32_t h = (uint32_t)(g - a.nfo);
-      uint32_t s = seg_of(a.di, a.ndiff, h, false);
-      const DiffInfo& d = a.di[s];
-      uint32_t i = h - d.sh_begin;
-      uint32_t node = rd32(d.base + d.map_off + 8ull * i), prev = rd32(d.base + d.map_off + 8ull * i + 4);
-      if (a.approach == APPROACH_TREE ? (node > a.M || prev > a.M) : node >= a.N) {
-        atomicOr(a.err, DERR_RANGE);
-        node = 0;
-        prev = 0;
-      }
-      a.sh_node[h] = node;
-      a.sh_prev[h] = prev;
-      a.sh_seg[h] = s;
-    }
+// Entries go in tiles of kEntryTile of one diff: FO tiles of every diff, then
+// shift tiles.  The diff that owns a tile: the last whose first tile is not
+// after it (whole warps call it).
+constexpr uint32_t kEntryTile = kScanTile;
+__device__ __forceinline__ uint32_t tile_diff(const DiffInfo* di, uint32_t ndiff, uint32_t tile, bool fo) {
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t n = 0;
+  for (uint32_t b = 0; b < ndiff; b += 32) {
+    const uint32_t s = b + lane;
+    n += __popc(__ballot_sync(0xffffffffu, s < ndiff && (fo ? di[s].fo_tile : di[s].sh_tile) <= tile));
   }
+  return n - 1;
 }
 
 // 2. inclusive prefix of the repeat-count table of every diff over ids 0..id
@@ -129,17 +118,16 @@ __global__ void load_entries_kernel(RArgs a) {
 //    The (checkpoint, count) pairs are read by the whole block and applied in
 //    table order by one thread (a repeated checkpoint keeps its last count);
 //    the prefix is a block scan (modulo 2^32, as the reference's uint32 sum).
-__global__ void rrs_kernel(RArgs a) {
-  __shared__ uint2 pairs[256];
-  __shared__ uint64_t sh[33];
-  for (uint32_t s = blockIdx.x; s < a.ndiff; s += gridDim.x) {
+__device__ void repeat_tables(const RArgs& a, uint32_t blk, uint32_t nblk, uint64_t* sh) {
+  __shared__ uint2 pairs[kScanThreads];
+  for (uint32_t s = blk; s < a.ndiff; s += nblk) {
     const DiffInfo& d = a.di[s];
     uint32_t* r = a.rrs + d.rrs_begin;
     for (uint32_t j = threadIdx.x; j <= d.id; j += blockDim.x) r[j] = 0;
     __syncthreads();
     for (uint32_t i0 = 0; i0 < d.P; i0 += blockDim.x) {
       const uint32_t i = i0 + threadIdx.x;
-      if (i < d.P && threadIdx.x < 256)
+      if (i < d.P)
         pairs[threadIdx.x] = make_uint2(rd32(d.base + d.cnt_off + 8ull * i), rd32(d.base + d.cnt_off + 8ull * i + 4));
       __syncthreads();
       if (threadIdx.x == 0) {
@@ -163,52 +151,6 @@ __global__ void rrs_kernel(RArgs a) {
     }
     __syncthreads();
   }
-}
-
-// 3. source checkpoint of every shift entry: the smallest j with i < prefix[j]
-//    (src/tree_approach.cpp:894-898), 0 if none
-__global__ void shift_tree_kernel(RArgs a) {
-  for (uint64_t h = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; h < a.nsh; h += (uint64_t)gridDim.x * blockDim.x) {
-    const DiffInfo& d = a.di[a.sh_seg[h]];
-    const uint32_t i = (uint32_t)h - d.sh_begin;
-    const uint32_t* r = a.rrs + d.rrs_begin;
-    uint32_t lo = 0, hi = d.id + 1;  // first j in [0, id] with r[j] > i
-    while (lo < hi) {
-      uint32_t mid = (lo + hi) >> 1;
-      if (r[mid] > i) hi = mid; else lo = mid + 1;
-    }
-    a.sh_tree[h] = lo <= d.id ? lo : 0;
-  }
-}
-
-// region length of an FO entry (tree: num_leaf_descendents, list/basic: 1)
-struct FoLen {
-  const uint32_t* node;
-  uint32_t M;
-  int tree;
-  __device__ __forceinline__ uint64_t operator()(uint64_t g) const { return tree ? num_leaf_descendents(node[g], M) : 1; }
-};
-struct StoreExcl {
-  uint64_t* out;
-  __device__ __forceinline__ void operator()(uint64_t g, uint64_t ex, uint64_t) const { out[g] = ex; }
-};
-// chunk_len of each FO entry relative to its own diff (src/tree_approach.cpp:803-816)
-// and the main checkpoint's item total (its entries lead the list, so their
-// prefix is fo_excl itself)
-__global__ void clen_kernel(RArgs a) {
-  for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < a.nfo; g += (uint64_t)gridDim.x * blockDim.x) {
-    const DiffInfo& d = a.di[a.fo_seg[g]];
-    a.fo_clen[g] = (uint32_t)(a.fo_excl[g] - a.fo_excl[d.fo_begin]);
-    if (g + 1 == a.F0)
-      a.tot[2] = a.fo_excl[g] + (a.approach == APPROACH_TREE ? num_leaf_descendents(a.fo_node[g], a.M) : 1);
-  }
-}
-
-// main checkpoint (segment 0): lowest FO entry per node / chunk
-__global__ void fo_at_kernel(RArgs a) {
-  const uint32_t F = a.di[0].F;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < F; i += (uint64_t)gridDim.x * blockDim.x)
-    atomicMin(&a.fo_at[a.fo_node[i]], (uint32_t)i);  // node range checked while decoding
 }
 
 // distinct_map lookup of (node, cur) in the main checkpoint's tree: the FO
@@ -245,9 +187,9 @@ __device__ uint64_t main_dm_lookup(const RArgs& a, uint32_t node) {
 
 // main shift entries: copy source offset (src/tree_approach.cpp:887-903,
 // src/list_approach.cpp:376-394)
-__global__ void main_shift_kernel(RArgs a) {
+__device__ __forceinline__ void main_shift(const RArgs& a, uint32_t blk, uint32_t nblk) {
   const DiffInfo& d = a.di[0];
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < d.S; i += (uint64_t)gridDim.x * blockDim.x) {
+  for (uint64_t i = (uint64_t)blk * blockDim.x + threadIdx.x; i < d.S; i += (uint64_t)nblk * blockDim.x) {
     const uint32_t prev = a.sh_prev[i], tree = a.sh_tree[i];
     uint64_t off = 0;
     if (tree == d.id) {
@@ -349,21 +291,27 @@ struct TwoLists {
 // tiles of 256 items: the main checkpoint holds a few percent of the chunks,
 // and tiles of 2048 left most SMs without one
 constexpr uint32_t kCoverTile = 256;
-__global__ void __launch_bounds__(256) main_cover_kernel(RArgs a) {
+// (list and basic: every entry is one item); the first n_shift blocks take the
+// shift entries' sources.
+__global__ void __launch_bounds__(256) main_cover_kernel(RArgs a, uint32_t n_shift) {
   __shared__ ExpandTile<kCoverTile> T;
-  const TwoLists<kCoverTile> L(a.tot[2], a.tot[3]);
+  if (blockIdx.x < n_shift) {
+    main_shift(a, blockIdx.x, n_shift);
+    return;
+  }
   const bool tree = a.approach == APPROACH_TREE;
-  for (uint64_t tile = blockIdx.x; tile < L.tiles(); tile += gridDim.x) {
+  const TwoLists<kCoverTile> L(tree ? a.tot[2] : a.F0, tree ? a.tot[3] : a.S0);
+  for (uint64_t tile = blockIdx.x - n_shift; tile < L.tiles(); tile += gridDim.x - n_shift) {
     const bool sh = tile >= L.nt0;
     const uint64_t total = sh ? L.tot1 : L.tot0;
     const uint64_t t0 = (sh ? tile - L.nt0 : tile) * kCoverTile;
     const uint64_t t1 = t0 + kCoverTile < total ? t0 + kCoverTile : total;
     const uint64_t* excl = sh ? a.sh_excl : a.fo_excl;
     const uint32_t n = sh ? a.S0 : a.F0;
-    expand_stage(T, excl, n, t0, t1);
+    if (tree) expand_stage(T, excl, n, t0, t1);
     for (uint64_t t = t0 + threadIdx.x; t < t1; t += blockDim.x) {
-      uint64_t j64;
-      const uint32_t i = expand_entry(T, excl, n, t, &j64);
+      uint64_t j64 = 0;
+      const uint32_t i = tree ? expand_entry(T, excl, n, t, &j64) : (uint32_t)t;
       const uint32_t j = (uint32_t)j64;
       if (!sh) {
         uint64_t c = tree ? (uint64_t)(uint32_t)(leftmost_leaf(a.fo_node[i], a.M) - (a.N - 1) + j) : a.fo_node[i];
@@ -408,169 +356,216 @@ __device__ __forceinline__ int fo_leaf_ranges(uint32_t u, uint32_t N, uint32_t M
   return n;
 }
 
-// Per chain FO entry, once: the (at most two) leaf ranges its distinct map
-// covers, or for the list and basic approaches its one chunk.
-__global__ void chain_ranges_kernel(RArgs a, uint32_t n) {
-  const bool tree = a.approach == APPROACH_TREE;
-  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t g = a.fo_cb + k;  // chain entries follow the main ones
-    uint4 r = make_uint4(0, 0, 0, 0);
-    if (tree) {
-      uint32_t lo[2], hi[2];
-      const int nr = fo_leaf_ranges(a.fo_node[g], a.N, a.M, lo, hi);
-      if (nr > 0) { r.x = lo[0]; r.y = hi[0] - lo[0] + 1; }
-      if (nr > 1) { r.z = lo[1]; r.w = hi[1] - lo[1] + 1; }
-    } else {
-      r.x = a.fo_node[g];
-      r.y = 1;
-    }
-    a.fo_rng[g] = r;
-  }
-}
-
 // Chain table items are segments of up to kSegKeys consecutive keys of one
 // entry, each handled by one thread.
 constexpr uint32_t kSegKeys = 32;
 __device__ __forceinline__ uint32_t segs_of(uint32_t keys) { return (keys + kSegKeys - 1) / kSegKeys; }
 
-struct ChainDmCount {
-  RArgs a;
-  __device__ __forceinline__ uint64_t operator()(uint64_t k) const {
-    const uint4 r = a.fo_rng[a.fo_cb + k];
-    return (uint64_t)segs_of(r.y) + segs_of(r.w);
-  }
-};
-struct ChainRmCount {
-  RArgs a;
-  __device__ __forceinline__ uint64_t operator()(uint64_t k) const {
-    const uint64_t h = a.sh_cb + k;
-    if (a.approach == APPROACH_LIST) return 1;
-    const uint32_t node = a.sh_node[h];
-    // repeat_map keys: the root (src/tree_approach.cpp:1069) and the leaf
-    // range of num_leaf_descendents(node) from leftmost_leaf(node) (:1073-1078);
-    // only keys in [N-1, M] can be looked up by a leaf
-    uint64_t c = segs_of(num_leaf_descendents(node, a.M));
-    if (node >= a.N - 1 && node <= a.M) c += 1;
-    return c;
-  }
-};
-
-// Items of every shift entry in one scan: the main checkpoint's regions
-// (num_leaf_descendents(prev) chunks each), then the chain entries' repeat-map
-// keys.  The main total goes to tot[3], the grand total to tot[4]; the chain
-// items are numbered from tot[3] on.
-struct ShiftItems {
-  RArgs a;
-  __device__ __forceinline__ uint64_t operator()(uint64_t h) const {
-    if (h < a.S0) return a.approach == APPROACH_TREE ? num_leaf_descendents(a.sh_prev[h], a.M) : 1;
-    return ChainRmCount{a}(h - a.sh_cb);
-  }
-};
-struct StoreShiftExcl {
-  RArgs a;
-  __device__ __forceinline__ void operator()(uint64_t h, uint64_t ex, uint64_t v) const {
-    a.sh_excl[h] = ex;
-    if (h + 1 == a.S0) a.tot[3] = ex + v;
-  }
-};
-
 __device__ __forceinline__ uint32_t key_of_leaf(const RArgs& a, uint32_t x) { return x - (a.N - 1); }
 
-// The three entry scans of a restart in one pair of launches, each segment
-// starting on a tile boundary and scanned on its own:
-//   0: region length of every FO entry (FoLen) -> fo_excl
-//   1: table segments of every chain FO entry, with its leaf ranges
-//      (ChainDmCount, chain_ranges_kernel; the ranges are kept by the first
-//      launch for the second) -> dm_excl, fo_rng, total tot[0]
-//   2: items of every shift entry (ShiftItems) -> sh_excl, tot[3], total tot[4]
-// Used when every segment fits the two-launch form (at most kReduceTiles
-// tiles); otherwise the three scans run separately.
-struct EntryScans {
-  RArgs a;
-  uint64_t n[3];
-  uint32_t first[4];  // first tile of each segment; first[3] = all tiles
-};
-__device__ __forceinline__ uint4 chain_ranges_of(const RArgs& a, uint32_t g) {
+// ---------------------------------------------------------------------------
+// entries, decoded and numbered
+// ---------------------------------------------------------------------------
+// Tree, a chain FO entry: the (at most two) leaf ranges its distinct map covers.
+__device__ __forceinline__ uint4 chain_ranges_of(const RArgs& a, uint32_t node) {
   uint4 r = make_uint4(0, 0, 0, 0);
-  if (a.approach == APPROACH_TREE) {
-    uint32_t lo[2], hi[2];
-    const int nr = fo_leaf_ranges(a.fo_node[g], a.N, a.M, lo, hi);
-    if (nr > 0) { r.x = lo[0]; r.y = hi[0] - lo[0] + 1; }
-    if (nr > 1) { r.z = lo[1]; r.w = hi[1] - lo[1] + 1; }
-  } else {
-    r.x = a.fo_node[g];
-    r.y = 1;
-  }
+  uint32_t lo[2], hi[2];
+  const int nr = fo_leaf_ranges(node, a.N, a.M, lo, hi);
+  if (nr > 0) { r.x = lo[0]; r.y = hi[0] - lo[0] + 1; }
+  if (nr > 1) { r.z = lo[1]; r.w = hi[1] - lo[1] + 1; }
   return r;
 }
-// `ranges`: compute a chain entry's leaf ranges and keep them (first pass),
-// or read the kept ones (second pass)
-__device__ __forceinline__ uint64_t entry_scan_val(const EntryScans& e, int k, uint64_t i, bool ranges) {
-  if (k == 0) return FoLen{e.a.fo_node, e.a.M, e.a.approach == APPROACH_TREE ? 1 : 0}(i);
-  if (k == 1) {
-    const uint32_t g = e.a.fo_cb + (uint32_t)i;
-    uint4 r;
-    if (ranges) {
-      r = chain_ranges_of(e.a, g);
-      e.a.fo_rng[g] = r;
-    } else {
-      r = e.a.fo_rng[g];
-    }
-    return (uint64_t)segs_of(r.y) + segs_of(r.w);
-  }
-  return ShiftItems{e.a}(i);
+// its ranges again: a leaf is its own, an interior node's were kept
+__device__ __forceinline__ uint4 chain_ranges_at(const RArgs& a, uint32_t g, uint32_t node) {
+  if (node < a.N - 1) return a.fo_rng[g];
+  return make_uint4(node, node <= a.M ? 1 : 0, 0, 0);
 }
-__device__ __forceinline__ int entry_scan_seg(const EntryScans& e, uint32_t b) {
-  return b < e.first[1] ? 0 : b < e.first[2] ? 1 : 2;
+
+// Table segments of a chain shift entry (tree).  repeat_map keys: the root
+// (src/tree_approach.cpp:1069) and the leaf range of num_leaf_descendents(node)
+// from leftmost_leaf(node) (:1073-1078); only keys in [N-1, M] can be looked up
+// by a leaf.
+__device__ __forceinline__ uint32_t chain_rm_items(const RArgs& a, uint32_t node) {
+  uint32_t c = segs_of(num_leaf_descendents(node, a.M));
+  if (node >= a.N - 1 && node <= a.M) c += 1;
+  return c;
 }
-__global__ void entry_scan_sums_kernel(EntryScans e, uint64_t* tile_sums) {
+
+// 1. Decode every entry of the chain, where it lies (device or host memory),
+// check its range, and (tree) sum each tile's chunks and table items; beside
+// it the repeat tables.  Tiles belong to one diff, so that a prefix within the
+// diff is a sum over the diff's own tiles.
+__global__ void __launch_bounds__(kScanThreads) entry_load_kernel(RArgs a) {
   __shared__ uint64_t sh[33];
-  const int k = entry_scan_seg(e, blockIdx.x);
-  const uint64_t base = (uint64_t)(blockIdx.x - e.first[k]) * kScanTile;
-  uint64_t sum = 0;
+  const uint32_t nt = a.n_fo_tiles + a.n_sh_tiles;
+  if (blockIdx.x >= nt) {
+    repeat_tables(a, blockIdx.x - nt, a.n_rrs, sh);
+    return;
+  }
+  const bool tree = a.approach == APPROACH_TREE;
+  const bool fo = blockIdx.x < a.n_fo_tiles;
+  const uint32_t tile = fo ? blockIdx.x : blockIdx.x - a.n_fo_tiles;
+  const uint32_t s = tile_diff(a.di, a.ndiff, tile, fo);
+  const DiffInfo d = a.di[s];
+  const uint32_t i0 = (tile - (fo ? d.fo_tile : d.sh_tile)) * kEntryTile, n = fo ? d.F : d.S;
+  uint64_t len = 0, items = 0;
+#pragma unroll 4
   for (int q = 0; q < kScanPerThread; q++) {
-    const uint64_t i = base + (uint64_t)q * kScanThreads + threadIdx.x;
-    if (i < e.n[k]) sum += entry_scan_val(e, k, i, true);
+    const uint32_t i = i0 + q * kScanThreads + threadIdx.x;
+    if (i >= n) break;
+    if (fo) {
+      uint32_t node = rd32(d.base + d.fo_off + 4ull * i);
+      if (tree ? node > a.M : node >= a.N) { atomicOr(a.err, DERR_RANGE); node = 0; }
+      const uint32_t g = d.fo_begin + i;
+      a.fo_node[g] = node;
+      a.fo_seg[g] = s;
+      if (tree) {
+        len += num_leaf_descendents(node, a.M);
+        if (s) {
+          const uint4 r = chain_ranges_of(a, node);
+          if (node < a.N - 1) a.fo_rng[g] = r;
+          items += segs_of(r.y) + segs_of(r.w);
+        }
+      }
+    } else {
+      uint32_t node = rd32(d.base + d.map_off + 8ull * i), prev = rd32(d.base + d.map_off + 8ull * i + 4);
+      if (tree ? (node > a.M || prev > a.M) : node >= a.N) {
+        atomicOr(a.err, DERR_RANGE);
+        node = 0;
+        prev = 0;
+      }
+      const uint32_t h = d.sh_begin + i;
+      a.sh_node[h] = node;
+      a.sh_prev[h] = prev;
+      a.sh_seg[h] = s;
+      if (tree) items += s ? chain_rm_items(a, node) : num_leaf_descendents(prev, a.M);
+    }
+  }
+  if (!tree) return;
+  uint64_t total;
+  block_excl_scan(items, sh, &total);
+  if (threadIdx.x == 0) (fo ? a.tile_items : a.tile_sh)[tile] = total;
+  if (!fo) return;
+  block_excl_scan(len, sh, &total);
+  if (threadIdx.x == 0) a.tile_len[tile] = total;
+}
+
+// Sum of v[lo .. hi), or with kScanned (v holds exclusive prefixes) their
+// difference.
+template <bool kScanned>
+__device__ __forceinline__ uint64_t sum_tiles(const uint64_t* v, uint32_t lo, uint32_t hi, uint64_t* sh) {
+  if (kScanned) return v[hi] - v[lo];
+  uint64_t part = 0, off;
+  for (uint32_t q = lo + threadIdx.x; q < hi; q += blockDim.x) part += v[q];
+  block_excl_scan(part, sh, &off);
+  return off;
+}
+
+// Exclusive prefix over a tile whose warps hold kScanPerThread rows of 32
+// consecutive values each (row r of warp w: entries (8 w + r) * 32 + lane):
+// coalesced, a shuffle scan per row and one block scan of the warps' sums.
+__device__ __forceinline__ uint64_t tile_prefix(uint64_t v[kScanPerThread], uint64_t* sh) {
+  const uint32_t lane = threadIdx.x & 31;
+  uint64_t run = 0;
+#pragma unroll
+  for (int r = 0; r < kScanPerThread; r++) {
+    const uint64_t x = v[r], incl = warp_incl_scan(x);
+    v[r] = run + incl - x;
+    run += __shfl_sync(0xffffffffu, incl, 31);
   }
   uint64_t total;
-  block_excl_scan(sum, sh, &total);
-  if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
+  const uint64_t before = block_excl_scan(lane == 31 ? run : 0, sh, &total);
+  const uint64_t mine = __shfl_sync(0xffffffffu, before, 31);
+#pragma unroll
+  for (int r = 0; r < kScanPerThread; r++) v[r] += mine;
+  return total;
 }
-__global__ void __launch_bounds__(kScanThreads, 3) entry_scan_emit_kernel(EntryScans e, const uint64_t* tile_sums) {
+
+// 2. Number the entries (tree: chunks before an FO entry in its diff, its table
+// items, a shift entry's items; totals in tot), find every shift entry's source
+// checkpoint -- the smallest j with i < prefix[j] (src/tree_approach.cpp
+// :894-898), 0 if none -- and the main checkpoint's lowest FO entry per node or
+// chunk.
+template <bool kScanned>
+__global__ void __launch_bounds__(kScanThreads) entry_number_kernel(RArgs a) {
   __shared__ uint64_t sh[33];
-  const int k = entry_scan_seg(e, blockIdx.x);
-  uint64_t part = 0;
-  for (uint32_t q = e.first[k] + threadIdx.x; q < blockIdx.x; q += blockDim.x) part += tile_sums[q];
-  uint64_t off;
-  block_excl_scan(part, sh, &off);
-  const uint64_t base = (uint64_t)(blockIdx.x - e.first[k]) * kScanTile;
-  uint64_t v[kScanPerThread];
-  uint64_t sum = 0;
+  const bool tree = a.approach == APPROACH_TREE;
+  const bool fo = blockIdx.x < a.n_fo_tiles;
+  const uint32_t tile = fo ? blockIdx.x : blockIdx.x - a.n_fo_tiles;
+  const uint32_t s = tile_diff(a.di, a.ndiff, tile, fo);
+  const DiffInfo d = a.di[s];
+  const uint32_t first = fo ? d.fo_tile : d.sh_tile, n = fo ? d.F : d.S, begin = fo ? d.fo_begin : d.sh_begin;
+  const uint32_t i0 = (tile - first) * kEntryTile + (threadIdx.x >> 5) * (32 * kScanPerThread) + (threadIdx.x & 31);
+  const bool last = (tile - first + 1) * (uint64_t)kEntryTile >= n;  // the diff's last tile
+  uint32_t node[kScanPerThread];
 #pragma unroll
-  for (int q = 0; q < kScanPerThread; q++) {
-    const uint64_t i = base + (uint64_t)threadIdx.x * kScanPerThread + q;
-    v[q] = i < e.n[k] ? entry_scan_val(e, k, i, false) : 0;
-    sum += v[q];
+  for (int r = 0; r < kScanPerThread; r++) {
+    const uint32_t i = i0 + 32 * r;
+    node[r] = i < n ? (fo ? a.fo_node : a.sh_node)[begin + i] : 0;
   }
-  uint64_t tile_total;
-  uint64_t ex = block_excl_scan(sum, sh, &tile_total) + off;
-  if (threadIdx.x == 0 && blockIdx.x + 1 == e.first[k + 1]) {
-    if (k == 1) e.a.tot[0] = off + tile_total;
-    if (k == 2) e.a.tot[4] = off + tile_total;
-  }
+  if (fo && s == 0 && a.S0) {
 #pragma unroll
-  for (int q = 0; q < kScanPerThread; q++) {
-    const uint64_t i = base + (uint64_t)threadIdx.x * kScanPerThread + q;
-    if (i < e.n[k]) {
-      if (k == 0) {
-        e.a.fo_excl[i] = ex;
-      } else if (k == 1) {
-        e.a.dm_excl[i] = ex;
-      } else {
-        StoreShiftExcl{e.a}(i, ex, v[q]);
+    for (int r = 0; r < kScanPerThread; r++)
+      if (i0 + 32 * r < n) atomicMin(&a.fo_at[node[r]], i0 + 32 * r);  // range checked while decoding
+  }
+  if (!fo) {
+    const uint32_t* r = a.rrs + d.rrs_begin;
+    for (int q = 0; q < kScanPerThread; q++) {
+      const uint32_t i = i0 + 32 * q;
+      if (i >= n) break;
+      uint32_t lo = 0, hi = d.id + 1;  // first j in [0, id] with r[j] > i
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (r[mid] > i) hi = mid; else lo = mid + 1;
       }
+      a.sh_tree[begin + i] = lo <= d.id ? lo : 0;
     }
-    ex += v[q];
+  }
+  if (!tree) return;
+  uint64_t v[kScanPerThread];
+  if (fo) {
+    const uint64_t off = sum_tiles<kScanned>(a.tile_len, first, tile, sh);
+#pragma unroll
+    for (int r = 0; r < kScanPerThread; r++) v[r] = i0 + 32 * r < n ? num_leaf_descendents(node[r], a.M) : 0;
+    const uint64_t total = tile_prefix(v, sh);
+#pragma unroll
+    for (int r = 0; r < kScanPerThread; r++) {
+      const uint32_t i = i0 + 32 * r;
+      if (i >= n) continue;
+      a.fo_clen[begin + i] = (uint32_t)(off + v[r]);
+      if (s == 0) a.fo_excl[i] = off + v[r];
+    }
+    if (s == 0) {
+      if (last && threadIdx.x == 0) a.tot[2] = off + total;
+      return;
+    }
+  }
+  const uint64_t* sums = fo ? a.tile_items : a.tile_sh;
+  const uint64_t off = sum_tiles<kScanned>(sums, 0, tile, sh);
+#pragma unroll
+  for (int r = 0; r < kScanPerThread; r++) {
+    const uint32_t i = i0 + 32 * r;
+    v[r] = 0;
+    if (i >= n) continue;
+    if (fo) {
+      const uint4 rg = chain_ranges_at(a, begin + i, node[r]);
+      v[r] = segs_of(rg.y) + segs_of(rg.w);
+    } else {
+      v[r] = s ? chain_rm_items(a, node[r]) : num_leaf_descendents(a.sh_prev[i], a.M);
+    }
+  }
+  const uint64_t total = tile_prefix(v, sh);
+#pragma unroll
+  for (int r = 0; r < kScanPerThread; r++) {
+    const uint32_t i = i0 + 32 * r;
+    if (i >= n) continue;
+    if (fo) a.dm_excl[begin + i - a.fo_cb] = off + v[r];
+    else a.sh_excl[begin + i] = off + v[r];
+  }
+  if (threadIdx.x == 0) {
+    if (fo && tile + 1 == a.n_fo_tiles) a.tot[0] = off + total;
+    if (!fo && s == 0 && last) a.tot[3] = off + total;
+    if (!fo && tile + 1 == a.n_sh_tiles) a.tot[4] = off + total;
   }
 }
 
@@ -604,9 +599,9 @@ __global__ void __launch_bounds__(256) chain_tables_kernel(RArgs a) {
   // (the per-segment work is a chain of dependent loads)
   __shared__ ExpandTile<kChainTile> T;
   if (a.nsteps == 0) return;
-  const uint64_t rbase = a.tot[3];  // repeat-map segments are numbered from here
-  const TwoLists<kChainTile> L(a.tot[0], a.tot[4] - rbase);
   const bool tree = a.approach == APPROACH_TREE;
+  const uint64_t rbase = tree ? a.tot[3] : 0;  // repeat-map segments are numbered from here
+  const TwoLists<kChainTile> L(tree ? a.tot[0] : a.nfo - a.fo_cb, tree ? a.tot[4] - rbase : a.nsh - a.sh_cb);
   const uint32_t leaf0 = a.N - 1;
   for (uint64_t tile = blockIdx.x; tile < L.tiles(); tile += gridDim.x) {
     const bool rm = tile >= L.nt0;
@@ -638,13 +633,14 @@ __global__ void __launch_bounds__(256) chain_tables_kernel(RArgs a) {
         uint32_t s = 0, x0 = 0, cnt = 0, pos0 = 0;
         if (in) {
           s = a.fo_seg[g] - 1;
-          const uint4 r = a.fo_rng[g];
+          const uint32_t node = a.fo_node[g];
+          const uint4 r = chain_ranges_at(a, g, node);
           const uint32_t n0 = segs_of(r.y);
           x0 = j < n0 ? r.x + j * kSegKeys : r.z + (j - n0) * kSegKeys;
           const uint32_t left = j < n0 ? r.y - j * kSegKeys : r.w - (j - n0) * kSegKeys;
           cnt = left < kSegKeys ? left : kSegKeys;
           // position of leaf x in the step's data: fo_clen + x - leftmost leaf
-          pos0 = a.fo_clen[g] + x0 - leftmost_leaf(a.fo_node[g], a.M);
+          pos0 = a.fo_clen[g] + x0 - leftmost_leaf(node, a.M);
         }
         k0 = x0 - leaf0;
         // 32 full, 32-key aligned, consecutive segments of one entry (the
@@ -673,10 +669,9 @@ __global__ void __launch_bounds__(256) chain_tables_kernel(RArgs a) {
         // list / basic: one chunk per entry
         const uint32_t g = a.fo_cb + k;
         const uint32_t s = a.fo_seg[g] - 1;
-        const uint4 r = a.fo_rng[g];
-        if (r.x >= a.N) continue;
-        k0 = r.x;
-        a.dm_off[(uint64_t)s * a.K + k0] = a.fo_clen[g];
+        k0 = a.fo_node[g];
+        if (k0 >= a.N) continue;
+        a.dm_off[(uint64_t)s * a.K + k0] = g - a.di[s + 1].fo_begin;
         lo = 1u << (k0 & 31);
         seg_bits(a, s, 0, k0, lo, hi);
       } else {
@@ -1133,7 +1128,7 @@ static uint32_t restart_parts(uint32_t N) {
 struct RestartScratch {
   DevBuf<DiffInfo> di;
   DevBuf<uint32_t> fo_node, fo_seg, fo_clen, sh_node, sh_prev, sh_tree, sh_seg, rrs, fo_at, dm_off, sbm;
-  DevBuf<uint64_t> fo_excl, sh_off, sh_excl, nl_rank, cp_rank, dm_excl, tot, scan, scan_total, rm_tab, srcp;
+  DevBuf<uint64_t> fo_excl, sh_off, sh_excl, nl_rank, cp_rank, dm_excl, tot, scan, rm_tab, srcp;
   DevBuf<uint32_t> nbv;
   DevBuf<uint4> fo_rng;
   // epochs: repeat-map cells and the main scatter ranks hold the epoch of
@@ -1165,7 +1160,6 @@ int Engine::read_headers(const std::vector<const uint8_t*>& ptrs, const std::vec
   const size_t n = ptrs.size(), bytes = n * sizeof(HeaderHost);
   out.assign(n, HeaderHost{});
   if (n == 0) return ST_OK;
-  MTC_CUDA_R(hdr_dev_.ensure(bytes, stream_));
   if (hdr_host_cap_ < bytes) {
     // grown geometrically, as the descriptors below
     const size_t cap = std::max<size_t>({bytes, 2 * hdr_host_cap_, 16u << 10});
@@ -1175,6 +1169,9 @@ int Engine::read_headers(const std::vector<const uint8_t*>& ptrs, const std::vec
     MTC_CUDA_R(cudaMallocHost(reinterpret_cast<void**>(&hdr_host_), cap));
     hdr_host_cap_ = cap;
   }
+  // written to the pinned memory by the kernel: a copy would queue on a copy
+  // engine
+  uint8_t* host_hdr = static_cast<uint8_t*>(host_alias(hdr_host_));
   for (size_t i0 = 0; i0 < n; i0 += kHeaderBatch) {
     HeaderSrc src{};
     src.n = (uint32_t)std::min<size_t>(kHeaderBatch, n - i0);
@@ -1183,11 +1180,10 @@ int Engine::read_headers(const std::vector<const uint8_t*>& ptrs, const std::vec
       src.len[k] = lens[i0 + k];
     }
     const uint32_t threads = src.n * (uint32_t)sizeof(HeaderHost);
-    header_gather_kernel<<<(threads + 255) / 256, 256, 0, stream_>>>(src, hdr_dev_.p + i0 * sizeof(HeaderHost));
+    header_gather_kernel<<<(threads + 255) / 256, 256, 0, stream_>>>(src, host_hdr + i0 * sizeof(HeaderHost));
     note_launch();
     MTC_CUDA_R(cudaGetLastError());
   }
-  MTC_CUDA_R(cudaMemcpyAsync(hdr_host_, hdr_dev_.p, bytes, cudaMemcpyDeviceToHost, stream_));
   MTC_CUDA_R(cudaStreamSynchronize(stream_));
   std::memcpy(out.data(), hdr_host_, bytes);
   return ST_OK;
@@ -1201,7 +1197,7 @@ uint64_t Engine::restart_scratch_bytes() const {
                         &R.fo_at, &R.dm_off, &R.sbm, &R.nbv})
     b += sizeof(uint32_t) * x->n;
   for (const auto* x : {&R.fo_excl, &R.sh_off, &R.sh_excl, &R.nl_rank, &R.cp_rank, &R.dm_excl, &R.tot, &R.scan,
-                        &R.scan_total, &R.rm_tab, &R.srcp})
+                        &R.rm_tab, &R.srcp})
     b += sizeof(uint64_t) * x->n;
   return b;
 }
@@ -1213,7 +1209,7 @@ static void set_scratch_pool(RestartScratch* r, cudaMemPool_t pool) {
                   &r->fo_at, &r->dm_off, &r->sbm})
     b->pool = pool;
   for (auto* b : {&r->fo_excl, &r->sh_off, &r->sh_excl, &r->nl_rank, &r->cp_rank, &r->dm_excl, &r->tot,
-                  &r->scan, &r->scan_total, &r->rm_tab, &r->srcp})
+                  &r->scan, &r->rm_tab, &r->srcp})
     b->pool = pool;
   r->nbv.pool = pool;
 }
@@ -1278,7 +1274,7 @@ int Engine::restart_enqueue(uint8_t* dev_out, uint64_t len, const std::vector<co
   std::vector<uint32_t> slots(1, id);
   for (uint32_t x : steps) slots.push_back(x);
   std::vector<DiffInfo> di(slots.size());
-  uint32_t nfo = 0, nsh = 0, nrrs = 0;
+  uint32_t nfo = 0, nsh = 0, nrrs = 0, n_fo_tiles = 0, n_sh_tiles = 0;
   for (size_t k = 0; k < slots.size(); k++) {
     const uint32_t idx = slots[k];
     const HeaderHost& h = headers[idx];
@@ -1303,6 +1299,8 @@ int Engine::restart_enqueue(uint8_t* dev_out, uint64_t len, const std::vector<co
     d.fo_begin = nfo;
     d.sh_begin = nsh;
     d.rrs_begin = nrrs;
+    d.fo_tile = n_fo_tiles;
+    d.sh_tile = n_sh_tiles;
     // entry indices are 32-bit on the device, shift entries doubled in the
     // table cells (2h + 1)
     if ((uint64_t)nfo + d.F >= 0xffffffffull || (uint64_t)nsh + d.S >= (1ull << 31) ||
@@ -1311,6 +1309,8 @@ int Engine::restart_enqueue(uint8_t* dev_out, uint64_t len, const std::vector<co
     nfo += d.F;
     nsh += d.S;
     nrrs += d.id + 1;
+    n_fo_tiles += (uint32_t)(((uint64_t)d.F + kEntryTile - 1) / kEntryTile);
+    n_sh_tiles += (uint32_t)(((uint64_t)d.S + kEntryTile - 1) / kEntryTile);
   }
   const uint32_t W = (nsteps + 31) / 32 ? (nsteps + 31) / 32 : 1;
   const uint32_t K = approach == APPROACH_TREE ? N + 1 : N;
@@ -1321,8 +1321,8 @@ int Engine::restart_enqueue(uint8_t* dev_out, uint64_t len, const std::vector<co
   RestartScratch& R = *rs_;
   StepTimer t_alloc("restart: table allocations", N);
   MTC_CUDA_R(R.di.ensure(di.size(), s));
-  // the chain descriptors go up from pinned memory: a copy from pageable
-  // memory would first wait for everything already on the stream
+  // the chain descriptors are read from pinned memory by the first kernel: a copy
+  // from pageable memory would first wait for everything already on the stream
   StepTimer t_up("restart: descriptor upload", N);
   const size_t di_bytes = sizeof(DiffInfo) * di.size();
   if (rdi_ev_) MTC_CUDA_R(cudaEventSynchronize(rdi_ev_));  // the previous restart's copy has read it
@@ -1338,26 +1338,27 @@ int Engine::restart_enqueue(uint8_t* dev_out, uint64_t len, const std::vector<co
     rdi_host_bytes_ = cap;
   }
   std::memcpy(rdi_host_, di.data(), di_bytes);
-  MTC_CUDA_R(cudaMemcpyAsync(R.di.p, rdi_host_, di_bytes, cudaMemcpyHostToDevice, s));
-  MTC_CUDA_R(cudaEventRecord(rdi_ev_, s));
+  const bool tree = approach == APPROACH_TREE;
   MTC_CUDA_R(R.fo_node.ensure(nfo + 1, s));
   MTC_CUDA_R(R.fo_seg.ensure(nfo + 1, s));
-  MTC_CUDA_R(R.fo_rng.ensure(nfo + 1, s));
-  MTC_CUDA_R(R.fo_clen.ensure(nfo + 1, s));
-  MTC_CUDA_R(R.fo_excl.ensure(nfo + 1, s));
   MTC_CUDA_R(R.sh_node.ensure(nsh + 1, s));
   MTC_CUDA_R(R.sh_prev.ensure(nsh + 1, s));
   MTC_CUDA_R(R.sh_tree.ensure(nsh + 1, s));
   MTC_CUDA_R(R.sh_seg.ensure(nsh + 1, s));
-  MTC_CUDA_R(R.sh_off.ensure(nsh + 1, s));
-  MTC_CUDA_R(R.sh_excl.ensure(nsh + 1, s));
+  MTC_CUDA_R(R.sh_off.ensure(di[0].S + 1, s));
+  if (tree) {  // list and basic: every entry is one chunk, and its own number
+    MTC_CUDA_R(R.fo_rng.ensure(nfo + 1, s));
+    MTC_CUDA_R(R.fo_clen.ensure(nfo + 1, s));
+    MTC_CUDA_R(R.fo_excl.ensure(di[0].F + 1, s));
+    MTC_CUDA_R(R.sh_excl.ensure(nsh + 1, s));
+    MTC_CUDA_R(R.dm_excl.ensure(nfo - di[0].F + 1, s));
+  }
   MTC_CUDA_R(R.rrs.ensure(nrrs + 1, s));
   MTC_CUDA_R(R.nl_rank.ensure(N, s));
   MTC_CUDA_R(R.cp_rank.ensure(N, s));
   MTC_CUDA_R(R.srcp.ensure(N, s));
   MTC_CUDA_R(R.nbv.ensure(N, s));
   MTC_CUDA_R(R.fo_at.ensure((size_t)M + 2, s));
-  MTC_CUDA_R(R.dm_excl.ensure(nfo + 1, s));
   MTC_CUDA_R(R.tot.ensure(5, s));
   const uint32_t KW = (K + 31) / 32;
   MTC_CUDA_R(R.dm_off.ensure((size_t)std::max<uint32_t>(nsteps, 1) * K, s));
@@ -1374,12 +1375,9 @@ int Engine::restart_enqueue(uint8_t* dev_out, uint64_t len, const std::vector<co
     R.epoch = 0;
   }
   R.epoch++;
-  const uint64_t scan_n = std::max<uint64_t>(nfo, nsh) + 1;
-  // tile sums: one scan at a time, or the three entry scans side by side
-  MTC_CUDA_R(R.scan.ensure(3 * (scan_n / kScanTile + 2), s));
-  MTC_CUDA_R(R.scan_total.ensure(1, s));
+  // per tile: FO chunks, FO table items, shift items
+  MTC_CUDA_R(R.scan.ensure(2 * (size_t)n_fo_tiles + n_sh_tiles + 3, s));
   MTC_CUDA_R(err_.ensure(1, s));
-  MTC_CUDA_R(cudaMemsetAsync(err_.p, 0, sizeof(uint32_t), s));
 
   RArgs a{};
   a.approach = approach;
@@ -1402,8 +1400,13 @@ int Engine::restart_enqueue(uint8_t* dev_out, uint64_t len, const std::vector<co
   a.dm_off = R.dm_off.p; a.rm_tab = R.rm_tab.p; a.sbm = R.sbm.p; a.KW = KW;
   a.dm_excl = R.dm_excl.p; a.tot = R.tot.p;
   a.fo_rng = R.fo_rng.p;
+  a.tile_len = R.scan.p;
+  a.tile_items = R.scan.p + n_fo_tiles + 1;
+  a.tile_sh = R.scan.p + 2 * (size_t)n_fo_tiles + 2;
+  a.n_fo_tiles = n_fo_tiles;
+  a.n_sh_tiles = n_sh_tiles;
+  a.n_rrs = basic ? 0 : std::min<uint32_t>((uint32_t)di.size(), 4 * num_sms());
   a.out = dev_out; a.err = err_.p;
-  const bool tree = approach == APPROACH_TREE;
 
   // The second stream: clears that depend on nothing run there at once; the
   // chain tables run there beside the main checkpoint's scatter; each range
@@ -1416,45 +1419,33 @@ int Engine::restart_enqueue(uint8_t* dev_out, uint64_t len, const std::vector<co
   StepTimer t_fork("restart: fork and clears", N);
   MTC_CUDA_R(cudaEventRecord(rev_[0], s));  // after the allocations and the previous restart
   MTC_CUDA_R(cudaStreamWaitEvent(side, rev_[0], 0));
-  MTC_CUDA_R(cudaMemsetAsync(R.fo_at.p, 0xff, sizeof(uint32_t) * ((size_t)M + 2), side));
-  if (nsteps) MTC_CUDA_R(cudaMemsetAsync(R.sbm.p, 0, sizeof(uint32_t) * (size_t)KW * W * 32 * 2, side));
+  // (the lowest entry per node only serves the main checkpoint's shift entries)
+  if (a.S0) MTC_CUDA_R(cudaMemsetAsync(R.fo_at.p, 0xff, sizeof(uint32_t) * ((size_t)M + 2), side));
   MTC_CUDA_R(cudaEventRecord(rev_[1], side));
+  if (nsteps) MTC_CUDA_R(cudaMemsetAsync(R.sbm.p, 0, sizeof(uint32_t) * (size_t)KW * W * 32 * 2, side));
 
-  // 1-3: decode entries, repeat tables, source checkpoints
+  // 1-2: decode and number the entries, repeat tables, source checkpoints
   StepTimer t_dec("restart: entry launches", N);
-  MTC_CUDA_R(cudaMemsetAsync(R.tot.p, 0, sizeof(uint64_t) * 5, s));
-  if (nfo + nsh) { load_entries_kernel<<<gsz((uint64_t)nfo + nsh), 256, 0, s>>>(a); note_launch(); }
-  rrs_kernel<<<gsz(di.size(), 1, 4), 256, 0, s>>>(a);
+  setup_kernel<<<1, 256, 0, s>>>(static_cast<const uint4*>(host_alias(rdi_host_)), reinterpret_cast<uint4*>(R.di.p),
+                                 (uint32_t)(di_bytes / 16), err_.p, R.tot.p);
+  MTC_CUDA_R(cudaEventRecord(rdi_ev_, s));
   note_launch();
-  if (nsh) { shift_tree_kernel<<<gsz(nsh), 256, 0, s>>>(a); note_launch(); }
-  const uint32_t nfo_chain = nsteps ? nfo - a.fo_cb : 0;
-  const uint64_t tiles[3] = {(nfo + kScanTile - 1) / kScanTile, (nfo_chain + kScanTile - 1) / kScanTile,
-                             (nsh + kScanTile - 1) / kScanTile};
-  const bool fused = tiles[0] <= reduce_tile_limit() && tiles[1] <= reduce_tile_limit() &&
-                     tiles[2] <= reduce_tile_limit() && tiles[0] + tiles[1] + tiles[2] > 0;
-  if (fused) {
-    // the three entry scans in one pair of launches
-    EntryScans e{a, {nfo, nfo_chain, nsh}, {0, (uint32_t)tiles[0], (uint32_t)(tiles[0] + tiles[1]),
-                                            (uint32_t)(tiles[0] + tiles[1] + tiles[2])}};
-    entry_scan_sums_kernel<<<e.first[3], kScanThreads, 0, s>>>(e, R.scan.p);
-    entry_scan_emit_kernel<<<e.first[3], kScanThreads, 0, s>>>(e, R.scan.p);
-    note_launch(2);
-  } else {
-    // chunk_len of every FO entry within its own diff
-    if (nfo) MTC_CUDA_R(grid_scan(FoLen{R.fo_node.p, M, tree ? 1 : 0}, StoreExcl{R.fo_excl.p}, nullptr, nfo,
-                                  R.scan.p, R.scan_total.p, s));
-    // items of the main shift regions and of the chain's repeat maps
-    if (nsh) MTC_CUDA_R(grid_scan(ShiftItems{a}, StoreShiftExcl{a}, nullptr, nsh, R.scan.p, R.tot.p + 4, s));
-    if (nfo_chain) {
-      chain_ranges_kernel<<<gsz(nfo_chain), 256, 0, s>>>(a, nfo_chain);
-      note_launch();
-      MTC_CUDA_R(grid_scan(ChainDmCount{a}, StoreExcl{R.dm_excl.p}, nullptr, nfo_chain, R.scan.p, R.tot.p + 0, s));
-    }
+  const uint32_t ntiles = n_fo_tiles + n_sh_tiles;
+  if (ntiles + a.n_rrs) {
+    entry_load_kernel<<<ntiles + a.n_rrs, kScanThreads, 0, s>>>(a);
+    note_launch();
   }
-  // chunk_len relative to each FO entry's own diff; the main checkpoint's FO
-  // items (tot[2])
-  if (nfo) {
-    clen_kernel<<<gsz(nfo), 256, 0, s>>>(a);
+  if (ntiles && !basic) {  // a basic entry's number is its index, and it has no shift entries
+    const bool scanned = tree && std::max(n_fo_tiles, n_sh_tiles) > reduce_tile_limit();
+    if (scanned) {
+      for (auto v : {std::make_pair(a.tile_len, n_fo_tiles), std::make_pair(a.tile_items, n_fo_tiles),
+                     std::make_pair(a.tile_sh, n_sh_tiles)})
+        scan_tile_offsets_kernel<<<1, 1024, 0, s>>>(v.first, v.second, nullptr);
+      note_launch(3);
+    }
+    MTC_CUDA_R(cudaStreamWaitEvent(s, rev_[1], 0));
+    if (scanned) entry_number_kernel<true><<<ntiles, kScanThreads, 0, s>>>(a);
+    else entry_number_kernel<false><<<ntiles, kScanThreads, 0, s>>>(a);
     note_launch();
   }
   // chain tables on the second stream, after the clears and the entries
@@ -1466,14 +1457,9 @@ int Engine::restart_enqueue(uint8_t* dev_out, uint64_t len, const std::vector<co
   }
   MTC_CUDA_R(cudaEventRecord(rev_[3], side));
   // main checkpoint, beside them
-  MTC_CUDA_R(cudaStreamWaitEvent(s, rev_[1], 0));
-  if (di[0].F) { fo_at_kernel<<<gsz(di[0].F), 256, 0, s>>>(a); note_launch(); }
-  if (di[0].S) {
-    main_shift_kernel<<<gsz(di[0].S), 256, 0, s>>>(a);
-    note_launch();
-  }
   if (di[0].F || di[0].S) {
-    main_cover_kernel<<<num_sms() * 8, 256, 0, s>>>(a);
+    const uint32_t n_shift = di[0].S ? std::min<uint32_t>(gsz(di[0].S), num_sms()) : 0;
+    main_cover_kernel<<<num_sms() * 8, 256, 0, s>>>(a, n_shift);
     note_launch();
   }
   MTC_CUDA_R(cudaStreamWaitEvent(s, rev_[3], 0));
