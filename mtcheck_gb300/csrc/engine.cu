@@ -71,7 +71,7 @@ static uint64_t next_pow2(uint64_t v) {
 }
 
 Engine::Engine(int mode, int hash_kind, uint32_t chunk_size)
-    : mode_(mode), hash_kind_(hash_kind), cs_(chunk_size), leaf_tune_(default_leaf_tune(hash_kind)) {
+    : mode_(mode), hash_kind_(hash_kind), cs_(chunk_size), leaf_tune_(default_leaf_tune(hash_kind, chunk_size)) {
   for (auto& e : ev_) cudaEventCreate(&e);
   cudaMallocHost(&lay_host_, sizeof(Layout));
   cudaMallocHost(&err_host_, 2 * sizeof(uint32_t));
@@ -190,7 +190,9 @@ int Engine::ensure_state(uint32_t N, bool fresh, uint32_t id_headroom) {
     M_ = M;
     const size_t nd = tree ? M : N;
     MTC_CUDA(digests_.ensure(nd, stream_));
-    MTC_CUDA(cudaMemsetAsync(digests_.p, 0, sizeof(Digest) * nd, stream_));
+    // a baseline writes every leaf's digest and, on the tree modes' baseline
+    // path, every interior node's before any is read
+    if (mode_ == MODE_TREE_LOW_OFFSET_REF) MTC_CUDA(cudaMemsetAsync(digests_.p, 0, sizeof(Digest) * nd, stream_));
     // read in 16-byte words by the list and basic compaction
     MTC_CUDA(labels_.ensure((nd + 15) / 16 * 16, stream_));
     // root flags, read in 16-byte words: zero between checkpoints (the root
@@ -335,6 +337,7 @@ int Engine::run_tree(const uint8_t* data, uint64_t len, bool baseline_path) {
   la.clk = timed_ ? clk_.p : nullptr;
   la.hash_kind = hash_kind_;
   la.epi = EPI_TREE;
+  la.fresh = fresh_ ? 1 : 0;
   la.changed_list = changed_list_.p;
   la.changed_count = changed_count_.p + COUNT_CHANGED;
   la.demoted = changed_count_.p + COUNT_DEMOTED;
@@ -392,6 +395,7 @@ int Engine::run_list_basic(const uint8_t* data, uint64_t len) {
   la.clk = timed_ ? clk_.p : nullptr;
   la.hash_kind = hash_kind_;
   la.epi = mode_ == MODE_LIST ? EPI_LIST : EPI_BASIC;
+  la.fresh = fresh_ ? 1 : 0;  // never true in a captured sequence
   la.basic_first = current_id == 0 ? 1 : 0;  // never true in a captured sequence
   la.changed_list = changed_list_.p;
   la.changed_count = changed_count_.p + COUNT_CHANGED;

@@ -39,14 +39,14 @@ __device__ __forceinline__ uint8_t child_flag(uint8_t lab) {
 
 // Passes.  0: first-occurrence forest (src/tree_approach.cpp:378-404); 1:
 // duplicate forest (:413-477); 2: both incremental passes in one traversal
-// (ForestArgs::fuse_gate); 3: both passes of a baseline (:115-227) on cleared
-// digests in one traversal, which hashes every node and leaves the inserts to
+// (ForestArgs::fuse_gate); 3: both passes of a baseline (:115-227) whose
+// digests count as cleared in one traversal, which hashes every node and leaves the inserts to
 // forest_insert_all_kernel.
 //
 // Pass 3.  A node is a first occurrence in the baseline's second pass exactly
 // when it is one in the first (both only look at the leaves' labels), with the
 // same digest, so its second hash and insert change nothing.  The shift test
-// reads a digest that is still cleared, so it asks one question of the map:
+// reads a digest that is still zero, so it asks one question of the map:
 // whether it holds the all-zero digest.  Which of the passes a node's insert
 // belongs to is kept in its epoch, and a map entry keeps the lowest (epoch,
 // priority), so the inserts may follow in any order.  4 GiB in 512-byte
@@ -204,7 +204,7 @@ __device__ __forceinline__ uint8_t span_node(const ForestArgs& a, int pass, uint
         dg = hash_pair(HK, dl, dr);
         st_digest(a.tree + n, dg);
       }
-      if (map_find(a.map, BASE ? ld_digest(a.tree + n) : dg, a.err) >= 0) lab_n = SHIFT_DUPL;
+      if (map_find(a.map, BASE ? Digest{{0, 0, 0, 0}} : dg, a.err) >= 0) lab_n = SHIFT_DUPL;
       else fl = fr = ROOT_SHIFT;
     } else if (ll == FIRST_OCUR) {
       lab_n = FIRST_OCUR;
@@ -415,7 +415,7 @@ __device__ __forceinline__ uint8_t thread_levels_bytewise(const ForestArgs& a, i
         }
         const Digest d = hash_pair(HK, dl, dr);
         if (BASE) {
-          if ((XS[q] >> (8 * b)) & 1 && map_find(a.map, ld_digest(a.tree + n), a.err) < 0) {
+          if ((XS[q] >> (8 * b)) & 1 && map_find(a.map, Digest{{0, 0, 0, 0}}, a.err) < 0) {
             set_byte(P[q], b, DONE);
             set_byte(FL[q], b, ROOT_SHIFT);
             set_byte(FR[q], b, ROOT_SHIFT);

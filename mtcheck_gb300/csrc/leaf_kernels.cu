@@ -67,7 +67,7 @@ __device__ __forceinline__ void leaf_epilogue(const LeafArgs& a, bool valid, uin
     if (!valid) return;
     uint8_t changed = 1;
     if (!a.basic_first && digest_eq(dg, old)) changed = 0;
-    if (changed) st_digest(a.prev + c, dg);
+    if (changed || a.fresh) st_digest(a.prev + c, dg);
     a.labels[c] = changed;
     return;
   }
@@ -75,12 +75,12 @@ __device__ __forceinline__ void leaf_epilogue(const LeafArgs& a, bool valid, uin
   bool changed = false;
   if (valid) {
     changed = !digest_eq(dg, old);
-    if (changed) st_digest(a.prev + c, dg);
+    if (changed || a.fresh) st_digest(a.prev + c, dg);
     a.labels[c] = changed ? PENDING : (EPI == EPI_TREE ? FIXED_DUPL : DONE);
     // A FIXED_DUPL leaf's insert() always finds its digest (every earlier
     // leaf digest was inserted) and changes nothing, so it is not repeated.
   }
-  append_changed(a, changed, c);
+  if (!a.fresh) append_changed(a, changed, c);
 }
 
 // A note for the demote pass (a changed-list position); kCheckCreator: the
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(256) leaf_insert_kernel(LeafArgs a) {
   pdl_enter();
   stamp(a.clk, CLK_LEAVES_DONE);
   __shared__ volatile uint32_t s_dups;
-  const uint32_t n = *a.changed_count;
+  const uint32_t n = a.fresh ? a.n_chunks : *a.changed_count;
   const uint32_t cur = a.sp->cur, epoch = a.sp->epoch;
   const uint32_t lane = threadIdx.x & 31;
   if (threadIdx.x == 0) s_dups = 0;
@@ -124,8 +124,9 @@ __global__ void __launch_bounds__(256) leaf_insert_kernel(LeafArgs a) {
   for (uint64_t kw = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); kw < n;
        kw += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t k = kw + lane;
-    const bool in = k < n;
-    const uint32_t c = in ? a.changed_list[k] : 0xffffffffu;
+    bool in = k < n;
+    const uint32_t c = !in ? 0xffffffffu : a.fresh ? (uint32_t)k : a.changed_list[k];
+    if (a.fresh) in = in && a.labels[c] == PENDING;
     Digest dg{{0, 0, 0, 0}};
     if (in) dg = map_key(ld_digest(a.prev + c));
     const unsigned act = __ballot_sync(0xffffffffu, in);
@@ -213,7 +214,7 @@ __global__ void leaf_demote_kernel(LeafArgs a) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t e = a.dup_list[i];
     const uint32_t k = e & ~kCheckCreator;
-    const uint32_t c = a.changed_list[k];
+    const uint32_t c = a.fresh ? k : a.changed_list[k];
     const MapSlot* s = &a.map.slots[a.chunk_slot[k]];
     demote_chunk(a, c, s, cur);
     if (e & kCheckCreator) demote_chunk(a, s->first_chunk, s, cur);
@@ -222,7 +223,7 @@ __global__ void leaf_demote_kernel(LeafArgs a) {
 
 template <int EPI>
 __device__ __forceinline__ bool needs_old(const LeafArgs& a) {
-  return EPI != EPI_HASH && !(EPI == EPI_BASIC && a.basic_first);
+  return EPI != EPI_HASH && !a.fresh && !(EPI == EPI_BASIC && a.basic_first);
 }
 
 // ---------------------------------------------------------------------------
@@ -375,7 +376,7 @@ constexpr uint32_t kMetaFirst = 1, kMetaLast = 2, kMetaDone = 4;
 constexpr uint32_t kBatchStageBytes = kBatchRows * 128;
 
 __device__ __forceinline__ bool needs_old_rt(const LeafArgs& a) {
-  return a.epi != EPI_HASH && !(a.epi == EPI_BASIC && a.basic_first);
+  return a.epi != EPI_HASH && !a.fresh && !(a.epi == EPI_BASIC && a.basic_first);
 }
 
 __global__ void __launch_bounds__(kBatchRows + 32, 3) batch_leaf_kernel(BatchLeafParams p) {

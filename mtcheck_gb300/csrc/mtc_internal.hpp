@@ -75,6 +75,12 @@ struct LeafArgs {
   int hash_kind = HASH_MURMUR3;
   int epi = EPI_HASH;
   int basic_first = 0;            // basic approach with current_id == 0: every chunk changed
+  // A baseline: the previous digests are all zero and not read (the buffer need
+  // not be cleared), every digest is stored, and the insert pass takes the
+  // chunks in order instead of a list.  An append per warp to one counter
+  // took a third of the hashing kernel of 2^23 chunks of 128 bytes (324 us,
+  // now 191-208), and more with more blocks per SM (480 us).
+  int fresh = 0;
   // Fault injection for the failure-detection tests: the TMA producer issues
   // no copy, so every consumer's bounded wait runs out after `spin_limit`
   // polls and the launch ends with DERR_SPIN, no copy in flight.  0 in
@@ -111,11 +117,17 @@ struct LeafTune {
   int direct = 0;
   int threads_per_chunk = 1;
 };
-// Default shape per digest, measured at 4 GiB / 512 B: Murmur3 tiles of 128
-// rows, two CTAs per SM (0.652 ms against 0.691 for 256 rows); MD5, whose
-// hashing is ALU-bound, 256 rows and as many CTAs as fit (0.948 ms).
-inline LeafTune default_leaf_tune(int hash_kind) {
-  return hash_kind == HASH_MD5 ? LeafTune{256, 0, 0} : LeafTune{128, 2, 0};
+// Default shape per digest and chunk size.  Murmur3: tiles of 128 rows and two
+// CTAs per SM (4 GiB in 512-byte chunks: 0.652 ms against 0.691 for 256 rows).
+// A tile of chunks below 128 bytes is one box of a few kilobytes, so it takes
+// more CTAs to keep the same bytes in flight (two / three / six per SM: 200 MB
+// in 64-byte chunks 65 / 56 / 52 us, 256 MiB in 32-byte chunks 135 / 102 / 87
+// us, 128 MiB in 16-byte chunks 131 / 95 / 67 us; 1 GiB in 128-byte chunks 202
+// / 194 / 205 us, in 256-byte chunks 178 / 187 / 194 us).  MD5, whose hashing
+// is ALU-bound: 256 rows and as many CTAs as fit (4 GiB: 0.948 ms).
+inline LeafTune default_leaf_tune(int hash_kind, uint32_t cs) {
+  if (hash_kind == HASH_MD5) return LeafTune{256, 0, 0};
+  return LeafTune{128, cs < 128 ? 6 : cs == 128 ? 3 : 2, 0};
 }
 
 // Launch the leaf hashing kernel(s) over every chunk.  Uses the TMA pipeline
