@@ -358,6 +358,179 @@ __global__ void leaf_direct_kernel(LeafArgs a, uint32_t c0, uint32_t c1) {
 }
 
 // ---------------------------------------------------------------------------
+// Staged kernel for what the tiled copies cannot take: chunk sizes that are no
+// supported box width, and buffers off a 16-byte boundary.  One thread hashes
+// one chunk, 128 chunks per tile, in panels of 128 bytes that come through
+// shared memory: a thread that reads its own chunk from global memory touches
+// a line per lane.  Rows of a panel start on 16 bytes of shared memory whatever
+// the chunk's address, so the copies are as wide as that allows (cp.async of 16,
+// 8 or 4 bytes) and a thread reads its row in 16-byte words, without bank
+// conflicts at a stride of 144 bytes; an address off a 4-byte boundary is
+// shifted in registers.  kStageBufs panels in flight per block.  Bound by HBM
+// for Murmur3 at 16 bytes per copy, by issue below, by the integer pipe for
+// MD5.  1 GiB in 4096-byte chunks 4 bytes off a boundary: 376 us (MD5 486), with
+// direct loads 1054 us (991).
+// ---------------------------------------------------------------------------
+constexpr int kStageRows = 128;
+constexpr int kStageBufs = 3;
+constexpr uint32_t kPanel = 128;                       // bytes of a chunk per step
+constexpr uint32_t kRowStride = kPanel + 16;
+constexpr uint32_t kStagedBytes = kStageRows * kRowStride;  // one buffer
+
+template <int B>
+__device__ __forceinline__ void cp_async(uint32_t smem, uint64_t gmem) {
+  if (B == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(gmem) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem), "l"(gmem), "n"(B) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Copies of one panel: each warp its own 32 rows, 128 / B lanes a row.  p0: the
+// panel's first byte in the warp's first row; n_rows of the warp's rows exist;
+// nb: bytes of a whole chunk in the panel; end: of the buffer.  Only words that
+// hold a byte of a chunk are read.  With B = 4 a row starts at the word that
+// holds its first byte, and may need a 33rd word.
+template <int B>
+__device__ __forceinline__ void stage_panel(uint32_t sm, uint64_t p0, uint64_t cs, uint32_t n_rows, uint32_t nb,
+                                            uint64_t end) {
+  constexpr uint32_t kLanes = kPanel / B, kRows = 32 / kLanes;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t sub = lane / kLanes, w = lane % kLanes;
+#pragma unroll 4
+  for (uint32_t r = sub; r < n_rows; r += kRows) {
+    const uint64_t p = p0 + r * cs, lo = p & ~(uint64_t)(B - 1);
+    const uint64_t stop = p + nb < end ? p + nb : end, at = lo + w * B;
+    if (at < stop) cp_async<B>(sm + r * kRowStride + w * B, at);
+  }
+  if (B == 4 && lane < n_rows) {
+    const uint64_t p = p0 + lane * cs, at = (p & ~3ull) + kPanel;
+    const uint64_t stop = p + nb < end ? p + nb : end;
+    if (at < stop) cp_async<B>(sm + lane * kRowStride + kPanel, at);
+  }
+}
+
+template <int HK, int EPI>
+__global__ void __launch_bounds__(kStageRows, 4) leaf_staged_kernel(LeafArgs a, uint32_t c0, uint32_t c1) {
+  pdl_enter();
+  extern __shared__ __align__(16) uint8_t sm_raw[];
+  const uint32_t tid = threadIdx.x, warp = tid >> 5;
+  const uint64_t cs = a.cs;
+  const uint64_t base = reinterpret_cast<uint64_t>(a.data), end = base + a.len;
+  const uint32_t steps = (uint32_t)((cs + kPanel - 1) / kPanel);
+  const uint32_t ntiles = (c1 - c0 + kStageRows - 1) / kStageRows;
+  const uint32_t mine = blockIdx.x < ntiles ? (ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+  const uint64_t total = (uint64_t)mine * steps;  // steps of this block, tile by tile
+  const uint32_t align = (uint32_t)(base | cs) & 15;  // of every row
+  const uint32_t sm0 = smem_u32(sm_raw);
+
+  uint32_t ld_tile = blockIdx.x, ld_step = 0;
+  auto load = [&](uint32_t buf) {
+    const uint64_t row0 = (uint64_t)c0 + (uint64_t)ld_tile * kStageRows + warp * 32;
+    const uint32_t n_rows = row0 >= c1 ? 0 : c1 - row0 < 32 ? (uint32_t)(c1 - row0) : 32;
+    const uint64_t done = (uint64_t)ld_step * kPanel;
+    const uint32_t nb = cs - done < kPanel ? (uint32_t)(cs - done) : kPanel;
+    const uint64_t p0 = base + row0 * cs + done;
+    const uint32_t sm = sm0 + buf * kStagedBytes + warp * 32 * kRowStride;
+    if (align == 0) stage_panel<16>(sm, p0, cs, n_rows, nb, end);
+    else if ((align & 7) == 0) stage_panel<8>(sm, p0, cs, n_rows, nb, end);
+    else stage_panel<4>(sm, p0, cs, n_rows, nb, end);
+    if (++ld_step == steps) {
+      ld_step = 0;
+      ld_tile += gridDim.x;
+    }
+  };
+
+  uint64_t issued = 0;
+#pragma unroll
+  for (int k = 0; k < kStageBufs - 1; k++) {
+    if (issued < total) load((uint32_t)(issued % kStageBufs));
+    issued++;
+    cp_async_commit();
+  }
+  Murmur3State mm;
+  Md5State md;
+  Digest old{{0, 0, 0, 0}};
+  uint32_t tile = blockIdx.x, step = 0, buf = 0;
+  for (uint64_t k = 0; k < total; k++) {
+    const uint64_t c = (uint64_t)c0 + (uint64_t)tile * kStageRows + tid;
+    const bool valid = c < c1;
+    if (step == 0) {
+      if (HK == HASH_MD5) md.init(); else mm.init();
+      old = Digest{{0, 0, 0, 0}};
+      if (valid && needs_old<EPI>(a)) old = ld_digest(a.prev + c);
+    }
+    // a warp reads only the rows it has copied itself
+    cp_async_wait<kStageBufs - 2>();
+    __syncwarp();
+    if (issued < total) load(buf == 0 ? kStageBufs - 1 : buf - 1);  // the buffer of step k - 1
+    issued++;
+    cp_async_commit();
+    if (valid) {
+      const uint4* src = reinterpret_cast<const uint4*>(sm_raw + buf * kStagedBytes + tid * kRowStride);
+      const uint64_t nb = min(cs, a.len - c * cs);  // bytes of the chunk
+      const uint64_t done = (uint64_t)step * kPanel;
+      const uint32_t rem = nb <= done ? 0 : nb - done < kPanel ? (uint32_t)(nb - done) : kPanel;
+      const uint32_t sh = ((uint32_t)(base + c * cs) & 3) * 8;
+      uint32_t y[33];
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const uint4 v = src[q];
+        y[4 * q] = v.x; y[4 * q + 1] = v.y; y[4 * q + 2] = v.z; y[4 * q + 3] = v.w;
+      }
+      if (sh) {
+        y[32] = src[8].x;
+#pragma unroll
+        for (int i = 0; i < 32; i++) y[i] = __funnelshift_r(y[i], y[i + 1], sh);
+      }
+      if (rem < kPanel) {  // words past the chunk's end read as zero
+#pragma unroll
+        for (int i = 0; i < 32; i++) {
+          const int left = (int)rem - 4 * i;
+          if (left < 4) y[i] &= left <= 0 ? 0u : (1u << (8 * left)) - 1;
+        }
+      }
+      const bool last = done < nb && nb <= done + kPanel;  // the chunk ends in this step
+      if (HK == HASH_MD5) {
+        if (rem >= 64) md.block(y);
+        if (rem == kPanel) md.block(y + 16);
+        if (last) {
+          // the final partial block: nothing, or the bytes after the last whole one
+          uint32_t X[16];
+          const uint32_t part = rem & 63;
+#pragma unroll
+          for (int i = 0; i < 16; i++) X[i] = part == 0 ? 0 : rem < 64 ? y[i] : y[16 + i];
+          const Digest dg = md.finish(X, part, nb);
+          leaf_epilogue<EPI>(a, true, (uint32_t)c, dg, old);
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+          if (16u * (q + 1) <= rem) mm.block(y[4 * q], y[4 * q + 1], y[4 * q + 2], y[4 * q + 3]);
+        if (last) {
+          const uint32_t part = rem & 15, q = rem >> 4;
+          uint32_t t[4] = {0, 0, 0, 0};
+#pragma unroll
+          for (int i = 0; i < 8; i++)
+            if ((uint32_t)i == q && part) {
+              t[0] = y[4 * i]; t[1] = y[4 * i + 1]; t[2] = y[4 * i + 2]; t[3] = y[4 * i + 3];
+            }
+          mm.tail(((uint64_t)t[1] << 32) | t[0], ((uint64_t)t[3] << 32) | t[2], part);
+          leaf_epilogue<EPI>(a, true, (uint32_t)c, mm.finish(nb), old);
+        }
+      }
+    }
+    __syncwarp();  // the row is read before the warp refills this buffer
+    if (++step == steps) {
+      step = 0;
+      tile += gridDim.x;
+    }
+    buf = buf + 1 == kStageBufs ? 0 : buf + 1;
+  }
+  cp_async_wait<0>();
+}
+
+// ---------------------------------------------------------------------------
 // One persistent launch for the leaf pass of many deduplicators (a batch).
 // A device work queue holds (member, tile) items; each CTA's producer lane
 // claims the next item with one atomicAdd and streams its boxes through the
@@ -691,6 +864,38 @@ cudaError_t launch_direct(const LeafArgs& a, uint32_t c0, uint32_t c1, cudaStrea
   return cudaGetLastError();
 }
 
+template <int HK, int EPI>
+cudaError_t launch_staged_t(const LeafArgs& a, uint32_t c0, uint32_t c1, cudaStream_t s) {
+  auto k = leaf_staged_kernel<HK, EPI>;
+  constexpr size_t smem = (size_t)kStageBufs * kStagedBytes;
+  static std::atomic<bool> attr_set{false};
+  if (!attr_set.load(std::memory_order_acquire)) {
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    attr_set.store(true, std::memory_order_release);
+  }
+  static const bool reg = (register_input_kernel(reinterpret_cast<const void*>(k), INPUT_LEAF_DIRECT), true);
+  (void)reg;
+  const uint32_t ntiles = (c1 - c0 + kStageRows - 1) / kStageRows;
+  const uint32_t cap = (uint32_t)num_sms() * 4;
+  launch_k(k, ntiles < cap ? ntiles : cap, kStageRows, smem, s, a, c0, c1);
+  note_launch();
+  return cudaGetLastError();
+}
+template <int EPI>
+cudaError_t launch_staged(const LeafArgs& a, uint32_t c0, uint32_t c1, cudaStream_t s) {
+  return a.hash_kind == HASH_MD5 ? launch_staged_t<HASH_MD5, EPI>(a, c0, c1, s)
+                                 : launch_staged_t<HASH_MURMUR3, EPI>(a, c0, c1, s);
+}
+cudaError_t dispatch_staged(const LeafArgs& a, uint32_t c0, uint32_t c1, cudaStream_t s) {
+  switch (a.epi) {
+    case EPI_TREE: return launch_staged<EPI_TREE>(a, c0, c1, s);
+    case EPI_LIST: return launch_staged<EPI_LIST>(a, c0, c1, s);
+    case EPI_BASIC: return launch_staged<EPI_BASIC>(a, c0, c1, s);
+    default: return launch_staged<EPI_HASH>(a, c0, c1, s);
+  }
+}
+
 cudaError_t dispatch_direct(const LeafArgs& a, uint32_t c0, uint32_t c1, cudaStream_t s) {
   switch (a.epi) {
     case EPI_TREE: return launch_direct<EPI_TREE>(a, c0, c1, s);
@@ -766,6 +971,12 @@ bool input_tmap(TmaCache* c, const uint8_t* data, uint64_t len, uint32_t cs, con
          make_tmap(c, data, len, cs, W, rows, n_full);
 }
 
+// Chunks up to here are read directly when no tiled copy fits: a warp's 32
+// chunks then share their lines in L1, and a panel is mostly padding (400 MB in
+// 100-byte chunks: 140 us direct, 226 us staged; 256 MiB in 128-byte chunks off a
+// boundary: 282 and 117 us).
+constexpr uint32_t kDirectMax = 100;
+
 cudaError_t launch_leaves(const LeafArgs& a, TmaCache* cache, cudaStream_t s, const LeafTune& tune) {
   if (a.n_chunks == 0) return cudaSuccess;
   const uint32_t n_full = (uint32_t)(a.len / a.cs);
@@ -779,6 +990,8 @@ cudaError_t launch_leaves(const LeafArgs& a, TmaCache* cache, cudaStream_t s, co
     cudaError_t e = dispatch_tma(a, cache->map, n_full, W, t, s);
     if (e != cudaSuccess) return e;
     done = n_full;
+  } else if (!t.direct && a.cs > kDirectMax) {
+    return dispatch_staged(a, 0, a.n_chunks, s);
   }
   return dispatch_direct(a, done, a.n_chunks, s);
 }
