@@ -345,25 +345,35 @@ int mtc_hash_chunks(int hash, const void* dev_data, uint64_t len, uint32_t chunk
   a.epi = mtc::EPI_HASH;
   mtc::TmaCache cache;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(cuda_stream);
-  // a device error word for the call (a bounded wait that runs out sets it):
-  // one per host thread and device, allocated on the thread's first call and
-  // kept (an allocation per call would go through the default memory pool,
-  // whose release at every synchronisation maps and unmaps device memory)
-  thread_local uint32_t* tl_err[64] = {};
+  // a device error word for the call (a bounded wait that runs out sets it) and
+  // a pinned word it is read through: one pair per host thread and device,
+  // allocated on the thread's first call and kept (an allocation per call would
+  // go through the default memory pool, whose release at every synchronisation
+  // maps and unmaps device memory).  The word is zero between calls: the kernel
+  // that reads it clears it.  A memset and a copy to pageable memory took 5 of
+  // a short call's 22 us.
+  struct ErrPair { uint32_t *dev, *host; };
+  thread_local ErrPair tl_err[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return ret(MTC_ENOTSUP, "device ordinal above 63");
+  ErrPair& p = tl_err[dev];
   cudaError_t e = cudaSuccess;
-  if (!tl_err[dev]) e = cudaMalloc(reinterpret_cast<void**>(&tl_err[dev]), sizeof(uint32_t));
-  uint32_t* err = e == cudaSuccess ? tl_err[dev] : nullptr;
-  uint32_t err_host = 0;
-  if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, sizeof(uint32_t), s);
-  a.err = err;
-  if (e == cudaSuccess) e = mtc::launch_leaves(a, &cache, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&err_host, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+  if (!p.host) e = cudaMallocHost(reinterpret_cast<void**>(&p.host), sizeof(uint32_t));
+  if (e == cudaSuccess && !p.dev) {
+    e = cudaMalloc(reinterpret_cast<void**>(&p.dev), sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemsetAsync(p.dev, 0, sizeof(uint32_t), s);
+  }
+  a.err = p.dev;
+  if (e == cudaSuccess) e = mtc::launch_leaves(a, &cache, s, mtc::default_leaf_tune(hash, chunk_size));
+  if (e == cudaSuccess) e = mtc::launch_take_word(p.dev, static_cast<uint32_t*>(mtc::host_alias(p.host)), s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return ret(e == cudaErrorMemoryAllocation ? MTC_ENOMEM : MTC_ECUDA, cudaGetErrorString(e));
-  if (err_host & mtc::DERR_SPIN) return ret(MTC_ETIMEOUT, "bounded device wait expired");
+  if (e != cudaSuccess) {
+    if (p.dev) cudaFree(p.dev);  // it may hold an error bit that no call has read
+    p.dev = nullptr;
+    return ret(e == cudaErrorMemoryAllocation ? MTC_ENOMEM : MTC_ECUDA, cudaGetErrorString(e));
+  }
+  if (*p.host & mtc::DERR_SPIN) return ret(MTC_ETIMEOUT, "bounded device wait expired");
   return MTC_OK;
 }
 

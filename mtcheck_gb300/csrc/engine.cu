@@ -55,6 +55,18 @@ cudaError_t launch_readback(const Readback& r, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+static __global__ void take_word_kernel(uint32_t* dev, uint32_t* host) {
+  pdl_enter();
+  *host = *dev;
+  *dev = 0;
+}
+
+cudaError_t launch_take_word(uint32_t* dev, uint32_t* host, cudaStream_t s) {
+  launch_k(take_word_kernel, 1, 1, 0, s, dev, host);
+  note_launch();
+  return cudaGetLastError();
+}
+
 void* host_alias(void* pinned) {
   void* d = nullptr;
   if (cudaHostGetDevicePointer(&d, pinned, 0) != cudaSuccess) {

@@ -179,6 +179,8 @@ struct Readback {
   uint64_t* clk;  // CLK_END is written here first (may be null)
 };
 cudaError_t launch_readback(const Readback& r, cudaStream_t s);
+// One device word moved to pinned memory the same way, and cleared.
+cudaError_t launch_take_word(uint32_t* dev, uint32_t* host, cudaStream_t s);
 // The device address of pinned host memory (the same pointer under unified
 // addressing).
 void* host_alias(void* pinned);
