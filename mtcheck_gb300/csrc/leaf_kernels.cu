@@ -227,8 +227,14 @@ __device__ __forceinline__ bool needs_old(const LeafArgs& a) {
 }
 
 // ---------------------------------------------------------------------------
-// TMA pipeline kernel.
+// TMA pipeline kernel.  A partial last chunk is hashed from global memory by an
+// idle lane of the last block's producer warp: a launch of its own took 3-4 us,
+// as long as the hashing of a 1 MB buffer.
 // ---------------------------------------------------------------------------
+__device__ __noinline__ Digest hash_bytes_call(int kind, const uint8_t* p, uint64_t len) {
+  return hash_bytes(kind, p, len);
+}
+
 template <int HK, int EPI, int W, int kRows>
 __global__ void __launch_bounds__(kRows + 32, 2) leaf_tma_kernel(const __grid_constant__ CUtensorMap tmap, LeafArgs a,
                                                               uint32_t n_full) {
@@ -253,6 +259,12 @@ __global__ void __launch_bounds__(kRows + 32, 2) leaf_tma_kernel(const __grid_co
   __syncthreads();
 
   if (tid >= kRows) {
+    if (tid == kRows + 1 && blockIdx.x == gridDim.x - 1 && n_full < a.n_chunks) {
+      Digest old{{0, 0, 0, 0}};
+      if (needs_old<EPI>(a)) old = ld_digest(a.prev + n_full);
+      const uint64_t off = (uint64_t)n_full * a.cs;
+      leaf_epilogue<EPI>(a, true, n_full, hash_bytes_call(HK, a.data + off, a.len - off), old);
+    }
     // producer warp: one elected lane issues every box in consumption order
     if (tid == kRows) {
       tma_prefetch_desc(&tmap);
@@ -985,15 +997,10 @@ cudaError_t launch_leaves(const LeafArgs& a, TmaCache* cache, cudaStream_t s, co
   LeafTune t = tune;
   if (t.rows != 128) t.rows = 256;
   if (t.threads_per_chunk == 32 && a.cs <= kWarpChunkMax) return dispatch_warp(a, 0, a.n_chunks, s);
-  uint32_t done = 0;
-  if (!t.direct && W && aligned && n_full > 0 && cache && make_tmap(cache, a.data, a.len, a.cs, W, t.rows, n_full)) {
-    cudaError_t e = dispatch_tma(a, cache->map, n_full, W, t, s);
-    if (e != cudaSuccess) return e;
-    done = n_full;
-  } else if (!t.direct && a.cs > kDirectMax) {
-    return dispatch_staged(a, 0, a.n_chunks, s);
-  }
-  return dispatch_direct(a, done, a.n_chunks, s);
+  if (!t.direct && W && aligned && n_full > 0 && cache && make_tmap(cache, a.data, a.len, a.cs, W, t.rows, n_full))
+    return dispatch_tma(a, cache->map, n_full, W, t, s);
+  if (!t.direct && a.cs > kDirectMax) return dispatch_staged(a, 0, a.n_chunks, s);
+  return dispatch_direct(a, 0, a.n_chunks, s);
 }
 
 bool batch_leaf_member(MemberLeaf* out, const LeafArgs& a) {

@@ -130,9 +130,10 @@ inline LeafTune default_leaf_tune(int hash_kind, uint32_t cs) {
   return LeafTune{128, cs < 128 ? 6 : cs == 128 ? 3 : 2, 0};
 }
 
-// Launch the leaf hashing kernel(s) over every chunk.  Uses the TMA pipeline
-// for chunk sizes that are a multiple of 128 bytes (or 16/32/64) on 16-byte
-// aligned buffers, and a thread-per-chunk kernel otherwise and for the tail.
+// Launch the leaf hashing kernel over every chunk: the TMA pipeline for chunk
+// sizes that are a multiple of 128 bytes (or 16/32/64) on 16-byte aligned
+// buffers, the staged kernel for other chunks above 100 bytes, and direct loads
+// for the rest.
 cudaError_t launch_leaves(const LeafArgs& a, TmaCache* cache, cudaStream_t s, const LeafTune& tune = LeafTune{});
 // The leaf pass of many deduplicators in one persistent launch (a batch):
 // one record per member (its TMA descriptor with boxes of kBatchRows rows,
