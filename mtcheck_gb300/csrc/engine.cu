@@ -307,6 +307,7 @@ GatherArgs Engine::gather_args(const uint8_t* data, uint64_t len) {
   g.n_flags = tree ? (uint64_t)M_ - 1 : N_;  // every node but the root, or every chunk
   g.labels = labels_.p;
   g.order = root_order();
+  g.all_own = fresh_ && baseline_path_ ? 1 : 0;
   if (tree && !baseline_path_) {
     g.fuse_gate = changed_count_.p + COUNT_DEMOTED;
     g.ins_queue = changed_list_.p;
@@ -382,8 +383,25 @@ int Engine::run_tree(const uint8_t* data, uint64_t len, bool baseline_path) {
   fa.ins_queue = changed_list_.p;
   fa.ins_count = changed_count_.p + COUNT_INSERTS;
   fa.span_done = span_done_.p;
+  fa.zero_found = changed_count_.p + COUNT_ZERO_FOUND;
   if (baseline_path && fresh_) {
-    MTC_CUDA(launch_forest(fa, 3, 1, N, stream_));  // both passes of a baseline on cleared digests
+    // both passes of a baseline; its map inserts, bound by random accesses, run
+    // beside the diff's assembly, which is a copy and looks up none of them (a
+    // baseline of 4 GiB in 512-byte chunks 3.31 -> 3.20 ms, of 64 MiB in 128-byte
+    // chunks 248 -> 221 us; fewer insert blocks are slower).  Below 2^18 chunks the extra launches
+    // cost as much; members of a batch or a server overlap with one another.
+    MTC_CUDA(launch_forest(fa, 3, 1, N, stream_));
+    if (N >= (1u << 18) && !pool_ && !order_after_legacy_) {
+      MTC_TRY(ensure_side());
+      MTC_CUDA(launch_forest_inserts(fa, INSERT_IF_ZERO, N, stream_));
+      MTC_CUDA(cudaEventRecord(rev_[0], stream_));
+      MTC_CUDA(cudaStreamWaitEvent(rside_, rev_[0], 0));
+      MTC_CUDA(launch_forest_inserts(fa, INSERT_UNLESS_ZERO, N, rside_));
+      MTC_CUDA(cudaEventRecord(rev_[1], rside_));
+      join_ = rev_[1];
+    } else {
+      MTC_CUDA(launch_forest_inserts(fa, INSERT_ALWAYS, N, stream_));
+    }
   } else {
     MTC_CUDA(launch_forest(fa, 0, 0, N, stream_));                      // first-occurrence forest
     MTC_CUDA(launch_forest(fa, 1, baseline_path ? 1 : 0, N, stream_));  // duplicate forest
@@ -480,9 +498,17 @@ int Engine::enqueue(const uint8_t* data, uint64_t len, bool timed) {
   }
   note_launch();
   MTC_CUDA(cudaGetLastError());
+  join_ = nullptr;
   int rc = (mode_ == MODE_LIST || mode_ == MODE_BASIC) ? run_list_basic(data, len) : run_tree(data, len, baseline_path_);
   if (rc) return rc;
-  MTC_CUDA(launch_assemble(gather_args(data, len), (uint64_t)N_ + 1, fresh_, stream_));
+  MTC_CUDA(launch_assemble(gather_args(data, len), (uint64_t)N_ + 1, fresh_, join_, stream_));
+  return ST_OK;
+}
+
+int Engine::ensure_side() {
+  if (rside_) return ST_OK;
+  MTC_CUDA(cudaStreamCreateWithFlags(&rside_, cudaStreamNonBlocking));
+  for (auto& e : rev_) MTC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   return ST_OK;
 }
 

@@ -330,11 +330,14 @@ class Engine {
   TmaCache tma_;
   cudaEvent_t ev_[3] = {nullptr, nullptr, nullptr};  // two timing events, one ordering event
   RestartScratch* rs_ = nullptr;  // restart buffers, created on first use
-  // restart: a second stream for the work that does not depend on the main
+  // a second stream, for a large baseline's map inserts beside the diff's
+  // assembly, and in a restart for the work that does not depend on the main
   // sequence (clears, the chain tables beside the main scatter, the copy of
   // resolved chunk ranges), and the events that fork and join it
   cudaStream_t rside_ = nullptr;
   cudaEvent_t rev_[12] = {};
+  int ensure_side();
+  cudaEvent_t join_ = nullptr;  // set while a baseline's map inserts run on the second stream
   // pinned staging of a restart's chain descriptors (kept when the restart
   // tables are released: freeing pinned memory waits for the device), and
   // the event after their last upload

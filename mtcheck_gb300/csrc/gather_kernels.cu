@@ -204,8 +204,12 @@ __device__ __forceinline__ uint8_t span_node(const ForestArgs& a, int pass, uint
         dg = hash_pair(HK, dl, dr);
         st_digest(a.tree + n, dg);
       }
-      if (map_find(a.map, BASE ? Digest{{0, 0, 0, 0}} : dg, a.err) >= 0) lab_n = SHIFT_DUPL;
-      else fl = fr = ROOT_SHIFT;
+      if (map_find(a.map, BASE ? Digest{{0, 0, 0, 0}} : dg, a.err) >= 0) {
+        lab_n = SHIFT_DUPL;
+        if (BASE) atomicOr(a.zero_found, 1u);
+      } else {
+        fl = fr = ROOT_SHIFT;
+      }
     } else if (ll == FIRST_OCUR) {
       lab_n = FIRST_OCUR;
       if (!BASE && pass == 2) {
@@ -415,10 +419,14 @@ __device__ __forceinline__ uint8_t thread_levels_bytewise(const ForestArgs& a, i
         }
         const Digest d = hash_pair(HK, dl, dr);
         if (BASE) {
-          if ((XS[q] >> (8 * b)) & 1 && map_find(a.map, Digest{{0, 0, 0, 0}}, a.err) < 0) {
-            set_byte(P[q], b, DONE);
-            set_byte(FL[q], b, ROOT_SHIFT);
-            set_byte(FR[q], b, ROOT_SHIFT);
+          if ((XS[q] >> (8 * b)) & 1) {
+            if (map_find(a.map, Digest{{0, 0, 0, 0}}, a.err) >= 0) {
+              atomicOr(a.zero_found, 1u);
+            } else {
+              set_byte(P[q], b, DONE);
+              set_byte(FL[q], b, ROOT_SHIFT);
+              set_byte(FR[q], b, ROOT_SHIFT);
+            }
           }
           st_digest(a.tree + n, d);
           a.labels[n] = (uint8_t)(P[q] >> (8 * b));
@@ -622,8 +630,9 @@ __device__ __forceinline__ void drain_inserts(const GatherArgs& g, uint32_t blk,
 // carry the first pass's epoch, the others the second's, among which equal
 // digests abound (runs of equal chunks): those of a warp insert once.  Bound by the
 // random accesses (two operations on each line).
-__global__ void __launch_bounds__(256) forest_insert_all_kernel(ForestArgs a, uint32_t n_interior) {
+__global__ void __launch_bounds__(256) forest_insert_all_kernel(ForestArgs a, int when, uint32_t n_interior) {
   pdl_enter();
+  if (when != INSERT_ALWAYS && (*a.zero_found != 0) != (when == INSERT_IF_ZERO)) return;
   const uint32_t cur_id = a.sp->cur, epoch = a.sp->epoch;
   const uint32_t lane = threadIdx.x & 31;
   uint32_t created = 0;
@@ -761,9 +770,11 @@ __global__ void __launch_bounds__(kScanThreads) root_count_kernel(GatherArgs g) 
 // First-occurrence root: (1 << 32) | chunks if it owns its digest, else 0.  A
 // first-occurrence leaf owns its digest: the leaf pass demotes every other one
 // (same checkpoint id, another owner).  The inserts of a fused pass may still
-// wait: a digest that is not in the map then is the root's own.
+// wait: a digest that is not in the map then is the root's own.  In a baseline
+// of an empty map every first occurrence owns its digest: its leaves own
+// theirs, and no second pair of the same leaves is a first occurrence.
 __device__ __forceinline__ uint64_t fo_region(const GatherArgs& g, uint32_t node, bool fused, uint32_t cur) {
-  bool owner = node >= g.N - 1;
+  bool owner = node >= g.N - 1 || g.all_own;
   if (!owner) {
     const int64_t slot = map_find(g.map, ld_digest(g.digests + node), g.err);
     const NodeIdDev prev = slot_value(g.map, slot);
@@ -1444,14 +1455,17 @@ cudaError_t launch_forest(const ForestArgs& a, int pass, int baseline, uint32_t 
              count);
   }
   note_launch();
-  if (pass == 3) {
-    launch_k(forest_insert_all_kernel, grid_for(N - 1, 256), 256, 0, s, a, N - 1);
-    note_launch();
-  }
   return cudaGetLastError();
 }
 
-cudaError_t launch_assemble(GatherArgs g, uint64_t max_entries, bool whole, cudaStream_t s) {
+cudaError_t launch_forest_inserts(const ForestArgs& a, int when, uint32_t N, cudaStream_t s) {
+  if (N < 2) return cudaSuccess;
+  launch_k(forest_insert_all_kernel, grid_for(N - 1, 256), 256, 0, s, a, when, N - 1);
+  note_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t launch_assemble(GatherArgs g, uint64_t max_entries, bool whole, cudaEvent_t join, cudaStream_t s) {
   const uint32_t tiles = (uint32_t)std::max<uint64_t>(1, (g.n_flags + kRootTile - 1) / kRootTile);
   const bool reduce = tiles <= std::min<uint32_t>(kRootReduceTiles, 2 * reduce_tile_limit());
   const bool tree = g.approach == APPROACH_TREE, basic = g.approach == APPROACH_BASIC;
@@ -1512,6 +1526,10 @@ cudaError_t launch_assemble(GatherArgs g, uint64_t max_entries, bool whole, cuda
     copies = 0;
   }
   g.n_drain = g.fuse_gate ? std::min<uint32_t>(2 * num_sms(), (g.N + 255) / 256) : 0;
+  if (join) {
+    const cudaError_t e = cudaStreamWaitEvent(s, join, 0);
+    if (e != cudaSuccess) return e;
+  }
   g.n_copy = copies;
   const uint32_t grid = std::max(1u, g.n_sort + g.n_drain + copies);
   launch_k(k, grid, 256, smem, s, g);

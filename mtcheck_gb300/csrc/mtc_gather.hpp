@@ -50,6 +50,7 @@ struct ForestArgs {
   uint32_t* ins_queue;  // first-occurrence nodes awaiting their map insert (N entries)
   uint32_t* ins_count;
   uint32_t* span_done;  // forest_done_words(N) counters, zero between passes
+  uint32_t* zero_found; // set by pass 3 when a shift test succeeds
 };
 
 // Position of node x (>= 1) in the canonical root order.
@@ -83,6 +84,7 @@ struct GatherArgs {
   uint64_t n_flags;
   const uint8_t* labels;  // tree: node labels
   RootOrder order;
+  int all_own;            // a baseline of an empty map: every first occurrence owns its digest
   uint64_t *tile_counts, *tile_regions;  // per tile of flags
   uint32_t* fo_list;
   uint32_t* sh_list;
@@ -104,13 +106,19 @@ struct GatherArgs {
 };
 
 // One forest pass.  pass 0 = first-occurrence forest, 1 = duplicate forest, 3 =
-// both, and the inserts, of a baseline whose digests were cleared (baseline =
-// 1).
+// both of a baseline whose digests count as cleared (baseline = 1), which
+// launch_forest_inserts completes.
 size_t forest_done_words(uint32_t N);
 cudaError_t launch_forest(const ForestArgs& a, int pass, int baseline, uint32_t N, cudaStream_t s);
+// The inserts of pass 3: all of them, or only if its shift test found the zero
+// digest (its shifted roots may then be interior nodes, which the root lookups
+// need in the map), or only if it did not (no lookup then waits for them).
+enum : int { INSERT_ALWAYS = 0, INSERT_IF_ZERO = 1, INSERT_UNLESS_ZERO = 2 };
+cudaError_t launch_forest_inserts(const ForestArgs& a, int when, uint32_t N, cudaStream_t s);
 // Roots listed and the diff assembled into g.stage; max_entries bounds F and S
-// (N + 1).  whole: most chunks are expected in the diff (a baseline).
-cudaError_t launch_assemble(GatherArgs g, uint64_t max_entries, bool whole, cudaStream_t s);
+// (N + 1).  whole: most chunks are expected in the diff (a baseline).  join: the
+// last launch waits for this event too (may be null).
+cudaError_t launch_assemble(GatherArgs g, uint64_t max_entries, bool whole, cudaEvent_t join, cudaStream_t s);
 // Rebuild `from` into the empty table `to` (capacity change), preserving values.
 cudaError_t launch_map_rehash(const DigestMap& from, uint64_t from_cap, const DigestMap& to, uint32_t* err,
                               cudaStream_t s);

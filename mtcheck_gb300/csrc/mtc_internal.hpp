@@ -46,10 +46,10 @@ struct ParamsOut {
 };
 // Counters of a checkpoint: changed chunks, demoted leaves, queued forest
 // inserts, notes of the insert pass; finished blocks of the assembly's
-// launches.
+// launches; whether a baseline's shift test found the all-zero digest.
 enum : int {
   COUNT_CHANGED = 0, COUNT_DEMOTED = 1, COUNT_INSERTS = 2, COUNT_NOTES = 3,
-  COUNT_ROOTS_DONE = 4, COUNT_SORT_DONE = 5, COUNT_FINAL_DONE = 6, kCounters = 8
+  COUNT_ROOTS_DONE = 4, COUNT_SORT_DONE = 5, COUNT_FINAL_DONE = 6, COUNT_ZERO_FOUND = 7, kCounters = 8
 };
 
 struct LeafArgs {

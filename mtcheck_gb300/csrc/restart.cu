@@ -1411,10 +1411,7 @@ int Engine::restart_enqueue(uint8_t* dev_out, uint64_t len, const std::vector<co
   // The second stream: clears that depend on nothing run there at once; the
   // chain tables run there beside the main checkpoint's scatter; each range
   // of resolved chunks is copied there while the next range is resolved.
-  if (!rside_) {
-    MTC_CUDA_R(cudaStreamCreateWithFlags(&rside_, cudaStreamNonBlocking));
-    for (auto& e : rev_) MTC_CUDA_R(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  }
+  if (const int rc = ensure_side()) return rc;
   cudaStream_t side = rside_;
   StepTimer t_fork("restart: fork and clears", N);
   MTC_CUDA_R(cudaEventRecord(rev_[0], s));  // after the allocations and the previous restart
