@@ -892,65 +892,126 @@ __device__ __forceinline__ uint32_t byte_mask(int lo, int hi, int q) {
   return below_b & ~below_a;
 }
 
+// Bytes [lo, hi) of the 16 bytes at address A, in place, the others zero: the
+// aligned words around them that hold one of these bytes, and the cut.
+struct Window { uint4 w0, w1; };
+__device__ __forceinline__ Window load_window(uint64_t A, int lo, int hi) {
+  Window v{make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+  const int d = (int)(A & 15);
+  const uint4* w = reinterpret_cast<const uint4*>(A - d);
+  if (hi > lo && lo + d < 16) v.w0 = __ldcs(w);
+  if (hi > lo && hi + d > 16) v.w1 = __ldcs(w + 1);
+  return v;
+}
+__device__ __forceinline__ void merge_window(const Window& x, uint64_t A, int lo, int hi, uint4& v, uint4& m) {
+  if (hi <= lo) return;
+  const uint4 c = cut16(x.w0, x.w1, (uint32_t)(A & 15));
+  const uint32_t m0 = byte_mask(lo, hi, 0), m1 = byte_mask(lo, hi, 1), m2 = byte_mask(lo, hi, 2),
+                 m3 = byte_mask(lo, hi, 3);
+  v.x |= c.x & m0; v.y |= c.y & m1; v.z |= c.z & m2; v.w |= c.w & m3;
+  m.x |= m0; m.y |= m1; m.z |= m2; m.w |= m3;
+}
+// a unit of which not every byte is restored is written byte by byte
+__device__ __forceinline__ void store_unit(uint64_t u, const uint4& v, const uint4& m) {
+  if ((m.x & m.y & m.z & m.w) == ~0u) {
+    *reinterpret_cast<uint4*>(u) = v;
+  } else if (m.x | m.y | m.z | m.w) {
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      const uint32_t vw = i < 4 ? v.x : i < 8 ? v.y : i < 12 ? v.z : v.w;
+      const uint32_t mw = i < 4 ? m.x : i < 8 ? m.y : i < 12 ? m.z : m.w;
+      if ((mw >> (8 * (i & 3))) & 1) *reinterpret_cast<uint8_t*>(u + i) = (uint8_t)(vw >> (8 * (i & 3)));
+    }
+  }
+}
+
 // Chunk sizes that are no multiple of 16 bytes, or an output that is not 16-byte
 // aligned: the warp writes the aligned 16-byte units of its 32 chunks' range,
-// each put together from the chunks it meets (two at most for chunks of 16
-// bytes or more), every piece cut out of the aligned words around it.  A unit
-// of which not every byte is restored is written byte by byte.  64 MB in chunks
-// of 100 bytes, a byte per lane: 218 us.
+// each cut out of the aligned words around its source.  A unit meets two
+// chunks at most (chunks of 16 bytes or more); where the second's bytes follow
+// the first's, as in a run of chunks, they are one piece.  Two units in flight
+// per lane, every load issued before the first is used: one unit and its
+// pieces in turn took 75 us for 64 MB in chunks of 100 bytes, a byte per lane
+// 218 us.
 __device__ __forceinline__ void copy_tile_any(const RArgs& a, uint64_t c0, const uint8_t* src, uint32_t nb) {
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t cs = a.cs, total = 32 * cs;
   const unsigned long long sp = reinterpret_cast<unsigned long long>(src);
   const uint64_t d0 = reinterpret_cast<uint64_t>(a.out) + c0 * cs;
   const uint64_t u0 = d0 & ~15ull, nu = (d0 + total - u0 + 15) / 16;
-  const int pieces = cs >= 16 ? 2 : (int)((15 + cs) / cs) + 1;
-  for (uint64_t f0 = 0; f0 < nu; f0 += 32) {
+  constexpr int kUnits = 2;
+  for (uint64_t f0 = 0; f0 < nu; f0 += 32 * kUnits) {
+    uint64_t A1[kUnits], A2[kUnits];
+    int lo1[kUnits], hi1[kUnits], lo2[kUnits], hi2[kUnits];
+    Window x1[kUnits], x2[kUnits];
+#pragma unroll
+    for (int k = 0; k < kUnits; k++) {
+      const uint64_t u = u0 + 16 * (f0 + 32 * k + lane);
+      const int pos = u < d0 ? (int)(d0 - u) : 0;
+      const int end = u >= d0 + total ? pos : d0 + total - u < 16 ? (int)(d0 + total - u) : 16;
+      const uint64_t x = u + pos - d0;
+      uint32_t q = 0;
+      if (pos < end && x >= cs) q = total <= 0xffffffffull ? (uint32_t)x / (uint32_t)cs : (uint32_t)(x / cs);
+      const uint64_t within = x - q * cs;
+      const unsigned long long s1 = __shfl_sync(0xffffffffu, sp, q), s2 = __shfl_sync(0xffffffffu, sp, (q + 1) & 31);
+      const uint32_t n1 = __shfl_sync(0xffffffffu, nb, q), n2 = __shfl_sync(0xffffffffu, nb, (q + 1) & 31);
+      lo1[k] = hi1[k] = lo2[k] = hi2[k] = pos;
+      A1[k] = A2[k] = 0;
+      if (pos < end) {
+        const int stop = cs - within < (uint64_t)(end - pos) ? pos + (int)(cs - within) : end;
+        // bytes pos .. hi of the unit come from s1 + within on, the next from s2
+        A1[k] = s1 + within - pos;
+        if (n1 > within) hi1[k] = n1 - within < (uint64_t)(stop - pos) ? pos + (int)(n1 - within) : stop;
+        A2[k] = s2 - stop;
+        lo2[k] = stop;
+        hi2[k] = n2 < (uint32_t)(end - stop) ? stop + (int)n2 : end;
+        if (A2[k] == A1[k] && hi1[k] == stop) {
+          hi1[k] = hi2[k];
+          hi2[k] = lo2[k];
+        }
+      }
+      x1[k] = load_window(A1[k], lo1[k], hi1[k]);
+      x2[k] = load_window(A2[k], lo2[k], hi2[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < kUnits; k++) {
+      uint4 v = make_uint4(0, 0, 0, 0), m = make_uint4(0, 0, 0, 0);
+      merge_window(x1[k], A1[k], lo1[k], hi1[k], v, m);
+      merge_window(x2[k], A2[k], lo2[k], hi2[k], v, m);
+      store_unit(u0 + 16 * (f0 + 32 * k + lane), v, m);
+    }
+  }
+}
+
+// Chunks of less than 16 bytes: a unit meets up to 17 of them.
+__device__ __forceinline__ void copy_tile_small(const RArgs& a, uint64_t c0, const uint8_t* src, uint32_t nb) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t cs = a.cs, total = 32 * cs;
+  const unsigned long long sp = reinterpret_cast<unsigned long long>(src);
+  const uint64_t d0 = reinterpret_cast<uint64_t>(a.out) + c0 * cs;
+  const uint64_t u0 = d0 & ~15ull;
+  const uint32_t nu = (uint32_t)((d0 + total - u0 + 15) / 16);
+  for (uint32_t f0 = 0; f0 < nu; f0 += 32) {
     const uint64_t u = u0 + 16 * (f0 + lane);
     int pos = u < d0 ? (int)(d0 - u) : 0;
     const int end = u >= d0 + total ? 0 : d0 + total - u < 16 ? (int)(d0 + total - u) : 16;
-    const uint64_t x = u + pos - d0;
-    uint64_t q64 = 0;
-    if (pos < end && x >= cs) q64 = total <= 0xffffffffull ? (uint32_t)x / (uint32_t)cs : x / cs;
-    uint32_t q = (uint32_t)q64;
-    uint64_t within = pos < end ? x - q64 * cs : 0;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    uint4 m = make_uint4(0, 0, 0, 0);  // bytes of v that are restored
-    for (int k = 0; k < pieces; k++) {
+    const uint32_t x = pos < end ? (uint32_t)(u + pos - d0) : 0;
+    uint32_t q = x / cs, within = x % cs;
+    uint4 v = make_uint4(0, 0, 0, 0), m = make_uint4(0, 0, 0, 0);
+    for (uint32_t k = 0; k < (15 + cs) / cs + 1; k++) {
       const unsigned long long s = __shfl_sync(0xffffffffu, sp, q & 31);
       const uint32_t n = __shfl_sync(0xffffffffu, nb, q & 31);
       if (pos < end) {
-        const int stop = cs - within < (uint64_t)(end - pos) ? pos + (int)(cs - within) : end;
-        // bytes pos .. hi of the unit come from s + within on
-        const int hi = within >= n ? pos : n - within < (uint64_t)(stop - pos) ? pos + (int)(n - within) : stop;
-        if (hi > pos) {
-          const uint64_t A = s + within - pos;
-          const int d = (int)(A & 15);
-          const uint4* w = reinterpret_cast<const uint4*>(A - d);
-          uint4 w0 = make_uint4(0, 0, 0, 0), w1 = make_uint4(0, 0, 0, 0);
-          if (pos + d < 16) w0 = __ldcs(w);
-          if (hi + d > 16) w1 = __ldcs(w + 1);
-          const uint4 c = cut16(w0, w1, (uint32_t)d);
-          const uint32_t m0 = byte_mask(pos, hi, 0), m1 = byte_mask(pos, hi, 1), m2 = byte_mask(pos, hi, 2),
-                         m3 = byte_mask(pos, hi, 3);
-          v.x |= c.x & m0; v.y |= c.y & m1; v.z |= c.z & m2; v.w |= c.w & m3;
-          m.x |= m0; m.y |= m1; m.z |= m2; m.w |= m3;
-        }
+        const int stop = min(pos + (int)(cs - within), end);
+        const int hi = n > within ? min(pos + (int)(n - within), stop) : pos;
+        const uint64_t A = s + within - pos;
+        merge_window(load_window(A, pos, hi), A, pos, hi, v, m);
         pos = stop;
         q++;
         within = 0;
       }
     }
-    if ((m.x & m.y & m.z & m.w) == ~0u) {
-      *reinterpret_cast<uint4*>(u) = v;
-    } else if (m.x | m.y | m.z | m.w) {
-#pragma unroll
-      for (int i = 0; i < 16; i++) {
-        const uint32_t vw = i < 4 ? v.x : i < 8 ? v.y : i < 12 ? v.z : v.w;
-        const uint32_t mw = i < 4 ? m.x : i < 8 ? m.y : i < 12 ? m.z : m.w;
-        if ((mw >> (8 * (i & 3))) & 1) *reinterpret_cast<uint8_t*>(u + i) = (uint8_t)(vw >> (8 * (i & 3)));
-      }
-    }
+    store_unit(u, v, m);
   }
 }
 
@@ -961,7 +1022,8 @@ __device__ __forceinline__ void copy_tile(const RArgs& a, uint64_t c0, const uin
   const unsigned long long sp = reinterpret_cast<unsigned long long>(src);
   uint8_t* out0 = a.out + c0 * cs;
   if ((cs & 15) != 0 || (reinterpret_cast<uintptr_t>(a.out) & 15) != 0) {
-    copy_tile_any(a, c0, src, nb);
+    if (cs >= 16) copy_tile_any(a, c0, src, nb);
+    else copy_tile_small(a, c0, src, nb);
     return;
   }
   const uint32_t upc = cs >> 4;

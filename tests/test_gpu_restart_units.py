@@ -10,7 +10,7 @@ FILL = 0xA5
 
 @pytest.mark.parametrize("approach", [2, 3, 4], ids=["basic", "list", "tree"])
 @pytest.mark.parametrize("offset", [0, 1, 8])
-@pytest.mark.parametrize("cs,n,tail", [(1, 100, 0), (7, 64, 3), (15, 33, 0), (17, 97, 16), (100, 64, 0), (100, 161, 9),
+@pytest.mark.parametrize("cs,n,tail", [(1, 100, 0), (7, 64, 3), (15, 33, 0), (16, 70, 5), (17, 97, 16), (100, 64, 0), (100, 161, 9),
                                        (129, 40, 1), (640, 33, 600), (5000, 9, 0)])
 def test_restart_units(cuda, mtc, oracle, approach, offset, cs, n, tail):
     if approach == 4:  # a power of two of whole chunks, of which a tree restart gives every one back
