@@ -6,10 +6,11 @@
 // box of 256 rows x W bytes (W = 128, 64, 32 or 16) with the matching TMA
 // swizzle so that the 256 consumer threads read their rows without bank
 // conflicts.  A dedicated producer warp keeps STAGES boxes in flight; full/empty
-// mbarriers hand stages between producer and consumers.  Odd chunk sizes,
-// unaligned buffers and the partial last chunk use a thread-per-chunk kernel
-// that reads global memory directly.  Both end in the same epilogue, which
-// restates the leaf loops of the reference:
+// mbarriers hand stages between producer and consumers; one more warp hashes a
+// partial last chunk.  Odd chunk sizes and unaligned buffers go through a staged
+// kernel, short odd chunks through a thread-per-chunk kernel that reads global
+// memory directly.  All end in the same epilogue, which restates the leaf loops
+// of the reference:
 //   tree  -- src/tree_approach.cpp:57-94 (baseline) and :309-351
 //   list  -- src/list_approach.cpp:38-61
 //   basic -- src/basic_approach.cpp:25-46
@@ -227,16 +228,69 @@ __device__ __forceinline__ bool needs_old(const LeafArgs& a) {
 }
 
 // ---------------------------------------------------------------------------
-// TMA pipeline kernel.  A partial last chunk is hashed from global memory by an
-// idle lane of the last block's producer warp: a launch of its own took 3-4 us,
-// as long as the hashing of a 1 MB buffer.
+// TMA pipeline kernel.  A partial last chunk is hashed from global memory by one
+// more warp of the last block: a launch of its own took 3-4 us, as long as the
+// hashing of a 1 MB buffer, and a lane of the producer warp hashes it before the
+// block's first box, since the warp's branches run one after the other.
 // ---------------------------------------------------------------------------
-__device__ __noinline__ Digest hash_bytes_call(int kind, const uint8_t* p, uint64_t len) {
-  return hash_bytes(kind, p, len);
+// Digest of `len` bytes at a 16-byte aligned address, one thread: a serial
+// chain, so what bounds it is the wait for its bytes.  They are loaded 64 bytes
+// ahead of the hashing, from L2.  Digests of 1.4 MB in chunks of 4096 bytes with
+// a tail of 3743: Murmur3 89 -> 36 us, MD5 127 -> 63 us; without
+// the tail 31 and 58 us.
+template <int HK>
+__device__ __noinline__ Digest hash_tail(const uint4* p, uint32_t len) {
+  constexpr uint32_t kWords = 4, kPiece = 16 * kWords;
+  uint4 v[kWords];
+  auto load = [&](uint64_t off) {
+#pragma unroll
+    for (uint32_t q = 0; q < kWords; q++)
+      v[q] = off + 16 * q < len ? __ldg(p + off / 16 + q) : make_uint4(0, 0, 0, 0);
+  };
+  Md5State md;
+  Murmur3State mm;
+  if (HK == HASH_MD5) md.init(); else mm.init();
+  uint32_t X[4 * kWords];
+  load(0);
+  uint64_t off = 0;
+  while (true) {
+#pragma unroll
+    for (uint32_t q = 0; q < kWords; q++) {
+      X[4 * q] = v[q].x; X[4 * q + 1] = v[q].y; X[4 * q + 2] = v[q].z; X[4 * q + 3] = v[q].w;
+    }
+    if (off + kPiece > len) break;
+    load(off + kPiece);
+    if (HK == HASH_MD5) {
+      md.block(X);
+    } else {
+#pragma unroll
+      for (uint32_t q = 0; q < kWords; q++) mm.block(X[4 * q], X[4 * q + 1], X[4 * q + 2], X[4 * q + 3]);
+    }
+    off += kPiece;
+  }
+  const uint32_t rem = (uint32_t)(len - off);
+#pragma unroll
+  for (uint32_t i = 0; i < 4 * kWords; i++) {  // zero past the end
+    const int k = (int)rem - 4 * (int)i;
+    X[i] &= k <= 0 ? 0u : k >= 4 ? ~0u : (1u << (8 * k)) - 1;
+  }
+  if (HK == HASH_MD5) return md.finish(X, rem, len);
+  uint64_t t0 = 0, t1 = 0;
+#pragma unroll
+  for (uint32_t q = 0; q < kWords; q++) {
+    if (16 * q + 16 <= rem) {
+      mm.block(X[4 * q], X[4 * q + 1], X[4 * q + 2], X[4 * q + 3]);
+    } else if (16 * q < rem) {
+      t0 = ((uint64_t)X[4 * q + 1] << 32) | X[4 * q];
+      t1 = ((uint64_t)X[4 * q + 3] << 32) | X[4 * q + 2];
+    }
+  }
+  mm.tail(t0, t1, rem & 15);
+  return mm.finish(len);
 }
 
 template <int HK, int EPI, int W, int kRows>
-__global__ void __launch_bounds__(kRows + 32, 2) leaf_tma_kernel(const __grid_constant__ CUtensorMap tmap, LeafArgs a,
+__global__ void __launch_bounds__(kRows + 64, 2) leaf_tma_kernel(const __grid_constant__ CUtensorMap tmap, LeafArgs a,
                                                               uint32_t n_full) {
   pdl_enter();
   extern __shared__ uint8_t smem_raw[];
@@ -259,11 +313,17 @@ __global__ void __launch_bounds__(kRows + 32, 2) leaf_tma_kernel(const __grid_co
   __syncthreads();
 
   if (tid >= kRows) {
-    if (tid == kRows + 1 && blockIdx.x == gridDim.x - 1 && n_full < a.n_chunks) {
+    if (tid >= kRows + 32) {  // launched only with a partial last chunk
+      if (blockIdx.x != gridDim.x - 1) return;
+      const uint8_t* tail = a.data + (uint64_t)n_full * a.cs;
+      const uint32_t nb = (uint32_t)(a.len - (uint64_t)n_full * a.cs);
+      for (uint64_t at = 128ull * (tid - kRows - 32); at < nb; at += 32 * 128)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(tail + at));
+      if (tid != kRows + 32) return;
       Digest old{{0, 0, 0, 0}};
       if (needs_old<EPI>(a)) old = ld_digest(a.prev + n_full);
-      const uint64_t off = (uint64_t)n_full * a.cs;
-      leaf_epilogue<EPI>(a, true, n_full, hash_bytes_call(HK, a.data + off, a.len - off), old);
+      leaf_epilogue<EPI>(a, true, n_full, hash_tail<HK>(reinterpret_cast<const uint4*>(tail), nb), old);
+      return;
     }
     // producer warp: one elected lane issues every box in consumption order
     if (tid == kRows) {
@@ -835,7 +895,7 @@ cudaError_t launch_tma_t(const LeafArgs& a, const CUtensorMap& m, uint32_t n_ful
   if (per_sm > fit) per_sm = fit > 0 ? fit : 1;
   uint32_t grid = (uint32_t)(num_sms() * per_sm);
   if (grid > ntiles) grid = ntiles;
-  launch_k(k, grid, R + 32, smem, s, m, a, n_full);
+  launch_k(k, grid, n_full < a.n_chunks ? R + 64 : R + 32, smem, s, m, a, n_full);
   note_launch();
   return cudaGetLastError();
 }

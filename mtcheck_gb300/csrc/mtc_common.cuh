@@ -193,8 +193,13 @@ struct Md5State {
   // Final padding for a message of `len` bytes whose last `rem` (< 64) bytes
   // are in words tw[0..15] (zero beyond rem, little-endian).
   MTC_HD Digest finish(uint32_t* tw, uint32_t rem, uint64_t len) {
-    // append 0x80 at byte `rem`
-    tw[rem >> 2] |= 0x80u << (8 * (rem & 3));
+    // append 0x80 at byte `rem`; every index is a constant, so that the block
+    // stays in registers
+#pragma unroll
+    for (uint32_t i = 0; i < 16; i++) {
+      const uint32_t d = rem - 4 * i;  // past 31 bits, or below 0: no byte of this word
+      tw[i] |= d < 4 ? 0x80u << (8 * d) : 0u;
+    }
     if (rem >= 56) {
       block(tw);
 #pragma unroll
