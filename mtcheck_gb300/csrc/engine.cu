@@ -211,7 +211,6 @@ int Engine::ensure_state(uint32_t N, bool fresh, uint32_t id_headroom) {
     // compaction clears what it has read)
     MTC_CUDA(rflag_.ensure(tree ? ((size_t)M + 15) / 16 * 16 : 16, stream_));
     MTC_CUDA(cudaMemsetAsync(rflag_.p, 0, rflag_.n, stream_));
-    MTC_CUDA(chunk_slot_.ensure(N, stream_));
     MTC_CUDA(changed_list_.ensure(N, stream_));
     if (tree) {
       MTC_CUDA(span_done_.ensure(forest_done_words(N), stream_));
@@ -342,7 +341,6 @@ int Engine::run_tree(const uint8_t* data, uint64_t len, bool baseline_path) {
   la.n_chunks = N;
   la.prev = digests_.p + (N - 1);
   la.labels = labels_.p + (N - 1);
-  la.chunk_slot = chunk_slot_.p;
   la.map = map;
   la.sp = sp_.p;
   la.leaf_base = N - 1;
@@ -353,11 +351,7 @@ int Engine::run_tree(const uint8_t* data, uint64_t len, bool baseline_path) {
   la.fresh = fresh_ ? 1 : 0;
   la.changed_list = changed_list_.p;
   la.changed_count = changed_count_.p + COUNT_CHANGED;
-  la.demoted = changed_count_.p + COUNT_DEMOTED;
-  // the first-occurrence root list is free until the root compaction
-  la.dup_list = fo_list_.p;
-  la.dup_count = changed_count_.p + COUNT_NOTES;
-  la.dup_cap = (uint32_t)fo_list_.n;
+  la.demoted = baseline_path ? nullptr : changed_count_.p + COUNT_DEMOTED;  // gates the fused forest pass
   if (stall_now_) {
     la.stall = 1;
     la.spin_limit = kInjectedSpinLimit;
@@ -377,7 +371,7 @@ int Engine::run_tree(const uint8_t* data, uint64_t len, bool baseline_path) {
   fa.order = root_order();
   // an incremental checkpoint without demoted leaves runs both passes in one
   // traversal (the launches of the duplicate pass then return at once)
-  fa.fuse_gate = baseline_path ? nullptr : la.demoted;
+  fa.fuse_gate = la.demoted;
   // the changed-chunk list is free once the leaf inserts are done: it queues
   // the forest's first-occurrence inserts
   fa.ins_queue = changed_list_.p;
@@ -417,7 +411,6 @@ int Engine::run_list_basic(const uint8_t* data, uint64_t len) {
   la.n_chunks = N_;
   la.prev = digests_.p;
   la.labels = labels_.p;
-  la.chunk_slot = chunk_slot_.p;
   la.map = DigestMap{slots_.p, map_cap_ ? map_cap_ - 1 : 0, map_size_.p};
   la.sp = sp_.p;
   la.leaf_base = 0;
@@ -429,9 +422,6 @@ int Engine::run_list_basic(const uint8_t* data, uint64_t len) {
   la.basic_first = current_id == 0 ? 1 : 0;  // never true in a captured sequence
   la.changed_list = changed_list_.p;
   la.changed_count = changed_count_.p + COUNT_CHANGED;
-  la.dup_list = fo_list_.p;  // free until the chunk compaction
-  la.dup_count = changed_count_.p + COUNT_NOTES;
-  la.dup_cap = (uint32_t)fo_list_.n;
   if (stall_now_) {
     la.stall = 1;
     la.spin_limit = kInjectedSpinLimit;
@@ -765,7 +755,7 @@ uint64_t Engine::shape_signature(const uint8_t* data, uint64_t len) const {
   // chooses the kernels that read it): a captured sequence follows a moved
   // input by retarget
   const uint64_t v[] = {(uint64_t)data & 15, len, (uint64_t)digests_.p, (uint64_t)labels_.p, (uint64_t)rflag_.p,
-                        (uint64_t)chunk_slot_.p, (uint64_t)changed_list_.p, (uint64_t)changed_count_.p,
+                        (uint64_t)changed_list_.p, (uint64_t)changed_count_.p,
                         (uint64_t)slots_.p, map_cap_, (uint64_t)map_size_.p, (uint64_t)err_.p, (uint64_t)fo_list_.p,
                         (uint64_t)sh_list_.p, (uint64_t)reg_chunk_.p, (uint64_t)reg_slot_.p, (uint64_t)fo_tile_.p,
                         (uint64_t)sh_key_.p, (uint64_t)sh_prev_.p, (uint64_t)hist_.p, hist_.n, (uint64_t)rep_.p,
@@ -781,7 +771,7 @@ uint64_t Engine::shape_signature(const uint8_t* data, uint64_t len) const {
 
 template <class F>
 void Engine::for_each_buf(F f) {
-  f(digests_); f(labels_); f(rflag_); f(chunk_slot_); f(changed_list_); f(changed_count_); f(slots_);
+  f(digests_); f(labels_); f(rflag_); f(changed_list_); f(changed_count_); f(slots_);
   f(map_size_); f(err_); f(fo_list_); f(sh_list_); f(reg_chunk_); f(reg_slot_); f(fo_tile_); f(sh_key_);
   f(sh_prev_); f(hist_); f(rep_); f(rank_); f(fo_val_); f(sort_mat_); f(scan_); f(scan2_);
   f(scan_total2_); f(stage_); f(lay_); f(sp_); f(clk_); f(span_done_);
@@ -856,7 +846,7 @@ void Engine::release_restart_scratch() {
 
 uint64_t Engine::device_bytes() const {
   return sizeof(Digest) * digests_.n + labels_.n + rflag_.n +
-         sizeof(uint32_t) * (chunk_slot_.n + changed_list_.n + changed_count_.n + map_size_.n + err_.n + fo_list_.n +
+         sizeof(uint32_t) * (changed_list_.n + changed_count_.n + map_size_.n + err_.n + fo_list_.n +
                              sh_list_.n + reg_chunk_.n + reg_slot_.n + fo_tile_.n + sh_key_.n + sh_prev_.n + hist_.n +
                              rep_.n + rank_.n + span_done_.n) +
          sizeof(MapSlot) * slots_.n +

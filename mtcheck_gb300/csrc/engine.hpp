@@ -311,7 +311,7 @@ class Engine {
 
   DevBuf<Digest> digests_;     // tree heap (M) or hash list (N)
   DevBuf<uint8_t> labels_, rflag_;
-  DevBuf<uint32_t> chunk_slot_, changed_list_, changed_count_;
+  DevBuf<uint32_t> changed_list_, changed_count_;
   DevBuf<MapSlot> slots_;
   DevBuf<uint32_t> map_size_, err_;
   DevBuf<uint32_t> fo_list_, sh_list_, reg_chunk_, reg_slot_, fo_tile_, sh_key_, sh_prev_, hist_, rep_, rank_;

@@ -1443,16 +1443,21 @@ cudaError_t launch_forest(const ForestArgs& a, int pass, int baseline, uint32_t 
     }
     return cudaGetLastError();
   }
+  // the first pass follows the leaf inserts and starts after them: its blocks
+  // beside theirs leave the inserts little L1 (a baseline of 64 MiB in 128-byte
+  // chunks with a fifth of them duplicates: 218 against 195 us, an increment 88
+  // against 84)
+  const bool beside = pass == 1;
   if (N <= kSmallLeaves) {
     auto k = pass == 3 ? (md5 ? forest_small_kernel<HASH_MD5, true> : forest_small_kernel<HASH_MURMUR3, true>)
                        : (md5 ? forest_small_kernel<HASH_MD5, false> : forest_small_kernel<HASH_MURMUR3, false>);
-    launch_k(k, 1, 512, 0, s, a, pass, N, dmax);
+    launch_with(beside, k, 1, 512, 0, s, a, pass, N, dmax);
   } else {
     auto k = pass == 3 ? (md5 ? forest_kernel<HASH_MD5, true> : forest_kernel<HASH_MURMUR3, true>)
                        : (md5 ? forest_kernel<HASH_MD5, false> : forest_kernel<HASH_MURMUR3, false>);
     const uint32_t top = dmax - (kBottomLevels - 1), count = 1u << top;
-    launch_k(k, pass == 1 ? std::min<uint32_t>(count, (uint32_t)num_sms() * 5) : count, 256, 0, s, a, pass, N, top,
-             count);
+    launch_with(beside, k, pass == 1 ? std::min<uint32_t>(count, (uint32_t)num_sms() * 5) : count, 256, 0, s, a,
+                pass, N, top, count);
   }
   note_launch();
   return cudaGetLastError();

@@ -38,8 +38,6 @@ __device__ __forceinline__ uint32_t swz(uint32_t logical) {
   return logical ^ (((logical >> 7) & mask) << 4);
 }
 
-constexpr uint8_t PENDING = 0xFE;  // changed chunk, classified by the insert pass
-
 // Append chunk c to the changed list (one atomic per warp).
 // Appends a changed chunk to the list the map inserts read (warp-aggregated).
 __device__ __forceinline__ void append_changed(const LeafArgs& a, bool changed, uint32_t c) {
@@ -77,33 +75,29 @@ __device__ __forceinline__ void leaf_epilogue(const LeafArgs& a, bool valid, uin
   if (valid) {
     changed = !digest_eq(dg, old);
     if (changed || a.fresh) st_digest(a.prev + c, dg);
-    a.labels[c] = changed ? PENDING : (EPI == EPI_TREE ? FIXED_DUPL : DONE);
+    // a changed chunk is a first occurrence until the insert pass finds its
+    // digest held by another
+    a.labels[c] = changed ? FIRST_OCUR : (EPI == EPI_TREE ? FIXED_DUPL : DONE);
     // A FIXED_DUPL leaf's insert() always finds its digest (every earlier
     // leaf digest was inserted) and changes nothing, so it is not repeated.
   }
   if (!a.fresh) append_changed(a, changed, c);
 }
 
-// A note for the demote pass (a changed-list position); kCheckCreator: the
-// chunk met an entry that another insert of this launch created, whose chunk
-// is checked too.
-constexpr uint32_t kCheckCreator = 1u << 31;  // chunk counts stay below 2^31
-// Every changed chunk notes itself at most once, so the notes never outnumber
-// the changed chunks (the list holds N + 1 entries).
-__device__ __forceinline__ void note_dup(const LeafArgs& a, uint32_t note) {
-  const uint32_t k = atomicAdd(a.dup_count, 1u);
-  if (k < a.dup_cap) a.dup_list[k] = note;
-  else raise_err(a.err, DERR_CAPACITY);
-}
-
-// Map insert of one changed chunk (src/tree_approach.cpp:325-349,
+// Map insert of one changed chunk (src/tree_approach.cpp:325-369,
 // src/list_approach.cpp:50-59): new digest -> first occurrence; a digest
-// already inserted by this launch -> first occurrence for now, the lowest
-// chunk keeping the entry; an older digest -> shifted duplicate, except (tree)
+// inserted by this launch too -> first occurrence of the lowest chunk, shifted
+// duplicates of the others; an older digest -> shifted duplicate, except (tree)
 // one whose entry carries this checkpoint's id, which an id that was not
 // advanced (the header overload) leaves in place: the reference lowers its
-// node and keeps the chunk a first occurrence there too.  The creator of an
-// entry waits for nothing after its claim.
+// node there too and keeps the chunk that has it a first occurrence.
+// Every insert lowers the entry's win word to its own, and the word it gets
+// back tells who lost: itself, where that is lower, else the chunk it names.  So
+// each loser is marked once by whoever passes it, in any order.  A second pass over
+// notes of the duplicates took a launch more (a 1 MB increment 63 against 58 us) and
+// an append to one list per duplicate (a list baseline of 256 MB in 64-byte
+// chunks, half of them copies: 799 against 586 us).  Labels only ever go from
+// first occurrence to shifted duplicate here.
 // Lanes of a warp that hold one digest (runs of equal chunks) insert it once,
 // through their first lane and with their lowest chunk, as if the lowest had
 // come first.  The slot is read before it is claimed only once the block has
@@ -119,7 +113,7 @@ __global__ void __launch_bounds__(256) leaf_insert_kernel(LeafArgs a) {
   const uint32_t lane = threadIdx.x & 31;
   if (threadIdx.x == 0) s_dups = 0;
   __syncthreads();
-  bool first = true;
+  bool first = true, lost = false;
   uint32_t created = 0;
   // whole warps step together
   for (uint64_t kw = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); kw < n;
@@ -127,7 +121,8 @@ __global__ void __launch_bounds__(256) leaf_insert_kernel(LeafArgs a) {
     const uint64_t k = kw + lane;
     bool in = k < n;
     const uint32_t c = !in ? 0xffffffffu : a.fresh ? (uint32_t)k : a.changed_list[k];
-    if (a.fresh) in = in && a.labels[c] == PENDING;
+    // (only a chunk that has been inserted is ever marked by another)
+    if (a.fresh) in = in && a.labels[c] == FIRST_OCUR;
     Digest dg{{0, 0, 0, 0}};
     if (in) dg = map_key(ld_digest(a.prev + c));
     const unsigned act = __ballot_sync(0xffffffffu, in);
@@ -146,80 +141,59 @@ __global__ void __launch_bounds__(256) leaf_insert_kernel(LeafArgs a) {
       }
     }
     const int lead = __ffs(peers) - 1;
-    uint64_t slot = 0;
     int r = INS_FAILED;
-    unsigned long long old = kWinEmpty;
-    bool here = false;  // an older entry that carries this checkpoint's id
+    // the entry is this launch's (or, tree, carries this checkpoint's id), and
+    // the lowest of these chunks has it so far
+    bool ours = false, wins = false;
     if (in && (int)lane == lead) {
       const uint32_t node = EPI == EPI_TREE ? a.leaf_base + low : low;
+      unsigned long long w = win_of(epoch, node), old = kWinEmpty;
+      uint64_t slot = 0;
       r = map_claim(a.map, dg, first || s_dups != 0, &slot, a.err);
       MapSlot* s = &a.map.slots[slot];
+      bool older = false;
       if (r == INS_NEW) {
-        slot_init(s, win_of(epoch, node), cur, low);
+        old = slot_init(s, w, cur);
+        ours = true;
         created++;
       } else if (r == INS_EXISTING) {
-        old = win_min(s, win_of(epoch, node));
-        if (old != kWinEmpty && win_epoch(old) != epoch && EPI == EPI_TREE && __ldcg(&s->tree) == cur) {
+        old = win_min(s, w);
+        older = old != kWinEmpty && win_epoch(old) != epoch;
+        ours = !older || (EPI == EPI_TREE && __ldcg(&s->tree) == cur);
+        if (older && ours) {
           // lowest node within the older entry (the reference's atomic_min,
           // src/tree_approach.cpp:337-339): the entry's high bits (epoch and
           // serial level) are fixed, since every insert of this launch carries
           // a larger epoch and leaves them alone, so lowering the whole word
           // lowers exactly its node
-          if (win_node(old) > node) win_min(s, (old & ~0xffffffffull) | node);
-          here = true;
+          w = (old & ~0xffffffffull) | node;
+          if (old > w) old = win_min(s, w);
+        }
+      }
+      wins = ours && old >= w;
+      if (wins && old > w && old != kWinEmpty) {
+        // the chunk that had it; an older entry's owner is one of this launch's
+        // only if it is a changed chunk with this digest
+        const uint32_t was = win_node(old) - (EPI == EPI_TREE ? a.leaf_base : 0u);
+        if (!older || (win_node(old) >= a.leaf_base && a.labels[was] == FIRST_OCUR &&
+                       digest_eq(map_key(ld_digest(a.prev + was)), dg))) {
+          a.labels[was] = SHIFT_DUPL;
+          lost = true;
         }
       }
     }
     first = false;
     if (__any_sync(0xffffffffu, r == INS_EXISTING) && lane == 0) s_dups = 1;
-    r = __shfl_sync(0xffffffffu, r, lead);
-    slot = __shfl_sync(0xffffffffu, slot, lead);
-    old = __shfl_sync(0xffffffffu, old, lead);
-    here = __shfl_sync(0xffffffffu, (int)here, lead) != 0;
-    if (!in) continue;
-    uint8_t label = SHIFT_DUPL;
-    if (r == INS_NEW) {
-      label = FIRST_OCUR;
-      if (c != low) note_dup(a, (uint32_t)k | kCheckCreator);
-    } else if (r == INS_EXISTING) {
-      if (old == kWinEmpty || win_epoch(old) == epoch) {
-        label = FIRST_OCUR;  // first seen by this launch: the lowest chunk keeps it
-        note_dup(a, (uint32_t)k | kCheckCreator);
-      } else if (here) {
-        label = FIRST_OCUR;
-        note_dup(a, (uint32_t)k);
-      }
-    }
-    a.chunk_slot[k] = (uint32_t)slot;  // by list position: a sequential write
-    a.labels[c] = label;
+    ours = __shfl_sync(0xffffffffu, (int)ours, lead) != 0;
+    wins = __shfl_sync(0xffffffffu, (int)wins, lead) != 0;
+    const bool dup = in && !(wins && c == low);
+    if (dup) a.labels[c] = SHIFT_DUPL;
+    lost |= dup && ours;
   }
+  // one store per block: with one per warp the word was what a baseline with
+  // duplicates all over it waited for
+  if (EPI == EPI_TREE && a.demoted && __syncthreads_or(lost) && threadIdx.x == 0) *a.demoted = 1;
   count_new_entries(a.map, created);
-}
-
-// Second pass (src/tree_approach.cpp:356-369): a first occurrence that does
-// not own its digest becomes a shifted duplicate.  Only the noted chunks and
-// the creators of their entries can be such.
-__device__ __forceinline__ void demote_chunk(const LeafArgs& a, uint32_t c, const MapSlot* s, uint32_t cur) {
-  if (a.labels[c] != FIRST_OCUR) return;
-  const uint32_t node = a.leaf_base + c;
-  const uint32_t owner = win_node(s->win);
-  if (a.epi == EPI_TREE ? (s->tree == cur && owner != node) : (owner != node)) {
-    a.labels[c] = SHIFT_DUPL;
-    if (a.demoted) atomicOr(a.demoted, 1u);
-  }
-}
-__global__ void leaf_demote_kernel(LeafArgs a) {
-  pdl_enter();
-  const uint32_t n = min(*a.dup_count, a.dup_cap);
-  const uint32_t cur = a.sp->cur;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t e = a.dup_list[i];
-    const uint32_t k = e & ~kCheckCreator;
-    const uint32_t c = a.fresh ? k : a.changed_list[k];
-    const MapSlot* s = &a.map.slots[a.chunk_slot[k]];
-    demote_chunk(a, c, s, cur);
-    if (e & kCheckCreator) demote_chunk(a, s->first_chunk, s, cur);
-  }
 }
 
 template <int EPI>
@@ -1118,8 +1092,7 @@ cudaError_t launch_leaf_inserts(const LeafArgs& a, cudaStream_t s) {
   // 2 GiB map: 0.16 ms slower, 1 GiB MD5 increments 6 us)
   if (a.epi == EPI_TREE) launch_with(false, leaf_insert_kernel<EPI_TREE>, grid, 256, 0, s, a);
   else launch_with(false, leaf_insert_kernel<EPI_LIST>, grid, 256, 0, s, a);
-  launch_k(leaf_demote_kernel, grid, 256, 0, s, a);
-  note_launch(2);
+  note_launch();
   return cudaGetLastError();
 }
 

@@ -338,8 +338,7 @@ __host__ __device__ __forceinline__ uint32_t leftmost_leaf(uint32_t node, uint32
 // and the old value an insert gets back tells whether the entry is older
 // than its launch.  The node is win's low 32 bits.  `tree` (the checkpoint id
 // of the first occurrence) is written by the creator and read by later
-// launches; so is `first_chunk`, the chunk whose leaf insert created the
-// entry (read by that checkpoint's demote pass).  Both halves of a slot are
+// launches.  Both halves of a slot are
 // only written by 16-byte compare-and-swaps.  No insert waits on another
 // thread.
 // ---------------------------------------------------------------------------
@@ -347,7 +346,7 @@ struct __align__(32) MapSlot {
   uint32_t key[4];
   unsigned long long win;
   uint32_t tree;
-  uint32_t first_chunk;
+  uint32_t pad;
 };
 struct DigestMap {
   MapSlot* slots;
@@ -410,16 +409,16 @@ __device__ __forceinline__ uint4 claim_key(MapSlot* s, const Digest& k) {
 
 // The values of an entry this thread has just created, in one operation: the
 // half is still empty unless another insert of the key has lowered its win
-// word first, and then keeps the lower one.  With the claim, two operations
-// per new entry; a claim, two stores and a minimum cost 865 us for 2^23 random
-// inserts into a 2 GiB table, these 665 us (470 us without the read before
-// the claim), each operation on the line costing about the same.
-__device__ __forceinline__ void slot_init(MapSlot* s, unsigned long long win, uint32_t tree, uint32_t first_chunk) {
-  const unsigned long long hi = ((unsigned long long)first_chunk << 32) | tree;
+// word first, and then keeps the lower one.  Returns the word that was there.
+// With the claim, two operations per new entry; a claim, two stores and a
+// minimum cost 865 us for 2^23 random inserts into a 2 GiB table, these 665 us
+// (470 us without the read before the claim), each operation on the line
+// costing about the same.
+__device__ __forceinline__ unsigned long long slot_init(MapSlot* s, unsigned long long win, uint32_t tree) {
   Half seen = empty_half();
   while (true) {
-    const Half o = cas_half(&s->win, seen, Half{seen.lo < win ? seen.lo : win, hi});
-    if (half_eq(o, seen)) return;
+    const Half o = cas_half(&s->win, seen, Half{seen.lo < win ? seen.lo : win, tree});
+    if (half_eq(o, seen)) return seen.lo;
     seen = o;
   }
 }
@@ -558,7 +557,7 @@ __device__ __forceinline__ uint32_t map_insert_serial(const DigestMap& m, const 
   uint64_t slot;
   const unsigned long long win = win_of(epoch, serial_prio(node));
   const int r = map_claim(m, map_key(k), read, &slot, err);
-  if (r == INS_NEW) slot_init(&m.slots[slot], win, tree, 0xffffffffu);
+  if (r == INS_NEW) slot_init(&m.slots[slot], win, tree);
   else if (r == INS_EXISTING) win_min(&m.slots[slot], win);
   return r == INS_NEW ? 1u : 0u;
 }

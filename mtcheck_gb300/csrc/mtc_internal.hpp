@@ -44,12 +44,13 @@ struct ParamsOut {
   uint64_t* clk;
   uint32_t* counters;  // kCounters words, cleared
 };
-// Counters of a checkpoint: changed chunks, demoted leaves, queued forest
-// inserts, notes of the insert pass; finished blocks of the assembly's
-// launches; whether a baseline's shift test found the all-zero digest.
+// Counters of a checkpoint: changed chunks, whether a leaf lost its digest to a
+// lower one of the same checkpoint, queued forest inserts; finished blocks of
+// the assembly's launches; whether a baseline's shift test found the all-zero
+// digest.
 enum : int {
-  COUNT_CHANGED = 0, COUNT_DEMOTED = 1, COUNT_INSERTS = 2, COUNT_NOTES = 3,
-  COUNT_ROOTS_DONE = 4, COUNT_SORT_DONE = 5, COUNT_FINAL_DONE = 6, COUNT_ZERO_FOUND = 7, kCounters = 8
+  COUNT_CHANGED = 0, COUNT_DEMOTED = 1, COUNT_INSERTS = 2, COUNT_ROOTS_DONE = 3,
+  COUNT_SORT_DONE = 4, COUNT_FINAL_DONE = 5, COUNT_ZERO_FOUND = 6, kCounters = 7
 };
 
 struct LeafArgs {
@@ -59,7 +60,6 @@ struct LeafArgs {
   uint32_t n_chunks = 0;          // ceil(len / cs)
   Digest* prev = nullptr;         // per-chunk digest of the previous checkpoint (tree leaves or hash list)
   uint8_t* labels = nullptr;      // per-chunk label / changed flag out
-  uint32_t* chunk_slot = nullptr; // map slot of each changed-list entry (by list position)
   Digest* out = nullptr;          // EPI_HASH output
   DigestMap map{};
   const StepParams* sp = nullptr; // current checkpoint id and launch epoch (device)
@@ -68,10 +68,7 @@ struct LeafArgs {
   uint64_t* clk = nullptr;        // CLK_LEAVES_DONE is written by the insert pass (may be null)
   uint32_t* changed_list = nullptr;  // chunks whose digest changed (tree, list)
   uint32_t* changed_count = nullptr;
-  uint32_t* demoted = nullptr;    // set to 1 when a first occurrence is demoted (tree; may be null)
-  uint32_t* dup_list = nullptr;   // changed-list positions that met a duplicate inserted by the same launch
-  uint32_t* dup_count = nullptr;  // appends (at most the changed chunks)
-  uint32_t dup_cap = 0;
+  uint32_t* demoted = nullptr;    // set to 1 when a chunk is a shifted duplicate of one of this checkpoint's (tree; may be null)
   int hash_kind = HASH_MURMUR3;
   int epi = EPI_HASH;
   int basic_first = 0;            // basic approach with current_id == 0: every chunk changed
