@@ -1491,7 +1491,8 @@ cudaError_t launch_assemble(GatherArgs g, uint64_t max_entries, bool whole, cuda
   // this launch sequence can see
   const uint32_t K = std::min<uint32_t>(g.k_cap, kSortFastKeys);
   const uint32_t T = (uint32_t)((max_entries + kSortTile - 1) / kSortTile) + 1;
-  g.n_emit = (uint32_t)std::min<uint64_t>((max_entries + 255) / 256, 4ull * num_sms());
+  const uint32_t emit_cap = 4 * num_sms();
+  g.n_emit = whole ? (uint32_t)std::min<uint64_t>((max_entries + 255) / 256, emit_cap) : sparse_grid(max_entries, emit_cap);
   // tiles of the actual shift entries, read on the device: small grids
   g.n_sort = basic ? 0 : std::min<uint32_t>(T, 2 * num_sms());
   // one block scans the counts of all tiles; for larger matrices two launches
@@ -1519,18 +1520,18 @@ cudaError_t launch_assemble(GatherArgs g, uint64_t max_entries, bool whole, cuda
   // A first or whole checkpoint gathers (nearly) every chunk: a block per tile
   // keeps the copy at the bandwidth of a plain one (4 GiB: 1.21 ms against
   // 1.46 ms for a persistent grid).  An incremental one gathers a few percent
-  // and gets one wave of blocks: a block per possible tile costs more to
-  // launch than the copy takes.
+  // and gets one wave of blocks at most: a block per possible tile costs more
+  // to launch than the copy takes.
   const uint64_t tile_bytes = 16ull * (g.cs >= 128 ? kCopyTileUnits : 16 * g.cs);
   const uint64_t ctiles = ((uint64_t)g.N * g.cs + tile_bytes - 1) / tile_bytes;
   const uint32_t wave = (uint32_t)num_sms() * 5;
-  uint32_t copies = (uint32_t)std::min<uint64_t>(ctiles, whole ? 1u << 20 : wave);
+  uint32_t copies = whole ? (uint32_t)std::min<uint64_t>(ctiles, 1u << 20) : sparse_grid(256 * ctiles, wave);
   if (whole && copies > wave) {  // never in a captured sequence
     launch_k(vec ? copy_kernel<true> : copy_kernel<false>, copies, 256, 0, s, g);
     note_launch();
     copies = 0;
   }
-  g.n_drain = g.fuse_gate ? std::min<uint32_t>(2 * num_sms(), (g.N + 255) / 256) : 0;
+  g.n_drain = g.fuse_gate ? sparse_grid(g.N, 2 * num_sms()) : 0;
   if (join) {
     const cudaError_t e = cudaStreamWaitEvent(s, join, 0);
     if (e != cudaSuccess) return e;

@@ -1086,7 +1086,8 @@ cudaError_t batch_leaf_node_params(const BatchLeafParams& p, cudaKernelNodeParam
 }
 
 cudaError_t launch_leaf_inserts(const LeafArgs& a, cudaStream_t s) {
-  const uint32_t grid = (uint32_t)num_sms() * 6;
+  const uint32_t wave = (uint32_t)num_sms() * 6;
+  const uint32_t grid = a.fresh ? wave : sparse_grid(a.n_chunks, wave);
   // not while the hashing kernel still holds its SMs: blocks that start beside
   // it run with the little L1 its shared memory leaves (2^23 inserts into a
   // 2 GiB map: 0.16 ms slower, 1 GiB MD5 increments 6 us)
