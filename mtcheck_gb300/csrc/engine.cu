@@ -44,17 +44,6 @@ static __global__ void params_host_kernel(const volatile StepParams* host, Param
 // Polls of an injected stall's bounded waits (about a millisecond).
 constexpr uint32_t kInjectedSpinLimit = 1u << 14;
 
-static __global__ void readback_kernel(Readback r) {
-  pdl_enter();
-  readback(r);
-}
-
-cudaError_t launch_readback(const Readback& r, cudaStream_t s) {
-  launch_k(readback_kernel, 1, 32, 0, s, r);
-  note_launch();
-  return cudaGetLastError();
-}
-
 static __global__ void take_word_kernel(uint32_t* dev, uint32_t* host) {
   pdl_enter();
   *host = *dev;

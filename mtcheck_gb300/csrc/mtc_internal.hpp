@@ -176,8 +176,7 @@ struct Readback {
   uint32_t words[4];
   uint64_t* clk;  // CLK_END is written here first (may be null)
 };
-cudaError_t launch_readback(const Readback& r, cudaStream_t s);
-// One device word moved to pinned memory the same way, and cleared.
+// One device word moved to pinned memory by a kernel, and cleared.
 cudaError_t launch_take_word(uint32_t* dev, uint32_t* host, cudaStream_t s);
 // The device address of pinned host memory (the same pointer under unified
 // addressing).

@@ -81,6 +81,7 @@ struct RArgs {
   uint8_t* out;
   uint32_t* err;
   uint32_t c_lo, c_hi;           // resolve / copy: chunks [c_lo, c_hi), c_lo a multiple of 32
+  uint32_t* err_host;            // pinned: the copy of the last range writes the error word here
 };
 
 __device__ __forceinline__ uint32_t rd32(const uint8_t* p) {
@@ -396,6 +397,7 @@ __device__ __forceinline__ uint32_t chain_rm_items(const RArgs& a, uint32_t node
 // it the repeat tables.  Tiles belong to one diff, so that a prefix within the
 // diff is a sum over the diff's own tiles.
 __global__ void __launch_bounds__(kScanThreads) entry_load_kernel(RArgs a) {
+  pdl_enter();
   __shared__ uint64_t sh[33];
   const uint32_t nt = a.n_fo_tiles + a.n_sh_tiles;
   if (blockIdx.x >= nt) {
@@ -1131,7 +1133,11 @@ __global__ void __launch_bounds__(256, 8) resolve_kernel(RArgs a) {
 }
 
 // 5. Each warp copies 32 consecutive chunks from the sources resolved above.
+// The error word, final once the last range is resolved, goes to the host from
+// here: a launch for it and the gap before it took 5 us.
 __global__ void __launch_bounds__(256, 3) restore_copy_kernel(RArgs a) {
+  pdl_enter();
+  if (a.err_host && blockIdx.x == 0 && threadIdx.x == 0) *a.err_host = *a.err;
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
   const uint64_t t_hi = ((uint64_t)a.c_hi + 31) / 32;
@@ -1487,13 +1493,13 @@ int Engine::restart_enqueue(uint8_t* dev_out, uint64_t len, const std::vector<co
   StepTimer t_dec("restart: entry launches", N);
   setup_kernel<<<1, 256, 0, s>>>(static_cast<const uint4*>(host_alias(rdi_host_)), reinterpret_cast<uint4*>(R.di.p),
                                  (uint32_t)(di_bytes / 16), err_.p, R.tot.p);
-  MTC_CUDA_R(cudaEventRecord(rdi_ev_, s));
   note_launch();
   const uint32_t ntiles = n_fo_tiles + n_sh_tiles;
   if (ntiles + a.n_rrs) {
-    entry_load_kernel<<<ntiles + a.n_rrs, kScanThreads, 0, s>>>(a);
+    launch_k(entry_load_kernel, ntiles + a.n_rrs, kScanThreads, 0, s, a);
     note_launch();
   }
+  MTC_CUDA_R(cudaEventRecord(rdi_ev_, s));
   if (ntiles && !basic) {  // a basic entry's number is its index, and it has no shift entries
     const bool scanned = tree && std::max(n_fo_tiles, n_sh_tiles) > reduce_tile_limit();
     if (scanned) {
@@ -1534,8 +1540,9 @@ int Engine::restart_enqueue(uint8_t* dev_out, uint64_t len, const std::vector<co
     r.c_lo = (uint32_t)lo;
     r.c_hi = (uint32_t)std::min<uint64_t>(N, lo + step);
     resolve_kernel<<<std::min(gsz(r.c_hi - r.c_lo), resolve_grid()), 256, 0, s>>>(r);
+    if (r.c_hi == N) r.err_host = static_cast<uint32_t*>(host_alias(err_host_));
     if (parts == 1) {
-      restore_copy_kernel<<<num_sms() * 3, 256, 0, s>>>(r);
+      launch_k(restore_copy_kernel, num_sms() * 3, 256, 0, s, r);
     } else {
       MTC_CUDA_R(cudaEventRecord(rev_[4 + launched], s));
       MTC_CUDA_R(cudaStreamWaitEvent(side, rev_[4 + launched], 0));
@@ -1547,12 +1554,8 @@ int Engine::restart_enqueue(uint8_t* dev_out, uint64_t len, const std::vector<co
     MTC_CUDA_R(cudaEventRecord(rev_[11], side));
     MTC_CUDA_R(cudaStreamWaitEvent(s, rev_[11], 0));
   }
+  MTC_CUDA_R(cudaGetLastError());
   cudaEventRecord(e1, s);
-  Readback rb{};
-  rb.src[0] = err_.p;
-  rb.dst[0] = static_cast<uint32_t*>(host_alias(err_host_));
-  rb.words[0] = 1;
-  MTC_CUDA_R(launch_readback(rb, s));
   return ST_OK;
 }
 
