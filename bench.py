@@ -365,8 +365,9 @@ def small_series_section(torch, mc, dev, peak):
             "ms_with_phase_events": round(t_timed * 1e3, 4),
             "leaf_ms": round(leaf * 1e3, 4),
             "roofline_frac": round(b / t / 1e9 / peak, 4),
-            "note": "value and ms: replayed as one graph (mtc_tune_t.untimed); ms_with_phase_events: the default "
-                    "five graph launches with events between the phases, which the leaf time comes from; "
+            "note": "value and ms: replayed as one graph without phase stamps (mtc_tune_t.untimed); "
+                    "ms_with_phase_events: the default, whose kernels stamp the device clock between the phases, "
+                    "which the leaf time comes from; "
                     "roofline_frac: B_dedup = D + 32 N + 2 S_data + S_meta per device-timed checkpoint over the "
                     "measured HBM copy bandwidth"}
 
