@@ -7,10 +7,10 @@
 // swizzle so that the 256 consumer threads read their rows without bank
 // conflicts.  A dedicated producer warp keeps STAGES boxes in flight; full/empty
 // mbarriers hand stages between producer and consumers; one more warp hashes a
-// partial last chunk.  Odd chunk sizes and unaligned buffers go through a staged
-// kernel, short odd chunks through a thread-per-chunk kernel that reads global
-// memory directly.  All end in the same epilogue, which restates the leaf loops
-// of the reference:
+// partial last chunk.  Other short chunks come as whole tiles by untiled bulk
+// copies, longer ones in panels through a staged kernel, the rest through a
+// thread-per-chunk kernel that reads global memory directly.  All end in the
+// same epilogue, which restates the leaf loops of the reference:
 //   tree  -- src/tree_approach.cpp:57-94 (baseline) and :309-351
 //   list  -- src/list_approach.cpp:38-61
 //   basic -- src/basic_approach.cpp:25-46
@@ -631,6 +631,128 @@ __global__ void __launch_bounds__(kStageRows, 4) leaf_staged_kernel(LeafArgs a, 
 }
 
 // ---------------------------------------------------------------------------
+// Short chunks that no box fits: the 128 chunks of a tile are contiguous, so one
+// untiled bulk copy of 128 * cs bytes (from the 16-byte boundary before them to
+// the one after) brings a tile in whatever its chunk size and alignment, and a
+// producer lane keeps two in flight.  A thread reads its row word by word: an
+// odd multiple of four bytes apart, rows lie in different banks.  Bound by the
+// integer pipe (hashing, and realigning words).  Two stages, for more CTAs per SM
+// (three: 250-byte chunks 73 us for 256 MiB, two 62).  Whole calls, two stages
+// against the kernels before: 400 MB in chunks of 100 bytes 130 -> 91 us
+// (Murmur3), 183 -> 174 (MD5); 256 MiB in 300 bytes 131 -> 69 and 166 -> 106.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kRowTile = 128;
+constexpr int kRowStages = 2;
+constexpr uint32_t kRowsMax = 440;
+__host__ __device__ constexpr uint32_t row_stage_bytes(uint32_t cs) { return (kRowTile * cs + 30) & ~15u; }
+// barriers, stages, and what a row's last words are read past its end (masked)
+__host__ __device__ constexpr uint32_t row_smem_bytes(uint32_t cs) {
+  return 128 + kRowStages * row_stage_bytes(cs) + 128;
+}
+
+template <int HK, int EPI>
+__global__ void __launch_bounds__(kRowTile + 32, HK == HASH_MD5 ? 5 : 8) leaf_rows_kernel(LeafArgs a, uint32_t c0,
+                                                                                        uint32_t c1) {
+  pdl_enter();
+  extern __shared__ __align__(128) uint8_t row_smem[];
+  uint64_t* full = reinterpret_cast<uint64_t*>(row_smem);
+  uint64_t* empty = full + kRowStages;
+  uint8_t* stages = row_smem + 128;
+  constexpr bool kLists = EPI == EPI_TREE || EPI == EPI_LIST;
+  __shared__ uint32_t changed_buf[kLists ? kRowTile / 32 : 1][64];
+  const uint32_t tid = threadIdx.x, cs = a.cs, stage_bytes = row_stage_bytes(cs);
+  const uint32_t ntiles = (c1 - c0 + kRowTile - 1) / kRowTile;
+  const uint32_t limit = a.spin_limit ? a.spin_limit : kMbarSpinLimit;
+  const uint64_t base = reinterpret_cast<uint64_t>(a.data) + (uint64_t)c0 * cs;
+  const uint64_t end = reinterpret_cast<uint64_t>(a.data) + min(a.len, (uint64_t)c1 * cs);
+  if (tid == 0) {
+    for (int s = 0; s < kRowStages; s++) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], kRowTile / 32);
+    }
+    mbar_fence_init();
+  }
+  __syncthreads();
+
+  if (tid >= kRowTile) {
+    if (tid != kRowTile) return;
+    uint32_t it = 0;
+    bool ok = !a.stall;  // injected fault: no copy is ever issued
+    for (uint32_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, it++) {
+      const uint32_t s = it % kRowStages, ph = (it / kRowStages) & 1;
+      if (!mbar_wait(&empty[s], ph ^ 1, limit)) { raise_err(a.err, DERR_SPIN); ok = false; break; }
+      const uint64_t p0 = (base + (uint64_t)tile * kRowTile * cs) & ~15ull;
+      const uint64_t p1 = min(end, base + (uint64_t)(tile + 1) * kRowTile * cs);
+      const uint32_t bytes = (uint32_t)(p1 - p0 + 15) & ~15u;
+      mbar_arrive_expect_tx(&full[s], bytes);
+      bulk_load(stages + s * stage_bytes, reinterpret_cast<const void*>(p0), bytes, &full[s]);
+    }
+    // drain: every issued copy must land before the CTA may exit
+    for (uint32_t j = it > (uint32_t)kRowStages ? it - kRowStages : 0; j < it; j++)
+      mbar_wait(&full[j % kRowStages], (j / kRowStages) & 1);
+    return;
+  }
+
+  const uint32_t lane = tid & 31;
+  ChangedBuf list{changed_buf[kLists ? tid >> 5 : 0], 0};
+  uint32_t it = 0;
+  for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
+    const uint64_t c = (uint64_t)c0 + (uint64_t)tile * kRowTile + tid;
+    const bool valid = c < c1;
+    Digest old{{0, 0, 0, 0}};
+    if (valid && needs_old<EPI>(a)) old = ld_digest(a.prev + c);
+    const uint32_t s = it % kRowStages, ph = (it / kRowStages) & 1;
+    if (!mbar_wait(&full[s], ph, limit)) { raise_err(a.err, DERR_SPIN); return; }
+    const uint32_t nb = !valid ? 0 : (uint32_t)min((uint64_t)cs, a.len - c * cs);
+    const uint32_t o = (uint32_t)((base + (uint64_t)tile * kRowTile * cs) & 15) + tid * cs;
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(stages + s * stage_bytes) + (o >> 2);
+    const uint32_t sh = (o & 3) * 8;
+    constexpr uint32_t kWords = HK == HASH_MD5 ? 16 : 4;
+    Md5State md;
+    Murmur3State mm;
+    if (HK == HASH_MD5) md.init(); else mm.init();
+    uint32_t X[kWords];
+    uint32_t left = nb;
+#pragma unroll 1
+    while (true) {
+      if (valid) {
+        uint32_t lo = w[0];
+#pragma unroll
+        for (uint32_t i = 0; i < kWords; i++) {
+          // past a short last chunk's copy the words are whatever the stage holds
+          const uint32_t hi = w[i + 1];
+          X[i] = __funnelshift_r(lo, hi, sh);
+          lo = hi;
+        }
+      }
+      if (left < 4 * kWords) break;
+      if (HK == HASH_MD5) md.block(X); else mm.block(X[0], X[1], X[2], X[3]);
+      left -= 4 * kWords;
+      w += kWords;
+    }
+    // the rows go back before the epilogue
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[s]);
+#pragma unroll
+    for (uint32_t i = 0; i < kWords; i++) {  // zero past the end
+      const int k = (int)left - 4 * (int)i;
+      X[i] &= k <= 0 ? 0u : k >= 4 ? ~0u : (1u << (8 * k)) - 1;
+    }
+    Digest dg;
+    if (HK == HASH_MD5) {
+      dg = md.finish(X, left, nb);
+    } else {
+      mm.tail(((uint64_t)X[1] << 32) | X[0], ((uint64_t)X[3 % kWords] << 32) | X[2], left);
+      dg = mm.finish(nb);
+    }
+    const bool changed = leaf_store<EPI>(a, valid, (uint32_t)c, dg, old);
+    if (appends<EPI>(a)) list.add(a, changed, (uint32_t)c);
+  }
+  if (appends<EPI>(a)) list.flush(a);
+}
+
+// ---------------------------------------------------------------------------
 // One persistent launch for the leaf pass of many deduplicators (a batch).
 // A device work queue holds (member, tile) items; each CTA's producer lane
 // claims the next item with one atomicAdd and streams its boxes through the
@@ -996,6 +1118,39 @@ cudaError_t dispatch_staged(const LeafArgs& a, uint32_t c0, uint32_t c1, cudaStr
   }
 }
 
+template <int HK, int EPI>
+cudaError_t launch_rows_t(const LeafArgs& a, cudaStream_t s) {
+  auto k = leaf_rows_kernel<HK, EPI>;
+  static const bool reg = (register_input_kernel(reinterpret_cast<const void*>(k), INPUT_LEAF_DIRECT), true);
+  (void)reg;
+  const size_t smem = row_smem_bytes(a.cs);
+  static std::atomic<bool> attr_set{false};
+  if (!attr_set.load(std::memory_order_acquire)) {
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)row_smem_bytes(kRowsMax));
+    if (e != cudaSuccess) return e;
+    attr_set.store(true, std::memory_order_release);
+  }
+  const uint32_t fit = (uint32_t)((227u * 1024u) / (smem + 2048));
+  const uint32_t per_sm = std::min<uint32_t>(fit, HK == HASH_MD5 ? 5 : 8);
+  const uint32_t tiles = (a.n_chunks + kRowTile - 1) / kRowTile;
+  launch_k(k, std::min<uint32_t>(tiles, num_sms() * per_sm), kRowTile + 32, smem, s, a, 0u, a.n_chunks);
+  note_launch();
+  return cudaGetLastError();
+}
+template <int EPI>
+cudaError_t launch_rows(const LeafArgs& a, cudaStream_t s) {
+  return a.hash_kind == HASH_MD5 ? launch_rows_t<HASH_MD5, EPI>(a, s) : launch_rows_t<HASH_MURMUR3, EPI>(a, s);
+}
+cudaError_t dispatch_rows(const LeafArgs& a, cudaStream_t s) {
+  switch (a.epi) {
+    case EPI_TREE: return launch_rows<EPI_TREE>(a, s);
+    case EPI_LIST: return launch_rows<EPI_LIST>(a, s);
+    case EPI_BASIC: return launch_rows<EPI_BASIC>(a, s);
+    default: return launch_rows<EPI_HASH>(a, s);
+  }
+}
+
 cudaError_t dispatch_direct(const LeafArgs& a, uint32_t c0, uint32_t c1, cudaStream_t s) {
   switch (a.epi) {
     case EPI_TREE: return launch_direct<EPI_TREE>(a, c0, c1, s);
@@ -1071,10 +1226,18 @@ bool input_tmap(TmaCache* c, const uint8_t* data, uint64_t len, uint32_t cs, con
          make_tmap(c, data, len, cs, W, rows, n_full);
 }
 
-// Chunks up to here are read directly when no tiled copy fits: a warp's 32
-// chunks then share their lines in L1, and a panel is mostly padding (400 MB in
-// 100-byte chunks: 140 us direct, 226 us staged; 256 MiB in 128-byte chunks off a
-// boundary: 282 and 117 us).
+// Chunks without a tiled copy whose tiles are copied whole (leaf_rows_kernel): up
+// to 440 bytes, where two stages of two CTAs still fit an SM (256 MiB in chunks
+// of 436 bytes: 70 us, staged 125; of 24 bytes: 106, direct 124; of 63: 70 and
+// 208); not multiples of 32 bytes (buffers off a boundary), whose rows share
+// banks (64 MiB in 128-byte chunks: 97 us, staged 33); not MD5 of less than a
+// block, which wants the direct kernel's warps (256 MiB in 56 bytes: 199, 174).
+bool rows_fit(const LeafArgs& a) {
+  return a.cs <= kRowsMax && a.cs % 32 != 0 && (a.hash_kind != HASH_MD5 || a.cs >= 64);
+}
+// Of the others, chunks up to here are read directly: a warp's 32 chunks share
+// their lines in L1, and a panel is mostly padding (64 MiB in 64-byte chunks off a
+// boundary: 50 us direct; in 128-byte chunks, 256 MiB: 282 us direct, 117 staged).
 constexpr uint32_t kDirectMax = 100;
 
 cudaError_t launch_leaves(const LeafArgs& a, TmaCache* cache, cudaStream_t s, const LeafTune& tune) {
@@ -1087,6 +1250,7 @@ cudaError_t launch_leaves(const LeafArgs& a, TmaCache* cache, cudaStream_t s, co
   if (t.threads_per_chunk == 32 && a.cs <= kWarpChunkMax) return dispatch_warp(a, 0, a.n_chunks, s);
   if (!t.direct && W && aligned && n_full > 0 && cache && make_tmap(cache, a.data, a.len, a.cs, W, t.rows, n_full))
     return dispatch_tma(a, cache->map, n_full, W, t, s);
+  if (!t.direct && rows_fit(a)) return dispatch_rows(a, s);
   if (!t.direct && a.cs > kDirectMax) return dispatch_staged(a, 0, a.n_chunks, s);
   return dispatch_direct(a, 0, a.n_chunks, s);
 }

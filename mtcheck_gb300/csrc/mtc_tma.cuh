@@ -52,6 +52,14 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
       "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
       : "memory");
 }
+// Copy of `bytes` contiguous bytes into shared memory, completing on `bar`: both
+// addresses on 16-byte boundaries, the size a multiple of 16.
+__device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_u32(smem_dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
 // Orders this thread's generic-proxy accesses to shared memory before later
 // async-proxy (TMA) accesses: a consumer runs it before releasing a stage
 // that the producer will refill, or the refill may land before its reads.
