@@ -557,7 +557,7 @@ int Engine::retarget(cudaGraphExec_t exec, std::vector<InputNode>& nodes, const 
       continue;
     }
     if (in.kind == INPUT_LEAF_TMA) {
-      if (!input_tmap(&tma_, data, len, cs_, leaf_tune_)) return fail(ST_ECUDA, "tensor map for the new input");
+      if (!input_tmap(&tma_, data, len, cs_, hash_kind_, leaf_tune_)) return fail(ST_ECUDA, "tensor map for the new input");
       in.tmap = tma_.map;
       in.la.data = data;
       args[0] = &in.tmap;

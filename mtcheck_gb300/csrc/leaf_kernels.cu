@@ -260,14 +260,21 @@ __device__ __forceinline__ bool needs_old(const LeafArgs& a) {
 // ahead of the hashing, from L2.  Digests of 1.4 MB in chunks of 4096 bytes with
 // a tail of 3743: Murmur3 89 -> 36 us, MD5 127 -> 63 us; without
 // the tail 31 and 58 us.
-template <int HK>
-__device__ __noinline__ Digest hash_tail(const uint4* p, uint32_t len) {
+// kShift: they start d bytes past p.
+template <int HK, bool kShift>
+__device__ __noinline__ Digest hash_tail(const uint4* p, uint32_t d, uint32_t len) {
   constexpr uint32_t kWords = 4, kPiece = 16 * kWords;
   uint4 v[kWords];
+  const uint64_t stop = (uint64_t)len + (kShift ? d : 0);  // from p
+  auto word = [&](uint64_t at) { return at < stop ? __ldg(p + at / 16) : make_uint4(0, 0, 0, 0); };
   auto load = [&](uint64_t off) {
 #pragma unroll
-    for (uint32_t q = 0; q < kWords; q++)
-      v[q] = off + 16 * q < len ? __ldg(p + off / 16 + q) : make_uint4(0, 0, 0, 0);
+    for (uint32_t q = 0; q < kWords; q++) v[q] = word(off + 16 * q);
+    if (kShift) {
+      const uint4 after = word(off + kPiece);
+#pragma unroll
+      for (uint32_t q = 0; q < kWords; q++) v[q] = cut16(v[q], q + 1 < kWords ? v[q + 1] : after, d);
+    }
   };
   Md5State md;
   Murmur3State mm;
@@ -311,7 +318,15 @@ __device__ __noinline__ Digest hash_tail(const uint4* p, uint32_t len) {
   return mm.finish(len);
 }
 
-template <int HK, int EPI, int W, int kRows>
+// kShift: a buffer off a 16-byte boundary is tiled from the boundary before it, so
+// chunk r starts d bytes into row r and ends d bytes into row r + 1.  Each 16
+// bytes are cut out of two words; the last word of a box waits for the next box,
+// and the first word of the next row is read with the row's first box (from
+// global memory for a tile's last row).  Against the staged kernel (64-byte
+// chunks: direct reads), 4 bytes off: 1 GiB in 4096-byte chunks 369 -> 216 us
+// (Murmur3), 480 -> 269 (MD5); 256 MiB in 128-byte chunks 107 -> 67, 168 -> 111; in
+// 64-byte chunks 150 -> 75, 221 -> 138.  On a boundary the 128-byte ones take 60.
+template <int HK, int EPI, int W, int kRows, bool kShift>
 __global__ void __launch_bounds__(kRows + 64, 2) leaf_tma_kernel(const __grid_constant__ CUtensorMap tmap, LeafArgs a,
                                                               uint32_t n_full) {
   pdl_enter();
@@ -324,6 +339,8 @@ __global__ void __launch_bounds__(kRows + 64, 2) leaf_tma_kernel(const __grid_co
   const uint32_t xsteps = a.cs / W;
   const uint32_t ntiles = (n_full + kRows - 1) / kRows;
   const uint32_t limit = a.spin_limit ? a.spin_limit : kMbarSpinLimit;
+  static_assert(!kShift || W >= 64, "whole MD5 blocks per box");
+  const uint32_t d = kShift ? (uint32_t)(reinterpret_cast<uintptr_t>(a.data) & 15) : 0;
 
   if (tid == 0) {
     for (int s = 0; s < kStages; s++) {
@@ -344,7 +361,8 @@ __global__ void __launch_bounds__(kRows + 64, 2) leaf_tma_kernel(const __grid_co
       if (tid != kRows + 32) return;
       Digest old{{0, 0, 0, 0}};
       if (needs_old<EPI>(a)) old = ld_digest(a.prev + n_full);
-      leaf_epilogue<EPI>(a, true, n_full, hash_tail<HK>(reinterpret_cast<const uint4*>(tail), nb), old);
+      const Digest dg = hash_tail<HK, kShift>(reinterpret_cast<const uint4*>(tail - d), d, nb);
+      leaf_epilogue<EPI>(a, true, n_full, dg, old);
       return;
     }
     // producer warp: one elected lane issues every box in consumption order
@@ -381,6 +399,7 @@ __global__ void __launch_bounds__(kRows + 64, 2) leaf_tma_kernel(const __grid_co
     Md5State md;
     if (HK == HASH_MD5) md.init(); else mm.init();
     uint32_t X[16];
+    uint4 carry = make_uint4(0, 0, 0, 0), next = carry;  // kShift
     for (uint32_t xs = 0; xs < xsteps; xs++, it++) {
       const uint32_t s = it % kStages, ph = (it / kStages) & 1;
       if (!mbar_wait(&full[s], ph, limit)) { raise_err(a.err, DERR_SPIN); return; }
@@ -391,11 +410,29 @@ __global__ void __launch_bounds__(kRows + 64, 2) leaf_tma_kernel(const __grid_co
       uint4 row[W / 16];
 #pragma unroll
       for (int q = 0; q < W / 16; q++) row[q] = *reinterpret_cast<const uint4*>(stage + swz<W>(rowbase + q * 16));
+      if (kShift && xs == 0 && valid) {
+        if (tid + 1 < kRows && c + 1 < n_full) next = *reinterpret_cast<const uint4*>(stage + swz<W>(rowbase + W));
+        else next = __ldg(reinterpret_cast<const uint4*>(a.data - d + (uint64_t)(c + 1) * a.cs));
+      }
       // release the stage: this thread's reads before the refill's TMA write
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[s]);
-      if (HK == HASH_MD5) {
+      if (kShift) {
+        auto put = [&](int slot, const uint4& v) {  // the next 16 bytes; MD5: fourth `slot` of its block
+          if (HK == HASH_MD5) {
+            X[4 * slot] = v.x; X[4 * slot + 1] = v.y; X[4 * slot + 2] = v.z; X[4 * slot + 3] = v.w;
+            if (slot == 3) md.block(X);
+          } else {
+            mm.block(v.x, v.y, v.z, v.w);
+          }
+        };
+        if (xs) put(3, cut16(carry, row[0], d));
+#pragma unroll
+        for (int q = 0; q + 1 < W / 16; q++) put(q & 3, cut16(row[q], row[q + 1], d));
+        carry = row[W / 16 - 1];
+        if (xs + 1 == xsteps) put(3, cut16(carry, next, d));
+      } else if (HK == HASH_MD5) {
         if (W >= 64) {
 #pragma unroll
           for (int blk = 0; blk < W / 64; blk++) {
@@ -458,8 +495,8 @@ __global__ void leaf_direct_kernel(LeafArgs a, uint32_t c0, uint32_t c1) {
 }
 
 // ---------------------------------------------------------------------------
-// Staged kernel for what the tiled copies cannot take: chunk sizes that are no
-// supported box width, and buffers off a 16-byte boundary.  One thread hashes
+// Staged kernel for what the tiled copies and whole tiles cannot take: longer chunk
+// sizes, and multiples of 32 bytes, that are no supported box width.  One thread hashes
 // one chunk, 128 chunks per tile, in panels of 128 bytes that come through
 // shared memory: a thread that reads its own chunk from global memory touches
 // a line per lane.  Rows of a panel start on 16 bytes of shared memory whatever
@@ -1026,9 +1063,9 @@ bool make_tmap(TmaCache* c, const uint8_t* data, uint64_t len, uint32_t cs, int 
   return true;
 }
 
-template <int HK, int EPI, int W, int R>
+template <int HK, int EPI, int W, int R, bool kShift = false>
 cudaError_t launch_tma_t(const LeafArgs& a, const CUtensorMap& m, uint32_t n_full, int ctas_per_sm, cudaStream_t s) {
-  auto k = leaf_tma_kernel<HK, EPI, W, R>;
+  auto k = leaf_tma_kernel<HK, EPI, W, R, kShift>;
   static const bool reg = (register_input_kernel(reinterpret_cast<const void*>(k), INPUT_LEAF_TMA), true);
   (void)reg;
   const size_t smem = 1024 + (size_t)kStages * R * W + 2 * kStages * sizeof(uint64_t);
@@ -1069,6 +1106,24 @@ cudaError_t launch_tma_e(const LeafArgs& a, const CUtensorMap& m, uint32_t n_ful
   }
   if (a.hash_kind == HASH_MD5) return launch_tma_w<HASH_MD5, EPI, 256>(a, m, n_full, W, t.ctas_per_sm, s);
   return launch_tma_w<HASH_MURMUR3, EPI, 256>(a, m, n_full, W, t.ctas_per_sm, s);
+}
+
+// Buffers off a 16-byte boundary, with the digest's default tile
+template <int EPI>
+cudaError_t launch_shift(const LeafArgs& a, const CUtensorMap& m, uint32_t n_full, int W, int per_sm, cudaStream_t s) {
+  if (a.hash_kind == HASH_MD5)
+    return W == 128 ? launch_tma_t<HASH_MD5, EPI, 128, 256, true>(a, m, n_full, per_sm, s)
+                    : launch_tma_t<HASH_MD5, EPI, 64, 256, true>(a, m, n_full, per_sm, s);
+  return W == 128 ? launch_tma_t<HASH_MURMUR3, EPI, 128, 128, true>(a, m, n_full, per_sm, s)
+                  : launch_tma_t<HASH_MURMUR3, EPI, 64, 128, true>(a, m, n_full, per_sm, s);
+}
+cudaError_t dispatch_shift(const LeafArgs& a, const CUtensorMap& m, uint32_t n_full, int W, int per_sm, cudaStream_t s) {
+  switch (a.epi) {
+    case EPI_TREE: return launch_shift<EPI_TREE>(a, m, n_full, W, per_sm, s);
+    case EPI_LIST: return launch_shift<EPI_LIST>(a, m, n_full, W, per_sm, s);
+    case EPI_BASIC: return launch_shift<EPI_BASIC>(a, m, n_full, W, per_sm, s);
+    default: return launch_shift<EPI_HASH>(a, m, n_full, W, per_sm, s);
+  }
 }
 
 template <int EPI>
@@ -1218,26 +1273,34 @@ int num_sms() {
   return n;
 }
 
-bool input_tmap(TmaCache* c, const uint8_t* data, uint64_t len, uint32_t cs, const LeafTune& tune) {
+static int shift_rows(int hash_kind) { return hash_kind == HASH_MD5 ? 256 : 128; }
+
+bool input_tmap(TmaCache* c, const uint8_t* data, uint64_t len, uint32_t cs, int hash_kind, const LeafTune& tune) {
   const uint32_t n_full = (uint32_t)(len / cs);
   const int W = tma_width(cs);
-  const int rows = tune.rows != 128 ? 256 : 128;
-  return W && n_full > 0 && (reinterpret_cast<uintptr_t>(data) & 15) == 0 &&
-         make_tmap(c, data, len, cs, W, rows, n_full);
+  int rows = tune.rows != 128 ? 256 : 128;
+  if (!W || n_full == 0) return false;
+  const uint32_t d = (uint32_t)(reinterpret_cast<uintptr_t>(data) & 15);
+  if (d) {
+    if (W < 64) return false;
+    rows = shift_rows(hash_kind);
+  }
+  return make_tmap(c, data - d, len, cs, W, rows, n_full);
 }
 
 // Chunks without a tiled copy whose tiles are copied whole (leaf_rows_kernel): up
 // to 440 bytes, where two stages of two CTAs still fit an SM (256 MiB in chunks
 // of 436 bytes: 70 us, staged 125; of 24 bytes: 106, direct 124; of 63: 70 and
-// 208); not multiples of 32 bytes (buffers off a boundary), whose rows share
-// banks (64 MiB in 128-byte chunks: 97 us, staged 33); not MD5 of less than a
+// 208); not multiples of 32 bytes, whose rows share banks (64 MiB in 128-byte
+// chunks, before shifted boxes took them: 97 us, staged 33); not MD5 of less than a
 // block, which wants the direct kernel's warps (256 MiB in 56 bytes: 199, 174).
 bool rows_fit(const LeafArgs& a) {
   return a.cs <= kRowsMax && a.cs % 32 != 0 && (a.hash_kind != HASH_MD5 || a.cs >= 64);
 }
 // Of the others, chunks up to here are read directly: a warp's 32 chunks share
-// their lines in L1, and a panel is mostly padding (64 MiB in 64-byte chunks off a
-// boundary: 50 us direct; in 128-byte chunks, 256 MiB: 282 us direct, 117 staged).
+// their lines in L1, and a panel is mostly padding (400 MB in 100-byte chunks: 140 us
+// direct, 226 staged; 256 MiB in 128-byte chunks off a boundary: 282 direct, 117
+// staged; both before other kernels took them).
 constexpr uint32_t kDirectMax = 100;
 
 cudaError_t launch_leaves(const LeafArgs& a, TmaCache* cache, cudaStream_t s, const LeafTune& tune) {
@@ -1248,8 +1311,10 @@ cudaError_t launch_leaves(const LeafArgs& a, TmaCache* cache, cudaStream_t s, co
   LeafTune t = tune;
   if (t.rows != 128) t.rows = 256;
   if (t.threads_per_chunk == 32 && a.cs <= kWarpChunkMax) return dispatch_warp(a, 0, a.n_chunks, s);
-  if (!t.direct && W && aligned && n_full > 0 && cache && make_tmap(cache, a.data, a.len, a.cs, W, t.rows, n_full))
-    return dispatch_tma(a, cache->map, n_full, W, t, s);
+  if (!t.direct && (W >= 64 || (W && aligned)) && n_full > 0 && cache &&
+      input_tmap(cache, a.data, a.len, a.cs, a.hash_kind, t))
+    return aligned ? dispatch_tma(a, cache->map, n_full, W, t, s)
+                   : dispatch_shift(a, cache->map, n_full, W, t.ctas_per_sm, s);
   if (!t.direct && rows_fit(a)) return dispatch_rows(a, s);
   if (!t.direct && a.cs > kDirectMax) return dispatch_staged(a, 0, a.n_chunks, s);
   return dispatch_direct(a, 0, a.n_chunks, s);

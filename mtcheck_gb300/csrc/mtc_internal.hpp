@@ -244,7 +244,7 @@ void register_input_kernel(const void* func, int kind);
 int input_kernel_kind(const void* func);
 // The descriptor launch_leaves gives the TMA leaf kernel for this buffer and
 // launch shape (in c->map); false when TMA does not apply.
-bool input_tmap(TmaCache* c, const uint8_t* data, uint64_t len, uint32_t cs, const LeafTune& tune);
+bool input_tmap(TmaCache* c, const uint8_t* data, uint64_t len, uint32_t cs, int hash_kind, const LeafTune& tune);
 // Message returned by mtc_last_error() on this thread.
 void set_last_error(const char* msg);
 
