@@ -29,3 +29,19 @@ def test_insert_duplicates(cuda, mtc, oracle, approach, advance, n, palette):
             state[n // 4:n // 2] = colours[0]
         if step >= 2:
             state[n // 2:] = old[rng.integers(0, n, n - n // 2)]
+
+
+@pytest.mark.parametrize("copies", [1, 2, 5])
+def test_list_bins_of_many_checkpoints(cuda, mtc, oracle, copies):
+    """A few shift entries with sources among many checkpoints: the sort's bins are
+    fewer than the keys, so keys share them."""
+    cs, n = 64, 400
+    rng = np.random.default_rng(copies)
+    state = rng.integers(0, 256, (n, cs), dtype=np.uint8)
+    ref, gpu = oracle.Deduplicator(3, cs, 0), mtc.Deduplicator(cs, 0, approach=3)
+    for step in range(220):
+        want = ref.checkpoint(state.reshape(-1), step == 0)
+        assert gpu.checkpoint(cuda.from_numpy(state.reshape(-1).copy()).cuda(), step == 0) == want, step
+        old = state.copy()
+        state[step] = rng.integers(0, 256, cs, dtype=np.uint8)  # this checkpoint's own content
+        state[300 + rng.choice(100, copies, replace=False)] = old[rng.integers(0, step + 1, copies)]
