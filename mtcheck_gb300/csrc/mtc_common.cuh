@@ -514,7 +514,9 @@ __device__ __forceinline__ void count_new_entries(const DigestMap& m, uint32_t n
   __syncthreads();
   if (threadIdx.x == 0) s_new = 0;
   __syncthreads();
-  const uint32_t w = __reduce_add_sync(0xffffffffu, n);
+  uint32_t w = n;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
   if ((threadIdx.x & 31) == 0 && w) atomicAdd(&s_new, w);
   __syncthreads();
   if (threadIdx.x == 0 && s_new) atomicAdd(m.size, s_new);
