@@ -349,24 +349,10 @@ int Engine::run_tree(const uint8_t* data, uint64_t len, bool baseline_path) {
   else MTC_CUDA(launch_leaves(la, &tma_, stream_, leaf_tune_));
   MTC_CUDA(launch_leaf_inserts(la, stream_));
 
-  ForestArgs fa{};
-  fa.tree = digests_.p;
-  fa.labels = labels_.p;
-  fa.rflag = rflag_.p;
-  fa.map = map;
-  fa.sp = sp_.p;
-  fa.err = err_.p;
-  fa.hash_kind = hash_kind_;
-  fa.order = root_order();
+  ForestArgs fa = forest_args();
   // an incremental checkpoint without demoted leaves runs both passes in one
   // traversal (the launches of the duplicate pass then return at once)
   fa.fuse_gate = la.demoted;
-  // the changed-chunk list is free once the leaf inserts are done: it queues
-  // the forest's first-occurrence inserts
-  fa.ins_queue = changed_list_.p;
-  fa.ins_count = changed_count_.p + COUNT_INSERTS;
-  fa.span_done = span_done_.p;
-  fa.zero_found = changed_count_.p + COUNT_ZERO_FOUND;
   if (baseline_path && fresh_) {
     // both passes of a baseline; its map inserts, bound by random accesses, run
     // beside the diff's assembly, which is a copy and looks up none of them (a
@@ -389,6 +375,49 @@ int Engine::run_tree(const uint8_t* data, uint64_t len, bool baseline_path) {
     MTC_CUDA(launch_forest(fa, 0, 0, N, stream_));                      // first-occurrence forest
     MTC_CUDA(launch_forest(fa, 1, baseline_path ? 1 : 0, N, stream_));  // duplicate forest
   }
+  return ST_OK;
+}
+
+ForestArgs Engine::forest_args() {
+  ForestArgs fa{};
+  fa.tree = digests_.p;
+  fa.labels = labels_.p;
+  fa.rflag = rflag_.p;
+  fa.map = DigestMap{slots_.p, map_cap_ - 1, map_size_.p};
+  fa.sp = sp_.p;
+  fa.err = err_.p;
+  fa.hash_kind = hash_kind_;
+  fa.order = root_order();
+  // the changed-chunk list is free once the leaf inserts are done: it queues
+  // the forest's first-occurrence inserts
+  fa.ins_queue = changed_list_.p;
+  fa.ins_count = changed_count_.p + COUNT_INSERTS;
+  fa.span_done = span_done_.p;
+  fa.zero_found = changed_count_.p + COUNT_ZERO_FOUND;
+  return fa;
+}
+
+// The checkpoint's roots and diff once more, now that every digest of its forest
+// is in the map: an insert found that two of its nodes share one (DERR_TWIN), and
+// the map tells which of them owns it.  The labels and digests of the leaves are
+// as they were; the flags, histogram and span counters are clear again.
+int Engine::redo_roots(uint64_t len) {
+  MTC_TRY(run_params(false));
+  const ForestArgs fa = forest_args();  // no fuse gate: first occurrences, then duplicates
+  if (baseline_path_ && fresh_) {
+    MTC_CUDA(launch_forest(fa, 3, 1, N_, stream_));
+  } else {
+    MTC_CUDA(launch_forest(fa, 0, 0, N_, stream_));
+    MTC_CUDA(launch_forest(fa, 1, 0, N_, stream_));
+  }
+  const bool timed = timed_;
+  timed_ = false;
+  GatherArgs g = gather_args(input_, len);
+  timed_ = timed;
+  g.all_own = 0;
+  g.fuse_gate = nullptr;
+  MTC_CUDA(launch_assemble(g, (uint64_t)N_ + 1, fresh_, nullptr, stream_));
+  MTC_CUDA(cudaStreamSynchronize(stream_));
   return ST_OK;
 }
 
@@ -439,6 +468,7 @@ int Engine::prepare(const uint8_t* data, uint64_t len, bool make_baseline, uint3
     if (rc) return rc;
   }
   data_len = len;
+  input_ = data;
   // TreeLowOffsetRef follows include/reference_impl.hpp:16-132, which has no
   // baseline special case; the tree modes follow dedup_data_baseline for
   // checkpoint 0 and every requested baseline (src/tree_approach.cpp:1644-1653)
@@ -465,8 +495,17 @@ int Engine::enqueue(const uint8_t* data, uint64_t len, bool timed) {
     if (timed) MTC_CUDA(cudaEventRecord(ev_[1], stream_));
     return ST_OK;
   }
-  // one kernel for the step values and every clear: each memset or copy of a
-  // few bytes was a node of its own in the replayed sequence
+  MTC_TRY(run_params(timed));
+  join_ = nullptr;
+  int rc = (mode_ == MODE_LIST || mode_ == MODE_BASIC) ? run_list_basic(data, len) : run_tree(data, len, baseline_path_);
+  if (rc) return rc;
+  MTC_CUDA(launch_assemble(gather_args(data, len), (uint64_t)N_ + 1, fresh_, join_, stream_));
+  return ST_OK;
+}
+
+// One kernel for the step values and every clear: each memset or copy of a
+// few bytes was a node of its own in the replayed sequence.
+int Engine::run_params(bool timed) {
   const ParamsOut po{sp_.p, err_.p, timed ? clk_.p : nullptr, changed_count_.p};
   if (params_by_value_) {
     static const bool reg = (register_input_kernel(reinterpret_cast<const void*>(params_in_kernel), INPUT_PARAMS), true);
@@ -477,10 +516,6 @@ int Engine::enqueue(const uint8_t* data, uint64_t len, bool timed) {
   }
   note_launch();
   MTC_CUDA(cudaGetLastError());
-  join_ = nullptr;
-  int rc = (mode_ == MODE_LIST || mode_ == MODE_BASIC) ? run_list_basic(data, len) : run_tree(data, len, baseline_path_);
-  if (rc) return rc;
-  MTC_CUDA(launch_assemble(gather_args(data, len), (uint64_t)N_ + 1, fresh_, join_, stream_));
   return ST_OK;
 }
 
@@ -699,6 +734,10 @@ int Engine::complete(uint64_t len, HeaderHost* header) {
     datasizes[1] = 0;
     if (header) std::memset(header, 0, sizeof(*header));
     return ST_OK;
+  }
+  if ((err_host_[0] & DERR_TWIN) && !(err_host_[0] & (DERR_SPIN | DERR_MAP_FULL))) {
+    const int rc = redo_roots(len);
+    if (rc) return rc;
   }
   const Layout& L = *lay_host_;
   last_device_error = err_host_[0];

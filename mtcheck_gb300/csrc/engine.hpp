@@ -273,6 +273,9 @@ class Engine {
   int ensure_map(uint64_t want_entries, bool reset);
   int ensure_sort(uint32_t K);
   int run_tree(const uint8_t* data, uint64_t len, bool baseline_path);
+  int run_params(bool timed);
+  ForestArgs forest_args();
+  int redo_roots(uint64_t len);
   int run_list_basic(const uint8_t* data, uint64_t len);
   GatherArgs gather_args(const uint8_t* data, uint64_t len);
   size_t root_tiles() const;
@@ -283,6 +286,7 @@ class Engine {
   cudaStream_t stream_ = nullptr;
   bool allocated_ = false;
   bool fresh_ = false, baseline_path_ = false, timed_ = true, order_after_legacy_ = false, spilled_ = false;
+  const uint8_t* input_ = nullptr;  // of the checkpoint under way
   cudaMemPool_t pool_ = nullptr;
   template <class F> void for_each_buf(F f);
   double max_load_ = 0.75;

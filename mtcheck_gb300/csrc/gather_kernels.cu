@@ -622,7 +622,7 @@ __device__ __forceinline__ void drain_inserts(const GatherArgs& g, uint32_t blk,
   uint32_t created = 0;
   for (uint32_t k = blk * blockDim.x + threadIdx.x; k < n; k += nblk * blockDim.x) {
     const uint32_t node = g.ins_queue[k];
-    created += map_insert_serial(g.map, ld_digest(g.digests + node), node, cur_id, epoch_fo, false, g.err);
+    created += map_insert_owner(g.map, ld_digest(g.digests + node), node, cur_id, epoch_fo, g.err);
   }
   count_new_entries(g.map, created);
 }
@@ -643,7 +643,7 @@ __global__ void __launch_bounds__(256) forest_insert_all_kernel(ForestArgs a, in
     const bool fo = in && a.labels[n] == FIRST_OCUR;
     Digest d{{0, 0, 0, 0}};
     if (in) d = ld_digest(a.tree + n);
-    if (fo) created += map_insert_serial(a.map, d, n, cur_id, epoch + 1, false, a.err);
+    if (fo) created += map_insert_owner(a.map, d, n, cur_id, epoch + 1, a.err);
     if (__any_sync(0xffffffffu, in && !fo))
       created += warp_insert_serial(a.map, in && !fo, d, n, cur_id, epoch + 2, a.err);
   }
@@ -772,7 +772,8 @@ __global__ void __launch_bounds__(kScanThreads) root_count_kernel(GatherArgs g) 
 // (same checkpoint id, another owner).  The inserts of a fused pass may still
 // wait: a digest that is not in the map then is the root's own.  In a baseline
 // of an empty map every first occurrence owns its digest: its leaves own
-// theirs, and no second pair of the same leaves is a first occurrence.
+// theirs, and no second pair of the same leaves is a first occurrence.  The
+// inserts check both (map_insert_owner).
 __device__ __forceinline__ uint64_t fo_region(const GatherArgs& g, uint32_t node, bool fused, uint32_t cur) {
   bool owner = node >= g.N - 1 || g.all_own;
   if (!owner) {

@@ -23,6 +23,7 @@ enum : uint32_t {
   DERR_RANGE = 1u << 5,         // restart metadata out of range
   DERR_INTERIOR = 1u << 6,      // restart provenance names an interior node
   DERR_SORTKEYS = 1u << 7,      // more distinct source checkpoints than the sort supports
+  DERR_TWIN = 1u << 8,          // a first occurrence's digest was another node's before: the roots are looked up again
 };
 
 // Programmatic dependent launch: a kernel launched with programmatic stream
@@ -553,15 +554,33 @@ __device__ __forceinline__ uint64_t serial_prio(uint32_t node) {
 // Insert for a pass that spans several levels in one launch: an entry from an
 // earlier launch is kept; among inserts of this pass the serially first wins.
 // Returns 1 when the entry is new; the caller adds it to m.size
-// (count_new_entries).  `read` as in map_claim.
+// (count_new_entries).  `read` as in map_claim; `old` receives the win word that
+// the insert met.
 __device__ __forceinline__ uint32_t map_insert_serial(const DigestMap& m, const Digest& k, uint32_t node,
-                                                      uint32_t tree, uint32_t epoch, bool read, uint32_t* err) {
+                                                      uint32_t tree, uint32_t epoch, bool read, uint32_t* err,
+                                                      unsigned long long* old = nullptr) {
   uint64_t slot;
   const unsigned long long win = win_of(epoch, serial_prio(node));
   const int r = map_claim(m, map_key(k), read, &slot, err);
-  if (r == INS_NEW) slot_init(&m.slots[slot], win, tree);
-  else if (r == INS_EXISTING) win_min(&m.slots[slot], win);
+  unsigned long long met = kWinEmpty;
+  if (r == INS_NEW) met = slot_init(&m.slots[slot], win, tree);
+  else if (r == INS_EXISTING) met = win_min(&m.slots[slot], win);
+  if (old) *old = met;
   return r == INS_NEW ? 1u : 0u;
+}
+
+// A first occurrence's insert after the roots have been looked up, which counted
+// it as its digest's owner unless an earlier launch had inserted the digest.  Its
+// children's digests are new, so its own can have been there only where a chunk
+// is the 32 bytes that it hashes (a buffer that keeps digests of its own chunks):
+// then the checkpoint's roots are looked up again (DERR_TWIN).  Whichever of two
+// such inserts comes second meets the other's word, or a lower one.
+__device__ __forceinline__ uint32_t map_insert_owner(const DigestMap& m, const Digest& k, uint32_t node, uint32_t tree,
+                                                     uint32_t epoch, uint32_t* err) {
+  unsigned long long old;
+  const uint32_t n = map_insert_serial(m, k, node, tree, epoch, false, err, &old);
+  if (win_epoch(old) <= epoch) raise_err(err, DERR_TWIN);
+  return n;
 }
 
 // The same for a whole warp: lanes that hold one digest insert it once, with
