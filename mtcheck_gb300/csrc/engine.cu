@@ -82,6 +82,7 @@ Engine::Engine(int mode, int hash_kind, uint32_t chunk_size)
   std::memset(sp_host_, 0, sizeof(StepParams));
   // test hook: start the launch epochs near their limit to exercise the rebase
   if (const char* e = std::getenv("MTCHECK_EPOCH_START")) epoch_ = (uint32_t)std::strtoul(e, nullptr, 10);
+  if (const char* e = std::getenv("MTCHECK_FAIL_GRAPH_OP")) fail_graph_op_ = (uint32_t)std::strtoul(e, nullptr, 10);
 }
 
 Engine::~Engine() {
@@ -543,6 +544,11 @@ void Engine::drop_own_graph() {
   own_data_ = nullptr;
 }
 
+int Engine::graph_op() {
+  if (fail_graph_op_ && --fail_graph_op_ == 0) return fail(ST_ECUDA, "injected failure of a graph update");
+  return ST_OK;
+}
+
 int Engine::collect_inputs(cudaGraph_t g, std::vector<InputNode>* out) {
   out->clear();
   size_t n = 0;
@@ -576,6 +582,7 @@ int Engine::collect_inputs(cudaGraph_t g, std::vector<InputNode>* out) {
       std::memcpy(&in.ga, in.p.kernelParams[0], sizeof(GatherArgs));
     }
     in.p.kernelParams = nullptr;
+    MTC_TRY(graph_op());
     out->push_back(in);
   }
   return ST_OK;
@@ -587,6 +594,7 @@ int Engine::retarget(cudaGraphExec_t exec, std::vector<InputNode>& nodes, const 
   for (auto& in : nodes) {
     void* args[3] = {nullptr, nullptr, nullptr};
     if (in.kind == INPUT_PARAMS) continue;
+    MTC_TRY(graph_op());
     if (in.kind == INPUT_COPY) {
       MTC_CUDA(cudaGraphExecMemcpyNodeSetParams1D(exec, in.node, stage_.p, data, len, cudaMemcpyDeviceToDevice));
       continue;
@@ -650,7 +658,10 @@ void Engine::set_own_graph(bool on) {
 int Engine::replay_own(const uint8_t* data, uint64_t len) {
   const uint64_t sig = shape_signature(data, len);
   if (own_exec_ && sig == own_sig_ && data != own_data_) {
-    MTC_TRY(retarget(own_exec_, input_nodes_, data, len));
+    if (const int rc = retarget(own_exec_, input_nodes_, data, len)) {
+      drop_own_graph();  // some of its nodes may read the new input, some the old one
+      return rc;
+    }
     own_data_ = data;
   }
   if (!own_exec_ || sig != own_sig_) {
@@ -660,11 +671,11 @@ int Engine::replay_own(const uint8_t* data, uint64_t len) {
     MTC_CUDA(cudaStreamBeginCapture(cap_stream_, cudaStreamCaptureModeRelaxed));
     cudaStream_t keep = stream_;
     stream_ = cap_stream_;
-    const int rc = enqueue(data, len, !untimed_);
+    int rc = enqueue(data, len, !untimed_);
     stream_ = keep;
     cudaError_t ce = cudaStreamEndCapture(cap_stream_, &own_seq_);
     if (rc == ST_OK && ce == cudaSuccess) ce = cudaGraphInstantiate(&own_exec_, own_seq_, 0);
-    if (rc == ST_OK && ce == cudaSuccess) MTC_TRY(collect_inputs(own_seq_, &input_nodes_));
+    if (rc == ST_OK && ce == cudaSuccess) rc = collect_inputs(own_seq_, &input_nodes_);
     if (rc != ST_OK || ce != cudaSuccess) {
       drop_own_graph();
       cudaGetLastError();

@@ -269,6 +269,10 @@ class Engine {
 
  private:
   int fail(int code, const std::string& msg);
+  // One query or update of a captured sequence's input nodes; fails on the one
+  // that MTCHECK_FAIL_GRAPH_OP counts to (a test hook, read on creation).
+  int graph_op();
+  uint32_t fail_graph_op_ = 0;
   int ensure_state(uint32_t N, bool fresh, uint32_t id_headroom);
   int ensure_map(uint64_t want_entries, bool reset);
   int ensure_sort(uint32_t K);
