@@ -279,12 +279,16 @@ int Batch::build_parent() {
     drop_parent();
     return fail(ST_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(ie));
   }
-  // the members' input nodes, as they lie in the step graph
+  // the members' input nodes, as they lie in the step graph; a graph whose nodes
+  // are not all known could not follow an input that moves
   for (size_t i = 0; i < engs_.size() && !leaf_batching_; i++) {
     cudaGraph_t g = nullptr;
-    MTC_BCUDA(cudaGraphChildGraphNodeGetGraph(children_[i], &g));
-    const int rc = engs_[i]->collect_inputs(g, &inputs_[i]);
-    if (rc) return fail(rc, "member " + std::to_string(i) + ": " + engs_[i]->last_error);
+    const cudaError_t e = cudaGraphChildGraphNodeGetGraph(children_[i], &g);
+    const int rc = e == cudaSuccess ? engs_[i]->collect_inputs(g, &inputs_[i]) : ST_ECUDA;
+    if (rc) {
+      drop_parent();
+      return fail(rc, "member " + std::to_string(i) + ": " + (e == cudaSuccess ? engs_[i]->last_error : cudaGetErrorString(e)));
+    }
   }
   exec_data_ = cap_data_;
   return ST_OK;

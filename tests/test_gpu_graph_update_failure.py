@@ -34,3 +34,28 @@ def test_lone_handle(cuda, mtc, oracle, monkeypatch, approach, op):
             continue
         assert got == ref.checkpoint(state, step == 0), step
     assert failed == 1
+
+
+@pytest.mark.parametrize("op", range(1, 6))
+def test_batch(cuda, mtc, oracle, monkeypatch, op):
+    monkeypatch.setenv("MTCHECK_FAIL_GRAPH_OP", str(op))
+    sizes = (1000, 5000)
+    batch = mtc.Batch([(4, 0, CS) for _ in sizes])
+    monkeypatch.delenv("MTCHECK_FAIL_GRAPH_OP")
+    refs = [oracle.Deduplicator(4, CS, 0) for _ in sizes]
+    bufs = [[cuda.zeros(n * CS, dtype=cuda.uint8, device="cuda") for n in sizes] for _ in range(3)]
+    failed = 0
+    for step, row in enumerate(zip(*[states(np.random.default_rng(n), n, 9) for n in sizes])):
+        for buf, state in zip(bufs[step % 3], row):
+            buf.copy_(cuda.from_numpy(state))
+        try:
+            batch.checkpoint(bufs[step % 3], make_baseline=step == 0)
+        except mtc.MtcError:
+            failed += 1
+            continue
+        for m, ref, state in zip(batch.members, refs, row):
+            host = np.empty(m.diff_device()[1], np.uint8)
+            m.copy_diff(host)
+            assert host.tobytes() == ref.checkpoint(state, step == 0), step
+    assert failed == len(sizes)
+    batch.close()
