@@ -1302,6 +1302,30 @@ bool rows_fit(const LeafArgs& a) {
 // direct, 226 staged; 256 MiB in 128-byte chunks off a boundary: 282 direct, 117
 // staged; both before other kernels took them).
 constexpr uint32_t kDirectMax = 100;
+// Of the longer ones, chunks of whole 4-byte words at word addresses that are read
+// directly all the same.  The direct kernel's 1536 threads per SM have three
+// times as many chunks in flight as the staged one's 512 (a wave), and a word
+// costs it no copy; the staged kernel's narrow copies take it one instruction per
+// 4 or 8 bytes, and a chunk's last panel is copied and hashed around whole.
+// Staged against direct, 4-byte aligned: MD5 1.0-1.5 from half a wave on; Murmur3
+// 0.3-0.95 up to half a wave, 1.0-1.25 from there to three waves (chunks above
+// about 1 KiB: from one and a half), 0.8-1.0 beyond, but 1.05-1.3 where the panels
+// are a sixth longer than the chunk (160, 288, 516 bytes).  8-byte aligned: MD5
+// 0.95-1.1 up to a wave, 1.0-1.2 beyond (but 0.9 for multiples of 16 above half a
+// KiB), Murmur3 0.6-1.05.  Multiples of 64 bytes (0.6-1.0: direct reads of a warp's
+// chunks meet in few L1 sets) and 16-byte aligned chunks (0.4-0.9) are always
+// staged.
+bool direct_words(const LeafArgs& a) {
+  const uint64_t align = reinterpret_cast<uintptr_t>(a.data) | a.cs;
+  if ((align & 3) != 0 || (align & 15) == 0 || a.cs % 64 == 0) return false;
+  const uint64_t n = a.n_chunks, wave = 512ull * num_sms();
+  const bool half8 = (align & 7) == 0;
+  if (a.hash_kind == HASH_MD5) return half8 ? n > wave && (a.cs % 16 != 0 || a.cs < 512) : n > wave / 2;
+  if (half8) return false;
+  const uint64_t panels = ((uint64_t)a.cs + kPanel - 1) / kPanel * kPanel;
+  if (6 * panels > 7ull * a.cs) return n > wave / 2;
+  return n > (a.cs < 1100 ? 3 * wave / 4 : 3 * wave / 2) && n <= 3 * wave;
+}
 
 cudaError_t launch_leaves(const LeafArgs& a, TmaCache* cache, cudaStream_t s, const LeafTune& tune) {
   if (a.n_chunks == 0) return cudaSuccess;
@@ -1316,7 +1340,7 @@ cudaError_t launch_leaves(const LeafArgs& a, TmaCache* cache, cudaStream_t s, co
     return aligned ? dispatch_tma(a, cache->map, n_full, W, t, s)
                    : dispatch_shift(a, cache->map, n_full, W, t.ctas_per_sm, s);
   if (!t.direct && rows_fit(a)) return dispatch_rows(a, s);
-  if (!t.direct && a.cs > kDirectMax) return dispatch_staged(a, 0, a.n_chunks, s);
+  if (!t.direct && a.cs > kDirectMax && !direct_words(a)) return dispatch_staged(a, 0, a.n_chunks, s);
   return dispatch_direct(a, 0, a.n_chunks, s);
 }
 
