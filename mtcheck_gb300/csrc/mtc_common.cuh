@@ -196,11 +196,9 @@ struct Md5State {
   MTC_HD Digest finish(uint32_t* tw, uint32_t rem, uint64_t len) {
     // append 0x80 at byte `rem`; every index is a constant, so that the block
     // stays in registers
+    const uint32_t at = rem >> 2, bit = 0x80u << (8 * (rem & 3));
 #pragma unroll
-    for (uint32_t i = 0; i < 16; i++) {
-      const uint32_t d = rem - 4 * i;  // past 31 bits, or below 0: no byte of this word
-      tw[i] |= d < 4 ? 0x80u << (8 * d) : 0u;
-    }
+    for (uint32_t i = 0; i < 16; i++) tw[i] |= i == at ? bit : 0u;
     if (rem >= 56) {
       block(tw);
 #pragma unroll
