@@ -3,6 +3,8 @@
 #include <cstdlib>
 #include <cstring>
 #include <fstream>
+#include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -328,6 +330,56 @@ int mtc_write_restart_log(const mtc_dedup_t* h, uint32_t select_chkpt, const cha
   return MTC_OK;
 }
 
+namespace {
+// A device error word for one call of mtc_hash_chunks (a bounded wait that runs
+// out sets it) and a pinned word it is read through, kept between calls: an
+// allocation per call would go through the default memory pool, whose release at
+// every synchronisation maps and unmaps device memory.  As many pairs exist as
+// calls have run at one time on the device.  The word is zero between calls: the
+// kernel that reads it clears it.  A memset and a copy to pageable memory took 5
+// of a short call's 22 us.
+struct ErrWord {
+  uint32_t *dev, *host;
+  ErrWord* next;
+};
+constexpr int kMaxDevices = 64;
+std::mutex g_err_mu;
+ErrWord* g_err_free[kMaxDevices];
+
+void free_err_word(ErrWord* p) {
+  if (p->dev) cudaFree(p->dev);
+  if (p->host) cudaFreeHost(p->host);
+  delete p;
+}
+void give_err_word(int dev, ErrWord* p) {
+  std::lock_guard<std::mutex> lk(g_err_mu);
+  p->next = g_err_free[dev];
+  g_err_free[dev] = p;
+}
+// A pair for a call on stream s of the current device.
+cudaError_t take_err_word(int dev, cudaStream_t s, ErrWord** out) {
+  {
+    std::lock_guard<std::mutex> lk(g_err_mu);
+    if (ErrWord* p = g_err_free[dev]) {
+      g_err_free[dev] = p->next;
+      *out = p;
+      return cudaSuccess;
+    }
+  }
+  auto* p = new (std::nothrow) ErrWord{nullptr, nullptr, nullptr};
+  if (!p) return cudaErrorMemoryAllocation;
+  cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&p->host), sizeof(uint32_t));
+  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&p->dev), sizeof(uint32_t));
+  if (e == cudaSuccess) e = cudaMemsetAsync(p->dev, 0, sizeof(uint32_t), s);
+  if (e != cudaSuccess) {
+    free_err_word(p);
+    return e;
+  }
+  *out = p;
+  return cudaSuccess;
+}
+}  // namespace
+
 int mtc_hash_chunks(int hash, const void* dev_data, uint64_t len, uint32_t chunk_size, void* dev_digests,
                     void* cuda_stream) {
   if (!dev_data || !dev_digests || chunk_size == 0) return ret(MTC_EINVAL, "bad argument");
@@ -345,35 +397,24 @@ int mtc_hash_chunks(int hash, const void* dev_data, uint64_t len, uint32_t chunk
   a.epi = mtc::EPI_HASH;
   mtc::TmaCache cache;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(cuda_stream);
-  // a device error word for the call (a bounded wait that runs out sets it) and
-  // a pinned word it is read through: one pair per host thread and device,
-  // allocated on the thread's first call and kept (an allocation per call would
-  // go through the default memory pool, whose release at every synchronisation
-  // maps and unmaps device memory).  The word is zero between calls: the kernel
-  // that reads it clears it.  A memset and a copy to pageable memory took 5 of
-  // a short call's 22 us.
-  struct ErrPair { uint32_t *dev, *host; };
-  thread_local ErrPair tl_err[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return ret(MTC_ENOTSUP, "device ordinal above 63");
-  ErrPair& p = tl_err[dev];
-  cudaError_t e = cudaSuccess;
-  if (!p.host) e = cudaMallocHost(reinterpret_cast<void**>(&p.host), sizeof(uint32_t));
-  if (e == cudaSuccess && !p.dev) {
-    e = cudaMalloc(reinterpret_cast<void**>(&p.dev), sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMemsetAsync(p.dev, 0, sizeof(uint32_t), s);
+  if (dev < 0 || dev >= kMaxDevices) return ret(MTC_ENOTSUP, "device ordinal above 63");
+  ErrWord* p = nullptr;
+  cudaError_t e = take_err_word(dev, s, &p);
+  if (e == cudaSuccess) {
+    a.err = p->dev;
+    e = mtc::launch_leaves(a, &cache, s, mtc::default_leaf_tune(hash, chunk_size));
   }
-  a.err = p.dev;
-  if (e == cudaSuccess) e = mtc::launch_leaves(a, &cache, s, mtc::default_leaf_tune(hash, chunk_size));
-  if (e == cudaSuccess) e = mtc::launch_take_word(p.dev, static_cast<uint32_t*>(mtc::host_alias(p.host)), s);
+  if (e == cudaSuccess) e = mtc::launch_take_word(p->dev, static_cast<uint32_t*>(mtc::host_alias(p->host)), s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {
-    if (p.dev) cudaFree(p.dev);  // it may hold an error bit that no call has read
-    p.dev = nullptr;
+    if (p) free_err_word(p);  // it may hold an error bit that no call has read
     return ret(e == cudaErrorMemoryAllocation ? MTC_ENOMEM : MTC_ECUDA, cudaGetErrorString(e));
   }
-  if (*p.host & mtc::DERR_SPIN) return ret(MTC_ETIMEOUT, "bounded device wait expired");
+  const uint32_t err = *p->host;
+  give_err_word(dev, p);
+  if (err & mtc::DERR_SPIN) return ret(MTC_ETIMEOUT, "bounded device wait expired");
   return MTC_OK;
 }
 
