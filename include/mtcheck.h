@@ -232,6 +232,9 @@ int mtc_batch_checkpoint(mtc_batch_t* b, const void* const* dev_data, const uint
  * id_headroom: checkpoint ids one captured graph serves before re-capture */
 int mtc_batch_set_options(mtc_batch_t* b, int use_graph, uint32_t id_headroom);
 int mtc_batch_get_info(const mtc_batch_t* b, mtc_batch_info_t* out);
+/* Of graph_captures, the inputs that had moved and were updated in place: the
+ * others are sequences captured. */
+int mtc_batch_moved_inputs(const mtc_batch_t* b, uint64_t* count);
 /* run the autotuner for every member (cached per approach, hash, chunk size
  * and power-of-two length; lengths above 64 MiB share one 64 MiB trial) and
  * apply the winners */

@@ -129,6 +129,7 @@ SIGNATURES = {
     "mtc_batch_checkpoint": (_I, [_VP, ctypes.POINTER(_VP), ctypes.POINTER(_U64), _I, ctypes.POINTER(_U64)]),
     "mtc_batch_set_options": (_I, [_VP, _I, _U32]),
     "mtc_batch_get_info": (_I, [_VP, ctypes.POINTER(BatchInfo)]),
+    "mtc_batch_moved_inputs": (_I, [_VP, ctypes.POINTER(_U64)]),
     "mtc_batch_autotune": (_I, [_VP, ctypes.POINTER(_U64)]),
     "mtc_batch_reserve": (_I, [_VP, ctypes.POINTER(_U64), ctypes.POINTER(_U64)]),
     "mtc_server_create": (_I, [ctypes.POINTER(ServerOptions), ctypes.POINTER(_VP)]),
@@ -435,6 +436,13 @@ class Batch:
         i = BatchInfo()
         _check(load().mtc_batch_get_info(self.b, ctypes.byref(i)))
         return i
+
+
+    def moved_inputs(self):
+        """Of info().graph_captures, the inputs that had moved and were updated in place."""
+        n = _U64()
+        _check(load().mtc_batch_moved_inputs(self.b, ctypes.byref(n)))
+        return int(n.value)
 
 
 class Server:

@@ -341,7 +341,10 @@ int Batch::checkpoint(const uint8_t* const* data, const uint64_t* lens, bool mak
         return fail(rc, "member " + std::to_string(i) + ": " + engs_[i]->last_error);
       }
       exec_data_[i] = data[i];
-      if (before[i] != data[i]) stats_.captures++;
+      if (before[i] != data[i]) {
+        stats_.captures++;
+        stats_.moved_inputs++;
+      }
     }
   }
   // 3. issue: the step starts after the work already on the legacy default

@@ -29,7 +29,8 @@ namespace mtc {
 
 struct BatchStats {
   uint64_t steps = 0;
-  uint64_t captures = 0;
+  uint64_t captures = 0;      // sequences captured, and inputs moved
+  uint64_t moved_inputs = 0;  // of those, updated in place
   uint64_t graph_nodes = 0;       // nodes of all members' graphs
   uint64_t batched_leaf_items = 0;  // work items of the batched leaf launch (0: none)
   uint32_t batched_leaf_members = 0;

@@ -513,6 +513,12 @@ int mtc_batch_get_info(const mtc_batch_t* b, mtc_batch_info_t* o) {
   return MTC_OK;
 }
 
+int mtc_batch_moved_inputs(const mtc_batch_t* b, uint64_t* count) {
+  if (!b || !count) return ret(MTC_EINVAL, "NULL argument");
+  *count = b->b->stats().moved_inputs;
+  return MTC_OK;
+}
+
 int mtc_batch_reserve(mtc_batch_t* b, const uint64_t* lens, uint64_t* bytes) {
   if (!b || !lens) return ret(MTC_EINVAL, "NULL argument");
   const int rc = b->b->reserve(lens, bytes);
