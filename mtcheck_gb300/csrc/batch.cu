@@ -73,6 +73,7 @@ Batch::~Batch() {
 
 int Batch::fail(int code, const std::string& msg) {
   last_error = msg;
+  if (code == ST_ECUDA || code == ST_ENOMEM) cudaGetLastError();
   return code;
 }
 

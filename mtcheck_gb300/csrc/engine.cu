@@ -108,6 +108,8 @@ Engine::~Engine() {
 
 int Engine::fail(int code, const std::string& msg) {
   last_error = msg;
+  // a failed CUDA call is reported here, not by the next call's launches
+  if (code == ST_ECUDA || code == ST_ENOMEM) cudaGetLastError();
   return code;
 }
 
@@ -454,7 +456,7 @@ int Engine::run_list_basic(const uint8_t* data, uint64_t len) {
 int Engine::prepare(const uint8_t* data, uint64_t len, bool make_baseline, uint32_t id_headroom) {
   if (!data || len == 0) return fail(ST_EINVAL, "empty buffer");
   if (spilled_) return fail(ST_EINVAL, "state spilled to host: restore it first");
-  if (need_baseline_) make_baseline = true;  // the last checkpoint timed out on the device
+  if (need_baseline_) make_baseline = true;  // the last baseline failed, or the last checkpoint timed out
   const uint64_t n64 = (len + cs_ - 1) / cs_;
   if (n64 >= (1ull << 31)) return fail(ST_ENOTSUP, "more than 2^31 chunks");
   const uint32_t N = (uint32_t)n64;
@@ -465,6 +467,9 @@ int Engine::prepare(const uint8_t* data, uint64_t len, bool make_baseline, uint3
     MTC_CUDA(stage_.ensure(len + 64, stream_));
     allocated_ = true;
   } else {
+    // until this baseline is complete there is no state to go on from: its
+    // buffers may be of one size and the next checkpoint's chunks of another
+    if (fresh_) need_baseline_ = true;
     int rc = ensure_state(N, fresh_, id_headroom);
     if (rc) return rc;
   }
