@@ -82,6 +82,7 @@ Engine::Engine(int mode, int hash_kind, uint32_t chunk_size)
   std::memset(sp_host_, 0, sizeof(StepParams));
   // test hook: start the launch epochs near their limit to exercise the rebase
   if (const char* e = std::getenv("MTCHECK_EPOCH_START")) epoch_ = (uint32_t)std::strtoul(e, nullptr, 10);
+  if (const char* e = std::getenv("MTCHECK_FAIL_RESTORE")) fail_restore_ = (uint32_t)std::strtoul(e, nullptr, 10);
   if (const char* e = std::getenv("MTCHECK_FAIL_GRAPH_OP")) fail_graph_op_ = (uint32_t)std::strtoul(e, nullptr, 10);
 }
 
@@ -856,11 +857,21 @@ int Engine::spill_to_host(uint8_t* host) {
 
 int Engine::restore_from_host(const uint8_t* host) {
   if (!spilled_) return ST_OK;
+  const int rc = load_spilled(host);
+  if (rc) {
+    // still spilled: the host copy is whole, the buffers may not be
+    for_each_buf([&](auto& b) { b.release(stream_); });
+    return rc;
+  }
   spilled_ = false;
+  return ST_OK;
+}
+
+int Engine::load_spilled(const uint8_t* host) {
   const bool tree = mode_ == MODE_TREE || mode_ == MODE_TREE_LOW_OFFSET || mode_ == MODE_TREE_LOW_OFFSET_REF;
   const uint32_t saved_size = [&] { uint32_t v; std::memcpy(&v, host + sizeof(Digest) * spill_nd_ + sizeof(MapSlot) * spill_cap_, 4); return v; }();
-  int rc = ensure_state(N_, true, 0);  // every buffer, zeroed; map sized for M
-  if (rc) return rc;
+  MTC_TRY(ensure_state(N_, true, 0));  // every buffer; map sized for M
+  if (fail_restore_ && --fail_restore_ == 0) return fail(ST_ENOMEM, "injected failure of a restore");
   if (mode_ != MODE_BASIC && slots_.n != spill_cap_) {
     slots_.release(stream_);
     MTC_CUDA(slots_.ensure(spill_cap_, stream_));

@@ -273,6 +273,8 @@ class Engine {
   // that MTCHECK_FAIL_GRAPH_OP counts to (a test hook, read on creation).
   int graph_op();
   uint32_t fail_graph_op_ = 0;
+  uint32_t fail_restore_ = 0;  // MTCHECK_FAIL_RESTORE: the same of restores of a spilled state
+  int load_spilled(const uint8_t* host);
   int ensure_state(uint32_t N, bool fresh, uint32_t id_headroom);
   int ensure_map(uint64_t want_entries, bool reset);
   int ensure_sort(uint32_t K);

@@ -103,3 +103,15 @@ def test_last_chunk_of_a_digest_pair(cuda, mtc, oracle, n):
         state[n * cs:] = pair(oracle, 0, rows[a], rows[a + 1])
         want = ref.checkpoint(state, step in (0, 2))
         assert gpu.checkpoint(cuda.from_numpy(state.copy()).cuda(), step in (0, 2)) == want, step
+
+
+@pytest.mark.parametrize("use_graph", [True, False], ids=["graph", "eager"])
+def test_served_digest_pairs(cuda, mtc, oracle, use_graph):
+    srv = mtc.Server(use_graph=use_graph)
+    pid, ref = srv.add_process(4, 0, CS), oracle.Deduplicator(4, CS, 0)
+    for step, state in enumerate(states(oracle, 0, 5000, 5)):
+        buf = cuda.from_numpy(state).cuda()
+        srv.submit_checkpoint(pid, buf, make_baseline=step == 0)
+        srv.drain()
+        assert srv.diff(pid, step) == ref.checkpoint(state, step == 0), step
+    srv.close()
