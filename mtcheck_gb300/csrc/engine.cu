@@ -34,8 +34,9 @@ static __global__ void params_in_kernel(StepParams p, ParamsOut o) {
   pdl_enter();
   params_store(p, o);
 }
-// A batch member's sequence, replayed inside the batch's graph, reads the step
-// values staged in the pinned block.
+// The sequence of a batch member, one of many in a graph that is launched as it
+// is, reads the step values staged in the pinned block: a few bytes over the
+// link, behind whatever transfer is under way there.
 static __global__ void params_host_kernel(const volatile StepParams* host, ParamsOut o) {
   pdl_enter();
   params_store(StepParams{host->cur, host->baseline_id, host->epoch, host->pad}, o);
@@ -441,7 +442,9 @@ int Engine::run_list_basic(const uint8_t* data, uint64_t len) {
   la.hash_kind = hash_kind_;
   la.epi = mode_ == MODE_LIST ? EPI_LIST : EPI_BASIC;
   la.fresh = fresh_ ? 1 : 0;  // never true in a captured sequence
-  la.basic_first = current_id == 0 ? 1 : 0;  // never true in a captured sequence
+  // captured as 1 by a second checkpoint under id 0; baseline_path_, part of the
+  // signature, keeps that sequence from other ids
+  la.basic_first = current_id == 0 ? 1 : 0;
   la.changed_list = changed_list_.p;
   la.changed_count = changed_count_.p + COUNT_CHANGED;
   if (stall_now_) {

@@ -335,7 +335,7 @@ class Engine {
   Layout* lay_host_ = nullptr;      // pinned
   uint32_t* err_host_ = nullptr;    // pinned [err, map size]
   uint64_t* clk_host_ = nullptr;    // pinned copy of clk_
-  bool params_by_value_ = true;     // false for batch members (their graphs copy sp_host_)
+  bool params_by_value_ = true;     // false for batch members (their first kernel reads sp_host_)
   uint64_t diff_len_ = 0, diff_pad_ = 0;
   TmaCache tma_;
   cudaEvent_t ev_[3] = {nullptr, nullptr, nullptr};  // two timing events, one ordering event

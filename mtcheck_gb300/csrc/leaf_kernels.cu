@@ -3,13 +3,15 @@
 // One thread owns one chunk (Murmur3 and MD5 are serial over a chunk).  On the
 // fast path the chunk bytes reach shared memory through TMA tiled loads: the
 // buffer is viewed as a 2-D tensor [n_full rows x cs bytes]; each stage moves a
-// box of 256 rows x W bytes (W = 128, 64, 32 or 16) with the matching TMA
-// swizzle so that the 256 consumer threads read their rows without bank
-// conflicts.  A dedicated producer warp keeps STAGES boxes in flight; full/empty
+// box of 128 (Murmur3) or 256 (MD5) rows x W bytes (W = 128, 64, 32 or 16) with
+// the matching TMA swizzle so that the consumer threads, one per row, read their
+// rows without bank conflicts.  A dedicated producer warp keeps STAGES boxes in flight; full/empty
 // mbarriers hand stages between producer and consumers; one more warp hashes a
-// partial last chunk.  Other short chunks come as whole tiles by untiled bulk
-// copies, longer ones in panels through a staged kernel, the rest through a
-// thread-per-chunk kernel that reads global memory directly.  All end in the
+// partial last chunk.  Buffers off a 16-byte boundary are tiled from the boundary
+// before them.  Other short chunks come as whole tiles by untiled bulk
+// copies, longer ones in panels through a staged kernel, the rest (and many
+// word-aligned chunks) through a thread-per-chunk kernel that reads global
+// memory directly.  All end in the
 // same epilogue, which restates the leaf loops of the reference:
 //   tree  -- src/tree_approach.cpp:57-94 (baseline) and :309-351
 //   list  -- src/list_approach.cpp:38-61

@@ -337,9 +337,9 @@ __host__ __device__ __forceinline__ uint32_t leftmost_leaf(uint32_t node, uint32
 // and the old value an insert gets back tells whether the entry is older
 // than its launch.  The node is win's low 32 bits.  `tree` (the checkpoint id
 // of the first occurrence) is written by the creator and read by later
-// launches.  Both halves of a slot are
-// only written by 16-byte compare-and-swaps.  No insert waits on another
-// thread.
+// launches.  Inserts write both halves of a slot by 16-byte compare-and-swaps
+// only (launches of their own that move the table or rebase its epochs store
+// plainly).  No insert waits on another thread.
 // ---------------------------------------------------------------------------
 struct __align__(32) MapSlot {
   uint32_t key[4];

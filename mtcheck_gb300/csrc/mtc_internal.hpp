@@ -127,10 +127,12 @@ inline LeafTune default_leaf_tune(int hash_kind, uint32_t cs) {
   return LeafTune{128, cs < 128 ? 6 : cs == 128 ? 3 : 2, 0};
 }
 
-// Launch the leaf hashing kernel over every chunk: the TMA pipeline for chunk
-// sizes that are a multiple of 128 bytes (or 16/32/64) on 16-byte aligned
-// buffers, the staged kernel for other chunks above 100 bytes, and direct loads
-// for the rest.
+// Launch the leaf hashing kernel over every chunk: tiled copies for chunk sizes
+// that are a multiple of 128 bytes or 64 on any buffer, and 16 or 32 on 16-byte
+// aligned ones; whole tiles by untiled copies for other sizes up to 440 bytes (not
+// multiples of 32, and for MD5 not below 64); of the rest the staged kernel
+// above 100 bytes, except word-aligned chunks that direct loads hash faster
+// (direct_words); direct loads otherwise.
 cudaError_t launch_leaves(const LeafArgs& a, TmaCache* cache, cudaStream_t s, const LeafTune& tune = LeafTune{});
 // The leaf pass of many deduplicators in one persistent launch (a batch):
 // one record per member (its TMA descriptor with boxes of kBatchRows rows,
@@ -158,9 +160,11 @@ cudaError_t batch_leaf_node_params(const BatchLeafParams& p, cudaKernelNodeParam
 // The leaf kernel for chunks [c0, c1) only, one thread per chunk.
 cudaError_t launch_leaf_range(const LeafArgs& a, uint32_t c0, uint32_t c1, cudaStream_t s);
 
-// Tree / list: map inserts of the changed chunks collected by launch_leaves,
-// then the lowest-offset demotion (src/tree_approach.cpp:356-369; for the
-// list a changed chunk is a first occurrence only if it owns its digest).
+// Tree / list: map inserts of the changed chunks collected by launch_leaves (in
+// a baseline of every chunk that is a first occurrence so far); each insert marks
+// the chunk that loses the digest as a shifted duplicate
+// (src/tree_approach.cpp:356-369; for the list a changed chunk is a first
+// occurrence only if it owns its digest).
 cudaError_t launch_leaf_inserts(const LeafArgs& a, cudaStream_t s);
 
 int num_sms();
