@@ -1142,12 +1142,6 @@ def main():
                "step_ms": [round((b - a) * 1e3, 2) for a, b in zip([t0] + marks[:-1], marks)]}
         del host, pinned_out, out_view, bufs
 
-    # the served stream and the batch run in processes of their own
-    srvd = None
-    if not a.no_serve and rank == 0:
-        torch.cuda.empty_cache()
-        srvd = section_in_subprocess("--only-serve", "served", a)
-
     md5 = small = None
     if rank == 0 and not a.no_sections:
         md5 = md5_section(torch, mc, dev, states[:1 + W + K], cs, W, peak)
@@ -1158,10 +1152,10 @@ def main():
         e2e["link"] = dict(link, note="pinned 1 GiB copies split over 1, 2 and 4 streams; kernels reading pinned "
                                       "or pageable host memory directly measured the same ceiling")
         e2e["link_frac"] = round(e2e["value"] / h2d, 3)
+    states = s = None
+    torch.cuda.empty_cache()
     rst = None
     if not a.no_restart and rank == 0:
-        del states
-        torch.cuda.empty_cache()
         rst = restart_bench(torch, mc, dev, a, kind)
         torch.cuda.empty_cache()
         rst["other_approaches"] = {}
@@ -1177,9 +1171,14 @@ def main():
         small = small_series_section(torch, mc, dev, peak)
         torch.cuda.empty_cache()
 
-    bat = None
-    if not a.no_batch and rank == 0:
+    # the served stream and the batch run in processes of their own, once this
+    # one's states are gone: 26 of them (20 steps after 5 warm-ups) left the
+    # served section without memory
+    srvd = bat = None
+    if not a.no_serve and rank == 0:
         torch.cuda.empty_cache()
+        srvd = section_in_subprocess("--only-serve", "served", a)
+    if not a.no_batch and rank == 0:
         bat = section_in_subprocess("--only-batch", "batched", a)
 
     cpu = None
