@@ -505,9 +505,10 @@ __global__ void leaf_direct_kernel(LeafArgs a, uint32_t c0, uint32_t c1) {
 // the chunk's address, so the copies are as wide as that allows (cp.async of 16,
 // 8 or 4 bytes) and a thread reads its row in 16-byte words, without bank
 // conflicts at a stride of 144 bytes; an address off a 4-byte boundary is
-// shifted in registers.  kStageBufs panels in flight per block.  Bound by HBM
-// for Murmur3 at 16 bytes per copy, by issue below, by the integer pipe for
-// MD5.  1 GiB in 4096-byte chunks 4 bytes off a boundary: 376 us (MD5 486), with
+// shifted in registers.  kStageBufs panels in flight per block.  They leave room
+// for 16 warps per SM, which wait for their own instructions: 441-byte chunks use
+// 63 % of the issue slots and 61 % of the integer pipe with Murmur3, 73 % of the
+// pipe with MD5, and a quarter of the bandwidth.  1 GiB in 4096-byte chunks 4 bytes off a boundary: 376 us (MD5 486), with
 // direct loads 1054 us (991).
 // ---------------------------------------------------------------------------
 constexpr int kStageRows = 128;
@@ -674,8 +675,9 @@ __global__ void __launch_bounds__(kStageRows, 4) leaf_staged_kernel(LeafArgs a, 
 // untiled bulk copy of 128 * cs bytes (from the 16-byte boundary before them to
 // the one after) brings a tile in whatever its chunk size and alignment, and a
 // producer lane keeps two in flight.  A thread reads its row word by word: an
-// odd multiple of four bytes apart, rows lie in different banks.  Bound by the
-// integer pipe (hashing, and realigning words).  Two stages, for more CTAs per SM
+// odd multiple of four bytes apart, rows lie in different banks.  100-byte chunks
+// use two thirds of the issue slots (hashing, and realigning words) and of the
+// bandwidth with Murmur3, 77 % of the integer pipe with MD5.  Two stages, for more CTAs per SM
 // (three: 250-byte chunks 73 us for 256 MiB, two 62).  Whole calls, two stages
 // against the kernels before: 400 MB in chunks of 100 bytes 130 -> 91 us
 // (Murmur3), 183 -> 174 (MD5); 256 MiB in 300 bytes 131 -> 69 and 166 -> 106.
